@@ -1,16 +1,17 @@
 // Decode attention with the learned relative-position bias: one query token per sequence against the
 // layer's K/V cache (a ring of `window` slots in a sliding layer, `slots` positions in a full one).
-// One block per (head, sequence); the relative logits of the head, the scores and the softmax live in
-// shared memory, K and V are read once per block (heads of one group share them through the L2).
 #include "../../include/inkling_b200.h"
 #include "common.cuh"
 
 namespace ink {
 
-constexpr int kAttnThreads = 256;   // (128 and 512 threads, i.e. 32 and 128 slots per block, measured the same)
+constexpr int kAttnThreads = 128;
 constexpr int kAttnWarps = kAttnThreads / 32;
-constexpr int kAttnKeys = 8;                                // cache slots a warp scores side by side
-constexpr int kAttnSlots = kAttnWarps * kAttnKeys;          // slots per block: 64
+constexpr int kAttnHeads = 8;                               // query heads that share a pass over the cache rows
+constexpr int kAttnUnit = 16;                               // cache slots per step of a warp
+constexpr int kAttnMinSlots = kAttnUnit * kAttnWarps;       // a block is not worth launching for fewer
+constexpr int kAttnMaxSplits = 64;
+constexpr int kAttnWaveBlocks = 148 * 3;                    // blocks resident at once
 constexpr int kAttnPartial = 2;                             // floats in front of a partial result: running maximum, sum
 
 struct AttnArgs {
@@ -26,31 +27,54 @@ struct AttnArgs {
   uint16_t* k_store;        // the caches again, writable: where the current token is stored when new_k is given
   uint16_t* v_store;
   float* partial;           // [bs, h, splits, 2 + c]: maximum, sum of exponentials, unnormalised weighted values
-  unsigned* arrived;        // [bs, h] blocks of a (sequence, head) that have stored their partial; zero between launches
+  unsigned* arrived;        // [bs, head groups] blocks of a group that have stored their partial; zero between launches
   uint16_t* out;            // [bs, h, c]
-  int heads, kv_heads, c, d_rel, extent, slots, window, n_floor, splits;
+  int heads, kv_heads, d_rel, extent, slots, window, n_floor, splits;
   float alpha, scale;
 };
 
-// One block per (head, sequence, group of 64 cache slots). A decode step has few (head, sequence) pairs and every
-// load is a trip to DRAM, so the work is cut along the cache (as in split-K / flash decoding) and every block asks
-// for ALL it needs at once: its key rows, its value rows (which slots are allowed is known before any score),
-// the query and the relative states. It leaves a partial softmax (maximum, sum, weighted values); the block that
-// stores the last partial of a (sequence, head) joins them.
+// D[16x8] += A[16x16] . B[16x8], BF16 in, FP32 out. Lane (g = lane / 4, t = lane % 4) holds of A: a0 = row g,
+// columns 2t, 2t+1; a1 = row g + 8, the same columns; a2, a3 = columns 2t+8, 2t+9 of these rows; of B: b0 = rows
+// 2t, 2t+1, b1 = rows 2t+8, 2t+9 of column g; of D: d0, d1 = row g, columns 2t, 2t+1; d2, d3 = row g + 8.
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
+// One block per (part of the cache, group of up to eight heads of one key/value head, sequence). Bound by reading
+// the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
+// deliver at HBM speed, so scores, bias and weighted values go through warp-level matrix instructions (M = heads: the
+// contraction is far too flat for the 128-row tcgen05 tiles). Measured on B200, batch 8, 64 heads on 8 key/value
+// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, see the table of the design notes for
+// this one.
+//
+// A warp takes 16 slots a step and keeps everything in registers; nothing of the cache passes through shared memory,
+// because the sums over channels may run in any order as long as both operands agree:
+//   scores  A = the queries (row g = head), B = the keys: lane (g, t) loads the 16-byte pieces t, t + 4, ... of the row
+//           of slot g; the four words of a piece are two k-steps' worth of B.
+//   values  A = the exponentials, which the score accumulators already hold in A's layout; B = the values: lane (g, t)
+//           loads the piece g (and g + 8) of the rows 2t, 2t+1, 2t+8, 2t+9, and word pairs of neighbouring rows are
+//           interleaved into B. The unused upper eight rows of A carry what BF16 cuts off the exponentials (p = hi + lo),
+//           so the weights keep 16 bits at no further instruction.
 template <int C>
-__global__ void __launch_bounds__(kAttnThreads) decode_attention_kernel(AttnArgs a) {
-  constexpr int kWords = C / 2;                          // 32-bit words of a row = channel pairs
-  constexpr int kPerLane = (kWords + 31) / 32;           // words of a key row per lane
-  constexpr int kParts = kAttnThreads / kWords;          // threads per channel pair in the value pass
-  constexpr int kValues = kAttnSlots / kParts;           // value rows per thread
-  static_assert(kAttnThreads % kWords == 0 && kAttnSlots % kParts == 0, "head_dim does not tile the block");
-  __shared__ float s_q[C];
-  __shared__ float s_bias[kAttnSlots];
-  __shared__ float s_scores[kAttnSlots];
-  __shared__ float s_part[kAttnThreads * 2];
-  const int head = blockIdx.x, b = blockIdx.y, split = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int kv_head = head / (a.heads / a.kv_heads);
-  const int slot_base = split * kAttnSlots;
+__global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attention_kernel(AttnArgs a) {
+  constexpr int kPieces = C / 32;       // 16-byte pieces of a key row per lane
+  constexpr int kHalves = C / 64;       // pieces of a value row per lane
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  float* s_acc = reinterpret_cast<float*>(s_raw);                                   // [warps][heads][C + 2]
+  uint16_t* s_r = reinterpret_cast<uint16_t*>(s_raw);                               // [heads][d_rel rounded up to 16]: before the sums
+  __shared__ bool s_last;
+  const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
+  const int kv_head = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
+  const int head0 = kv_head * group + chunk * kAttnHeads, n_heads = min(kAttnHeads, group - chunk * kAttnHeads);
   // positions fit 32 bits; the ring arithmetic is done once per block (position modulo the window), not per slot
   const int position = (int)*a.position;
   const int reach = position - (int)(a.pad_counts ? a.pad_counts[b] : 0);   // largest distance that is not padding
@@ -64,186 +88,244 @@ __global__ void __launch_bounds__(kAttnThreads) decode_attention_kernel(AttnArgs
     const int d = distance_of(slot);
     return slot < a.slots && d >= 0 && d <= reach;
   };
-  // ---- everything from memory, in flight together
-  const uint16_t* keys = a.k + ((size_t)b * a.kv_heads + kv_head) * a.slots * C;
-  const uint16_t* values = a.v + ((size_t)b * a.kv_heads + kv_head) * a.slots * C;
+  const size_t row0 = ((size_t)b * a.kv_heads + kv_head) * a.slots;
+  const uint16_t* keys = a.k + row0 * C;
+  const uint16_t* values = a.v + row0 * C;
   // The current token may not be in the caches yet (new_k / new_v given): every block takes its row from there, and
-  // the block of the group's first head whose slots include it stores it for the steps to come.
+  // one block stores it for the steps to come.
   const int fresh_slot = a.new_k ? (a.window ? ring_position : position) : -1;
   const uint16_t* fresh_k = a.new_k ? a.new_k + ((size_t)b * a.kv_heads + kv_head) * C : nullptr;
   const uint16_t* fresh_v = a.new_k ? a.new_v + ((size_t)b * a.kv_heads + kv_head) * C : nullptr;
-  if (a.new_k && head % (a.heads / a.kv_heads) == 0 && fresh_slot >= slot_base && fresh_slot < slot_base + kAttnSlots &&
-      fresh_slot < a.slots && tid < kWords) {
-    const size_t at = (((size_t)b * a.kv_heads + kv_head) * a.slots + fresh_slot) * C;
-    reinterpret_cast<uint32_t*>(a.k_store + at)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_k) + tid);
-    reinterpret_cast<uint32_t*>(a.v_store + at)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_v) + tid);
+  if (a.new_k && chunk == 0 && split == 0 && fresh_slot < a.slots) {
+    for (int i = tid; i < C / 2; i += kAttnThreads) {
+      reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[i] = __ldg(reinterpret_cast<const uint32_t*>(fresh_k) + i);
+      reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[i] = __ldg(reinterpret_cast<const uint32_t*>(fresh_v) + i);
+    }
   }
-  bool k_allowed[kAttnKeys];
-  uint32_t kw[kAttnKeys][kPerLane];
+  // The slots that can count at all (a full layer: from the end of the padding to the position; a ring: all that have
+  // been written) are dealt evenly to the splits, so that the blocks of a short context are as busy as those of a long one.
+  const int lo = a.window ? 0 : max(0, position - reach);
+  const int hi = (a.window == 0 || a.slots <= a.window) ? min(a.slots, position + 1) : a.slots;
+  const int units = hi > lo ? (hi - lo + kAttnUnit - 1) / kAttnUnit : 0;
+  const int unit0 = (int)((long long)units * split / a.splits), unit1 = (int)((long long)units * (split + 1) / a.splits);
+
+  uint4 kq[2][kPieces];
+  auto load_keys = [&](int unit) {
 #pragma unroll
-  for (int j = 0; j < kAttnKeys; ++j) {
-    const int slot = slot_base + warp * kAttnKeys + j;
-    k_allowed[j] = allowed_at(slot);
-    const uint32_t* row = reinterpret_cast<const uint32_t*>(slot == fresh_slot ? fresh_k : keys + (size_t)slot * C);
+    for (int n = 0; n < 2; ++n) {
+      const int slot = lo + unit * kAttnUnit + n * 8 + g;
+      const bool ok = unit < unit1 && allowed_at(slot);
+      const uint4* row = reinterpret_cast<const uint4*>(slot == fresh_slot ? fresh_k : keys + (size_t)slot * C);
 #pragma unroll
-    for (int i = 0; i < kPerLane; ++i) kw[j][i] = (k_allowed[j] && i * 32 + lane < kWords) ? __ldg(row + i * 32 + lane) : 0u;
-  }
-  const int pair = tid % kWords, part = tid / kWords;   // value pass: this thread's channel pair, its slots part, part + kParts, ...
-  uint32_t vw[kValues];
-#pragma unroll
-  for (int n = 0; n < kValues; ++n) {
-    const int slot = slot_base + part + n * kParts;
-    // (a slot that is not allowed may hold anything: it is not read)
-    vw[n] = allowed_at(slot) ? __ldg(reinterpret_cast<const uint32_t*>(slot == fresh_slot ? fresh_v : values + (size_t)slot * C) + pair) : 0u;
-  }
+      for (int i = 0; i < kPieces; ++i) kq[n][i] = ok ? ldg_stream_16(row + t + 4 * i) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  int unit = unit0 + warp;
+  load_keys(unit);
+
   // logarithmic scaling of full-attention layers: query and bias times tau, each rounded to BF16 (the reference
   // multiplies in FP32 and casts back, my_inkling/model.py:583-590)
   const bool scaled = a.window == 0 && a.n_floor > 0;
   float tau = 1.f;
   if (scaled) tau = 1.f + a.alpha * logf(fmaxf((float)(position + 1) / (float)a.n_floor, 1.f));
-  if (tid < C) {
-    const float x = bf16_to_f32(a.q[((size_t)b * a.heads + head) * C + tid]);
-    s_q[tid] = scaled ? round_bf16(x * tau) : x;
-  }
-  // relative bias of this block's slots: (r @ proj)[distance], a BF16 matmul (FP32 sum, rounded once)
-  if (tid >= kAttnThreads - kAttnSlots) {
-    const int i = tid - (kAttnThreads - kAttnSlots), slot = slot_base + i;
-    const int d = distance_of(slot);
-    float bias = 0.f;
-    if (slot < a.slots && d >= 0 && d < a.extent) {
-      const uint16_t* r = a.r + ((size_t)b * a.heads + head) * a.d_rel;
-      float sum = 0.f;
-#pragma unroll 8
-      for (int j = 0; j < a.d_rel; ++j) sum = fmaf(bf16_to_f32(r[j]), bf16_to_f32(__ldg(a.proj + (size_t)j * a.extent + d)), sum);
-      bias = round_bf16(sum);
-      if (scaled) bias = round_bf16(bias * tau);
+  uint4 qf[kPieces];
+#pragma unroll
+  for (int i = 0; i < kPieces; ++i) {
+    qf[i] = g < n_heads ? __ldg(reinterpret_cast<const uint4*>(a.q + ((size_t)b * a.heads + head0 + g) * C) + t + 4 * i) : make_uint4(0, 0, 0, 0);
+    if (scaled) {
+      qf[i].x = pack_bf16(bf16lo(qf[i].x) * tau, bf16hi(qf[i].x) * tau);
+      qf[i].y = pack_bf16(bf16lo(qf[i].y) * tau, bf16hi(qf[i].y) * tau);
+      qf[i].z = pack_bf16(bf16lo(qf[i].z) * tau, bf16hi(qf[i].z) * tau);
+      qf[i].w = pack_bf16(bf16lo(qf[i].w) * tau, bf16hi(qf[i].w) * tau);
     }
-    s_bias[i] = bias;
+  }
+  const int rel_steps = (a.d_rel + 15) / 16, rel_pitch = rel_steps * 16;
+  for (int i = tid; i < kAttnHeads * rel_pitch; i += kAttnThreads) {
+    const int h = i / rel_pitch, j = i % rel_pitch;
+    s_r[i] = (h < n_heads && j < a.d_rel) ? a.r[((size_t)b * a.heads + head0 + h) * a.d_rel + j] : (uint16_t)0;
   }
   __syncthreads();
-  // ---- scores: warp w holds the key rows of the slots w * 8 .. w * 8 + 7 of the block
-  {
-    float dot[kAttnKeys];
+
+  float acc[kHalves * 8][4];
 #pragma unroll
-    for (int j = 0; j < kAttnKeys; ++j) {
-      float sum = 0.f;
+  for (int i = 0; i < kHalves * 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  float top = -INFINITY, total = 0.f;   // of head g over this warp's slots (total: this lane's slots only)
+#pragma unroll 1
+  for (; unit < unit1; unit += kAttnWarps) {
+    const int slot0 = lo + unit * kAttnUnit;
+    // ---- the values of the step are asked for before its scores are computed ...
+    const uint4* vrow[4];
+    bool vok[4];
 #pragma unroll
-      for (int i = 0; i < kPerLane; ++i) {
-        const int at = i * 32 + lane;
-        if (at < kWords) {
-          sum = fmaf(s_q[2 * at], bf16lo(kw[j][i]), sum);
-          sum = fmaf(s_q[2 * at + 1], bf16hi(kw[j][i]), sum);
+    for (int i = 0; i < 4; ++i) {
+      const int slot = slot0 + 2 * t + (i & 1) + (i >> 1) * 8;
+      vok[i] = allowed_at(slot);   // (a slot that is not allowed may hold anything: it is not read)
+      vrow[i] = reinterpret_cast<const uint4*>(slot == fresh_slot ? fresh_v : values + (size_t)slot * C);
+    }
+    constexpr int kAhead = kHalves > 2 ? 1 : kHalves;   // (256 channels: half of the row at a time, for the registers)
+    uint4 vv[kAhead][4];
+    auto load_values = [&](int h, uint4 (&to)[4]) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) to[i] = vok[i] ? ldg_stream_16(vrow[i] + g + 8 * h) : make_uint4(0, 0, 0, 0);
+    };
+#pragma unroll
+    for (int h = 0; h < kAhead; ++h) load_values(h, vv[h]);
+    // ---- scores
+    float sc[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) {
+        mma_bf16(sc[n], qf[i].x, 0u, qf[i].y, 0u, kq[n][i].x, kq[n][i].y);
+        mma_bf16(sc[n], qf[i].z, 0u, qf[i].w, 0u, kq[n][i].z, kq[n][i].w);
+      }
+    }
+    // ---- ... and the next step's keys before the softmax
+    load_keys(unit + kAttnWarps);
+    float s[2][2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      // relative bias of the step's slots: (r @ proj)[distance], a BF16 matmul (FP32 sum, rounded once)
+      const int d_mine = distance_of(slot0 + n * 8 + g);
+      const bool rel = slot0 + n * 8 + g < a.slots && d_mine >= 0 && d_mine < a.extent;
+      float bias[4] = {0.f, 0.f, 0.f, 0.f};
+      if (__any_sync(0xffffffffu, rel)) {
+#pragma unroll 1
+        for (int step = 0; step < rel_steps; ++step) {
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int j = step * 16 + 2 * t + (i & 1) + (i >> 1) * 8;
+            w[i] = (rel && j < a.d_rel) ? (uint32_t)__ldg(a.proj + (size_t)j * a.extent + d_mine) : 0u;
+          }
+          const uint32_t* r2 = reinterpret_cast<const uint32_t*>(s_r + g * rel_pitch + step * 16) + t;
+          mma_bf16(bias, r2[0], 0u, r2[4], 0u, w[0] | (w[1] << 16), w[2] | (w[3] << 16));
         }
       }
-      dot[j] = sum;
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int j = 0; j < kAttnKeys; ++j) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int j = 0; j < kAttnKeys; ++j)
-        s_scores[warp * kAttnKeys + j] = k_allowed[j] ? dot[j] * a.scale + s_bias[warp * kAttnKeys + j] : -INFINITY;
-    }
-  }
-  __syncthreads();
-  // the block's 64 scores: every warp finds the maximum for itself (two scores per lane, five shuffles), the
-  // first two warps turn the scores into exponentials once for everybody
-  static_assert(kAttnSlots % 32 == 0, "whole scores per lane");
-  float top = s_scores[lane];
-#pragma unroll
-  for (int i = 1; i < kAttnSlots / 32; ++i) top = fmaxf(top, s_scores[lane + 32 * i]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  if (tid < kAttnSlots) {
-    const float sc = s_scores[tid];
-    s_bias[tid] = (sc == -INFINITY) ? 0.f : __expf(sc - top);   // (the biases are in the scores by now)
-  }
-  __syncthreads();
-  float acc0 = 0.f, acc1 = 0.f, sum = 0.f;
-#pragma unroll
-  for (int n = 0; n < kValues; ++n) {
-    const float p = s_bias[part + n * kParts];
-    acc0 = fmaf(p, bf16lo(vw[n]), acc0);
-    acc1 = fmaf(p, bf16hi(vw[n]), acc1);
-    sum += p;
-  }
-  s_part[2 * tid] = acc0;
-  s_part[2 * tid + 1] = acc1;
-  __syncthreads();
-  if (pair == 0) s_scores[part] = sum;   // (the scores are not needed any more) one partial sum of exponentials per part
-  __syncthreads();
-  if (tid < kWords) {
-    float o0 = 0.f, o1 = 0.f, total = 0.f;
-#pragma unroll
-    for (int p = 0; p < kParts; ++p) {
-      o0 += s_part[2 * (p * kWords + tid)];
-      o1 += s_part[2 * (p * kWords + tid) + 1];
-      total += s_scores[p];
-    }
-    if (a.splits == 1) {
-      const float inv = 1.f / total;
-      uint32_t* out = reinterpret_cast<uint32_t*>(a.out + ((size_t)b * a.heads + head) * C);
-      out[tid] = f32_to_bf16_bits(o0 * inv) | (f32_to_bf16_bits(o1 * inv) << 16);
-    } else {
-      float* mine = a.partial + (((size_t)b * a.heads + head) * a.splits + split) * (kAttnPartial + C);
-      if (tid == 0) {
-        mine[0] = top;
-        mine[1] = total;
+      for (int i = 0; i < 2; ++i) {
+        float add = round_bf16(bias[i]);
+        if (scaled) add = round_bf16(add * tau);
+        s[n][i] = allowed_at(slot0 + n * 8 + 2 * t + i) ? fmaf(sc[n][i], a.scale, add) : -INFINITY;
       }
-      mine[kAttnPartial + 2 * tid] = o0;
-      mine[kAttnPartial + 2 * tid + 1] = o1;
-      __threadfence();   // every writer pushes its own stores out before the block is counted
+    }
+    float step_top = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+    step_top = fmaxf(step_top, __shfl_xor_sync(0xffffffffu, step_top, 1));
+    step_top = fmaxf(step_top, __shfl_xor_sync(0xffffffffu, step_top, 2));
+    if (__any_sync(0xffffffffu, step_top > top)) {   // rare after the first steps: what has been summed moves to the new maximum
+      const float next = fmaxf(top, step_top);
+      const float factor = top == -INFINITY ? 0.f : __expf(top - next);
+      top = next;
+      total *= factor;
+#pragma unroll
+      for (int i = 0; i < kHalves * 8; ++i) {
+        acc[i][0] *= factor;
+        acc[i][1] *= factor;
+        acc[i][2] *= factor;
+        acc[i][3] *= factor;
+      }
+    }
+    uint32_t p_hi[2], p_lo[2];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const float p0 = s[n][0] == -INFINITY ? 0.f : __expf(s[n][0] - top), p1 = s[n][1] == -INFINITY ? 0.f : __expf(s[n][1] - top);
+      total += p0 + p1;
+      p_hi[n] = pack_bf16(p0, p1);
+      p_lo[n] = pack_bf16(p0 - bf16lo(p_hi[n]), p1 - bf16hi(p_hi[n]));
+    }
+    // ---- weighted values: 8 channels of the lane's piece, one instruction each
+#pragma unroll
+    for (int h = 0; h < kHalves; ++h) {
+      uint4(&v4)[4] = vv[h < kAhead ? h : 0];
+      if (h >= kAhead) load_values(h, v4);
+      const uint32_t w0[4] = {v4[0].x, v4[0].y, v4[0].z, v4[0].w}, w1[4] = {v4[1].x, v4[1].y, v4[1].z, v4[1].w};
+      const uint32_t w2[4] = {v4[2].x, v4[2].y, v4[2].z, v4[2].w}, w3[4] = {v4[3].x, v4[3].y, v4[3].z, v4[3].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        mma_bf16(acc[h * 8 + 2 * j], p_hi[0], p_lo[0], p_hi[1], p_lo[1], __byte_perm(w0[j], w1[j], 0x5410), __byte_perm(w2[j], w3[j], 0x5410));
+        mma_bf16(acc[h * 8 + 2 * j + 1], p_hi[0], p_lo[0], p_hi[1], p_lo[1], __byte_perm(w0[j], w1[j], 0x7632), __byte_perm(w2[j], w3[j], 0x7632));
+      }
+    }
+  }
+  total += __shfl_xor_sync(0xffffffffu, total, 1);
+  total += __shfl_xor_sync(0xffffffffu, total, 2);
+  __syncthreads();   // (the relative states make room)
+  // ---- the warps' sums, then the block's: thread = (head, channels)
+  {
+    float* mine = s_acc + (warp * kAttnHeads + g) * (C + 2);
+    if (t == 0) {
+      mine[C] = top;
+      mine[C + 1] = total;
+    }
+#pragma unroll
+    for (int h = 0; h < kHalves; ++h)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mine[h * 64 + 16 * t + 8 * n + j] = acc[h * 8 + j][n] + acc[h * 8 + j][2 + n];
+  }
+  __syncthreads();
+  constexpr int kPairs = C / 2;                       // channel pairs of a head
+  const int stride = kAttnPartial + C;
+  for (int i = tid; i < n_heads * kPairs; i += kAttnThreads) {
+    const int h = i / kPairs, pair = i % kPairs;
+    float all_top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) all_top = fmaxf(all_top, s_acc[(w * kAttnHeads + h) * (C + 2) + C]);
+    float o0 = 0.f, o1 = 0.f, sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kAttnWarps; ++w) {
+      const float* from = s_acc + (w * kAttnHeads + h) * (C + 2);
+      const float weight = from[C] == -INFINITY ? 0.f : __expf(from[C] - all_top);
+      o0 = fmaf(from[2 * pair], weight, o0);
+      o1 = fmaf(from[2 * pair + 1], weight, o1);
+      sum = fmaf(from[C + 1], weight, sum);
+    }
+    const size_t row = (size_t)b * a.heads + head0 + h;
+    if (a.splits == 1) {
+      const float inv = 1.f / sum;
+      reinterpret_cast<uint32_t*>(a.out + row * C)[pair] = pack_bf16(o0 * inv, o1 * inv);
+    } else {
+      float* mine = a.partial + (row * a.splits + split) * stride;
+      if (pair == 0) *reinterpret_cast<float2*>(mine) = make_float2(all_top, sum);
+      *reinterpret_cast<float2*>(mine + kAttnPartial + 2 * pair) = make_float2(o0, o1);
     }
   }
   if (a.splits == 1) return;
-  // The block that stores the last partial of its (sequence, head) joins them all:
+  // The block that stores the last partial of its heads joins them all:
   //   out = sum_i acc_i e^(m_i - M) / sum_i l_i e^(m_i - M)
-  __shared__ bool s_last;
+  __threadfence();   // every writer pushes its own stores out before the block is counted
   __syncthreads();
   if (tid == 0) {
-    unsigned* arrived = a.arrived + (size_t)b * a.heads + head;
+    unsigned* arrived = a.arrived + (size_t)b * gridDim.y + blockIdx.y;
     s_last = atomicAdd(arrived, 1u) + 1u == (unsigned)a.splits;
     if (s_last) *arrived = 0u;   // left as found, for the next launch
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  const int stride = kAttnPartial + C;
-  const float* base = a.partial + ((size_t)b * a.heads + head) * a.splits * stride;
-  float all_top = -INFINITY;
-  for (int i = lane; i < a.splits; i += 32) all_top = fmaxf(all_top, __ldcg(base + (size_t)i * stride));
+  for (int i = tid; i < n_heads * kPairs; i += kAttnThreads) {
+    const int h = i / kPairs, pair = i % kPairs;
+    const size_t row = (size_t)b * a.heads + head0 + h;
+    const float* base = a.partial + row * a.splits * stride;
+    float all_top = -INFINITY;
+    for (int s = lane; s < a.splits; s += 32) all_top = fmaxf(all_top, __ldcg(base + (size_t)s * stride));   // (a warp is inside one head)
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, o));
-  // thread = (channel pair, part): every part takes every kParts-th partial, then the parts are added up
-  float o0 = 0.f, o1 = 0.f, total = 0.f;
-  for (int i = part; i < a.splits; i += kParts) {
-    const float* from = base + (size_t)i * stride;
-    const float m = __ldcg(from);
-    if (m == -INFINITY) continue;
-    const float weight = __expf(m - all_top);
-    total = fmaf(__ldcg(from + 1), weight, total);
-    const float2 acc = __ldcg(reinterpret_cast<const float2*>(from + kAttnPartial) + pair);
-    o0 = fmaf(acc.x, weight, o0);
-    o1 = fmaf(acc.y, weight, o1);
-  }
-  s_part[2 * tid] = o0;
-  s_part[2 * tid + 1] = o1;
-  if (pair == 0) s_scores[part] = total;
-  __syncthreads();
-  if (tid < kWords) {
-    float f0 = 0.f, f1 = 0.f, sum_all = 0.f;
-#pragma unroll
-    for (int p = 0; p < kParts; ++p) {
-      f0 += s_part[2 * (p * kWords + tid)];
-      f1 += s_part[2 * (p * kWords + tid) + 1];
-      sum_all += s_scores[p];
+    for (int o = 16; o > 0; o >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, o));
+    float o0 = 0.f, o1 = 0.f, sum = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < a.splits; ++s) {
+      const float* from = base + (size_t)s * stride;
+      const float2 head = __ldcg(reinterpret_cast<const float2*>(from));
+      const float2 val = __ldcg(reinterpret_cast<const float2*>(from + kAttnPartial) + pair);
+      const float weight = head.x == -INFINITY ? 0.f : __expf(head.x - all_top);
+      sum = fmaf(head.y, weight, sum);
+      o0 = fmaf(val.x, weight, o0);
+      o1 = fmaf(val.y, weight, o1);
     }
-    const float inv = 1.f / sum_all;
-    uint32_t* out = reinterpret_cast<uint32_t*>(a.out + ((size_t)b * a.heads + head) * C);
-    out[tid] = f32_to_bf16_bits(f0 * inv) | (f32_to_bf16_bits(f1 * inv) << 16);
+    const float inv = 1.f / sum;
+    reinterpret_cast<uint32_t*>(a.out + row * C)[pair] = pack_bf16(o0 * inv, o1 * inv);
   }
 }
 
@@ -267,9 +349,25 @@ using namespace ink;
 
 static size_t attention_counter_bytes(int batch, int heads) { return ((size_t)batch * heads * sizeof(unsigned) + 255) / 256 * 256; }
 
+// Splits along the cache at most: what the workspace is sized for, whatever the number of key/value heads.
+static int attention_max_splits(int slots) {
+  const int whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
+  return whole < kAttnMaxSplits ? whole : kAttnMaxSplits;
+}
+
 extern "C" size_t ink_decode_attention_workspace_bytes(int batch, int heads, int head_dim, int slots) {
-  const size_t splits = ((size_t)slots + kAttnSlots - 1) / kAttnSlots;
+  const size_t splits = (size_t)attention_max_splits(slots);
   return splits <= 1 ? 0 : attention_counter_bytes(batch, heads) + sizeof(float) * (size_t)batch * heads * splits * (kAttnPartial + head_dim);
+}
+
+template <int C>
+static int launch_decode_attention(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
+  const size_t sums = sizeof(float) * kAttnWarps * kAttnHeads * (C + 2), rel = sizeof(uint16_t) * kAttnHeads * ((size_t)(a.d_rel + 15) / 16 * 16);
+  const size_t smem = sums > rel ? sums : rel;
+  INK_REQUIRE(smem <= 48 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
+  decode_attention_kernel<C><<<grid, kAttnThreads, smem, stream>>>(a);
+  INK_CHECK_LAUNCH("decode_attention");
+  return kOk;
 }
 
 extern "C" int ink_decode_attention(const void* q, const void* r, const void* proj, void* k_cache,
@@ -285,24 +383,30 @@ extern "C" int ink_decode_attention(const void* q, const void* r, const void* pr
   INK_REQUIRE(d_rel > 0 && rel_extent > 0 && slots > 0 && window >= 0 && (window == 0 || window <= slots), kBadArgument,
               "decode_attention: d_rel=%d rel_extent=%d slots=%d window=%d", d_rel, rel_extent, slots, window);
   INK_REQUIRE((new_k == nullptr) == (new_v == nullptr), kBadArgument, "decode_attention: new_k and new_v come together");
-  const int splits = (slots + kAttnSlots - 1) / kAttnSlots;
-  INK_REQUIRE(splits <= 65535 && batch <= 65535, kUnsupportedShape, "decode_attention: %d slots or %d sequences exceed the grid", slots, batch);
+  const int group = heads / kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
+  INK_REQUIRE((long long)kv_heads * chunks <= 65535 && batch <= 65535, kUnsupportedShape,
+              "decode_attention: %d heads or %d sequences exceed the grid", heads, batch);
   const size_t need = ink_decode_attention_workspace_bytes(batch, heads, head_dim, slots);
   INK_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), kBadArgument,
               "decode_attention: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-  INK_REQUIRE(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out) && (need == 0 || aligned16(workspace)),
+  INK_REQUIRE(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out) && aligned16(new_k) && aligned16(new_v) &&
+                  (need == 0 || aligned16(workspace)),
               kMisaligned, "decode_attention: buffers must be 16-byte aligned");
   if (batch == 0) return kOk;
+  // Parts of the cache: enough blocks to fill the GPU (three of four warps fit on an SM), none with less than a step
+  // per warp. Where one wave of long parts would leave SMs idle at its end (few pairs of sequence and head group), the
+  // parts are small anyway; with many pairs there are two waves' worth, so that shorter sequences even out.
+  const int pairs = batch * kv_heads * chunks, most = attention_max_splits(slots);
+  const int wanted = (kAttnWaveBlocks * 2 + pairs - 1) / pairs;
+  const int splits = wanted < 1 ? 1 : wanted < most ? wanted : most;
   AttnArgs a{(const uint16_t*)q, (const uint16_t*)r, (const uint16_t*)proj, (const uint16_t*)k_cache, (const uint16_t*)v_cache,
              position, pad_counts, (const uint16_t*)new_k, (const uint16_t*)new_v, (uint16_t*)k_cache, (uint16_t*)v_cache,
-             (float*)((char*)workspace + attention_counter_bytes(batch, heads)), (unsigned*)workspace, (uint16_t*)out, heads, kv_heads, head_dim, d_rel, rel_extent, slots, window,
-             n_floor, splits, alpha, scale};
-  const dim3 grid(heads, batch, splits);
-  if (head_dim == 64) decode_attention_kernel<64><<<grid, kAttnThreads, 0, (cudaStream_t)stream>>>(a);
-  else if (head_dim == 128) decode_attention_kernel<128><<<grid, kAttnThreads, 0, (cudaStream_t)stream>>>(a);
-  else decode_attention_kernel<256><<<grid, kAttnThreads, 0, (cudaStream_t)stream>>>(a);
-  INK_CHECK_LAUNCH("decode_attention");
-  return kOk;
+             (float*)((char*)workspace + attention_counter_bytes(batch, heads)), (unsigned*)workspace, (uint16_t*)out, heads, kv_heads,
+             d_rel, rel_extent, slots, window, n_floor, splits, alpha, scale};
+  const dim3 grid((unsigned)splits, (unsigned)(kv_heads * chunks), (unsigned)batch);
+  if (head_dim == 64) return launch_decode_attention<64>(a, grid, (cudaStream_t)stream);
+  if (head_dim == 128) return launch_decode_attention<128>(a, grid, (cudaStream_t)stream);
+  return launch_decode_attention<256>(a, grid, (cudaStream_t)stream);
 }
 
 extern "C" int ink_update_kv(const void* new_k, const void* new_v, void* k_cache, void* v_cache, const int64_t* position,

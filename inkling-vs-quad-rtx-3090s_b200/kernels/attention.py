@@ -57,6 +57,8 @@ def decode_attention(query, relative_states, proj, k_cache, v_cache, position, p
         new_k = new_key.reshape(bs, hk, c).contiguous()
         new_v = new_value.reshape(bs, hk, c).contiguous()
         assert new_k.dtype == new_v.dtype == torch.bfloat16
+        if (new_k.data_ptr() | new_v.data_ptr()) & 15:   # the kernel reads rows 16 bytes at a time
+            new_k, new_v = new_k.clone(), new_v.clone()
     if out is None:
         out = torch.empty((bs, h, 1, c), dtype=torch.bfloat16, device=q.device)
     need = _abi.lib().ink_decode_attention_workspace_bytes(bs, h, c, slots)

@@ -355,3 +355,35 @@ def test_a_decode_step_of_the_whole_model(ib, step):
     assert (got[same] - want[same]).abs().max() <= TOL * scale, float((got[same] - want[same]).abs().max() / scale)
     assert (got - want).abs().max() <= 0.15 * scale
     assert torch.equal(got.argmax(-1), want.argmax(-1))          # the same next token
+
+
+@pytest.mark.parametrize("c,h,hk,slots,window,position,d_rel", [
+    (128, 8, 8, 64, 0, 0, 16),            # one slot in use, one head per key/value head
+    (128, 9, 1, 65, 0, 64, 16),           # nine heads on one key/value head (a second, nearly empty group), one slot past a part
+    (64, 32, 2, 300, 0, 271, 20),         # two full groups of eight per key/value head; relative states that end inside a step
+    (256, 8, 2, 1000, 0, 999, 7),         # the cache full
+    (128, 12, 4, 5000, 0, 4100, 16),      # more parts than blocks have steps for in places
+    (128, 8, 1, 80, 48, 31, 16),          # a ring shorter than its cache, not yet full
+    (64, 8, 2, 48, 48, 1000, 16),         # a ring that is not a multiple of a step, wrapped
+])
+def test_decode_attention_at_the_edges_of_its_parts(ib, c, h, hk, slots, window, position, d_rel):
+    """Steps of 16 slots, groups of eight heads, parts along the cache: remainders of each, against the oracle with
+    the module's roundings (bar: BF16 results of a softmax-weighted sum, as above)."""
+    device = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(17)
+    bs, extent = 2, max(8, slots // 2)
+    draw = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()  # noqa: E731
+    q, r, proj = draw(bs, h, c), draw(bs, h, d_rel), draw(d_rel, extent)
+    k, v, new_k, new_v = draw(bs, hk, slots, c), draw(bs, hk, slots, c), draw(bs, hk, c), draw(bs, hk, c)
+    slot = position % window if window else position
+    before = [t.clone().to(device) for t in (k, v)]
+    k[:, :, slot], v[:, :, slot] = new_k, new_v
+    pad = torch.tensor([0, min(position, 19)])
+    want = oa.decode_attention(q, r, proj, k, v, position, pad, window, 40, 0.1, 1.0 / c).float()
+    for _ in range(2):   # the second call finds the arrival counters as the first left them
+        got = ib.kernels.decode_attention(q.to(device), r.to(device), proj.to(device), *before, torch.tensor(position, device=device),
+                                          pad.to(device), window=window, log_scaling_n_floor=40, new_key=new_k.to(device).unsqueeze(2),
+                                          new_value=new_v.to(device).unsqueeze(2))
+    torch.cuda.synchronize()
+    assert (got[:, :, 0].float().cpu() - want).abs().max() <= TOL * want.abs().max()
+    assert torch.equal(before[0].cpu(), k) and torch.equal(before[1].cpu(), v)
