@@ -247,20 +247,45 @@ int ink_expert_reduce(const void* down, const int64_t* indices, const void* weig
  * ink_expert_gemm): the packed E2M1 codes of an expert's 128-row tile and their E4M3 block scales are the
  * M operand of tcgen05.mma.kind::mxf4nvf4.block_scale.block16 straight from the checkpoint layout -- no
  * conversion on the CUDA cores -- and the tokens routed to the expert are the N operand as four E2M1 digit
- * rows each (power-of-two block scales; exact to 2^-9 of the block's largest magnitude), eight tokens per
- * pass. Each active expert's bytes cross HBM once per eight of its tokens.
+ * rows each (power-of-two block scales; exact to 2^-9 of the block's largest magnitude).
  *  bank_maps  device copy (128-byte aligned) of the 512 bytes ink_moe_stack_encode_banks wrote for this
  *             layer's banks, which must therefore be evenly spaced in memory; `start` is the expert id of
  *             the first bank the descriptors cover (experts[g] - start indexes them)
  *  pointers   as for ink_expert_gemm: the FP32 scale2 is read through it, a zero row skips the expert
- *  scratch    ink_expert_gemm_tc_scratch_bytes(input_rows, k) bytes: a kernel in front writes every input row's
- *             normaliser, digit rows and block scales there once; the main kernel reads them per expert tile
+ *  scratch    ink_expert_gemm_tc_scratch_bytes(input_rows, k) bytes (of up to eight choices a row; more choices: as if
+ *             for proportionally more rows): a kernel in front writes the N operand there
  * Constraints: n a multiple of 128, k a multiple of 256 up to 4096, groups <= 1024. */
 size_t ink_expert_gemm_tc_scratch_bytes(int input_rows, int k);
 int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, const int64_t* pointers,
                        const int32_t* experts, const int32_t* rows, const int32_t* counts, void* y, int capacity,
                        int n, int k, int top_k, int projection, int groups, int start, void* scratch,
                        size_t scratch_bytes, int32_t* status, ink_stream_t stream);
+
+/* The whole layer after the routing for several tokens, on the same kernels (my_inkling/offloaded_experts.py:249-310 and
+ * my_inkling/model.py:192-226): both routed projections and the weighted sum, and -- with n_shared > 0 -- the shared
+ * experts as further tiles of the same launches. Each active expert's bytes cross HBM once.
+ *  indices, weights, experts, rows, counts, pointers   as for ink_expert_gemm / ink_expert_reduce, of ink_expert_plan
+ *  quantized   1: NVFP4 banks, bank_maps of ink_moe_stack_encode_banks (512 bytes); 0: BF16 banks (pointer stride 2),
+ *              bank_maps of ink_encode_bf16_banks (256 bytes); device copies, 128-byte aligned
+ *  shared_maps device copy of ink_encode_shared's 384 bytes, gammas BF16 [tokens, n_shared] (both unused for n_shared = 0)
+ *  activated   scratch BF16 [tokens * top_k, intermediate]: left holding the routes' gate/up results; down likewise BF16
+ *              [tokens * top_k, hidden]: their down projections before the router weights
+ *  output      FP32 [tokens, hidden], fully overwritten, or NULL; output_bf16 the same rounded to BF16, or NULL
+ *  groups      entries of experts / counts to visit; start, local: first expert and number of experts of this rank
+ *  status      bit 0: a route named an expert outside [0, max_expert] (it is skipped); bit 1: a bounded wait gave up
+ * Constraints: hidden and intermediate up to 4096, multiples of 256 (BF16 banks: of 64, hidden of 128); groups <= 1024. */
+int ink_encode_bf16_banks(void* out_host_256, const void* gate_up, uint64_t gate_up_stride, const void* down,
+                          uint64_t down_stride, int experts, int hidden, int intermediate);
+int ink_encode_shared(void* out_host_384, const void* gate, const void* up, const void* down, int n_shared, int hidden,
+                      int intermediate);
+size_t ink_moe_grouped_scratch_bytes(int tokens, int top_k, int n_shared, int hidden, int intermediate, int groups,
+                                     int quantized);
+int ink_moe_grouped(const void* x, const int64_t* indices, const void* weights, const int64_t* pointers,
+                    const int32_t* experts, const int32_t* rows, const int32_t* counts, const void* bank_maps,
+                    const void* shared_maps, const void* gammas, void* activated, void* down, float* output,
+                    void* output_bf16, int tokens, int top_k, int n_shared, int hidden, int intermediate, int groups, int start, int local, int capacity,
+                    int max_expert, int quantized, void* scratch, size_t scratch_bytes, int32_t* status,
+                    ink_stream_t stream);
 
 /* ------------------------------------------------- whole stack, one launch ------
  * One decode token through n_layers MoE blocks in ONE persistent cooperative kernel:

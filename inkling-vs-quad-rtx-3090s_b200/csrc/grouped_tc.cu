@@ -1,70 +1,77 @@
-// Grouped expert projections on the block-scaled tensor-core path: the packed NVFP4 codes of an
-// expert's 128-row weight tile are the M operand of tcgen05.mma.kind::mxf4nvf4.block_scale.block16
-// straight from the checkpoint layout (tiled TMA into a ring of 18 KB units: 128 rows x 256 columns of
-// codes and their E4M3 block scales), nothing is converted on the CUDA cores; the tokens routed to the
-// expert are the N operand, each as four E2M1 digit rows with power-of-two block scales (tc_path.cuh),
-// up to eight tokens (N = 32) per pass. Every active expert's bytes cross HBM once per eight of its
-// tokens; accumulators live in tensor memory and are read back once per tile. The digit rows of every
-// input row are made ONCE, by a small kernel in front, as ready-to-use pieces of the swizzled operand
-// (a piece's swizzle depends on whether its token sits in an even or an odd slot of the batch, so both
-// are kept); the main kernel only copies the pieces of a batch's tokens into place. (Making them per
-// work item -- thirty-two tiles per expert need the same rows -- cost two thirds of the kernel's time.)
+// Expert projections for more than one token on the tcgen05 tensor cores. One kernel takes every weight tile of a
+// projection: the routed experts' (packed NVFP4 through tcgen05.mma.kind::mxf4nvf4.block_scale straight from the
+// checkpoint layout, or BF16 banks through kind::f16) and the shared experts' (BF16). The weights are the M operand and
+// stream from HBM; the tokens of an expert are the N operand.
 //
-// Persistent blocks, one per SM. A work item is (expert group, batch of <= 8 routes, 128-row tile), tile
-// fastest; every block takes a contiguous run of items, so it stages the activations of only one or two
-// batches (the tiles of a batch share them). Warp 0 lane 0 streams weight units (it runs ahead of everything
-// else: addresses do not depend on activations), warp 1 lane 0 issues the MMAs, warps 2..5 move each
-// unit's weight scales from shared to tensor memory, warps 6..9 read the accumulators and write the
-// outputs; warps 2..9 together turn the batch's activations into digit rows before its first MMA.
-// Every wait is bounded; a wait that gives up sets kFlagWaitTimedOut and the block drains.
-#include <stdlib.h>
-
+// The N operand is laid out by a small kernel in front (`stage_rows_kernel`) exactly as the main kernel's ring wants it,
+// tile by tile, so that the main kernel fetches it with one bulk copy per stage next to the weights and never gathers:
+//   NVFP4  a token is four E2M1 digit rows with power-of-two block scales (tc_path.cuh); a tile is up to 32 tokens;
+//   BF16   a token is a row of 64-column pieces; a tile is up to 128 tokens.
+// (Gathering the digit rows in the main kernel, eight tokens a pass, stalled its MMAs at the head of every pass, and every
+// expert's bank was read once per eight of its tokens: 64 tokens of one block 0.42 ms, 1 024 tokens 2.8 ms.)
+//
+// A ring stage is two weight units of 128 rows x 128 bytes (plus their block scales) and the N operand that goes with
+// them. TALL: the units are the two halves of a 256-row tile, so that each fetch of the N operand serves 256 rows -- for
+// prompts, where L2 traffic counts. Else (a few tokens per expert, everything waits for HBM) they are two consecutive
+// chunks of the contraction of a 128-row tile: smaller work items, which even out better over the SMs.
+//
+// Persistent blocks, one per SM. The shared experts' items (long) are dealt evenly, the routed items by cost in what is
+// left of each block's share. Warp 0 produces (its lanes issue a stage's copies side by side), warp 1 issues the MMAs,
+// warps 2..5 move block scales to tensor memory, warps 6..9 read accumulators and write outputs. The kernel is launched
+// while its predecessor runs (programmatic dependent launch): until that is done it only streams weights, whose
+// addresses depend on nothing but the plan. Every wait is bounded; one that gives up sets kFlagWaitTimedOut.
 #include "../../include/inkling_b200.h"
 #include "common.cuh"
 #include "decode_args.cuh"
 #include "pipe.cuh"
 #include "tc_path.cuh"
+#include "tensor_map.cuh"
 
 namespace ink {
 
-constexpr int kGtBatch = 8;                      // routes per pass (x 4 digit rows = MMA N 32)
-constexpr int kGtN = kGtBatch * kTcDigits;       // 32
-constexpr int kGtUnits = 7;                      // ring depth, units of kTcUnitBytes
-constexpr int kGtThreads = 320;
-constexpr int kGtWorkers = 256;                  // warps 2..9
-constexpr int kGtMaxGroups = 1024;
-constexpr int kGtMaxK = 4096;                    // activation scales of a whole row must fit the tensor-memory columns
+constexpr int kGgStages = 4;
+constexpr int kGgUnitBytes = kTcUnitBytes;                       // 128 rows x 128 B of codes, 2 KB of block scales: 18 KB
+constexpr int kGgRowsBytes = 18 * 1024;                          // the stage's N operand: up to 16 KB, and its block scales
+constexpr int kGgStageBytes = 2 * kGgUnitBytes + kGgRowsBytes;   // 54 KB
+constexpr int kGgThreads = 320;
+constexpr int kGgMaxGroups = 1024;
+constexpr int kGgSharedBox = 16;                                 // gate and up rows of a shared expert alternate by so many
+constexpr int kGgColD = 0, kGgColSf = 256, kGgSfPerStage = 64;   // tensor memory: accumulators, then each stage's scales
 
-struct GemmTcArgs {
-  const uint16_t* X;            // BF16 [*, K]
-  const unsigned char* maps;    // the layer's four TMA descriptors (gate/up codes, scales, down codes, scales)
-  const int64_t* pointers;      // [(max_expert + 1) * 6]: scale2 is read through it, a zero row is an inactive expert
+// tokens in a tile
+__host__ __device__ constexpr int gg_tile(bool fp4, bool tall) { return fp4 ? (tall ? 32 : 16) : (tall ? 128 : 64); }
+// slots of a group are padded to whole 1024-byte swizzle atoms of its tiles
+__host__ __device__ constexpr int gg_pad(bool fp4) { return fp4 ? 2 : 8; }
+
+struct GgArgs {
+  // routed experts
+  const unsigned char* maps;    // descriptors of this projection: codes and scales (NVFP4), or one (BF16)
+  const int64_t* pointers;      // [(max_expert + 1) * stride]: a zero row is an inactive expert; scale2 is read through it
   const int32_t* experts;       // [groups]
-  const int32_t* rows;          // [groups, capacity]
   const int32_t* counts;        // [groups]
-  uint16_t* Y;
-  const float2* row_scale;      // per row of X: {power-of-two multiplier, its inverse}
-  const unsigned char* digits;  // per row of X: [K/256 chunks][slot parity][4 digit rows][128 B], swizzled as the operand wants them
-  const unsigned char* digit_scales;   // per row of X: [4 digit rows][kGtMaxK / 16] E4M3 block scales
-  int capacity, n, k, top_k, groups, start;
+  const int32_t* rows;          // [groups, capacity]
+  const unsigned char* image;   // N operand, group after group (see stage_rows_kernel)
+  const unsigned char* image_scales;
+  const float* slot_scale;      // [slots] (NVFP4)
+  uint16_t* y;                  // BF16 [route][n / 2] (gate/up) or [route][n]
+  int groups, start, capacity, stride, bank, k, n;
+  // shared experts
+  const unsigned char* shared_maps;    // gate and up, or down
+  const unsigned char* shared_image;   // [tile][k / 64][tokens of the tile, padded to 8][128 B]; down: the same per expert
+  uint16_t* shared_y;           // gate/up: the image of the down projection; down: BF16 [tokens][n_shared][n]
+  const uint16_t* gammas;       // [tokens, n_shared]
+  int n_shared, tokens;
   int32_t* status;
-  long long* prof;              // optional [blocks][8] clock totals per phase (INKLING_GROUPED_PROFILE=1)
 };
 
-struct GtShared {
-  uint64_t full[kGtUnits], empty[kGtUnits];
-  uint64_t sf_full[kTcSfSlots], sf_empty[kTcSfSlots];
-  uint64_t d_full[2], d_empty[2];      // two accumulators: the next tile's MMAs run while this one is read
+struct GgShared {
+  uint64_t full[kGgStages], empty[kGgStages], sf_full[kGgStages];
+  uint64_t d_full[2], d_empty[2];
   uint32_t tmem_base;
-  volatile int staged;                 // items whose activations are staged as digit rows
   volatile int failed;
-  int first_item[kGtMaxGroups + 1];    // items before each group
-  int route[kGtBatch];
-  float out_scale[kGtBatch];
-  uint8_t sfb[kGtN][kGtMaxK / 16];     // block scales of the digit rows
 };
 
-__device__ __forceinline__ bool gt_wait(uint64_t* bar, uint32_t parity, GtShared* sh) {
+__device__ __forceinline__ bool gg_wait(uint64_t* bar, uint32_t parity, GgShared* sh) {
   if (sh->failed) return false;
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
@@ -77,369 +84,873 @@ __device__ __forceinline__ bool gt_wait(uint64_t* bar, uint32_t parity, GtShared
   }
   return true;
 }
-__device__ __forceinline__ void gt_worker_sync() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// batches of a group (0: nothing to do for it)
-__device__ __forceinline__ int gt_batches(const GemmTcArgs& a, int g, int bank) {
-  const int count = a.counts[g], expert = a.experts[g];
-  if (count <= 0 || expert < 0) return 0;
-  if (a.pointers[(size_t)expert * kBank + bank] == 0) return 0;
-  return (count + kGtBatch - 1) / kGtBatch;
+// routes of a group that have something to do
+__device__ __forceinline__ int gg_count(const int32_t* counts, const int32_t* experts, const int64_t* pointers, int stride, int bank, int g) {
+  const int count = counts[g], expert = experts[g];
+  if (count <= 0 || expert < 0 || pointers[(size_t)expert * stride + bank] == 0) return 0;
+  return count;
 }
 
-struct GtItem { int group, batch, tile, batches; };
-__device__ __forceinline__ GtItem gt_item(const GtShared& sh, int groups, int tiles, int index) {
-  int lo = 0, hi = groups;   // largest g with first_item[g] <= index
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (sh.first_item[mid] <= index) lo = mid;
-    else hi = mid;
-  }
-  GtItem it;
-  it.group = lo;
-  it.batches = (sh.first_item[lo + 1] - sh.first_item[lo]) / tiles;
-  const int local = index - sh.first_item[lo];
-  it.batch = local / tiles;
-  it.tile = local % tiles;
-  return it;
-}
-
-template <int PROJ>
-__global__ void __launch_bounds__(kGtThreads, 1) expert_gemm_tc_kernel(GemmTcArgs a) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ GtShared sh;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char* units = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
-  unsigned char* s_b = units + (size_t)kGtUnits * kTcUnitBytes;                          // [K/256][32 rows][128 B] digit rows
-  const int K = a.k, chunks = K / kTcChunkK, tiles = a.n / kTcRows;
-  const int bank = PROJ ? 3 : 0;
-  const unsigned char* map_codes = a.maps + (PROJ ? 256 : 0);
-  const unsigned char* map_scales = map_codes + 128;
-
-  // ---- items before each group: all threads fetch the groups' sizes, one warp adds them up
-  for (int g = threadIdx.x; g < a.groups; g += kGtThreads) sh.first_item[g + 1] = gt_batches(a, g, bank) * tiles;
-  __syncthreads();
-  if (warp == 0) {
-    const int per_lane = (a.groups + 31) / 32;
-    int mine = 0;
-    for (int i = 0; i < per_lane; ++i) {
-      const int g = lane * per_lane + i;
-      if (g < a.groups) mine += sh.first_item[g + 1];
-    }
-    int before = mine;
+// Exclusive prefix sums of `mine` over a warp's lanes; *total gets the sum.
+__device__ __forceinline__ int warp_before(int mine, int lane, int* total) {
+  int up_to = mine;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, before, o);
-      if (lane >= o) before += v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, up_to, o);
+    if (lane >= o) up_to += v;
+  }
+  *total = __shfl_sync(0xffffffffu, up_to, 31);
+  return up_to - mine;
+}
+
+// The groups' tables in shared memory: slot0[g] = first slot | padding slots of the group, cost[g] = cost of all groups
+// before. `slot0[g]` holds the group's count on entry.
+struct GgTables { int* slot0; int* cost; };
+template <typename CostOf>
+__device__ __forceinline__ void gg_scan(const GgTables& t, int groups, int pad, int lane, CostOf cost_of) {
+  int slots = 0, cost = 0;
+  for (int g0 = 0; g0 < groups; g0 += 32) {
+    const int g = g0 + lane, count = g < groups ? t.slot0[g] : 0;
+    const int padded = (count + pad - 1) / pad * pad, c = cost_of(count);
+    int all_slots, all_cost;
+    const int s = slots + warp_before(padded, lane, &all_slots), w = cost + warp_before(c, lane, &all_cost);
+    if (g < groups) {
+      t.slot0[g] = s | (padded - count);
+      t.cost[g] = w;
     }
-    before -= mine;
-    for (int i = 0; i < per_lane; ++i) {
-      const int g = lane * per_lane + i;
-      if (g < a.groups) {
-        before += sh.first_item[g + 1];
-        sh.first_item[g + 1] = before;   // items up to and including group g
-      }
+    slots += all_slots;
+    cost += all_cost;
+  }
+  if (lane == 0) {
+    t.slot0[groups] = slots;
+    t.cost[groups] = cost;
+  }
+}
+__device__ __forceinline__ int gg_first_slot(const int* slot0, int g, int pad) { return slot0[g] & ~(pad - 1); }
+__device__ __forceinline__ int gg_group_count(const int* slot0, int g, int pad) {
+  return gg_first_slot(slot0, g + 1, pad) - gg_first_slot(slot0, g, pad) - (slot0[g] & (pad - 1));
+}
+
+// One work item: a 128 (256) row tile of one expert's matrix against one tile of its tokens.
+struct GgItem {
+  bool shared;
+  int group;      // group of routes, or shared expert
+  int m0;         // first weight row
+  int tile, n;    // tile of tokens, and how many
+  int slot;       // first slot of the tile (routed)
+};
+
+template <bool FP4, bool TALL>
+struct GgWalk {
+  static constexpr int kM = TALL ? 256 : 128;
+  static constexpr int kTile = gg_tile(FP4, TALL), kPad = gg_pad(FP4), kSharedTile = gg_tile(false, TALL);
+  const GgArgs* a;
+  GgTables t;
+  int m_tiles, shared_tiles;
+  int shared_next, shared_end;   // shared items left
+  int group, mt, tile, limit;    // next routed item; it is this block's while its cost offset is below `limit`
+  int count;                     // routes of `group`
+
+  __device__ __forceinline__ int stages_of(bool shared) const {
+    const int chunks = a->k / ((FP4 && !shared) ? kTcChunkK : 64);
+    return TALL ? chunks : (chunks + 1) / 2;
+  }
+  // cost of one item with n tokens: its bytes, the streamed weights weighing most
+  __device__ static __forceinline__ int tile_cost(int n, int stages) { return stages * (64 + (TALL ? n : 2 * n) / (FP4 ? 1 : 4)); }
+  __device__ __forceinline__ int cost_per_mt(int c, int stages) const {
+    return c / kTile * tile_cost(kTile, stages) + (c % kTile ? tile_cost(c % kTile, stages) : 0);
+  }
+  __device__ __forceinline__ void find(int from) {   // the first routed item whose cost offset is at least `from`
+    const int stages = stages_of(false);
+    int lo = 0, hi = a->groups;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (t.cost[mid] <= from) lo = mid;
+      else hi = mid;
     }
-    if (lane == 0) sh.first_item[0] = 0;
-    if (lane == 0) {
-      for (int s = 0; s < kGtUnits; ++s) {
-        mbar_init(&sh.full[s], 1);
-        mbar_init(&sh.empty[s], 1);
+    group = lo;
+    mt = tile = 0;
+    count = a->groups > 0 ? gg_group_count(t.slot0, group, kPad) : 0;
+    const int cm = cost_per_mt(count, stages);
+    if (cm > 0) {
+      const int off = from - t.cost[group], ct = tile_cost(kTile, stages);
+      mt = off / cm;
+      tile = (off % cm + ct - 1) / ct;
+      if (tile * kTile >= count) {
+        tile = 0;
+        ++mt;
       }
-      for (int s = 0; s < kTcSfSlots; ++s) {
-        mbar_init(&sh.sf_full[s], 4);
-        mbar_init(&sh.sf_empty[s], 1);
-      }
-      for (int s = 0; s < 2; ++s) {
-        mbar_init(&sh.d_full[s], 1);
-        mbar_init(&sh.d_empty[s], 4);
-      }
-      sh.staged = 0;
-      sh.failed = 0;
-      mbar_init_fence();
+    } else {
+      mt = m_tiles;
+    }
+    skip();
+  }
+  __device__ __forceinline__ void skip() {
+    while (group < a->groups && (mt >= m_tiles || count == 0)) {
+      ++group;
+      mt = 0;
+      count = group < a->groups ? gg_group_count(t.slot0, group, kPad) : 0;
     }
   }
-  __syncthreads();
-  const int total = sh.first_item[a.groups];
-  const int item_lo = (int)((long long)blockIdx.x * total / gridDim.x), item_hi = (int)((long long)(blockIdx.x + 1) * total / gridDim.x);
-  if (item_hi <= item_lo) return;   // (before any tensor memory is taken)
+  __device__ __forceinline__ bool next(GgItem& it) {
+    if (shared_next < shared_end) {
+      const int s = shared_next++, per_e = (a->n + kM - 1) / kM * shared_tiles;
+      it.shared = true;
+      it.group = s / per_e;
+      it.m0 = s % per_e / shared_tiles * kM;
+      it.tile = s % shared_tiles;
+      it.n = min(kSharedTile, a->tokens - it.tile * kSharedTile);
+      it.slot = 0;
+      return true;
+    }
+    if (group >= a->groups) return false;
+    const int stages = stages_of(false);
+    if (t.cost[group] + mt * cost_per_mt(count, stages) + tile * tile_cost(kTile, stages) >= limit) return false;
+    it.shared = false;
+    it.group = group;
+    it.m0 = mt * kM;
+    it.tile = tile;
+    it.n = min(kTile, count - tile * kTile);
+    it.slot = gg_first_slot(t.slot0, group, kPad) + tile * kTile;
+    if (++tile * kTile >= count) {
+      tile = 0;
+      ++mt;
+      skip();
+    }
+    return true;
+  }
+};
+
+// E2M1 (block-scaled) items use tc_idesc / tc_mma; BF16 x BF16 -> FP32, M = 128:
+__device__ __forceinline__ uint32_t gg_idesc_bf16(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24); }
+__device__ __forceinline__ void gg_mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(ad),
+               "l"(bd), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+
+template <bool FP4, int PROJ, bool TALL>
+__global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __grid_constant__ GgArgs a) {
+  using Walk = GgWalk<FP4, TALL>;
+  constexpr int kAccs = TALL ? 1 : 2;            // accumulators in turn: the next item's MMAs run while one is read
+  constexpr int kAccCols = TALL ? 256 : 128;     // columns of one (TALL: 128 per half)
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ GgShared sh;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
+  GgTables tables;
+  tables.slot0 = reinterpret_cast<int*>(ring + (size_t)kGgStages * kGgStageBytes);
+  tables.cost = tables.slot0 + a.groups + 1;
+  Walk walk;
+  walk.a = &a;
+  walk.t = tables;
+  walk.m_tiles = (a.n + Walk::kM - 1) / Walk::kM;
+  walk.shared_tiles = a.n_shared > 0 ? (a.tokens + Walk::kSharedTile - 1) / Walk::kSharedTile : 0;
+
+  for (int g = threadIdx.x; g < a.groups; g += kGgThreads) tables.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kGgStages; ++s) {
+      mbar_init(&sh.full[s], 1);
+      mbar_init(&sh.empty[s], 1);
+      mbar_init(&sh.sf_full[s], 4);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&sh.d_full[s], 1);
+      mbar_init(&sh.d_empty[s], 4);
+    }
+    sh.failed = 0;
+    mbar_init_fence();
+  }
   if (warp == 1) tc_alloc(&sh.tmem_base, 512);
   tc_fence_before();
   __syncthreads();
+  if (warp == 0) {
+    const int stages = walk.stages_of(false), m_tiles = walk.m_tiles;
+    gg_scan(tables, a.groups, Walk::kPad, lane, [&](int count) { return m_tiles * walk.cost_per_mt(count, stages); });
+  }
+  __syncthreads();
   tc_fence_after();
+  pdl_trigger();
+  // ---- this block's share: its shared items, and the routed items in what remains of total / blocks
+  {
+    const int shared_items = a.n_shared * walk.m_tiles * walk.shared_tiles, G = gridDim.x, b = blockIdx.x;
+    const long long shared_cost = a.n_shared > 0 ? (long long)walk.stages_of(true) * (64 + min(a.tokens, Walk::kSharedTile) / 4) : 0;
+    const long long routed = tables.cost[a.groups], total = routed + shared_cost * shared_items;
+    // routed cost taken by the blocks before block x (a block whose shared items exceed its share takes none)
+    auto before = [&](int x) -> long long { return total * x / G - shared_cost * ((long long)shared_items * x / G); };
+    long long from = 0, to = 0;
+    for (int x = lane; x <= b + 1; x += 32) {
+      const long long v = before(x) < 0 ? 0 : before(x);
+      if (x <= b && v > from) from = v;
+      if (v > to) to = v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      from = max(from, __shfl_xor_sync(0xffffffffu, from, o));
+      to = max(to, __shfl_xor_sync(0xffffffffu, to, o));
+    }
+    walk.shared_next = (int)((long long)shared_items * b / G);
+    walk.shared_end = (int)((long long)shared_items * (b + 1) / G);
+    walk.limit = (int)(b + 1 == G ? routed : min(to, routed));
+    walk.find((int)min(from, routed));
+  }
   const uint32_t tmem = sh.tmem_base;
 
   if (warp == 0) {
-    // =========================================================== producer
-    if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(map_codes) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(map_scales) : "memory");
-      long long seq = 0;
-      for (int index = item_lo; index < item_hi && !sh.failed; ++index) {
-        const GtItem it = gt_item(sh, a.groups, tiles, index);
-        const int z = a.experts[it.group] - a.start;
-        for (int c = 0; c < chunks; ++c, ++seq) {
-          const int u = (int)(seq % kGtUnits);
-          if (seq >= kGtUnits && !gt_wait(&sh.empty[u], (uint32_t)((seq / kGtUnits) - 1) & 1u, &sh)) break;
-          unsigned char* dst = units + (size_t)u * kTcUnitBytes;
-          mbar_expect_tx(&sh.full[u], kTcUnitBytes);
-          tc_tma_3d(dst, map_codes, c * 128, it.tile * kTcRows, z, &sh.full[u]);
-          tc_tma_3d(dst + kTcCodeBytes, map_scales, c * 16, it.tile * kTcRows, z, &sh.full[u]);
-        }
+    // =========================================================== producer: every lane issues one of the stage's copies
+    const int k_routed = FP4 ? kTcChunkK : 64;
+    auto rows_bytes = [&](const GgItem& it) -> uint32_t {   // one chunk of the tile's N operand
+      return (FP4 && !it.shared) ? (uint32_t)((it.n + 1) / 2 * 2) * 512u : (uint32_t)((it.n + 7) / 8 * 8) * 128u;
+    };
+    auto chunks_of = [&](const GgItem& it) -> int { return a.k / (it.shared ? 64 : k_routed); };
+    auto units_of = [&](const GgItem& it, int s) -> int { return TALL ? 2 : min(2, chunks_of(it) - 2 * s); };
+    auto expect = [&](const GgItem& it, int s, int u) {
+      if (lane == 0) {
+        const int units = units_of(it, s), b_chunks = TALL ? 1 : units;
+        uint32_t bytes = (uint32_t)units * ((FP4 && !it.shared) ? kTcUnitBytes : kTcCodeBytes) + (uint32_t)b_chunks * rows_bytes(it);
+        if (FP4 && !it.shared) bytes += (uint32_t)b_chunks * (uint32_t)((it.n + 1) / 2 * 2) * 64u;
+        mbar_expect_tx(&sh.full[u], bytes);
+      }
+      __syncwarp();
+    };
+    auto issue_weights = [&](const GgItem& it, int s, int u) {
+      unsigned char* dst = ring + (size_t)u * kGgStageBytes;
+      const int units = units_of(it, s);
+      if (PROJ == 0 && it.shared) {
+        // 16 gate rows, 16 up rows, ... : lane = (unit, box)
+        constexpr int kBoxes = kTcRows / kGgSharedBox;
+        const int unit = lane / kBoxes, box = lane % kBoxes;
+        if (unit < units)
+          tc_tma_3d(dst + unit * kGgUnitBytes + box * (kGgSharedBox * 128), a.shared_maps + (box & 1) * 128, (TALL ? s : 2 * s + unit) * 64,
+                    it.m0 / 2 + (TALL ? unit * (kTcRows / 2) : 0) + (box >> 1) * kGgSharedBox, it.group, &sh.full[u]);
+        return;
+      }
+      const int unit = lane & 1, chunk = TALL ? s : 2 * s + unit, row = it.m0 + (TALL ? unit * kTcRows : 0);
+      if (unit >= units) return;
+      const int z = it.shared ? it.group : a.experts[it.group] - a.start;
+      const unsigned char* map = it.shared ? a.shared_maps : a.maps;
+      if (FP4 && !it.shared) {
+        if (lane < 2) tc_tma_3d(dst + unit * kGgUnitBytes, map, chunk * 128, row, z, &sh.full[u]);
+        else if (lane < 4) tc_tma_3d(dst + unit * kGgUnitBytes + kTcCodeBytes, map + 128, chunk * 16, row, z, &sh.full[u]);
+      } else if (lane < 2) {
+        tc_tma_3d(dst + unit * kGgUnitBytes, map, chunk * 64, row, z, &sh.full[u]);
+      }
+    };
+    auto issue_rows = [&](const GgItem& it, int s, int u) {
+      unsigned char* dst = ring + (size_t)u * kGgStageBytes + 2 * kGgUnitBytes;
+      const int c = lane & 1, chunk = TALL ? s : 2 * s + c;
+      if (c >= (TALL ? 1 : units_of(it, s))) return;
+      const uint32_t bytes = rows_bytes(it);
+      if (it.shared) {
+        const int padded = (a.tokens + 7) / 8 * 8, chunks = a.k / 64;
+        const unsigned char* from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2;
+        if (lane < 2) bulk_g2s(dst + c * 8192, from + (size_t)chunk * bytes, bytes, &sh.full[u]);
+        (void)chunks;
+      } else if (FP4) {
+        if (lane < 2) bulk_g2s(dst + c * 8192, a.image + (size_t)it.slot * a.k * 2 + (size_t)chunk * bytes, bytes, &sh.full[u]);
+        else if (lane < 4) bulk_g2s(dst + 16384 + c * 1024, a.image_scales + (size_t)it.slot * (a.k / 4) + (size_t)chunk * (bytes / 8), bytes / 8, &sh.full[u]);
+      } else {
+        if (lane < 2) bulk_g2s(dst + c * 8192, a.image + (size_t)it.slot * a.k * 2 + (size_t)chunk * bytes, bytes, &sh.full[u]);
+      }
+    };
+    auto stages = [&](const GgItem& it) -> int { return walk.stages_of(it.shared); };
+    // The first stages' weights are asked for before the kernel in front has finished; their N operand after.
+    Walk ahead = walk;
+    GgItem it;
+    bool have = ahead.next(it);
+    int s = 0, early = 0;
+    for (; early < kGgStages && have; ++early) {
+      expect(it, s, early);
+      issue_weights(it, s, early);
+      if (++s == stages(it)) {
+        s = 0;
+        have = ahead.next(it);
+      }
+    }
+    pdl_wait();
+    GgItem late;
+    int ls = 0;
+    bool more = walk.next(late);
+    for (int i = 0; i < early && more; ++i) {
+      issue_rows(late, ls, i);
+      if (++ls == stages(late)) {
+        ls = 0;
+        more = walk.next(late);
+      }
+    }
+    for (long long seq = early; have; ++seq) {
+      const int u = (int)(seq % kGgStages);
+      if (!__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / kGgStages) - 1) & 1u, &sh))) break;
+      expect(it, s, u);
+      issue_weights(it, s, u);
+      issue_rows(it, s, u);
+      if (++s == stages(it)) {
+        s = 0;
+        have = ahead.next(it);
       }
     }
   } else if (warp == 1) {
     // =========================================================== MMA issue
     if (lane == 0) {
+      GgItem it;
       long long seq = 0;
-      int item_count = 0;
-      long long t_wait_staged = 0, t_loop = 0;
-      const uint32_t idesc = tc_idesc(kGtN);
-      int stagings = 0;
-      for (int index = item_lo; index < item_hi && !sh.failed; ++index, ++item_count) {
-        const long long t_a = clock64();
-        const GtItem it = gt_item(sh, a.groups, tiles, index);
-        if (index == item_lo || it.tile == 0) {   // a new batch: its digit rows and their scales must be in place
-          const long long t0 = clock64();
-          while (sh.staged <= stagings && !sh.failed)
-            if (clock64() - t0 > kWaitLimitCycles) sh.failed = 1;
-          __threadfence_block();
-          ++stagings;
-        }
-        const long long t_b = clock64();
-        t_wait_staged += t_b - t_a;
-        const int dbuf = item_count & 1;
-        if (!gt_wait(&sh.d_empty[dbuf], (uint32_t)((item_count >> 1) & 1) ^ 1u, &sh)) break;   // this accumulator's previous tile has been read
+      for (int item = 0; walk.next(it) && !sh.failed; ++item) {
+        const bool fp4 = FP4 && !it.shared;
+        const int buf = kAccs == 2 ? item & 1 : 0;
+        const int columns = fp4 ? (it.n + 1) / 2 * 8 : (it.n + 15) / 16 * 16;
+        const uint32_t idesc = fp4 ? tc_idesc(columns) : gg_idesc_bf16(columns);
+        const int chunks = a.k / (fp4 ? kTcChunkK : 64), stages = walk.stages_of(it.shared);
+        if (!gg_wait(&sh.d_empty[buf], (uint32_t)((item / kAccs) & 1) ^ 1u, &sh)) break;   // this accumulator's previous item has been read
         tc_fence_after();
-        for (int c = 0; c < chunks; ++c, ++seq) {
-          const int u = (int)(seq % kGtUnits), sfs = (int)(seq % kTcSfSlots);
-          if (!gt_wait(&sh.full[u], (uint32_t)(seq / kGtUnits) & 1u, &sh)) break;
-          if (!gt_wait(&sh.sf_full[sfs], (uint32_t)(seq / kTcSfSlots) & 1u, &sh)) break;
+        for (int s = 0; s < stages; ++s, ++seq) {
+          const int u = (int)(seq % kGgStages);
+          const uint32_t parity = (uint32_t)(seq / kGgStages) & 1u;
+          if (!gg_wait(&sh.full[u], parity, &sh)) break;
+          if (FP4 && !gg_wait(&sh.sf_full[u], parity, &sh)) break;
           tc_fence_after();
-          const uint64_t ad = tc_desc_sw128(smem_u32(units + (size_t)u * kTcUnitBytes));
-          const uint64_t bd = tc_desc_sw128(smem_u32(s_b + (size_t)c * kGtN * 128));
+          const uint32_t base = smem_u32(ring + (size_t)u * kGgStageBytes), sf = tmem + kGgColSf + u * kGgSfPerStage;
+          const int units = TALL ? 2 : min(2, chunks - 2 * s);
+          for (int unit = 0; unit < units; ++unit) {
+            const uint64_t ad = tc_desc_sw128(base + unit * kGgUnitBytes);
+            const uint64_t bd = tc_desc_sw128(base + 2 * kGgUnitBytes + (TALL ? 0 : unit * 8192));
+            const uint32_t d = tmem + kGgColD + buf * kAccCols + (TALL ? unit * 128 : 0);
+            const bool fresh = s == 0 && (TALL || unit == 0);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc_mma(tmem + kTcColD + dbuf * kGtN, ad + 2 * k, bd + 2 * k, idesc, (c == 0 && k == 0) ? 0u : 1u,
-                   tmem + kTcColSfa + sfs * 16 + k * 4, tmem + kTcColSfb + (c * 4 + k) * 4);
+            for (int k = 0; k < 4; ++k) {
+              const uint32_t accumulate = (fresh && k == 0) ? 0u : 1u;
+              if (fp4) tc_mma(d, ad + 2 * k, bd + 2 * k, idesc, accumulate, sf + unit * 16 + k * 4, sf + 32 + (TALL ? 0 : unit * 16) + k * 4);
+              else gg_mma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
+            }
+          }
           tc_commit(&sh.empty[u]);
-          tc_commit(&sh.sf_empty[sfs]);
-          if (c == chunks - 1) tc_commit(&sh.d_full[dbuf]);
         }
-        t_loop += clock64() - t_b;
+        tc_commit(&sh.d_full[buf]);
       }
-      if (a.prof) {
-        a.prof[blockIdx.x * 8 + 4] = t_wait_staged;
-        a.prof[blockIdx.x * 8 + 5] = t_loop;
+    }
+  } else if (warp < 6) {
+    // =========================================================== block scales: shared -> tensor memory
+    if constexpr (FP4) {
+      const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;   // the tensor-memory subpartition this warp reaches
+      GgItem it;
+      long long seq = 0;
+      bool ok = true;
+      while (ok && walk.next(it)) {
+        const int chunks = a.k / (it.shared ? 64 : kTcChunkK), stages = walk.stages_of(it.shared);
+        for (int s = 0; s < stages; ++s, ++seq) {
+          const int u = (int)(seq % kGgStages);
+          ok = __all_sync(0xffffffffu, gg_wait(&sh.full[u], (uint32_t)(seq / kGgStages) & 1u, &sh));
+          if (!ok) break;
+          if (!it.shared) {
+            const unsigned char* stage = ring + (size_t)u * kGgStageBytes;
+            const int units = TALL ? 2 : min(2, chunks - 2 * s);
+            // a unit's scales lie as 128 rows of 16 bytes; row r belongs to lane r % 32, column r / 32, four bytes a 64-column step
+            auto upload = [&](const unsigned char* sc, int column) {
+              const uint4 r0 = *reinterpret_cast<const uint4*>(sc + lane * 16), r1 = *reinterpret_cast<const uint4*>(sc + (lane + 32) * 16);
+              uint4 r2 = make_uint4(0, 0, 0, 0), r3 = r2;
+              if (TALL || column < 32) {
+                r2 = *reinterpret_cast<const uint4*>(sc + (lane + 64) * 16);
+                r3 = *reinterpret_cast<const uint4*>(sc + (lane + 96) * 16);
+              }
+              const uint32_t w[16] = {r0.x, r1.x, r2.x, r3.x, r0.y, r1.y, r2.y, r3.y, r0.z, r1.z, r2.z, r3.z, r0.w, r1.w, r2.w, r3.w};
+              tc_st16(tmem + lane_base + kGgColSf + u * kGgSfPerStage + column, w);
+            };
+            tc_fence_after();
+            for (int unit = 0; unit < units; ++unit) upload(stage + unit * kGgUnitBytes + kTcCodeBytes, unit * 16);
+            for (int c = 0; c < (TALL ? 1 : units); ++c) upload(stage + 2 * kGgUnitBytes + 16384 + c * 1024, 32 + c * 16);
+            tc_wait_st();
+            tc_fence_before();
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.sf_full[u]);
+        }
       }
     }
   } else {
-    // =========================================================== workers: warps 2..5 scales, 6..9 accumulators
-    const int wt = threadIdx.x - 64;
-    const bool scale_warp = warp < 6;
-    const int sub = warp & 3;                                   // the tensor-memory subpartition this warp reaches
+    // =========================================================== accumulators -> outputs
+    pdl_wait();   // (the tokens' scales come from the kernel in front)
+    const int sub = warp & 3;
     const uint32_t lane_base = (uint32_t)(sub * 32) << 16;
-    long long seq = 0;
-    int item_count = 0;
-    long long t_stage = 0, t_upload = 0, t_main = 0;
-    const long long t_begin = clock64();
-    int stagings = 0;
-    long long t_1 = 0, t_2 = 0;
-    for (int index = item_lo; index < item_hi; ++index, ++item_count) {
-      const long long t_0 = clock64();
-      const GtItem it = gt_item(sh, a.groups, tiles, index);
-      const bool fresh = index == item_lo || it.tile == 0;                        // a new batch: stage its activations
-      const bool last_of_batch = index + 1 == item_hi || it.tile + 1 == tiles;   // the next item (if any) stages again
-      t_1 = t_2 = t_0;
-      if (fresh) {
-      const int expert = a.experts[it.group];
-      const int count = a.counts[it.group];
-      // ---- the batch's routes
-      if (wt < kGtBatch) {
-        const int at = it.batch * kGtBatch + wt;
-        int route = -1;
-        float out_scale = 0.f;
-        if (at < count) {
-          route = a.rows[(size_t)it.group * a.capacity + at];
-          const int in_row = PROJ == 0 ? route / a.top_k : route;
-          const float scale2 = *reinterpret_cast<const float*>(a.pointers[(size_t)expert * kBank + bank + 2]);
-          out_scale = scale2 * a.row_scale[in_row].y * (1.f / 512.f);
-        }
-        sh.route[wt] = route;
-        sh.out_scale[wt] = out_scale;
-      }
-      gt_worker_sync();
-      // ---- the digit rows of the batch's tokens into place: 16-byte pieces, consecutive pieces to consecutive threads,
-      // eight loads in flight per thread
-      {
-        const int pieces_per_route = chunks * 32;   // 512 bytes per chunk
-        const int n_pieces = kGtBatch * pieces_per_route;
+    GgItem it;
+    for (int item = 0; walk.next(it); ++item) {
+      const bool fp4 = FP4 && !it.shared;
+      const int buf = kAccs == 2 ? item & 1 : 0;
+      const int expert = it.shared ? 0 : a.experts[it.group];
+      const float scale2 = fp4 ? *reinterpret_cast<const float*>(a.pointers[(size_t)expert * a.stride + a.bank + 2]) : 1.f;
+      const int per_chunk = fp4 ? 8 : 32, token_chunks = (it.n + per_chunk - 1) / per_chunk;
+      // lane i holds token i of a chunk: its route (or token number), and its scale
+      auto token_of = [&](int chunk, float& scale) -> int {
+        const int i = chunk * per_chunk + lane;
+        scale = 0.f;
+        if (lane >= per_chunk || i >= it.n) return -1;
+        if (it.shared) return it.tile * Walk::kSharedTile + i;
+        if (fp4) scale = scale2 * a.slot_scale[it.slot + i];
+        return a.rows[(size_t)it.group * a.capacity + it.tile * Walk::kTile + i];
+      };
+      float my_scale;
+      int my_token = token_of(0, my_scale);
+      const bool ok = __all_sync(0xffffffffu, gg_wait(&sh.d_full[buf], (uint32_t)((item / kAccs) & 1), &sh));
+      if (!ok) break;
+      tc_fence_after();
 #pragma unroll 1
-        for (int p0 = wt; p0 < n_pieces; p0 += 8 * kGtWorkers) {
-          uint4 v[8];
+      for (int half = 0; half < (TALL ? 2 : 1); ++half) {
+        const int r = it.m0 + half * kTcRows + sub * 32 + lane;   // this thread's weight row
+#pragma unroll 1
+        for (int chunk = 0; chunk < token_chunks; ++chunk) {
+          if (token_chunks > 1) my_token = token_of(chunk, my_scale);
+          float v[32];
+          tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, v);
+          if (fp4) {
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int p = p0 + q * kGtWorkers;
-            v[q] = make_uint4(0, 0, 0, 0);
-            if (p < n_pieces) {
-              const int j = p / pieces_per_route, rem = p % pieces_per_route, c = rem >> 5, piece = rem & 31;
-              const int route = sh.route[j];
-              if (route >= 0) {
-                const int in_row = PROJ == 0 ? route / a.top_k : route;
-                v[q] = __ldg(reinterpret_cast<const uint4*>(a.digits + (((size_t)in_row * chunks + c) * 2 + (j & 1)) * 512) + piece);
+            for (int j = 0; j < 8; ++j) v[j] = ((v[4 * j] + v[4 * j + 1]) + (v[4 * j + 2] + v[4 * j + 3])) * __shfl_sync(0xffffffffu, my_scale, j);
+          }
+          const int here = min(per_chunk, it.n - chunk * per_chunk);
+          if (PROJ == 0) {
+            // gate and up rows sit in lanes that differ in one bit (routed banks interleave single rows, the shared experts'
+            // boxes sixteen): of two tokens each of the two lanes finishes one
+            const int bit = it.shared ? kGgSharedBox : 1;
+            const bool second = (lane & bit) != 0;
+            const int pair = it.shared ? it.m0 / 2 + half * (kTcRows / 2) + sub * kGgSharedBox + (lane & (kGgSharedBox - 1)) : r >> 1;
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              if (j >= here) break;
+              const float other = __shfl_xor_sync(0xffffffffu, second ? v[j] : v[j + 1], bit);
+              const float gate = second ? other : v[j], up = second ? v[j + 1] : other;
+              const int token = __shfl_sync(0xffffffffu, my_token, second ? j + 1 : j);
+              if (token >= 0 && 2 * pair < a.n) {
+                if (!it.shared) {
+                  a.y[(size_t)token * (a.n / 2) + pair] = (uint16_t)f32_to_bf16_bits(silu_mul(gate, up));
+                } else {
+                  // the reference's BF16 tensor ops: both bmm outputs, silu, the product and the product with gamma round
+                  const float g = round_bf16(gate), u = round_bf16(up);
+                  const float act = round_bf16(round_bf16(g / (1.f + expf(-g))) * u);
+                  const float gamma = bf16_to_f32(a.gammas[(size_t)token * a.n_shared + it.group]);
+                  const int padded = (a.tokens + 7) / 8 * 8, f = a.n / 2, row = token - it.tile * Walk::kSharedTile;
+                  unsigned char* at = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
+                                      (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + row * 128 + ((((pair & 63) >> 3) ^ (row & 7)) << 4) + (pair & 7) * 2;
+                  *reinterpret_cast<uint16_t*>(at) = (uint16_t)f32_to_bf16_bits(act * gamma);
+                }
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              if (j >= here) break;
+              const int token = __shfl_sync(0xffffffffu, my_token, j);
+              if (r < a.n) {
+                uint16_t* y = it.shared ? a.shared_y + ((size_t)token * a.n_shared + it.group) * a.n : a.y + (size_t)token * a.n;
+                y[r] = (uint16_t)f32_to_bf16_bits(v[j]);
               }
             }
           }
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int p = p0 + q * kGtWorkers;
-            if (p < n_pieces) {
-              const int j = p / pieces_per_route, rem = p % pieces_per_route, c = rem >> 5, piece = rem & 31;
-              *reinterpret_cast<uint4*>(s_b + (size_t)c * kGtN * 128 + (size_t)j * 512 + piece * 16) = v[q];
-            }
-          }
-        }
-        constexpr int kScalePieces = kTcDigits * (kGtMaxK / 16) / 16;   // 16-byte pieces of a token's scale rows: 64
-        for (int p = wt; p < kGtBatch * kScalePieces; p += kGtWorkers) {
-          const int j = p / kScalePieces, piece = p % kScalePieces;
-          const int route = sh.route[j];
-          uint4 v = make_uint4(0, 0, 0, 0);
-          if (route >= 0) {
-            const int in_row = PROJ == 0 ? route / a.top_k : route;
-            v = __ldg(reinterpret_cast<const uint4*>(a.digit_scales + (size_t)in_row * kTcDigits * (kGtMaxK / 16)) + piece);
-          }
-          reinterpret_cast<uint4*>(&sh.sfb[kTcDigits * j][0])[piece] = v;
         }
       }
-      tc_proxy_fence();   // the digit rows are read by the tensor core
-      gt_worker_sync();
-      t_1 = clock64();
-      if (scale_warp) tc_upload_scales(tmem, sub, &sh.sfb[0][0], kGtMaxK / 16, kGtN, K / 64, lane);
-      gt_worker_sync();
-      t_2 = clock64();
-      if (wt == 0) {
-        __threadfence_block();
-        sh.staged = ++stagings;
-      }
-      }   // fresh
-      if (scale_warp) {
-        // ---- weight scales of every unit: shared -> tensor memory (lane = row % 32, column = row / 32)
-        for (int c = 0; c < chunks; ++c, ++seq) {
-          const int u = (int)(seq % kGtUnits), sfs = (int)(seq % kTcSfSlots);
-          bool ok = gt_wait(&sh.full[u], (uint32_t)(seq / kGtUnits) & 1u, &sh);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) continue;
-          const unsigned char* sc = units + (size_t)u * kTcUnitBytes + kTcCodeBytes;
-          const uint4 r0 = *reinterpret_cast<const uint4*>(sc + lane * 16);
-          const uint4 r1 = *reinterpret_cast<const uint4*>(sc + (lane + 32) * 16);
-          const uint4 r2 = *reinterpret_cast<const uint4*>(sc + (lane + 64) * 16);
-          const uint4 r3 = *reinterpret_cast<const uint4*>(sc + (lane + 96) * 16);
-          ok = gt_wait(&sh.sf_empty[sfs], (uint32_t)((seq / kTcSfSlots) & 1) ^ 1u, &sh);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) continue;
-          tc_fence_after();
-          const uint32_t w[16] = {r0.x, r1.x, r2.x, r3.x, r0.y, r1.y, r2.y, r3.y, r0.z, r1.z, r2.z, r3.z, r0.w, r1.w, r2.w, r3.w};
-          tc_st16(tmem + lane_base + kTcColSfa + sfs * 16, w);
-          tc_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.sf_full[sfs]);
-        }
-      } else {
-        // ---- the tile's accumulator: row = tensor-memory lane, four digit columns per route
-        const int dbuf = item_count & 1;
-        bool ok = gt_wait(&sh.d_full[dbuf], (uint32_t)((item_count >> 1) & 1), &sh);
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
-          tc_fence_after();
-          float v[kGtN];
-          tc_ld32(tmem + lane_base + kTcColD + dbuf * kGtN, v);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh.d_empty[dbuf]);
-          const int r = it.tile * kTcRows + sub * 32 + lane;
-#pragma unroll
-          for (int j = 0; j < kGtBatch; ++j) {
-            const int route = sh.route[j];
-            const float mine = ((v[4 * j] + v[4 * j + 1]) + (v[4 * j + 2] + v[4 * j + 3])) * sh.out_scale[j];
-            if (PROJ == 0) {
-              const float up = __shfl_xor_sync(0xffffffffu, mine, 1);   // even rows are gate, odd rows up
-              if (route >= 0 && (lane & 1) == 0)
-                a.Y[(size_t)route * (a.n / 2) + (r >> 1)] = (uint16_t)f32_to_bf16_bits(mine / (1.f + __expf(-mine)) * up);
-            } else {
-              if (route >= 0) a.Y[(size_t)route * a.n + r] = (uint16_t)f32_to_bf16_bits(mine);
-            }
-          }
-        }
-      }
-      // before the next batch is staged every MMA of this one must be done: the accumulator warps have seen the last
-      // tile's accumulator complete, which the tensor core signals only after all earlier MMAs
-      if (last_of_batch) gt_worker_sync();
-      t_stage += t_1 - t_0;
-      t_upload += t_2 - t_1;
-      t_main += clock64() - t_2;
-    }
-    if (a.prof && wt == 0) {
-      a.prof[blockIdx.x * 8 + 0] = t_stage;
-      a.prof[blockIdx.x * 8 + 1] = t_upload;
-      a.prof[blockIdx.x * 8 + 2] = t_main;
-      a.prof[blockIdx.x * 8 + 3] = clock64() - t_begin;
-      a.prof[blockIdx.x * 8 + 6] = item_count;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
     }
   }
+  __syncwarp();
+  pdl_wait();   // whoever waits for this kernel may rely on the ones before it too
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tc_dealloc(tmem, 512);
   if (threadIdx.x == 0 && sh.failed && a.status) atomicOr(a.status, kFlagWaitTimedOut);
 }
 
-// One block per row of X: its power-of-two normaliser, its four E2M1 digit rows as 512-byte pieces of the swizzled
-// operand (per 256-column chunk, once for an even and once for an odd slot of a batch), and their block scales.
-__global__ void __launch_bounds__(256) digit_rows_kernel(const uint16_t* __restrict__ X, int k, float2* row_scale,
-                                                         unsigned char* digits, unsigned char* digit_scales) {
-  extern __shared__ __align__(1024) unsigned char image[];   // [k/256][8 rows][128 B]: rows 0..3 even slot, 4..7 odd slot
-  __shared__ __align__(16) uint8_t sf[8][kGtMaxK / 16];
-  __shared__ uint32_t s_amax[8];
-  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint4* x = reinterpret_cast<const uint4*>(X + (size_t)row * k);
-  uint32_t amax = 0;
-  for (int g = threadIdx.x; g < k / 8; g += 256) {
-    const uint4 v = x[g];
-    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) amax = max(amax, max(w4[j] & 0x7fffu, (w4[j] >> 16) & 0x7fffu));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if (lane == 0) s_amax[warp] = amax;
-  __syncthreads();
-#pragma unroll
-  for (int w = 0; w < 8; ++w) amax = max(amax, s_amax[w]);
-  float inverse;
-  const float scale = pow2_normaliser(amax, &inverse);
-  if (threadIdx.x == 0) row_scale[row] = make_float2(scale, inverse);
-  for (int g = threadIdx.x; g < k / 8; g += 256) {   // (k / 8 is a multiple of 32: whole warps stay in the call)
-    const uint4 v = x[g];
-    tc_stage8(v, 512.f * scale, image, 8, 0, g * 8, &sf[0][0], kGtMaxK / 16);
-    tc_stage8(v, 512.f * scale, image, 8, 4, g * 8, &sf[0][0], kGtMaxK / 16);
-  }
-  __syncthreads();
-  uint4* out = reinterpret_cast<uint4*>(digits + (size_t)row * k * 4);
-  for (int i = threadIdx.x; i < k * 4 / 16; i += 256) out[i] = reinterpret_cast<const uint4*>(image)[i];
-  uint4* out_sf = reinterpret_cast<uint4*>(digit_scales + (size_t)row * kTcDigits * (kGtMaxK / 16));
-  for (int i = threadIdx.x; i < kTcDigits * (kGtMaxK / 16) / 16; i += 256) out_sf[i] = reinterpret_cast<const uint4*>(&sf[0][0])[i];
+// ---------------------------------------------------------------------------- N operand
+struct StageArgs {
+  const uint16_t* x;            // BF16 [*, k]
+  const int64_t* pointers;
+  const int32_t *experts, *counts, *rows;
+  unsigned char* image;         // routed slots; a tile of n tokens: [chunk][n padded][4 digit rows x 128 B] or [chunk][n padded][128 B]
+  unsigned char* image_scales;  // NVFP4: [chunk][n padded][4 digit rows x 16 B] per tile
+  float* slot_scale;
+  unsigned char* shared_image;  // the tokens themselves for the shared experts, or null
+  int groups, capacity, stride, bank, k, div;   // div: routes per row of x
+  int tokens, tile, shared_tile;
+};
+
+constexpr int kStageThreads = 128;
+
+// 16-byte pieces of a BF16 row into a [k / 64][rows][128 B] swizzled image
+__device__ __forceinline__ void stage_bf16_row(const uint16_t* from, unsigned char* tile, int row, int padded, int k) {
+  for (int p = threadIdx.x; p < k / 8; p += kStageThreads)
+    *reinterpret_cast<uint4*>(tile + (size_t)(p >> 3) * padded * 128 + row * 128 + (((p & 7) ^ (row & 7)) << 4)) = reinterpret_cast<const uint4*>(from)[p];
 }
+
+// Blocks take routed slots in turn, then the tokens for the shared experts. Bound by the digit arithmetic (about a hundred
+// instructions per eight elements) and, for prompts, by the image's bytes; a token is converted once per route, which
+// costs less than gathering it from one copy sixteen times per expert in the main kernel.
+template <bool FP4>
+__global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) {
+  extern __shared__ __align__(16) int s_tables[];
+  __shared__ uint32_t s_amax[kStageThreads / 32];
+  constexpr int kPad = gg_pad(FP4);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  GgTables t{s_tables, s_tables + a.groups + 1};
+  pdl_wait();
+  pdl_trigger();   // the main kernel may read the plan now
+  for (int g = threadIdx.x; g < a.groups; g += kStageThreads) t.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
+  __syncthreads();
+  if (warp == 0) gg_scan(t, a.groups, kPad, lane, [](int count) { return count; });
+  __syncthreads();
+  const int routed = t.cost[a.groups], total = routed + (a.shared_image ? a.tokens : 0);
+  for (int i = blockIdx.x; i < total; i += gridDim.x) {
+    if (i >= routed) {
+      const int token = i - routed, tile = token / a.shared_tile, row = token % a.shared_tile;
+      const int padded = (min(a.shared_tile, a.tokens - tile * a.shared_tile) + 7) / 8 * 8;
+      stage_bf16_row(a.x + (size_t)token * a.k, a.shared_image + (size_t)tile * a.shared_tile * a.k * 2, row, padded, a.k);
+      continue;
+    }
+    int lo = 0, hi = a.groups;   // the group of active route i
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (t.cost[mid] <= i) lo = mid;
+      else hi = mid;
+    }
+    const int pos = i - t.cost[lo], count = t.cost[lo + 1] - t.cost[lo];
+    const int tile = pos / a.tile, row = pos % a.tile, slot0 = gg_first_slot(t.slot0, lo, kPad) + tile * a.tile;
+    const int padded = (min(a.tile, count - tile * a.tile) + kPad - 1) / kPad * kPad;
+    const uint16_t* from = a.x + (size_t)(a.rows[(size_t)lo * a.capacity + pos] / a.div) * a.k;
+    if constexpr (!FP4) {
+      stage_bf16_row(from, a.image + (size_t)slot0 * a.k * 2, row, padded, a.k);
+    } else {
+      const uint4* x = reinterpret_cast<const uint4*>(from);
+      constexpr int kMost = kTcMaxK / 8 / kStageThreads;
+      uint4 v[kMost];
+      uint32_t amax = 0;
+#pragma unroll
+      for (int n = 0; n < kMost; ++n) {
+        const int p = n * kStageThreads + threadIdx.x;
+        v[n] = p < a.k / 8 ? x[p] : make_uint4(0, 0, 0, 0);
+        const uint32_t w4[4] = {v[n].x, v[n].y, v[n].z, v[n].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) amax = max(amax, max(w4[j] & 0x7fffu, (w4[j] >> 16) & 0x7fffu));
+      }
+      amax = __reduce_max_sync(0xffffffffu, amax);
+      __syncthreads();   // (the previous slot's maxima have been read)
+      if (lane == 0) s_amax[warp] = amax;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kStageThreads / 32; ++w) amax = max(amax, s_amax[w]);
+      float inverse;
+      const float scale = pow2_normaliser(amax, &inverse);
+      if (threadIdx.x == 0) a.slot_scale[slot0 + row] = inverse * (1.f / 512.f);
+      unsigned char* image = a.image + (size_t)slot0 * a.k * 2 + (size_t)row * 512;
+      unsigned char* scales = a.image_scales + (size_t)slot0 * (a.k / 4) + (size_t)row * 64;
+#pragma unroll
+      for (int n = 0; n < kMost; ++n) {
+        const int p = n * kStageThreads + threadIdx.x, chunk = p >> 5;   // a warp holds a chunk of 256 elements
+        if (chunk * kTcChunkK < a.k)
+          tc_stage8_row(v[n], 512.f * scale, image + (size_t)chunk * padded * 512, 4 * (row & 1), scales + (size_t)chunk * padded * 64, lane);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------- combine
+// out[token] = sum over choices of fp32(bf16(y[route] * w)) in choice order, then the shared experts: eight columns a thread
+__global__ void __launch_bounds__(256) combine_kernel(const uint16_t* __restrict__ y, const int64_t* __restrict__ indices,
+                                                      const uint16_t* __restrict__ weights, const int64_t* __restrict__ pointers, int stride, int max_expert,
+                                                      const uint16_t* __restrict__ shared_y, int n_shared, float* out, uint16_t* out_bf16,
+                                                      int width, int top_k, int32_t* status) {
+  pdl_wait();
+  pdl_trigger();
+  const int token = blockIdx.x, piece = blockIdx.y * 256 + threadIdx.x;
+  if (piece * 8 >= width) return;
+  float sum[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) sum[i] = 0.f;
+  for (int j = 0; j < top_k; ++j) {
+    const size_t route = (size_t)token * top_k + j;
+    const int64_t expert = indices[route];
+    if (expert < 0 || expert > max_expert) {
+      if (piece == 0 && status) atomicOr(status, kFlagExpertOutOfRange);
+      continue;
+    }
+    if (pointers[expert * stride] == 0) continue;
+    const float w = bf16_to_f32(weights[route]);
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(y + route * width) + piece);
+    const uint32_t q4[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sum[2 * i] += round_bf16(bf16lo(q4[i]) * w);
+      sum[2 * i + 1] += round_bf16(bf16hi(q4[i]) * w);
+    }
+  }
+  for (int e = 0; e < n_shared; ++e) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(shared_y + ((size_t)token * n_shared + e) * width) + piece);
+    const uint32_t q4[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      sum[2 * i] += bf16lo(q4[i]);
+      sum[2 * i + 1] += bf16hi(q4[i]);
+    }
+  }
+  if (out) {
+    float4* to = reinterpret_cast<float4*>(out + (size_t)token * width) + 2 * piece;
+    to[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+    to[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
+  }
+  if (out_bf16) {
+    uint4 p;
+    p.x = f32_to_bf16_bits(sum[0]) | (f32_to_bf16_bits(sum[1]) << 16);
+    p.y = f32_to_bf16_bits(sum[2]) | (f32_to_bf16_bits(sum[3]) << 16);
+    p.z = f32_to_bf16_bits(sum[4]) | (f32_to_bf16_bits(sum[5]) << 16);
+    p.w = f32_to_bf16_bits(sum[6]) | (f32_to_bf16_bits(sum[7]) << 16);
+    reinterpret_cast<uint4*>(out_bf16 + (size_t)token * width)[piece] = p;
+  }
+}
+
+// ---------------------------------------------------------------------------- host side
+static size_t gg_pad256(size_t n) { return (n + 255) / 256 * 256; }
+
+// what one projection's N operand takes: images of the routed slots, of the tokens for the shared experts
+struct GgScratch {
+  size_t slots, image, image_scales, slot_scale, total;
+  GgScratch(bool fp4, size_t routes, size_t groups, int k) {
+    const size_t active = routes < groups ? routes : groups;
+    slots = routes + active * (gg_pad(fp4) - 1);
+    image = gg_pad256(slots * (size_t)k * 2);
+    image_scales = fp4 ? gg_pad256(slots * (size_t)k / 4) : 0;
+    slot_scale = fp4 ? gg_pad256(slots * sizeof(float)) : 0;
+    total = image + image_scales + slot_scale;
+  }
+};
+
+static int gg_sms() {
+  constexpr int kMaxDevices = 64;
+  static int sms_of[kMaxDevices] = {};
+  int device = 0;
+  cudaGetDevice(&device);
+  if (device < 0 || device >= kMaxDevices) return 148;
+  if (sms_of[device] == 0) {
+    int count = 0;
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+    sms_of[device] = count < 1 ? 148 : count;
+  }
+  return sms_of[device];
+}
+
+// launched while the kernel in front runs (both sides use griddepcontrol)
+template <typename Args>
+static cudaError_t launch_dependent(void (*kernel)(Args), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args& args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, args);
+}
+
+template <bool FP4, int PROJ, bool TALL>
+static int launch_grouped(const GgArgs& a, cudaStream_t stream) {
+  constexpr size_t kRing = (size_t)kGgStages * kGgStageBytes + 1024;
+  constexpr int kMaxDevices = 64;
+  static bool configured[kMaxDevices] = {};
+  int device = 0;
+  cudaGetDevice(&device);
+  INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "grouped projections: device ordinal %d", device);
+  if (!configured[device]) {
+    const size_t most = kRing + 2 * sizeof(int) * (kGgMaxGroups + 1);
+    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<FP4, PROJ, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "grouped projections: %zu bytes of shared memory refused: %s", most, cudaGetErrorString(e));
+    configured[device] = true;
+  }
+  const cudaError_t e = launch_dependent(grouped_gemm_kernel<FP4, PROJ, TALL>, dim3(gg_sms()), kGgThreads,
+                                         kRing + 2 * sizeof(int) * (a.groups + 1), stream, a);
+  INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "grouped projections: launch failed: %s", cudaGetErrorString(e));
+  return kOk;
+}
+template <bool FP4, int PROJ>
+static int launch_grouped(bool tall, const GgArgs& a, cudaStream_t s) {
+  return tall ? launch_grouped<FP4, PROJ, true>(a, s) : launch_grouped<FP4, PROJ, false>(a, s);
+}
+
+static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStream_t stream) {
+  const size_t smem = 2 * sizeof(int) * (a.groups + 1), most = (size_t)gg_sms() * 8;
+  const dim3 grid((unsigned)(most_rows < most ? most_rows : most));
+  const cudaError_t e = fp4 ? launch_dependent(stage_rows_kernel<true>, grid, kStageThreads, smem, stream, a)
+                            : launch_dependent(stage_rows_kernel<false>, grid, kStageThreads, smem, stream, a);
+  INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "grouped projections: launch failed: %s", cudaGetErrorString(e));
+  return kOk;
+}
+
+// Tall tiles pay where an expert has more than a few tokens: below, every weight tile meets one tile of tokens anyway and
+// the smaller items even out better (measured: see the table of the design notes).
+static bool gg_tall(long long routes, int experts) { return routes > 8LL * experts; }
 
 }  // namespace ink
 
 using namespace ink;
 
-static size_t gt_pad256(size_t n) { return (n + 255) / 256 * 256; }
-// row scales, digit-row pieces (4 k bytes per row) and their block scales (4 x 256 bytes per row)
+extern "C" int ink_encode_bf16_banks(void* out_host_256, const void* gate_up, uint64_t gate_up_stride, const void* down, uint64_t down_stride,
+                                     int experts, int hidden, int intermediate) {
+  INK_REQUIRE(out_host_256 != nullptr && experts >= 1, kBadArgument, "encode_bf16_banks: null output or no experts");
+  INK_REQUIRE(hidden % 64 == 0 && intermediate % 64 == 0, kUnsupportedShape, "encode_bf16_banks: hidden=%d intermediate=%d", hidden, intermediate);
+  CUtensorMap maps[2];
+  int rc = encode_rows(&maps[0], gate_up, 2, gate_up_stride, experts, 2 * intermediate, hidden, 64, kTcRows, true);
+  if (rc == kOk) rc = encode_rows(&maps[1], down, 2, down_stride, experts, hidden, intermediate, 64, kTcRows, true);
+  if (rc == kOk) memcpy(out_host_256, maps, sizeof(maps));
+  return rc;
+}
+
+extern "C" int ink_encode_shared(void* out_host_384, const void* gate, const void* up, const void* down, int n_shared, int hidden, int intermediate) {
+  INK_REQUIRE(out_host_384 != nullptr && n_shared >= 1, kBadArgument, "encode_shared: null output or no experts");
+  INK_REQUIRE(hidden % 64 == 0 && intermediate % 64 == 0, kUnsupportedShape, "encode_shared: hidden=%d intermediate=%d", hidden, intermediate);
+  CUtensorMap maps[3];
+  const uint64_t stride = 2ull * hidden * intermediate;
+  int rc = encode_rows(&maps[0], gate, 2, stride, n_shared, intermediate, hidden, 64, kGgSharedBox, true);
+  if (rc == kOk) rc = encode_rows(&maps[1], up, 2, stride, n_shared, intermediate, hidden, 64, kGgSharedBox, true);
+  if (rc == kOk) rc = encode_rows(&maps[2], down, 2, stride, n_shared, hidden, intermediate, 64, kTcRows, true);
+  if (rc == kOk) memcpy(out_host_384, maps, sizeof(maps));
+  return rc;
+}
+
+static int check_grouped_shape(bool fp4, int n, int k, int groups) {
+  const int step = fp4 ? kTcChunkK : 64;
+  INK_REQUIRE(k % step == 0 && k >= step && k <= kTcMaxK && n % kTcRows == 0 && n > 0, kUnsupportedShape,
+              "grouped projections: n=%d k=%d unsupported (n a multiple of %d, k a multiple of %d up to %d)", n, k, kTcRows, step, kTcMaxK);
+  INK_REQUIRE(groups >= 0 && groups <= kGgMaxGroups, kBadArgument, "grouped projections: %d groups, at most %d", groups, kGgMaxGroups);
+  return kOk;
+}
+
+extern "C" size_t ink_moe_grouped_scratch_bytes(int tokens, int top_k, int n_shared, int hidden, int intermediate, int groups, int quantized) {
+  const size_t routes = (size_t)(tokens > 0 ? tokens : 0) * top_k, padded = ((size_t)(tokens > 0 ? tokens : 0) + 7) / 8 * 8;
+  const GgScratch a(quantized != 0, routes, groups, hidden), b(quantized != 0, routes, groups, intermediate);
+  return a.total + b.total + gg_pad256(n_shared ? padded * hidden * 2 : 0) + gg_pad256(padded * n_shared * intermediate * 2) +
+         gg_pad256((size_t)(tokens > 0 ? tokens : 0) * n_shared * hidden * 2);
+}
+
+extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void* weights, const int64_t* pointers, const int32_t* experts,
+                               const int32_t* rows, const int32_t* counts, const void* bank_maps, const void* shared_maps, const void* gammas,
+                               void* activated, void* down, float* output, void* output_bf16, int tokens, int top_k, int n_shared, int hidden, int intermediate, int groups,
+                               int start, int local, int capacity, int max_expert, int quantized, void* scratch, size_t scratch_bytes, int32_t* status,
+                               ink_stream_t stream) {
+  INK_REQUIRE(x && indices && weights && pointers && experts && rows && counts && bank_maps && activated && down && scratch && (output || output_bf16), kBadArgument,
+              "moe_grouped: null pointer argument");
+  INK_REQUIRE(n_shared == 0 || (shared_maps && gammas), kBadArgument, "moe_grouped: shared experts need their descriptors and weights");
+  INK_REQUIRE(tokens >= 0 && top_k >= 1 && n_shared >= 0 && capacity >= 1 && start >= 0 && local >= 1, kBadArgument,
+              "moe_grouped: tokens=%d top_k=%d n_shared=%d capacity=%d", tokens, top_k, n_shared, capacity);
+  const bool fp4 = quantized != 0;
+  if (int rc = check_grouped_shape(fp4, 2 * intermediate, hidden, groups)) return rc;
+  if (int rc = check_grouped_shape(fp4, hidden, intermediate, groups)) return rc;
+  INK_REQUIRE(scratch_bytes >= ink_moe_grouped_scratch_bytes(tokens, top_k, n_shared, hidden, intermediate, groups, quantized), kBadArgument,
+              "moe_grouped: scratch of %zu bytes is too small", scratch_bytes);
+  INK_REQUIRE(aligned16(x) && aligned16(activated) && aligned16(down) && aligned16(output) && aligned16(output_bf16) && (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0 &&
+                  (reinterpret_cast<uintptr_t>(bank_maps) & 127u) == 0 && (reinterpret_cast<uintptr_t>(shared_maps) & 127u) == 0,
+              kMisaligned, "moe_grouped: misaligned buffer (scratch 256 bytes, descriptors 128, x and outputs 16)");
+  if (tokens == 0) return kOk;
+  cudaStream_t s = (cudaStream_t)stream;
+  const size_t routes = (size_t)tokens * top_k, padded = ((size_t)tokens + 7) / 8 * 8;
+  const GgScratch in(fp4, routes, groups, hidden), act(fp4, routes, groups, intermediate);
+  unsigned char* p = (unsigned char*)scratch;
+  auto take = [&](size_t n) { unsigned char* q = p; p += gg_pad256(n); return q; };
+  unsigned char *in_image = take(in.image), *in_scales = take(in.image_scales), *in_slot = take(in.slot_scale);
+  unsigned char *act_image = take(act.image), *act_scales = take(act.image_scales), *act_slot = take(act.slot_scale);
+  unsigned char *x_image = take(n_shared ? padded * hidden * 2 : 0), *sact_image = take(padded * n_shared * intermediate * 2);
+  unsigned char* shared_out = take((size_t)tokens * n_shared * hidden * 2);
+  const bool tall = gg_tall((long long)routes, local);
+  const int bank = fp4 ? 3 : 1, stride = fp4 ? kBank : 2;
+
+  StageArgs st = {};
+  st.x = (const uint16_t*)x;
+  st.pointers = pointers;
+  st.experts = experts;
+  st.counts = counts;
+  st.rows = rows;
+  st.image = in_image;
+  st.image_scales = in_scales;
+  st.slot_scale = (float*)in_slot;
+  st.shared_image = n_shared ? x_image : nullptr;
+  st.groups = groups;
+  st.capacity = capacity;
+  st.stride = stride;
+  st.bank = 0;
+  st.k = hidden;
+  st.div = top_k;
+  st.tokens = tokens;
+  st.tile = gg_tile(fp4, tall);
+  st.shared_tile = gg_tile(false, tall);
+  if (int rc = launch_stage(fp4, st, routes + (n_shared ? tokens : 0), s)) return rc;
+
+  GgArgs g = {};
+  g.maps = (const unsigned char*)bank_maps;
+  g.pointers = pointers;
+  g.experts = experts;
+  g.counts = counts;
+  g.rows = rows;
+  g.image = in_image;
+  g.image_scales = in_scales;
+  g.slot_scale = (const float*)in_slot;
+  g.y = (uint16_t*)activated;
+  g.groups = groups;
+  g.start = start;
+  g.capacity = capacity;
+  g.stride = stride;
+  g.bank = 0;
+  g.k = hidden;
+  g.n = 2 * intermediate;
+  g.shared_maps = (const unsigned char*)shared_maps;
+  g.shared_image = x_image;
+  g.shared_y = (uint16_t*)sact_image;
+  g.gammas = (const uint16_t*)gammas;
+  g.n_shared = n_shared;
+  g.tokens = tokens;
+  g.status = status;
+  if (int rc = fp4 ? launch_grouped<true, 0>(tall, g, s) : launch_grouped<false, 0>(tall, g, s)) return rc;
+
+  st.x = (const uint16_t*)activated;
+  st.image = act_image;
+  st.image_scales = act_scales;
+  st.slot_scale = (float*)act_slot;
+  st.shared_image = nullptr;
+  st.bank = bank;
+  st.k = intermediate;
+  st.div = 1;
+  if (int rc = launch_stage(fp4, st, routes, s)) return rc;
+
+  g.maps += fp4 ? 256 : 128;
+  g.image = act_image;
+  g.image_scales = act_scales;
+  g.slot_scale = (const float*)act_slot;
+  g.y = (uint16_t*)down;
+  g.bank = bank;
+  g.k = intermediate;
+  g.n = hidden;
+  g.shared_maps = n_shared ? g.shared_maps + 256 : nullptr;
+  g.shared_image = sact_image;
+  g.shared_y = (uint16_t*)shared_out;
+  if (int rc = fp4 ? launch_grouped<true, 1>(tall, g, s) : launch_grouped<false, 1>(tall, g, s)) return rc;
+
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)tokens, (unsigned)((hidden / 8 + 255) / 256));
+  config.blockDim = dim3(256);
+  config.stream = s;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&config, combine_kernel, (const uint16_t*)down, indices, (const uint16_t*)weights, pointers, stride, max_expert,
+                                           (const uint16_t*)shared_out, n_shared, output, (uint16_t*)output_bf16, hidden, top_k, status);
+  INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "moe_grouped: launch failed: %s", cudaGetErrorString(e));
+  return kOk;
+}
+
+// The two projections on their own, as the reference's expert_gemm calls them.
+static size_t expert_gemm_tc_bytes(size_t routes, size_t groups, int k) { return GgScratch(true, routes, groups, k).total; }
 extern "C" size_t ink_expert_gemm_tc_scratch_bytes(int input_rows, int k) {
-  const size_t rows = input_rows > 0 ? (size_t)input_rows : 0;
-  return gt_pad256(sizeof(float2) * rows) + gt_pad256(rows * (size_t)k * 4) + gt_pad256(rows * kTcDigits * (kGtMaxK / 16)) +
-         8 * 8 * 256;   // (+ the optional per-block phase clocks)
+  const size_t routes = 8 * (size_t)(input_rows > 0 ? input_rows : 0);   // of up to eight choices a row
+  return expert_gemm_tc_bytes(routes, kGgMaxGroups, k);
 }
 
 extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, const int64_t* pointers,
@@ -449,65 +960,54 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   INK_REQUIRE(x && bank_maps && pointers && experts && rows && counts && y && scratch, kBadArgument,
               "expert_gemm_tc: null pointer argument");
   INK_REQUIRE(projection == 0 || projection == 1, kBadArgument, "expert_gemm_tc: projection=%d", projection);
-  INK_REQUIRE(k % kTcChunkK == 0 && k >= kTcChunkK && k <= kGtMaxK && n % kTcRows == 0 && n > 0, kUnsupportedShape,
-              "expert_gemm_tc: n=%d k=%d unsupported (n a multiple of %d, k a multiple of %d up to %d)", n, k, kTcRows,
-              kTcChunkK, kGtMaxK);
-  INK_REQUIRE(groups >= 0 && groups <= kGtMaxGroups && capacity >= 1 && top_k >= 1 && input_rows >= 0 && start >= 0, kBadArgument,
-              "expert_gemm_tc: bad sizes (groups=%d, at most %d)", groups, kGtMaxGroups);
-  INK_REQUIRE(scratch_bytes >= ink_expert_gemm_tc_scratch_bytes(input_rows, k), kBadArgument,
-              "expert_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, ink_expert_gemm_tc_scratch_bytes(input_rows, k));
+  if (int rc = check_grouped_shape(true, n, k, groups)) return rc;
+  INK_REQUIRE(capacity >= 1 && top_k >= 1 && input_rows >= 0 && start >= 0, kBadArgument, "expert_gemm_tc: bad sizes (capacity=%d top_k=%d rows=%d)",
+              capacity, top_k, input_rows);
+  const long long all = projection == 0 ? (long long)input_rows * top_k : input_rows;
+  const size_t routes = (size_t)(all < capacity ? all : capacity);
+  INK_REQUIRE(scratch_bytes >= expert_gemm_tc_bytes(routes, groups, k), kBadArgument,
+              "expert_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, expert_gemm_tc_bytes(routes, groups, k));
   INK_REQUIRE(aligned16(x) && aligned16(y) && aligned16(scratch) && (reinterpret_cast<uintptr_t>(bank_maps) & 127u) == 0,
               kMisaligned, "expert_gemm_tc: misaligned buffer (the descriptors need 128-byte alignment)");
-  if (groups == 0 || input_rows == 0) return kOk;
+  if (groups == 0 || routes == 0) return kOk;
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned char* digits = (unsigned char*)scratch + gt_pad256(sizeof(float2) * (size_t)input_rows);
-  unsigned char* digit_scales = digits + gt_pad256((size_t)input_rows * k * 4);
-  digit_rows_kernel<<<input_rows, 256, (size_t)k * 4, s>>>((const uint16_t*)x, k, (float2*)scratch, digits, digit_scales);
-  INK_CHECK_LAUNCH("expert_gemm_tc (digit rows)");
-  GemmTcArgs a;
-  a.X = (const uint16_t*)x;
-  a.maps = (const unsigned char*)bank_maps;
-  a.pointers = pointers;
-  a.experts = experts;
-  a.rows = rows;
-  a.counts = counts;
-  a.Y = (uint16_t*)y;
-  a.row_scale = (const float2*)scratch;
-  a.digits = digits;
-  a.digit_scales = digit_scales;
-  a.capacity = capacity;
-  a.n = n;
-  a.k = k;
-  a.top_k = top_k;
-  a.groups = groups;
-  a.start = start;
-  a.status = status;
-  a.prof = nullptr;
-  {
-    // INKLING_GROUPED_PROFILE=1: the tail of the scratch (8 x 8 bytes per block after the row scales) gets per-phase clock totals
-    const char* on = getenv("INKLING_GROUPED_PROFILE");
-    if (on && on[0] == '1') a.prof = (long long*)((char*)scratch + ink_expert_gemm_tc_scratch_bytes(input_rows, k) - 8 * 8 * 256);
-  }
-  const size_t smem = (size_t)kGtUnits * kTcUnitBytes + (size_t)k * 16 + 1024;
-  constexpr int kMaxDevices = 64;
-  static int sms_of[2][kMaxDevices] = {};
-  int device = 0;
-  cudaGetDevice(&device);
-  INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "expert_gemm_tc: device ordinal %d", device);
-  if (sms_of[projection][device] == 0) {
-    const size_t most = (size_t)kGtUnits * kTcUnitBytes + (size_t)kGtMaxK * 16 + 1024;
-    cudaError_t e = projection == 0
-                        ? cudaFuncSetAttribute(expert_gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)
-                        : cudaFuncSetAttribute(expert_gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "expert_gemm_tc: %zu bytes of shared memory refused: %s", most, cudaGetErrorString(e));
-    int count = 0;
-    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-    INK_REQUIRE(count >= 1, kLaunchFailed, "expert_gemm_tc: no multiprocessors reported");
-    sms_of[projection][device] = count;
-  }
-  const int blocks = sms_of[projection][device];
-  if (projection == 0) expert_gemm_tc_kernel<0><<<blocks, kGtThreads, smem, s>>>(a);
-  else expert_gemm_tc_kernel<1><<<blocks, kGtThreads, smem, s>>>(a);
-  INK_CHECK_LAUNCH("expert_gemm_tc");
-  return kOk;
+  const GgScratch sizes(true, routes, groups, k);
+  const bool tall = gg_tall((long long)routes, groups);
+  StageArgs st = {};
+  st.x = (const uint16_t*)x;
+  st.pointers = pointers;
+  st.experts = experts;
+  st.counts = counts;
+  st.rows = rows;
+  st.image = (unsigned char*)scratch;
+  st.image_scales = st.image + sizes.image;
+  st.slot_scale = (float*)(st.image_scales + sizes.image_scales);
+  st.groups = groups;
+  st.capacity = capacity;
+  st.stride = kBank;
+  st.bank = projection ? 3 : 0;
+  st.k = k;
+  st.div = projection ? 1 : top_k;
+  st.tile = gg_tile(true, tall);
+  st.shared_tile = gg_tile(false, tall);
+  if (int rc = launch_stage(true, st, routes, s)) return rc;
+  GgArgs g = {};
+  g.maps = (const unsigned char*)bank_maps + (projection ? 256 : 0);
+  g.pointers = pointers;
+  g.experts = experts;
+  g.counts = counts;
+  g.rows = rows;
+  g.image = st.image;
+  g.image_scales = st.image_scales;
+  g.slot_scale = st.slot_scale;
+  g.y = (uint16_t*)y;
+  g.groups = groups;
+  g.start = start;
+  g.capacity = capacity;
+  g.stride = kBank;
+  g.bank = st.bank;
+  g.k = k;
+  g.n = n;
+  g.status = status;
+  return projection == 0 ? launch_grouped<true, 0>(tall, g, s) : launch_grouped<true, 1>(tall, g, s);
 }

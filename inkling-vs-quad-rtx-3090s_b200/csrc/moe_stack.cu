@@ -35,6 +35,7 @@
 #include "pipe.cuh"
 #include "stream_math.cuh"
 #include "tc_path.cuh"
+#include "tensor_map.cuh"
 
 namespace ink {
 
@@ -2267,38 +2268,6 @@ using namespace ink;
 
 extern "C" size_t ink_moe_stack_layer_bytes(void) { return sizeof(StackLayer); }
 
-// ---- TMA descriptors of a layer's banks (driver entry point resolved at first use; no link to libcuda)
-typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                      const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                      CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static TensorMapEncodeFn tensor_map_encoder() {
-  static TensorMapEncodeFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (TensorMapEncodeFn)p;
-  }
-  return fn;
-}
-// bytes [row_bytes] x rows x experts, box of `box_bytes` x 128 rows x 1 expert
-static int encode_bank(CUtensorMap* out, const void* base, uint64_t expert_stride, int experts, int rows, int row_bytes,
-                       int box_bytes, bool swizzle) {
-  TensorMapEncodeFn enc = tensor_map_encoder();
-  INK_REQUIRE(enc != nullptr, kLaunchFailed, "encode_banks: the driver has no cuTensorMapEncodeTiled");
-  INK_REQUIRE(base != nullptr && aligned16(base) && expert_stride % 16 == 0 && expert_stride >= (uint64_t)rows * row_bytes,
-              kBadArgument, "encode_banks: bank at %p with expert stride %llu", base, (unsigned long long)expert_stride);
-  cuuint64_t dims[3] = {(cuuint64_t)row_bytes, (cuuint64_t)rows, (cuuint64_t)experts};
-  cuuint64_t strides[2] = {(cuuint64_t)row_bytes, (cuuint64_t)expert_stride};
-  cuuint32_t box[3] = {(cuuint32_t)box_bytes, (cuuint32_t)kTcRows, 1}, elem[3] = {1, 1, 1};
-  const CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, elem,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  INK_REQUIRE(r == CUDA_SUCCESS, kBadArgument, "encode_banks: cuTensorMapEncodeTiled returned %d", (int)r);
-  return kOk;
-}
-
 extern "C" int ink_moe_stack_encode_banks(void* out_host_512, const void* gate_up_codes, uint64_t gate_up_codes_stride,
                                           const void* gate_up_scales, uint64_t gate_up_scales_stride, const void* down_codes,
                                           uint64_t down_codes_stride, const void* down_scales, uint64_t down_scales_stride,
@@ -2309,10 +2278,10 @@ extern "C" int ink_moe_stack_encode_banks(void* out_host_512, const void* gate_u
               kUnsupportedShape, "encode_banks: hidden=%d intermediate=%d do not tile by 128 rows x 256 columns", hidden,
               intermediate);
   CUtensorMap maps[4];
-  int rc = encode_bank(&maps[0], gate_up_codes, gate_up_codes_stride, experts, 2 * intermediate, hidden / 2, 128, true);
-  if (rc == kOk) rc = encode_bank(&maps[1], gate_up_scales, gate_up_scales_stride, experts, 2 * intermediate, hidden / 16, 16, false);
-  if (rc == kOk) rc = encode_bank(&maps[2], down_codes, down_codes_stride, experts, hidden, intermediate / 2, 128, true);
-  if (rc == kOk) rc = encode_bank(&maps[3], down_scales, down_scales_stride, experts, hidden, intermediate / 16, 16, false);
+  int rc = encode_rows(&maps[0], gate_up_codes, 1, gate_up_codes_stride, experts, 2 * intermediate, hidden / 2, 128, kTcRows, true);
+  if (rc == kOk) rc = encode_rows(&maps[1], gate_up_scales, 1, gate_up_scales_stride, experts, 2 * intermediate, hidden / 16, 16, kTcRows, false);
+  if (rc == kOk) rc = encode_rows(&maps[2], down_codes, 1, down_codes_stride, experts, hidden, intermediate / 2, 128, kTcRows, true);
+  if (rc == kOk) rc = encode_rows(&maps[3], down_scales, 1, down_scales_stride, experts, hidden, intermediate / 16, 16, kTcRows, false);
   if (rc != kOk) return rc;
   static_assert(sizeof(CUtensorMap) == 128, "a TMA descriptor is 128 bytes");
   memcpy(out_host_512, maps, sizeof(maps));

@@ -19,6 +19,7 @@ constexpr int kTcChunkK = 256;               // K elements per unit: one 128-byt
 constexpr int kTcCodeBytes = kTcRows * kTcChunkK / 2;    // 16384
 constexpr int kTcScaleBytes = kTcRows * kTcChunkK / 16;  // 2048
 constexpr int kTcUnitBytes = kTcCodeBytes + kTcScaleBytes;
+constexpr int kTcMaxK = 4096;               // widest contraction
 constexpr int kTcSfSlots = 8;                // units whose weight scales sit in tensor memory
 // tensor memory columns (512 allocated): two accumulators, the weight-scale ring, the activation scales
 constexpr int kTcColD = 0, kTcColSfa = 64, kTcColSfb = 256;
@@ -115,16 +116,11 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float (&v)[32]) {
 
 // 2^p as an E4M3 byte, -9 <= p <= 8 (the three lowest are subnormals)
 __device__ __forceinline__ uint32_t tc_e4m3_pow2(int p) { return p >= -6 ? (uint32_t)(p + 7) << 3 : (uint32_t)(4 >> (-7 - p)); }
-// Eight consecutive elements k0 .. k0+7 (k0 a multiple of 8) of a BF16 vector whose largest
-// magnitude `scale` brings into [512, 1024): their digit codes go to rows row0 .. row0+3 of a
-// [K/256][rows][128 B] swizzled N operand, one 32-bit store per row, and the block's four scale
-// bytes to sf[(row0 + t) * sf_pitch + k0 / 16]. A 16-element block is two such groups held by
-// the lanes 2m and 2m+1 of a warp (the caller deals consecutive groups to consecutive lanes and
-// keeps the whole warp in the call). Per element: q = round(v * 2^(9-e)) lies in [-2048, 2048];
-// adding 4 * (512 + 64 + 8 + 1) turns its balanced base-8 digits (-4..3, the leading one up to 4)
-// into plain ones, which index a table of E2M1 codes.
-__device__ __forceinline__ void tc_stage8(uint4 raw, float scale, unsigned char* operand, int rows, int row0, int k0, uint8_t* sf,
-                                          int sf_pitch) {
+// Digits of eight consecutive elements, one word of eight E2M1 codes per digit row; a lane pair 2m, 2m+1 holds a block of
+// sixteen elements (`scale` brings the vector's largest magnitude into [512, 1024)). Returns the block's exponent e: its
+// scale bytes are 2^(e - 3t). Per element: q = round(v * 2^(9-e)) lies in [-2048, 2048]; adding 4 * (512 + 64 + 8 + 1)
+// turns its balanced base-8 digits (-4..3, the leading one up to 4) into plain ones, which index a table of E2M1 codes.
+__device__ __forceinline__ int tc_digits8(uint4 raw, float scale, uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
   const uint32_t in[4] = {raw.x, raw.y, raw.z, raw.w};
   float v[8];
   float m = 0.f;
@@ -139,7 +135,7 @@ __device__ __forceinline__ void tc_stage8(uint4 raw, float scale, unsigned char*
   e = e < 0 ? 0 : (e > 8 ? 8 : e);
   const float mult = __uint_as_float((uint32_t)(127 + 9 - e) << 23);
   constexpr uint32_t kCodes = 0x5420ACDEu;   // E2M1 codes of -4, -3, -2, -1, 0, 1, 2, 3
-  uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+  w0 = w1 = w2 = w3 = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     int q = __float2int_rn(v[i] * mult);
@@ -151,6 +147,18 @@ __device__ __forceinline__ void tc_stage8(uint4 raw, float scale, unsigned char*
     w2 |= ((kCodes >> (4u * ((u >> 3) & 7u))) & 15u) << (4 * i);
     w3 |= ((kCodes >> (4u * (u & 7u))) & 15u) << (4 * i);
   }
+  return e;
+}
+// Eight consecutive elements k0 .. k0+7 (k0 a multiple of 8) of a BF16 vector whose largest
+// magnitude `scale` brings into [512, 1024): their digit codes go to rows row0 .. row0+3 of a
+// [K/256][rows][128 B] swizzled N operand, one 32-bit store per row, and the block's four scale
+// bytes to sf[(row0 + t) * sf_pitch + k0 / 16]. A 16-element block is two such groups held by
+// the lanes 2m and 2m+1 of a warp (the caller deals consecutive groups to consecutive lanes and
+// keeps the whole warp in the call).
+__device__ __forceinline__ void tc_stage8(uint4 raw, float scale, unsigned char* operand, int rows, int row0, int k0, uint8_t* sf,
+                                          int sf_pitch) {
+  uint32_t w0, w1, w2, w3;
+  const int e = tc_digits8(raw, scale, w0, w1, w2, w3);
   const int chunk = k0 >> 8, in256 = k0 & 255, unit = in256 >> 5, byte = (in256 & 31) >> 1;
   unsigned char* at = operand + (size_t)chunk * rows * 128 + byte;
   *reinterpret_cast<uint32_t*>(at + (row0 + 0) * 128 + ((unit ^ ((row0 + 0) & 7)) << 4)) = w0;
@@ -161,6 +169,26 @@ __device__ __forceinline__ void tc_stage8(uint4 raw, float scale, unsigned char*
 #pragma unroll
     for (int t = 0; t < kTcDigits; ++t) sf[(row0 + t) * sf_pitch + (k0 >> 4)] = (uint8_t)tc_e4m3_pow2(e - 3 * t);
   }
+}
+
+// One warp: the digit rows of 256 consecutive elements (eight per lane) as a 512-byte piece of the swizzled N operand
+// (rows row0 .. row0 + 3 of an eight-row atom) and its 4 x 16 scale bytes, to global memory: a line per digit row, one word
+// of scales per lane of the lower half-warp.
+__device__ __forceinline__ void tc_stage8_row(uint4 raw, float scale, unsigned char* piece, int row0, unsigned char* scales, int lane) {
+  uint32_t w0, w1, w2, w3;
+  const int e = tc_digits8(raw, scale, w0, w1, w2, w3);
+  const int unit = lane >> 2, byte = (lane & 3) * 4;
+  *reinterpret_cast<uint32_t*>(piece + 0 * 128 + ((unit ^ (row0 + 0)) << 4) + byte) = w0;
+  *reinterpret_cast<uint32_t*>(piece + 1 * 128 + ((unit ^ (row0 + 1)) << 4) + byte) = w1;
+  *reinterpret_cast<uint32_t*>(piece + 2 * 128 + ((unit ^ (row0 + 2)) << 4) + byte) = w2;
+  *reinterpret_cast<uint32_t*>(piece + 3 * 128 + ((unit ^ (row0 + 3)) << 4) + byte) = w3;
+  uint32_t word = 0;   // of digit row lane / 4, blocks 4 * (lane % 4) ..
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int of = __shfl_sync(0xffffffffu, e, ((lane & 3) * 4 + i) * 2);
+    word |= tc_e4m3_pow2(of - 3 * ((lane >> 2) & 3)) << (8 * i);
+  }
+  if (lane < 16) reinterpret_cast<uint32_t*>(scales)[lane] = word;
 }
 
 // Block scales of `rows` digit rows (`bytes_per_row` each, row r at table + r * pitch) into the

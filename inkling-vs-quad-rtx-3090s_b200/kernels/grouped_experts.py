@@ -18,35 +18,63 @@ def expert_bank_names(quantized: bool) -> list[str]:
     return [projection + suffix for projection in ("gate_up_proj", "down_proj") for suffix in suffixes]
 
 
-_SCRATCH: dict[tuple, torch.Tensor] = {}
+def _scratch(need: int, device) -> torch.Tensor:
+    """Scratch of one call, from the caching allocator: it belongs to the call's stream (or to the graph being captured),
+    so calls on several streams and threads do not share it and a captured graph keeps its own."""
+    return torch.empty(need, dtype=torch.uint8, device=device)
 
 
-def _scratch(rows: int, device, k: int = 0) -> torch.Tensor:
-    """Per-device buffer for the activations' row normalisers (and, for the block-scaled
-    kernel, their digit rows: pass `k`); grows to the largest request and is then reused, so
-    a captured step never allocates once it has been warmed up at its largest shape."""
-    key = (device.type, device.index)
-    need = _abi.lib().ink_expert_gemm_tc_scratch_bytes(rows, k) if k else _abi.lib().ink_expert_gemm_scratch_bytes(rows)
-    buf = _SCRATCH.get(key)
-    if buf is None or buf.numel() < need:
-        buf = torch.empty(max(need, 1 << 16), dtype=torch.uint8, device=device)
-        _SCRATCH[key] = buf
-    return buf
+def _maps_to_device(size: int, device, encode) -> torch.Tensor:
+    import ctypes
+
+    host = bytearray(size)
+    _abi.check(encode((ctypes.c_char * size).from_buffer(host)))
+    maps = torch.frombuffer(host, dtype=torch.uint8).to(device)
+    assert maps.data_ptr() % 128 == 0
+    return maps
 
 
 def encode_bank_maps(layout, experts: int, hidden: int, intermediate: int, device) -> torch.Tensor:
     """The four TMA descriptors of one layer's evenly spaced NVFP4 banks as a 512-byte device
     tensor (ink_moe_stack_encode_banks). `layout` = ((address of expert 0, byte distance between
     experts) for gate_up_proj, gate_up_proj_scale, down_proj, down_proj_scale)."""
-    import ctypes
-
-    host = bytearray(512)
-    out = (ctypes.c_char * 512).from_buffer(host)
     (gc, gcs), (gs, gss), (dc, dcs), (ds, dss) = layout
-    _abi.check(_abi.lib().ink_moe_stack_encode_banks(out, gc, gcs, gs, gss, dc, dcs, ds, dss, experts, hidden, intermediate))
-    maps = torch.frombuffer(host, dtype=torch.uint8).to(device)
-    assert maps.data_ptr() % 128 == 0
-    return maps
+    return _maps_to_device(512, device, lambda out: _abi.lib().ink_moe_stack_encode_banks(
+        out, gc, gcs, gs, gss, dc, dcs, ds, dss, experts, hidden, intermediate))
+
+
+def encode_bf16_bank_maps(layout, experts: int, hidden: int, intermediate: int, device) -> torch.Tensor:
+    """The same for evenly spaced BF16 banks (ink_encode_bf16_banks): `layout` = ((address of expert 0, byte distance
+    between experts) for gate_up_proj, down_proj)."""
+    (g, gs), (d, ds) = layout
+    return _maps_to_device(256, device, lambda out: _abi.lib().ink_encode_bf16_banks(out, g, gs, d, ds, experts, hidden, intermediate))
+
+
+def encode_shared_maps(gate, up, down) -> torch.Tensor:
+    """The descriptors of a block's shared experts (ink_encode_shared): gate, up BF16 [n, f, d], down BF16 [n, d, f]."""
+    n, f, d = gate.shape
+    assert up.shape == gate.shape and down.shape == (n, d, f) and all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (gate, up, down))
+    return _maps_to_device(384, gate.device, lambda out: _abi.lib().ink_encode_shared(out, gate.data_ptr(), up.data_ptr(), down.data_ptr(), n, d, f))
+
+
+def moe_grouped(x, indices, weights, pointers, experts, rows, counts, bank_maps, activated, down, *, output=None, output_bf16=None,
+                groups: int, start: int, local: int, capacity: int, max_expert: int, quantized: bool, shared_maps=None, gammas=None,
+                n_shared: int = 0, status=None) -> None:
+    """Everything of a layer after the plan, for several tokens (ink_moe_grouped): the routed experts, with `n_shared`
+    the shared ones too, summed per token into `output` (FP32) and / or `output_bf16`, both fully overwritten; `activated`, `down` [routes, f | d] are scratch."""
+    tokens, hidden = x.shape
+    top_k, intermediate = indices.shape[1], activated.shape[1]
+    assert x.dtype == weights.dtype == activated.dtype == down.dtype == torch.bfloat16 and indices.dtype == pointers.dtype == torch.int64
+    assert x.is_contiguous() and indices.is_contiguous() and weights.is_contiguous() and x.is_cuda
+    assert activated.shape[0] >= tokens * top_k and down.shape[0] >= tokens * top_k
+    lib = _abi.lib()
+    need = lib.ink_moe_grouped_scratch_bytes(tokens, top_k, n_shared, hidden, intermediate, groups, int(quantized))
+    scratch = _scratch(need, x.device)
+    _abi.check(lib.ink_moe_grouped(
+        x.data_ptr(), indices.data_ptr(), weights.data_ptr(), pointers.data_ptr(), experts.data_ptr(), rows.data_ptr(), counts.data_ptr(),
+        bank_maps.data_ptr(), _abi.ptr(shared_maps), _abi.ptr(gammas), activated.data_ptr(), down.data_ptr(), _abi.ptr(output), _abi.ptr(output_bf16), tokens, top_k, n_shared,
+        hidden, intermediate, groups, start, local, capacity, max_expert, int(quantized), scratch.data_ptr(), need, _abi.ptr(status),
+        _abi.stream()))
 
 
 def block_scaled_supported(n: int, k: int, groups: int) -> bool:
@@ -68,13 +96,14 @@ def _expert_gemm(X, Pointers, Experts, Rows, Counts, Y, CAPACITY, N, K, TOP_K, P
     _abi.require_cuda(X, Pointers, Experts, Rows, Counts, Y)
     groups = Experts.numel() if groups is None else groups
     if bank_maps is not None and QUANTIZED and block_scaled_supported(N, K, groups):
-        scratch = _scratch(X.shape[0], X.device, K)
+        routes = min(X.shape[0] * (TOP_K if PROJECTION == 0 else 1), CAPACITY)
+        scratch = _scratch(_abi.lib().ink_expert_gemm_tc_scratch_bytes((routes + 7) // 8, K), X.device)
         _abi.check(_abi.lib().ink_expert_gemm_tc(
             X.data_ptr(), X.shape[0], bank_maps.data_ptr(), Pointers.data_ptr(), Experts.data_ptr(), Rows.data_ptr(),
             Counts.data_ptr(), Y.data_ptr(), CAPACITY, N, K, TOP_K, PROJECTION, groups, start, scratch.data_ptr(),
             scratch.numel(), _abi.ptr(status), _abi.stream()))
         return
-    scratch = _scratch(X.shape[0], X.device)
+    scratch = _scratch(_abi.lib().ink_expert_gemm_scratch_bytes(X.shape[0]), X.device)
     _abi.check(_abi.lib().ink_expert_gemm(
         X.data_ptr(), X.shape[0], Pointers.data_ptr(), Experts.data_ptr(), Rows.data_ptr(), Counts.data_ptr(),
         Y.data_ptr(), CAPACITY, N, K, TOP_K, PROJECTION, int(bool(QUANTIZED)), groups, scratch.data_ptr(),

@@ -17,9 +17,9 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .kernels import (StackDescriptor, encode_bank_maps, expert_bank_names, expert_copy, expert_gemm, expert_plan, expert_reduce,
-                      moe_decode, routed_decode, router_forward, router_plan_forward, router_workspace,
-                      stack_supported)
+from .kernels import (StackDescriptor, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
+                      expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode, router_forward,
+                      router_plan_forward, router_workspace, stack_supported)
 from .kernels.paired_all_reduce import all_reduce
 
 # Up to this many tokens each route runs its own matrix-vector product
@@ -79,13 +79,15 @@ class ResidentExperts(nn.Module):
                                     dtype=torch.int64, device=self.device)
         # banks of one kind evenly spaced in memory (one allocation per kind, say): (address of the first,
         # byte distance) per kind, for the TMA descriptors of the one-launch kernel; otherwise None
-        kinds = ("gate_up_proj", "gate_up_proj_scale", "down_proj", "down_proj_scale")
+        kinds = ("gate_up_proj", "gate_up_proj_scale", "down_proj", "down_proj_scale") if self.quantized else ("gate_up_proj", "down_proj")
         self.bank_layout = self._even_spacing([[weights[e][n].data_ptr() for e in ids] for n in kinds],
-                                              [first[n].numel() * first[n].element_size() for n in kinds]) if self.quantized else None
-        # TMA descriptors of the banks for the block-scaled grouped kernel, where they are evenly spaced
+                                              [first[n].numel() * first[n].element_size() for n in kinds])
+        # TMA descriptors of the banks for the grouped tensor-core kernel, where they are evenly spaced
         self.bank_maps = None
-        if self.bank_layout is not None and hidden_dim % 256 == 0 and intermediate_dim % 256 == 0:
-            self.bank_maps = encode_bank_maps(self.bank_layout, self.local, hidden_dim, intermediate_dim, self.device)
+        step, widest = (256 if self.quantized else 128), max(hidden_dim, intermediate_dim)
+        if self.bank_layout is not None and hidden_dim % step == 0 and intermediate_dim % step == 0 and widest <= 4096 and self.local <= 1024:
+            encode = encode_bank_maps if self.quantized else encode_bf16_bank_maps
+            self.bank_maps = encode(self.bank_layout, self.local, hidden_dim, intermediate_dim, self.device)
         self.resident = torch.ones(self.local, **i32)
         self.destinations = torch.zeros((0, self.stride), dtype=torch.int64, device=self.device)
         self.slot_experts = torch.full((0,), -1, **i32)
@@ -130,14 +132,15 @@ class ResidentExperts(nn.Module):
         expert_copy[(128, 0)](self.sources, self.destinations, self.copy_experts, (), self.stride, 1024, 128)
 
     def grouped_supported(self) -> bool:
-        """The tensor-core path takes NVFP4 banks whose contraction widths are multiples of 128."""
-        return self.quantized and self.hidden_dim % 128 == 0 and self.intermediate_dim % 128 == 0
+        """Banks the grouped tensor-core path takes: evenly spaced in memory, or NVFP4 banks anywhere whose contraction
+        widths are multiples of 128."""
+        return self.bank_maps is not None or (self.quantized and self.hidden_dim % 128 == 0 and self.intermediate_dim % 128 == 0)
 
     def _project(self, x, indices, weights, output) -> None:
-        """GEMV per route up to MATVEC_TOKENS tokens, grouped tensor-core GEMMs above
-        (my_inkling/offloaded_experts.py:224-296). `output` must be zero on entry."""
+        """GEMV per route for one token (up to MATVEC_TOKENS where the banks are not evenly spaced), grouped tensor-core
+        GEMMs above (my_inkling/offloaded_experts.py:224-296). `output` must be zero on entry."""
         tokens = x.shape[0]
-        if tokens > MATVEC_TOKENS and self.grouped_supported():
+        if tokens > (1 if self.bank_maps is not None else MATVEC_TOKENS) and self.grouped_supported():
             self._project_grouped(x, indices, weights, output)
             return
         for t0 in range(0, tokens, MATVEC_TOKENS):
@@ -146,9 +149,20 @@ class ResidentExperts(nn.Module):
                           self.activated[t0 * indices.shape[1]:], output[t0:t1], self.max_expert, self.quantized,
                           status=self.status)
 
+    def grouped(self, x, indices, weights, output=None, output_bf16=None, shared_maps=None, gammas=None, n_shared: int = 0) -> None:
+        """Both projections and the weighted sum over the plan's groups in one call (banks with `bank_maps`); with
+        `shared_maps` the block's shared experts too. The outputs are overwritten."""
+        moe_grouped(x, indices, weights, self.pointers, self.experts, self.rows, self.counts, self.bank_maps, self.activated,
+                    self.down, output=output, output_bf16=output_bf16, groups=min(indices.numel(), self.local), start=self.start,
+                    local=self.local, capacity=self.capacity, max_expert=self.max_expert, quantized=self.quantized,
+                    shared_maps=shared_maps, gammas=gammas, n_shared=n_shared, status=self.status)
+
     def _project_grouped(self, x, indices, weights, output) -> None:
         """Both projections as grouped tensor-core GEMMs over the plan's groups, then the weighted
         sum per token (my_inkling/offloaded_experts.py:249-296). `output` must be zero on entry."""
+        if self.bank_maps is not None:
+            self.grouped(x, indices, weights, output)
+            return
         tokens, routes, top_k = x.shape[0], indices.numel(), indices.shape[1]
         groups = min(routes, self.local)
         for projection, inputs, target, n, k in (
@@ -156,8 +170,7 @@ class ResidentExperts(nn.Module):
                 (1, self.activated, self.down, self.hidden_dim, self.intermediate_dim)):
             grid = (triton_cdiv(routes, 16), triton_cdiv(n, 64), groups)
             expert_gemm[grid](inputs, self.pointers, self.experts, self.rows, self.counts, target, self.capacity,
-                              n, k, top_k, projection, True, self.stride, 16, 64, 64, status=self.status,
-                              bank_maps=self.bank_maps, start=self.start)
+                              n, k, top_k, projection, True, self.stride, 16, 64, 64, status=self.status)
         expert_reduce[(tokens, triton_cdiv(self.hidden_dim, 256))](
             self.down, indices, weights, self.pointers, output, self.hidden_dim, top_k, self.stride,
             self.max_expert, 256)
@@ -206,6 +219,7 @@ class FusedMoE(nn.Module):
         self.device_mesh = device_mesh
         self._tokens = 0
         self._fused = None   # one-launch descriptor for a single token, built on first use
+        self._maps_of = None
 
     def block_descriptor(self, norm_weight=None) -> dict:
         """This block as the one-launch kernel takes it (addresses of the module's tensors)."""
@@ -245,6 +259,13 @@ class FusedMoE(nn.Module):
         self.partial = torch.empty(tokens, self.experts.hidden_dim, dtype=torch.float32, device=dev)
         self.experts._reserve(tokens * self.top_k)
 
+    def _shared_maps(self):
+        """TMA descriptors of the shared experts, made when they are first needed (and again if the tensors are replaced)."""
+        at = (self.shared_gate.data_ptr(), self.shared_up.data_ptr(), self.shared_down.data_ptr())
+        if self._maps_of != at:
+            self._maps, self._maps_of = encode_shared_maps(self.shared_gate, self.shared_up, self.shared_down), at
+        return self._maps
+
     def route(self, flat):
         """Router and plan for `flat` [t, d]; fills the module's routing buffers."""
         t = flat.shape[0]
@@ -278,6 +299,10 @@ class FusedMoE(nn.Module):
             self._fused.decode(flat, self.partial[:1])
             return self.partial[:1]
         self.route(flat)
+        if t > 1 and ex.bank_maps is not None:
+            ex.grouped(flat, self.topk_indices[:t], self.topk_weights[:t], self.partial[:t], shared_maps=self._shared_maps() if self.n_shared else None,
+                       gammas=self.gammas[:t], n_shared=self.n_shared)
+            return all_reduce(self.partial[:t], _group_of(self.device_mesh))
         for t0 in range(0, t, MATVEC_TOKENS):
             t1 = min(t, t0 + MATVEC_TOKENS)
             moe_decode(flat[t0:t1], self.topk_indices[t0:t1], self.topk_weights[t0:t1], ex.pointers,
