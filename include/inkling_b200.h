@@ -81,7 +81,7 @@ int ink_router_forward_static(const void* x, const void* weight, const float* bi
                               void* routed_logits, void* topk_weights, int64_t* topk_indices,
                               void* shared_gammas, ink_stream_t stream);
 
-/* Router and expert plan in ONE launch (decode: tokens * top_k <= 512 routes); the
+/* Router and expert plan in one call (up to eight tokens in ONE launch); the
  * plan arguments are those of ink_expert_plan below. */
 int ink_router_plan_forward(const void* x, const void* weight, const float* bias, const void* global_scale,
                             float route_scale, int tokens, int hidden, int n_routed, int n_shared, int top_k,

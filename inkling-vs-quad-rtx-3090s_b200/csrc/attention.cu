@@ -10,9 +10,10 @@ constexpr int kAttnWarps = kAttnThreads / 32;
 constexpr int kAttnHeads = 8;                               // query heads that share a pass over the cache rows
 constexpr int kAttnUnit = 16;                               // cache slots per step of a warp
 constexpr int kAttnMinSlots = kAttnUnit * kAttnWarps;       // a block is not worth launching for fewer
+constexpr int kAttnCluster = 8;                             // parts that can meet in one thread-block cluster
 constexpr int kAttnMaxSplits = 64;
 constexpr int kAttnWaveBlocks = 148 * 3;                    // blocks resident at once
-constexpr int kAttnPartial = 2;                             // floats in front of a partial result: running maximum, sum
+constexpr int kAttnPartial = 4;                             // floats in front of a partial result: running maximum, sum, padding
 
 struct AttnArgs {
   const uint16_t* q;        // [bs, h, c] after q_norm
@@ -47,6 +48,19 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return r;
 }
 
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// two floats at this block's address `p` in the shared memory of block `rank` of the cluster
+__device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
+  float2 v;
+  asm volatile("{\n .reg .u32 at;\n mapa.shared::cluster.u32 at, %2, %3;\n ld.shared::cluster.v2.f32 {%0, %1}, [at];\n}\n"
+               : "=f"(v.x), "=f"(v.y)
+               : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank)
+               : "memory");
+  return v;
+}
+
 // One block per (part of the cache, group of up to eight heads of one key/value head, sequence). Bound by reading
 // the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
 // deliver at HBM speed, so scores, bias and weighted values go through warp-level matrix instructions (M = heads: the
@@ -62,7 +76,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 //           loads the piece g (and g + 8) of the rows 2t, 2t+1, 2t+8, 2t+9, and word pairs of neighbouring rows are
 //           interleaved into B. The unused upper eight rows of A carry what BF16 cuts off the exponentials (p = hi + lo),
 //           so the weights keep 16 bits at no further instruction.
-template <int C>
+//
+// The parts of a group of heads are joined in one of two ways. Up to eight of them form a thread-block cluster (CLUSTER)
+// and read one another's sums through distributed shared memory; more leave their sums in global memory and the block that
+// finishes last adds them up. The second way costs a fence, an atomic and two more round trips.
+template <int C, bool CLUSTER>
 __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attention_kernel(AttnArgs a) {
   constexpr int kPieces = C / 32;       // 16-byte pieces of a key row per lane
   constexpr int kHalves = C / 64;       // pieces of a value row per lane
@@ -70,6 +88,7 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
   float* s_acc = reinterpret_cast<float*>(s_raw);                                   // [warps][heads][C + 2]
   uint16_t* s_r = reinterpret_cast<uint16_t*>(s_raw);                               // [heads][d_rel rounded up to 16]: before the sums
   __shared__ bool s_last;
+  __shared__ __align__(16) float s_block[CLUSTER ? kAttnHeads * (C + 2) : 1];   // this block's sums, for its cluster
   const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
@@ -286,6 +305,10 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
     if (a.splits == 1) {
       const float inv = 1.f / sum;
       reinterpret_cast<uint32_t*>(a.out + row * C)[pair] = pack_bf16(o0 * inv, o1 * inv);
+    } else if (CLUSTER) {
+      float* mine = s_block + h * (C + 2);
+      if (pair == 0) *reinterpret_cast<float2*>(mine + C) = make_float2(all_top, sum);
+      *reinterpret_cast<float2*>(mine + 2 * pair) = make_float2(o0, o1);
     } else {
       float* mine = a.partial + (row * a.splits + split) * stride;
       if (pair == 0) *reinterpret_cast<float2*>(mine) = make_float2(all_top, sum);
@@ -293,8 +316,34 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
     }
   }
   if (a.splits == 1) return;
-  // The block that stores the last partial of its heads joins them all:
   //   out = sum_i acc_i e^(m_i - M) / sum_i l_i e^(m_i - M)
+  if constexpr (CLUSTER) {
+    cluster_sync();
+    for (int i = split * kAttnThreads + tid; i < n_heads * kPairs; i += a.splits * kAttnThreads) {
+      const int h = i / kPairs, pair = i % kPairs;
+      float2 head[kAttnCluster], val[kAttnCluster];
+      float all_top = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kAttnCluster; ++s) {
+        head[s] = s < a.splits ? ld_cluster_float2(s_block + h * (C + 2) + C, s) : make_float2(-INFINITY, 0.f);
+        val[s] = s < a.splits ? ld_cluster_float2(s_block + h * (C + 2) + 2 * pair, s) : make_float2(0.f, 0.f);
+        all_top = fmaxf(all_top, head[s].x);
+      }
+      float o0 = 0.f, o1 = 0.f, sum = 0.f;
+#pragma unroll
+      for (int s = 0; s < kAttnCluster; ++s) {
+        const float weight = head[s].x == -INFINITY ? 0.f : __expf(head[s].x - all_top);
+        sum = fmaf(head[s].y, weight, sum);
+        o0 = fmaf(val[s].x, weight, o0);
+        o1 = fmaf(val[s].y, weight, o1);
+      }
+      const float inv = 1.f / sum;
+      reinterpret_cast<uint32_t*>(a.out + ((size_t)b * a.heads + head0 + h) * C)[pair] = pack_bf16(o0 * inv, o1 * inv);
+    }
+    cluster_sync();   // (a block's sums stay until everybody has read them)
+    return;
+  }
+  // The block that stores the last partial of its heads joins them all.
   __threadfence();   // every writer pushes its own stores out before the block is counted
   __syncthreads();
   if (tid == 0) {
@@ -305,27 +354,54 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int i = tid; i < n_heads * kPairs; i += kAttnThreads) {
-    const int h = i / kPairs, pair = i % kPairs;
-    const size_t row = (size_t)b * a.heads + head0 + h;
-    const float* base = a.partial + row * a.splits * stride;
-    float all_top = -INFINITY;
-    for (int s = lane; s < a.splits; s += 32) all_top = fmaxf(all_top, __ldcg(base + (size_t)s * stride));   // (a warp is inside one head)
+  // first every part's weight, all parts at once: [head][part]; then the sums, sixteen parts in flight
+  float* s_weight = s_acc;
+  float* s_inv = s_acc + kAttnHeads * kAttnMaxSplits;
+  for (int h = warp; h < n_heads; h += kAttnWarps) {
+    const float* base = a.partial + ((size_t)b * a.heads + head0 + h) * a.splits * stride;
+    constexpr int kPerLane = kAttnMaxSplits / 32;
+    float2 head[kPerLane];
+    float all_top = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int n = 0; n < kPerLane; ++n) {
+      const int s = n * 32 + lane;
+      head[n] = s < a.splits ? __ldcg(reinterpret_cast<const float2*>(base + (size_t)s * stride)) : make_float2(-INFINITY, 0.f);
+      all_top = fmaxf(all_top, head[n].x);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, o));
-    float o0 = 0.f, o1 = 0.f, sum = 0.f;
-#pragma unroll 8
-    for (int s = 0; s < a.splits; ++s) {
-      const float* from = base + (size_t)s * stride;
-      const float2 head = __ldcg(reinterpret_cast<const float2*>(from));
-      const float2 val = __ldcg(reinterpret_cast<const float2*>(from + kAttnPartial) + pair);
-      const float weight = head.x == -INFINITY ? 0.f : __expf(head.x - all_top);
-      sum = fmaf(head.y, weight, sum);
-      o0 = fmaf(val.x, weight, o0);
-      o1 = fmaf(val.y, weight, o1);
+#pragma unroll
+    for (int n = 0; n < kPerLane; ++n) {
+      const float weight = head[n].x == -INFINITY ? 0.f : __expf(head[n].x - all_top);
+      s_weight[h * kAttnMaxSplits + n * 32 + lane] = weight;
+      sum = fmaf(head[n].y, weight, sum);
     }
-    const float inv = 1.f / sum;
-    reinterpret_cast<uint32_t*>(a.out + row * C)[pair] = pack_bf16(o0 * inv, o1 * inv);
+    sum = warp_sum(sum);
+    if (lane == 0) s_inv[h] = 1.f / sum;
+  }
+  __syncthreads();
+  for (int i = tid; i < n_heads * (C / 4); i += kAttnThreads) {
+    const int h = i / (C / 4), quad = i % (C / 4);
+    const size_t row = (size_t)b * a.heads + head0 + h;
+    const float* base = a.partial + row * a.splits * stride + kAttnPartial + 4 * quad;
+    const float* weights = s_weight + h * kAttnMaxSplits;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int s0 = 0; s0 < a.splits; s0 += 16) {
+      float4 v[16];
+#pragma unroll
+      for (int n = 0; n < 16; ++n) v[n] = s0 + n < a.splits ? __ldcg(reinterpret_cast<const float4*>(base + (size_t)(s0 + n) * stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int n = 0; n < 16; ++n) {
+        const float weight = weights[s0 + n];   // (zero beyond the last part)
+        o.x = fmaf(v[n].x, weight, o.x);
+        o.y = fmaf(v[n].y, weight, o.y);
+        o.z = fmaf(v[n].z, weight, o.z);
+        o.w = fmaf(v[n].w, weight, o.w);
+      }
+    }
+    const float inv = s_inv[h];
+    reinterpret_cast<uint2*>(a.out + row * C)[quad] = make_uint2(pack_bf16(o.x * inv, o.y * inv), pack_bf16(o.z * inv, o.w * inv));
   }
 }
 
@@ -364,9 +440,23 @@ template <int C>
 static int launch_decode_attention(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
   const size_t sums = sizeof(float) * kAttnWarps * kAttnHeads * (C + 2), rel = sizeof(uint16_t) * kAttnHeads * ((size_t)(a.d_rel + 15) / 16 * 16);
   const size_t smem = sums > rel ? sums : rel;
-  INK_REQUIRE(smem <= 48 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
-  decode_attention_kernel<C><<<grid, kAttnThreads, smem, stream>>>(a);
-  INK_CHECK_LAUNCH("decode_attention");
+  static_assert(kAttnWarps * (C + 2) > kAttnMaxSplits + 1, "the join's weights fit where the warps' sums were");
+  INK_REQUIRE(smem <= 40 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(kAttnThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeClusterDimension;
+  attribute.val.clusterDim.x = grid.x;
+  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+  config.attrs = &attribute;
+  const bool cluster = a.splits > 1 && a.splits <= kAttnCluster;
+  config.numAttrs = cluster ? 1 : 0;
+  const cudaError_t e = cluster ? cudaLaunchKernelEx(&config, decode_attention_kernel<C, true>, a)
+                                : cudaLaunchKernelEx(&config, decode_attention_kernel<C, false>, a);
+  INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "decode_attention: launch failed: %s", cudaGetErrorString(e));
   return kOk;
 }
 
@@ -393,10 +483,12 @@ extern "C" int ink_decode_attention(const void* q, const void* r, const void* pr
                   (need == 0 || aligned16(workspace)),
               kMisaligned, "decode_attention: buffers must be 16-byte aligned");
   if (batch == 0) return kOk;
-  // Parts of the cache: enough blocks to fill the GPU (three of four warps fit on an SM), none with less than a step
-  // per warp. Where one wave of long parts would leave SMs idle at its end (few pairs of sequence and head group), the
-  // parts are small anyway; with many pairs there are two waves' worth, so that shorter sequences even out.
-  const int pairs = batch * kv_heads * chunks, most = attention_max_splits(slots);
+  // Parts of the cache: two waves of blocks where there is that much to read (three of four warps fit on an SM; two, so that
+  // shorter sequences even out). Short caches are cut no finer than one step per warp while the parts fit a cluster, and no
+  // finer than two steps beyond, where each further part lengthens the join.
+  const int pairs = batch * kv_heads * chunks, whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
+  const int short_most = whole <= kAttnCluster ? whole : whole / 2 > kAttnCluster ? whole / 2 : kAttnCluster;
+  const int most = short_most < attention_max_splits(slots) ? short_most : attention_max_splits(slots);
   const int wanted = (kAttnWaveBlocks * 2 + pairs - 1) / pairs;
   const int splits = wanted < 1 ? 1 : wanted < most ? wanted : most;
   AttnArgs a{(const uint16_t*)q, (const uint16_t*)r, (const uint16_t*)proj, (const uint16_t*)k_cache, (const uint16_t*)v_cache,

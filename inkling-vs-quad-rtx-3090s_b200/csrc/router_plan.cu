@@ -20,7 +20,10 @@ void set_error(const char* fmt, ...) {
 constexpr int kTokenGroup = 8;           // tokens whose accumulators a warp holds at once
 constexpr int kMaxScoresPerLane = 16;    // n_routed <= 512
 constexpr int kFinishThreads = 256;
-constexpr int kPlanSmallRoutes = 512;    // routes the single-block plan keeps in shared memory
+constexpr int kFewTokens = 8;            // tokens the one-launch router takes
+constexpr int kFusedRoutes = 32 * kFewTokens;   // their routes
+constexpr int kFusedRuns = kFinishThreads / 32;
+constexpr size_t kPlanSmem = 200 * 1024; // most shared memory of the plan's tables
 
 struct RouterArgs {
   const uint16_t* x;
@@ -49,47 +52,44 @@ struct PlanArgs {
 };
 
 // ------------------------------------------------------------------ one token
-// Executed by one warp. `score` is this warp's shared-memory scratch of n_routed floats:
-// score[e] = bf16(sigmoid(logit_e)) + bias_e, computed by the blocks that produced the
-// logits. Small loops on purpose: this code runs once, on one warp, straight out of a
-// cold instruction cache.
-__device__ void router_finish_token(const RouterArgs& a, int token, float* score, int* ids_out) {
+// Executed by one warp, scores and selection in registers: lane l holds the experts l, l + 32, ... (up to 32 * K).
+// A round of the selection is the lane's own best, then two hardware reductions over the warp (largest score as an
+// order-preserving integer, then the lowest expert id among the lanes that hold it).
+template <int K>
+__device__ __forceinline__ void router_finish_token(const RouterArgs& a, int token, int* ids_out) {
   const int lane = threadIdx.x & 31;
   const int total = a.n_routed + a.n_shared;
   const float* logit = a.logits + (size_t)token * total;
   const float* scores = a.scores + (size_t)token * a.n_routed;
-  for (int e = lane; e < a.n_routed; e += 32) {
-    score[e] = __ldcg(scores + e);
-    if (a.routed_logits) a.routed_logits[(size_t)token * a.n_routed + e] = (uint16_t)f32_to_bf16_bits(__ldcg(logit + e));
+  float sc[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const int e = i * 32 + lane;
+    sc[i] = e < a.n_routed ? __ldcg(scores + e) : -INFINITY;
+    if (a.routed_logits && e < a.n_routed) a.routed_logits[(size_t)token * a.n_routed + e] = (uint16_t)f32_to_bf16_bits(__ldcg(logit + e));
   }
-  __syncwarp();
   // top-k by repeated arg-max; ties go to the lower expert id
   int my_choice = 0;  // lane r < top_k ends up holding the r-th choice
 #pragma unroll 1
   for (int r = 0; r < a.top_k; ++r) {
     float best = -INFINITY;
     int best_e = 0x7fffffff;
-#pragma unroll 1
-    for (int e = lane; e < a.n_routed; e += 32) {
-      const float v = score[e];
-      if (v > best) {  // ascending e within a lane: a later equal value never replaces
-        best = v;
-        best_e = e;
-      }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ov > best || (ov == best && oe < best_e)) {
-        best = ov;
-        best_e = oe;
+    for (int i = 0; i < K; ++i) {
+      if (sc[i] > best) {  // ascending e within a lane: a later equal value never replaces
+        best = sc[i];
+        best_e = i * 32 + lane;
       }
     }
-    if (best_e == 0x7fffffff) best_e = r;  // every score is -inf/NaN: fall back to a valid id
-    if (lane == 0) score[best_e] = -INFINITY;
-    if (lane == r) my_choice = best_e;
-    __syncwarp();
+    const unsigned bits = __float_as_uint(best + 0.f);   // (-0 counts as 0)
+    const unsigned key = (bits & 0x80000000u) ? ~bits : (bits | 0x80000000u);   // a > b  <=>  key(a) > key(b)
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    int winner = (int)__reduce_min_sync(0xffffffffu, key == top ? (unsigned)best_e : 0x7fffffffu);
+    if (winner == 0x7fffffff) winner = r;  // every score is -inf/NaN: fall back to a valid id
+#pragma unroll
+    for (int i = 0; i < K; ++i)
+      if (i * 32 + lane == winner) sc[i] = -INFINITY;
+    if (lane == r) my_choice = winner;
   }
   // weights over the top_k selected logits followed by the shared logits
   const int n = a.top_k + a.n_shared;
@@ -121,37 +121,67 @@ __device__ void router_finish_token(const RouterArgs& a, int token, float* score
   }
 }
 
-// ------------------------------------------------------------- single-block plan
-// routes <= kPlanSmallRoutes. Whole block; `ids` is shared memory for the routes.
-__device__ void plan_small(const PlanArgs& p, int* ids, int* warp_totals, bool ids_loaded) {
+__device__ __forceinline__ void router_finish_token(const RouterArgs& a, int token, int* ids_out) {
+  if (a.n_routed <= 256) router_finish_token<8>(a, token, ids_out);
+  else router_finish_token<kMaxScoresPerLane>(a, token, ids_out);
+}
+
+// ------------------------------------------------------------------------ the plan
+// One block: a stable counting sort of the routes by expert. Warp w takes the w-th run of routes, counts them per expert
+// (lanes with equal ids find each other with a match, so nothing is atomic), the counts become offsets by a prefix sum over
+// the warps, and a second pass over the same runs hands out the places in order. `hist` is [runs][local] and `group_of`
+// [local] in shared memory. (One warp per expert walking all routes took 105 us for 12 000 of them, the compare loop of a
+// single block 18 us for 366; this one is two passes over routes / 1024 steps.)
+constexpr int kPlanRuns = 32;
+__device__ void plan_block(const PlanArgs& p, const int* ids, int* hist, int* group_of, int* warp_totals, int runs) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  for (int r = tid; r < p.routes; r += blockDim.x) {
-    const int64_t id = ids_loaded ? (int64_t)ids[r] : p.indices[r];
-    ids[r] = (id >= p.start && id < (int64_t)p.start + p.local) ? (int)(id - p.start) : -1;
+  const int per_run = ((p.routes + runs - 1) / runs + 31) / 32 * 32;
+  auto id_of = [&](int r, int end) -> int {   // local id, -1: not on this rank
+    if (r >= end) return -1;
+    const int64_t id = ids ? (int64_t)ids[r] : __ldcg(p.indices + r);
+    return (id >= p.start && id < (int64_t)p.start + p.local) ? (int)(id - p.start) : -1;
+  };
+  for (int i = tid; i < runs * p.local; i += blockDim.x) hist[i] = 0;
+  __syncthreads();
+  const int first = warp * per_run, end = min(p.routes, first + per_run);
+  if (warp < runs) {
+    int* mine = hist + warp * p.local;
+    int next = id_of(first + lane, end);
+    for (int r = first; r < end; r += 32) {
+      const int id = next;
+      next = id_of(r + 32 + lane, end);
+      const unsigned same = __match_any_sync(0xffffffffu, id);
+      if (id >= 0 && lane == __ffs(same) - 1) mine[id] += __popc(same);
+      __syncwarp();
+    }
   }
   __syncthreads();
   int groups_before = 0;
   for (int base = 0; base < p.local; base += blockDim.x) {
     const int e = base + tid;
     int count = 0;
-    if (e < p.local)
-      for (int r = 0; r < p.routes; ++r) count += (ids[r] == e);
+    if (e < p.local) {
+      for (int w = 0; w < runs; ++w) {
+        const int n = hist[w * p.local + e];
+        hist[w * p.local + e] = count;
+        count += n;
+      }
+    }
     const bool active = count > 0;
     const unsigned ballot = __ballot_sync(0xffffffffu, active);
     if (lane == 0) warp_totals[warp] = __popc(ballot);
     __syncthreads();
-    int before = groups_before;
-    for (int w = 0; w < warp; ++w) before += warp_totals[w];
-    int chunk_total = 0;
-    for (int w = 0; w < warps; ++w) chunk_total += warp_totals[w];
+    int before = groups_before, chunk_total = 0;
+    for (int w = 0; w < warps; ++w) {
+      if (w < warp) before += warp_totals[w];
+      chunk_total += warp_totals[w];
+    }
     const int group = before + __popc(ballot & ((1u << lane) - 1u));
     if (e < p.local) {
+      group_of[e] = group;
       if (active) {
         p.experts[group] = p.start + e;
         p.counts[group] = count;
-        int pos = 0;
-        for (int r = 0; r < p.routes; ++r)
-          if (ids[r] == e) p.rows[(size_t)group * p.capacity + pos++] = r;
       }
       for (int b = 0; b < p.stride; ++b)
         p.pointers[(size_t)(p.start + e) * p.stride + b] = active ? p.sources[(size_t)e * p.stride + b] : 0;
@@ -162,6 +192,23 @@ __device__ void plan_small(const PlanArgs& p, int* ids, int* warp_totals, bool i
   for (int g = groups_before + tid; g < p.local; g += blockDim.x) {
     p.experts[g] = -1;
     p.counts[g] = 0;
+  }
+  if (warp < runs) {
+    int* mine = hist + warp * p.local;
+    int next = id_of(first + lane, end);
+    for (int r = first; r < end; r += 32) {
+      const int id = next;
+      next = id_of(r + 32 + lane, end);
+      const unsigned same = __match_any_sync(0xffffffffu, id);
+      int at = 0;
+      if (id >= 0) at = mine[id] + __popc(same & ((1u << lane) - 1u));
+      __syncwarp();
+      if (id >= 0) {
+        p.rows[(size_t)group_of[id] * p.capacity + at] = r + lane;
+        if (lane == __ffs(same) - 1) mine[id] += __popc(same);
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -174,10 +221,10 @@ constexpr int kWarpsPerRow = kFinishThreads / 32 / kRowsPerBlock;
 
 template <bool kFusePlan, int TG>
 __global__ void __launch_bounds__(kFinishThreads) router_kernel(RouterArgs a, PlanArgs p) {
-  __shared__ int s_ids[kPlanSmallRoutes];
+  __shared__ int s_ids[kFusedRoutes];
   __shared__ int s_warp_totals[32];
+  __shared__ int s_hist[kFusePlan ? kFusedRuns * 32 * kMaxScoresPerLane : 1], s_group_of[kFusePlan ? 32 * kMaxScoresPerLane : 1];
   __shared__ float s_part[kRowsPerBlock][kWarpsPerRow][TG];
-  __shared__ float s_score[kFinishThreads / 32][32 * kMaxScoresPerLane];
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int total = a.n_routed + a.n_shared;
@@ -244,80 +291,119 @@ __global__ void __launch_bounds__(kFinishThreads) router_kernel(RouterArgs a, Pl
   if (!s_last) return;
   __threadfence();
   for (int token = warp; token < a.tokens; token += warps)
-    router_finish_token(a, token, s_score[warp], kFusePlan ? s_ids : nullptr);
+    router_finish_token(a, token, kFusePlan ? s_ids : nullptr);
   if (kFusePlan) {
     __syncthreads();
-    plan_small(p, s_ids, s_warp_totals, true);
+    plan_block(p, s_ids, s_hist, s_group_of, s_warp_totals, kFusedRuns);
   }
   if (threadIdx.x == 0) *a.counter = 0u;  // leave the workspace ready for the next call
 }
 
-__global__ void __launch_bounds__(kFinishThreads) plan_small_kernel(PlanArgs p) {
-  __shared__ int s_ids[kPlanSmallRoutes];
+__global__ void __launch_bounds__(1024) plan_kernel(PlanArgs p, int runs) {
+  extern __shared__ int s_plan[];   // [runs][local] counts, [local] groups
   __shared__ int s_warp_totals[32];
-  plan_small(p, s_ids, s_warp_totals, false);
+  plan_block(p, nullptr, s_plan, s_plan + runs * p.local, s_warp_totals, runs);
 }
 
-// ------------------------------------------------------------- plan, any size
-// Pass 1 (one block): histogram of routes per expert, then compaction of the active
-// experts and the pointer table. Pass 2 (one warp per expert): ordered list of routes.
-__global__ void __launch_bounds__(1024) plan_count_kernel(PlanArgs p, int* histogram /* [local] zeroed by this kernel */) {
-  __shared__ int s_warp_totals[32];
-  __shared__ int s_base;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  for (int e = tid; e < p.local; e += blockDim.x) histogram[e] = 0;
-  if (tid == 0) s_base = 0;
-  __syncthreads();
-  for (int r = tid; r < p.routes; r += blockDim.x) {
-    const int64_t id = p.indices[r];
-    if (id >= p.start && id < (int64_t)p.start + p.local) atomicAdd(&histogram[(int)(id - p.start)], 1);
-  }
-  __syncthreads();
-  for (int base = 0; base < p.local; base += blockDim.x) {
-    const int e = base + tid;
-    const int count = e < p.local ? histogram[e] : 0;
-    const bool active = count > 0;
-    const unsigned ballot = __ballot_sync(0xffffffffu, active);
-    if (lane == 0) s_warp_totals[warp] = __popc(ballot);
-    __syncthreads();
-    int before = s_base, chunk_total = 0;
-    for (int w = 0; w < warps; ++w) {
-      if (w < warp) before += s_warp_totals[w];
-      chunk_total += s_warp_totals[w];
+// ------------------------------------------------------------- router, many tokens
+// The logits of more than a handful of tokens: a block takes eight router rows and sixteen tokens, every thread the
+// partial sums of all 128 pairs over its columns. A thread's columns, the order of its sums and the order in which the
+// threads' sums are added are those of router_kernel, so a token's logits do not depend on how many others there are (the
+// selection compares BF16 values: a last-bit difference picks another expert). Bound by the FMA pipes (2.1 G FMAs for
+// 1 999 tokens: 58 us); router_kernel, two rows a block and its tail on one block, took 3 270 us for them.
+constexpr int kManyRows = 8, kManyTokens = 16, kManyThreads = 128;
+
+// Sums N per-lane values over the warp in the order of warp_sum; lane l keeps the values first, first + 1, ... (N / 32).
+template <int N>
+__device__ __forceinline__ int wide_reduce(float (&v)[N], int lane) {
+  int first = 0;
+#pragma unroll
+  for (int o = 16, n = N; o > 0; o >>= 1, n >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const float send = upper ? v[i] : v[i + n / 2];
+      const float keep = upper ? v[i + n / 2] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
-    const int group = before + __popc(ballot & ((1u << lane) - 1u));
-    if (e < p.local) {
-      if (active) {
-        p.experts[group] = p.start + e;
-        p.counts[group] = count;
+    first += upper ? n / 2 : 0;
+  }
+  return first;
+}
+
+__global__ void __launch_bounds__(kManyThreads, 2) router_logits_kernel(RouterArgs a) {
+  constexpr int kPairs = kManyRows * kManyTokens, kParts = kManyThreads / 32;
+  __shared__ float s_part[kParts][kPairs];
+  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+  const int total = a.n_routed + a.n_shared, chunks = a.hidden / 8;
+  const int row0 = blockIdx.x * kManyRows, token0 = blockIdx.y * kManyTokens;
+  float acc[kPairs];   // [token][row]
+#pragma unroll
+  for (int i = 0; i < kPairs; ++i) acc[i] = 0.f;
+#pragma unroll 1
+  for (int c = tid; c < chunks; c += kManyThreads) {
+    float w[kManyRows][8];
+#pragma unroll
+    for (int r = 0; r < kManyRows; ++r) {
+      const int row = min(row0 + r, total - 1);
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(a.weight + (size_t)row * a.hidden) + c);
+      w[r][0] = bf16lo(q.x); w[r][1] = bf16hi(q.x); w[r][2] = bf16lo(q.y); w[r][3] = bf16hi(q.y);
+      w[r][4] = bf16lo(q.z); w[r][5] = bf16hi(q.z); w[r][6] = bf16lo(q.w); w[r][7] = bf16hi(q.w);
+    }
+#pragma unroll
+    for (int t0 = 0; t0 < kManyTokens; t0 += 4) {
+      uint4 x4[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) x4[t] = __ldg(reinterpret_cast<const uint4*>(a.x + (size_t)min(token0 + t0 + t, a.tokens - 1) * a.hidden) + c);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float x[8] = {bf16lo(x4[t].x), bf16hi(x4[t].x), bf16lo(x4[t].y), bf16hi(x4[t].y),
+                            bf16lo(x4[t].z), bf16hi(x4[t].z), bf16lo(x4[t].w), bf16hi(x4[t].w)};
+#pragma unroll
+        for (int r = 0; r < kManyRows; ++r) {
+          float s = acc[(t0 + t) * kManyRows + r];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) s = fmaf(w[r][k], x[k], s);
+          acc[(t0 + t) * kManyRows + r] = s;
+        }
       }
-      for (int b = 0; b < p.stride; ++b)
-        p.pointers[(size_t)(p.start + e) * p.stride + b] = active ? p.sources[(size_t)e * p.stride + b] : 0;
     }
-    __syncthreads();
-    if (tid == 0) s_base += chunk_total;
-    __syncthreads();
   }
-  for (int g = s_base + tid; g < p.local; g += blockDim.x) {
-    p.experts[g] = -1;
-    p.counts[g] = 0;
+  const int first = wide_reduce<kPairs>(acc, lane);
+#pragma unroll
+  for (int i = 0; i < kPairs / 32; ++i) s_part[part][first + i] = acc[i];
+  __syncthreads();
+  for (int i = tid; i < kPairs; i += kManyThreads) {
+    const int row = row0 + i % kManyRows, token = token0 + i / kManyRows;
+    if (row >= total || token >= a.tokens) continue;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < kParts; ++w) s += s_part[w][i];
+    const float l = round_bf16(s);
+    a.logits[(size_t)token * total + row] = l;
+    if (row < a.n_routed) a.scores[(size_t)token * a.n_routed + row] = round_bf16(1.f / (1.f + __expf(-l))) + a.bias[row];
   }
 }
 
-__global__ void __launch_bounds__(256) plan_rows_kernel(PlanArgs p) {
-  const int lane = threadIdx.x & 31;
-  const int group = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (group >= p.local) return;
-  const int expert = p.experts[group];
-  if (expert < 0) return;
-  int pos = 0;
-  for (int base = 0; base < p.routes; base += 32) {
-    const int r = base + lane;
-    const bool match = r < p.routes && p.indices[r] == (int64_t)expert;
-    const unsigned ballot = __ballot_sync(0xffffffffu, match);
-    if (match) p.rows[(size_t)group * p.capacity + pos + __popc(ballot & ((1u << lane) - 1u))] = r;
-    pos += __popc(ballot);
+// One warp per token; the block that is done last makes the plan, if one is asked for.
+template <bool kFusePlan>
+__global__ void __launch_bounds__(1024) router_select_kernel(RouterArgs a, PlanArgs p, int runs) {
+  extern __shared__ int s_plan[];
+  __shared__ int s_warp_totals[32];
+  __shared__ bool s_last;
+  const int token = blockIdx.x * 32 + (threadIdx.x >> 5);
+  if (token < a.tokens) router_finish_token(a, token, nullptr);
+  if (!kFusePlan) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
+    if (s_last) *a.counter = 0u;   // leave the workspace ready for the next call
   }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  plan_block(p, nullptr, s_plan, s_plan + runs * p.local, s_warp_totals, runs);
 }
 
 static int check_router(const RouterArgs& a, size_t workspace_bytes) {
@@ -342,7 +428,57 @@ static int check_plan(const PlanArgs& p) {
   INK_REQUIRE(p.local > 0 && p.start >= 0 && p.stride > 0 && p.routes >= 0 && p.capacity >= 1, kBadArgument,
               "expert_plan: start=%d local=%d stride=%d routes=%d capacity=%d", p.start, p.local, p.stride,
               p.routes, p.capacity);
-  INK_REQUIRE(p.capacity >= p.routes || p.capacity >= 1, kBadArgument, "expert_plan: capacity too small");
+  INK_REQUIRE((size_t)p.local * 2 * sizeof(int) <= kPlanSmem, kUnsupportedShape, "expert_plan: %d experts on this rank", p.local);
+  return kOk;
+}
+
+// Runs of routes the plan sorts side by side: as many warps as have a step's worth, as far as their tables fit.
+static int plan_runs(const PlanArgs& p) {
+  const int fit = (int)(kPlanSmem / sizeof(int) / p.local) - 1, whole = (p.routes + 31) / 32;
+  const int runs = fit < kPlanRuns ? fit : kPlanRuns;
+  return whole < 1 ? 1 : whole < runs ? whole : runs;
+}
+template <typename Kernel>
+static int allow_plan_smem(Kernel kernel) {
+  constexpr int kMaxDevices = 64;
+  static bool done[kMaxDevices] = {};
+  int device = 0;
+  cudaGetDevice(&device);
+  INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "expert_plan: device ordinal %d", device);
+  if (!done[device]) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanSmem);
+    INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "expert_plan: shared memory opt-in refused: %s", cudaGetErrorString(e));
+    done[device] = true;
+  }
+  return kOk;
+}
+
+// The router, with the plan if `p` is given. Up to eight tokens: one launch, whose last block selects and plans; more: the
+// logits by themselves (the last block of one launch would select for thousands of tokens alone), then selection and plan.
+static int launch_router(const RouterArgs& a, const PlanArgs* p, cudaStream_t stream) {
+  const int rows = a.n_routed + a.n_shared, blocks = (rows + kRowsPerBlock - 1) / kRowsPerBlock;
+  if (a.tokens <= kFewTokens && (!p || p->local <= 32 * kMaxScoresPerLane)) {
+    const PlanArgs plan = p ? *p : PlanArgs{};
+    if (p && a.tokens == 1) router_kernel<true, 1><<<blocks, kFinishThreads, 0, stream>>>(a, plan);
+    else if (p) router_kernel<true, kTokenGroup><<<blocks, kFinishThreads, 0, stream>>>(a, plan);
+    else if (a.tokens == 1) router_kernel<false, 1><<<blocks, kFinishThreads, 0, stream>>>(a, plan);
+    else router_kernel<false, kTokenGroup><<<blocks, kFinishThreads, 0, stream>>>(a, plan);
+    INK_CHECK_LAUNCH("ink_router_forward");
+    return kOk;
+  }
+  const dim3 grid((unsigned)((rows + kManyRows - 1) / kManyRows), (unsigned)((a.tokens + kManyTokens - 1) / kManyTokens));
+  INK_REQUIRE(grid.y <= 65535, kUnsupportedShape, "router: %d tokens in one call", a.tokens);
+  router_logits_kernel<<<grid, kManyThreads, 0, stream>>>(a);
+  INK_CHECK_LAUNCH("ink_router_forward (logits)");
+  const unsigned selects = (unsigned)((a.tokens + 31) / 32);
+  if (!p) {
+    router_select_kernel<false><<<selects, 1024, 0, stream>>>(a, PlanArgs{}, 0);
+  } else {
+    if (int rc = allow_plan_smem(router_select_kernel<true>)) return rc;
+    const int runs = plan_runs(*p);
+    router_select_kernel<true><<<selects, 1024, sizeof(int) * (size_t)(runs + 1) * p->local, stream>>>(a, *p, runs);
+  }
+  INK_CHECK_LAUNCH("ink_router_forward (selection)");
   return kOk;
 }
 
@@ -392,15 +528,7 @@ extern "C" int ink_router_forward(const void* x, const void* weight, const float
                                   top_k, routed_logits, topk_weights, topk_indices, shared_gammas, workspace);
   if (int rc = check_router(a, workspace_bytes)) return rc;
   if (tokens == 0) return kOk;
-  const int blocks = (n_routed + n_shared + kRowsPerBlock - 1) / kRowsPerBlock;
-  INK_PREFER_MAX_SMEM((router_kernel<false, 1>));
-  INK_PREFER_MAX_SMEM((router_kernel<false, kTokenGroup>));
-  if (tokens == 1)
-    router_kernel<false, 1><<<blocks, kFinishThreads, 0, (cudaStream_t)stream>>>(a, PlanArgs{});
-  else
-    router_kernel<false, kTokenGroup><<<blocks, kFinishThreads, 0, (cudaStream_t)stream>>>(a, PlanArgs{});
-  INK_CHECK_LAUNCH("ink_router_forward");
-  return kOk;
+  return launch_router(a, nullptr, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------ router, no allocation
@@ -463,20 +591,9 @@ extern "C" int ink_router_plan_forward(const void* x, const void* weight, const 
   if (int rc = check_router(a, workspace_bytes)) return rc;
   PlanArgs p{topk_indices, sources, pointers, experts, counts, rows, start, local, stride, tokens * top_k, capacity};
   if (int rc = check_plan(p)) return rc;
-  INK_REQUIRE(p.routes <= kPlanSmallRoutes, kUnsupportedShape,
-              "router_plan: %d routes exceed the fused limit of %d; call the router and the plan separately",
-              p.routes, kPlanSmallRoutes);
   INK_REQUIRE(capacity >= p.routes || capacity >= tokens, kBadArgument, "router_plan: capacity=%d too small", capacity);
   if (tokens == 0) return kOk;
-  const int blocks = (n_routed + n_shared + kRowsPerBlock - 1) / kRowsPerBlock;
-  INK_PREFER_MAX_SMEM((router_kernel<true, 1>));
-  INK_PREFER_MAX_SMEM((router_kernel<true, kTokenGroup>));
-  if (tokens == 1)
-    router_kernel<true, 1><<<blocks, kFinishThreads, 0, (cudaStream_t)stream>>>(a, p);
-  else
-    router_kernel<true, kTokenGroup><<<blocks, kFinishThreads, 0, (cudaStream_t)stream>>>(a, p);
-  INK_CHECK_LAUNCH("ink_router_plan_forward");
-  return kOk;
+  return launch_router(a, &p, (cudaStream_t)stream);
 }
 
 extern "C" int ink_expert_plan(const int64_t* indices, const int64_t* sources, int64_t* pointers,
@@ -484,20 +601,9 @@ extern "C" int ink_expert_plan(const int64_t* indices, const int64_t* sources, i
                                int stride, int routes, int capacity, ink_stream_t stream) {
   PlanArgs p{indices, sources, pointers, experts, counts, rows, start, local, stride, routes, capacity};
   if (int rc = check_plan(p)) return rc;
-  if (routes <= kPlanSmallRoutes) {
-    INK_PREFER_MAX_SMEM(plan_small_kernel);
-    plan_small_kernel<<<1, kFinishThreads, 0, (cudaStream_t)stream>>>(p);
-    INK_CHECK_LAUNCH("ink_expert_plan");
-    return kOk;
-  }
-  // large plans borrow counts[] as the histogram: pass 1 rewrites it in compacted order
-  // only after every histogram entry has been read into a register.
-  INK_PREFER_MAX_SMEM(plan_count_kernel);
-  INK_PREFER_MAX_SMEM(plan_rows_kernel);
-  plan_count_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(p, p.counts);
-  INK_CHECK_LAUNCH("ink_expert_plan(count)");
-  const int warps = 8;
-  plan_rows_kernel<<<(local + warps - 1) / warps, warps * 32, 0, (cudaStream_t)stream>>>(p);
-  INK_CHECK_LAUNCH("ink_expert_plan(rows)");
+  if (int rc = allow_plan_smem(plan_kernel)) return rc;
+  const int runs = plan_runs(p);
+  plan_kernel<<<1, 1024, sizeof(int) * (size_t)(runs + 1) * local, (cudaStream_t)stream>>>(p, runs);
+  INK_CHECK_LAUNCH("ink_expert_plan");
   return kOk;
 }

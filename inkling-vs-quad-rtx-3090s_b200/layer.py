@@ -18,7 +18,7 @@ import torch
 from torch import nn
 
 from .kernels import (StackDescriptor, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
-                      expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode, router_forward,
+                      expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode,
                       router_plan_forward, router_workspace, stack_supported)
 from .kernels.paired_all_reduce import all_reduce
 
@@ -272,12 +272,8 @@ class FusedMoE(nn.Module):
         ex = self.experts
         args = (flat, self.router_weight, self.router_bias, self.global_scale, self.route_scale, self.top_k,
                 self.n_shared, self.topk_weights[:t], self.topk_indices[:t], self.gammas[:t], self.workspace)
-        if t * self.top_k <= 512:
-            router_plan_forward(*args, ex.sources, ex.pointers, ex.experts, ex.counts, ex.rows, ex.start,
-                                ex.local, ex.stride, ex.capacity)
-        else:
-            router_forward(*args)
-            ex._plan(self.topk_indices[:t])
+        router_plan_forward(*args, ex.sources, ex.pointers, ex.experts, ex.counts, ex.rows, ex.start,
+                            ex.local, ex.stride, ex.capacity)
 
     def forward(self, hidden_states):
         shape = hidden_states.shape

@@ -1,0 +1,124 @@
+"""Several tokens at once: the grouped kernel behind FusedMoE and ResidentExperts, the router and the plan, at the sizes where
+their tiles end."""
+import pytest
+import torch
+
+import cases
+from helpers import BF16, layer_on_device, max_rel
+from oracle import moe as oracle_moe
+
+pytestmark = pytest.mark.gpu
+TOL = 2e-2   # of the largest magnitude, the bar of the other expert kernels: FP16 / digit operands, BF16 intermediates
+
+
+@pytest.fixture(scope="module")
+def ib():
+    import inkling_b200
+
+    return inkling_b200
+
+
+@pytest.fixture(scope="module")
+def device():
+    return torch.device("cuda", 0)
+
+
+def one_allocation_per_kind(banks, device):
+    """Banks the way a loader lays them out: one tensor per kind, the experts views into it."""
+    stacked = {n: torch.stack([banks[e][n].reshape(1).float() if n.endswith("scale2") else banks[e][n] for e in sorted(banks)]).to(device)
+               for n in banks[0]}
+    return {e: {n: t[e] for n, t in stacked.items()} for e in banks}
+
+
+@pytest.mark.parametrize("d,f,experts,tokens", [
+    (1024, 512, 32, 2), (1024, 512, 32, 15), (1024, 512, 32, 17), (1024, 512, 32, 65),   # tiles of 16 and 64 tokens
+    (512, 256, 4, 33), (512, 256, 4, 129),                                                # tall tiles of 32 and 128
+    (512, 768, 4, 31), (256, 256, 16, 9),                                                 # an odd number of chunks; a single one
+])
+def test_a_block_of_several_tokens(ib, device, d, f, experts, tokens):
+    p, banks, x = cases.make_layer(d, f, experts, 2, 3, tokens, seed=tokens, bias="randn")
+    dp = layer_on_device(p, device)
+    module = ib.ResidentExperts(d, f, None, one_allocation_per_kind(banks, device))
+    assert module.bank_maps is not None
+    layer = ib.FusedMoE(dp["router_weight"], dp["router_bias"], dp["global_scale"], p["route_scale"], p["top_k"],
+                        dp["shared_gate"], dp["shared_up"], dp["shared_down"], module, None)
+    for _ in range(2):
+        got = layer(x.to(device).unsqueeze(0))[0].float().cpu()
+    module.check_status()
+    idx, w, gam = layer.topk_indices[:tokens].cpu(), layer.topk_weights[:tokens].cpu(), layer.gammas[:tokens].cpu()
+    assert max_rel(got, oracle_moe.moe_layer_fp32(x, p, banks, idx, w, gam)) <= TOL
+    alone = module(x.to(device), idx.to(device), w.to(device)).float().cpu()
+    assert max_rel(alone, oracle_moe.routed_experts_fp32(x, idx, w, banks)) <= TOL
+
+
+@pytest.mark.parametrize("d,f,experts,tokens", [(256, 128, 8, 2), (256, 128, 8, 70), (384, 128, 2, 131), (512, 256, 5, 17)])
+def test_unquantised_banks_of_several_tokens(ib, device, d, f, experts, tokens):
+    gen = torch.Generator().manual_seed(tokens)
+    banks = {e: dict(gate_up_proj=(torch.randn(2 * f, d, generator=gen) * 0.05).to(BF16), down_proj=(torch.randn(d, f, generator=gen) * 0.05).to(BF16))
+             for e in range(experts)}
+    x = torch.randn(tokens, d, generator=gen).to(BF16)
+    idx = torch.stack([torch.randperm(experts, generator=gen)[:2] for _ in range(tokens)])
+    w = torch.rand(tokens, 2, generator=gen).to(BF16)
+    module = ib.ResidentExperts(d, f, None, one_allocation_per_kind(banks, device), quantized=False)
+    assert module.bank_maps is not None
+    got = module(x.to(device), idx.to(device), w.to(device)).float().cpu()
+    module.check_status()
+    assert max_rel(got, oracle_moe.routed_experts_bf16_fp32(x, idx, w, banks)) <= TOL
+
+
+def test_experts_that_are_not_there_are_skipped_and_reported(ib, device):
+    """A rank that holds the experts 2..5 of 8: routes to the others add nothing; an id beyond the table sets the status."""
+    d, f, tokens = 512, 256, 20
+    p, banks, x = cases.make_layer(d, f, 8, 2, 3, tokens, seed=6, bias="randn")
+    mine = {e: b for e, b in one_allocation_per_kind(banks, device).items() if 2 <= e <= 5}
+    module = ib.ResidentExperts(d, f, None, mine)
+    gen = torch.Generator().manual_seed(1)
+    idx = torch.stack([torch.randperm(6, generator=gen)[:3] for _ in range(tokens)])
+    w = torch.rand(tokens, 3, generator=gen).to(BF16)
+    got = module(x.to(device), idx.to(device), w.to(device)).float().cpu()
+    module.check_status()
+    assert max_rel(got, oracle_moe.routed_experts_fp32(x, idx, w, {e: banks[e] for e in mine})) <= TOL
+    idx[3, 1] = 7
+    module(x.to(device), idx.to(device), w.to(device))
+    with pytest.raises(RuntimeError, match="outside"):
+        module.check_status()
+
+
+@pytest.mark.parametrize("hidden,routed,shared,top_k,tokens", [(4096, 256, 2, 6, 17), (1024, 61, 1, 4, 33), (264, 300, 0, 8, 9), (8, 8, 2, 8, 100)])
+def test_a_token_is_routed_the_same_in_any_company(ib, device, hidden, routed, shared, top_k, tokens):
+    """Bit-exact: the many-token router against the one-launch router on the same tokens in groups of at most eight."""
+    gen = torch.Generator().manual_seed(hidden)
+    weight = (torch.randn(routed + shared, hidden, generator=gen) * 1.3 / hidden ** 0.5).to(BF16).to(device)
+    bias = (torch.randn(routed, generator=gen) * 0.05).to(device)
+    scale = torch.full((1,), 1.25).to(BF16).to(device)
+    x = torch.randn(tokens, hidden, generator=gen).to(BF16).to(device)
+
+    def route(x):
+        t = x.shape[0]
+        out = (torch.empty(t, top_k, dtype=BF16, device=device), torch.empty(t, top_k, dtype=torch.int64, device=device),
+               torch.empty(t, shared, dtype=BF16, device=device))
+        logits = torch.empty(t, routed, dtype=BF16, device=device)
+        ib.kernels.router_forward(x, weight, bias, scale, 8.0, top_k, shared, *out, ib.kernels.router_workspace(t, routed + shared, device),
+                                  routed_logits=logits)
+        return (*out, logits)
+
+    whole = route(x)
+    parts = [route(x[i:i + 8]) for i in range(0, tokens, 8)]
+    for i, got in enumerate(whole):
+        assert torch.equal(got, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.parametrize("local,start,routes", [(256, 0, 1), (3, 5, 31), (256, 0, 33), (40, 100, 1025), (257, 3, 5000), (2000, 0, 20000)])
+def test_the_plan_is_a_stable_sort_at_any_size(ib, device, local, start, routes):
+    gen = torch.Generator().manual_seed(routes)
+    idx = torch.randint(0, start + local + 2, (routes,), generator=gen)   # some on other ranks
+    sources = torch.randint(1, 1 << 40, (local, 2), generator=gen)
+    i32 = dict(dtype=torch.int32, device=device)
+    pointers = torch.zeros((start + local) * 2, dtype=torch.int64, device=device)
+    experts, counts, rows = torch.empty(local, **i32), torch.empty(local, **i32), torch.full((local, routes), -1, **i32)
+    ib.kernels.expert_plan[(1,)](idx.to(device), sources.to(device), None, None, None, None, None, torch.empty(0, **i32), pointers, experts,
+                                 counts, rows, start, local, 0, 2, routes, routes)
+    want = oracle_moe.expert_plan(idx.view(-1, 1), sources, start, local, 2, routes)
+    for got, name in ((experts, "experts"), (counts, "counts"), (rows, "rows")):
+        assert torch.equal(got.cpu(), torch.as_tensor(want[name]).to(torch.int32)), name
+    assert torch.equal(pointers.cpu(), torch.as_tensor(want["pointers"]))
