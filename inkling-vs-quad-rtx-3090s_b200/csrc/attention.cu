@@ -2,6 +2,7 @@
 // layer's K/V cache (a ring of `window` slots in a sliding layer, `slots` positions in a full one).
 #include "../../include/inkling_b200.h"
 #include "common.cuh"
+#include "stream_math.cuh"
 
 namespace ink {
 
@@ -405,6 +406,319 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
   }
 }
 
+// The form for small problems, where all parts are resident at once and latency counts: one block per (64 slots, group of
+// up to eight heads of one key/value head, sequence), on the CUDA cores in FP32. Every thread asks for its share of the key
+// rows and value rows at once (which slots are allowed is known before any score) and keeps them for all heads of the
+// group; with one block per head, as before, eight blocks read the same rows and the join of a head waited for eight times as
+// many of them. The order of all sums is that of one block per head, so the results are the same bits: a decode step of
+// several layers turns any last-bit difference into another routing weight, another rounding, and so on.
+constexpr int kSmallThreads = 256;
+constexpr int kSmallMostBlocks = 148 * 4;
+constexpr int kSmallKeys = 8;                                        // slots a warp scores
+constexpr int kSmallSlots = kSmallThreads / 32 * kSmallKeys;         // slots per block: 64
+
+template <int C, bool CLUSTER>
+__global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(AttnArgs a) {
+  constexpr int kWords = C / 2;                          // 32-bit words of a row = channel pairs
+  constexpr int kPerLane = (kWords + 31) / 32;           // words of a key row per lane
+  constexpr int kParts = kSmallThreads / kWords;         // threads per channel pair in the value pass
+  constexpr int kValues = kSmallSlots / kParts;          // value rows per thread
+  static_assert(kSmallThreads % kWords == 0 && kSmallSlots % kParts == 0, "head_dim does not tile the block");
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  float2* s_part = reinterpret_cast<float2*>(s_raw);                                // [heads][parts][pairs]
+  float* s_q = reinterpret_cast<float*>(s_part + kAttnHeads * kSmallThreads);       // [heads][C]
+  float* s_scores = s_q + kAttnHeads * C;                                           // [heads][64]: biases, scores, exponentials
+  float* s_sum = s_scores + kAttnHeads * kSmallSlots;                               // [heads][parts]
+  float* s_block = s_sum + kAttnHeads * kParts;                                     // [heads][C + 2]: this block's sums, for its cluster
+  uint16_t* s_r = reinterpret_cast<uint16_t*>(s_block + kAttnHeads * (C + 2));      // [heads][d_rel]
+  __shared__ float s_top[kAttnHeads];
+  __shared__ bool s_last;
+  const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
+  const int kv_head = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
+  const int head0 = kv_head * group + chunk * kAttnHeads, n_heads = min(kAttnHeads, group - chunk * kAttnHeads);
+  const int slot_base = split * kSmallSlots;
+  const size_t row0 = ((size_t)b * a.kv_heads + kv_head) * a.slots;
+  const uint16_t* keys = a.k + row0 * C;
+  const uint16_t* values = a.v + row0 * C;
+  const uint16_t* fresh_k = a.new_k ? a.new_k + ((size_t)b * a.kv_heads + kv_head) * C : nullptr;
+  const uint16_t* fresh_v = a.new_k ? a.new_v + ((size_t)b * a.kv_heads + kv_head) * C : nullptr;
+  const int pair = tid % kWords, part = tid / kWords;   // value pass: this thread's channel pair, its slots part, part + kParts, ...
+  // All rows of the block are asked for before the position is known (a short cache is mostly in use); what turns out not
+  // to be allowed is dropped below. In a long one that would read far beyond the position: there the position comes first.
+  constexpr bool kEarly = CLUSTER;
+  uint32_t kw[kSmallKeys][kPerLane], vw[kValues];
+  if (kEarly) {
+#pragma unroll
+    for (int j = 0; j < kSmallKeys; ++j) {
+      const int slot = slot_base + warp * kSmallKeys + j;
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(keys + (size_t)slot * C);
+#pragma unroll
+      for (int i = 0; i < kPerLane; ++i) kw[j][i] = (slot < a.slots && i * 32 + lane < kWords) ? __ldcg(row + i * 32 + lane) : 0u;
+    }
+#pragma unroll
+    for (int n = 0; n < kValues; ++n) {
+      const int slot = slot_base + part + n * kParts;
+      vw[n] = slot < a.slots ? __ldcg(reinterpret_cast<const uint32_t*>(values + (size_t)slot * C) + pair) : 0u;
+    }
+  }
+  const int position = (int)*a.position;
+  const int reach = position - (int)(a.pad_counts ? a.pad_counts[b] : 0);
+  const int ring_position = a.window ? position % a.window : 0;
+  auto distance_of = [&](int slot) -> int {
+    if (!a.window) return position - slot;
+    const int d = ring_position - (slot < a.window ? slot : slot % a.window);
+    return d < 0 ? d + a.window : d;
+  };
+  auto allowed_at = [&](int slot) -> bool {
+    const int d = distance_of(slot);
+    return slot < a.slots && d >= 0 && d <= reach;
+  };
+  // parts beyond the position have nothing to add (in a full layer; a ring's slots beyond it are masked one by one)
+  const int active = a.window || position + 1 >= a.slots ? a.splits : position / kSmallSlots + 1;
+  if (!CLUSTER && split >= active) return;
+  const int fresh_slot = a.new_k ? (a.window ? ring_position : position) : -1;
+  const bool fresh_here = fresh_slot >= slot_base && fresh_slot < slot_base + kSmallSlots && fresh_slot < a.slots;
+  bool k_allowed[kSmallKeys];
+#pragma unroll
+  for (int j = 0; j < kSmallKeys; ++j) {
+    const int slot = slot_base + warp * kSmallKeys + j;
+    k_allowed[j] = allowed_at(slot);
+    if (!kEarly || (fresh_here && slot == fresh_slot)) {
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(slot == fresh_slot ? fresh_k : keys + (size_t)slot * C);
+#pragma unroll
+      for (int i = 0; i < kPerLane; ++i) kw[j][i] = (k_allowed[j] && i * 32 + lane < kWords) ? __ldcg(row + i * 32 + lane) : 0u;
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < kValues; ++n) {
+    const int slot = slot_base + part + n * kParts;
+    const bool ok = allowed_at(slot);   // (a slot that is not allowed may hold anything: it does not count)
+    if (!kEarly || (fresh_here && slot == fresh_slot))
+      vw[n] = ok ? __ldcg(reinterpret_cast<const uint32_t*>(slot == fresh_slot ? fresh_v : values + (size_t)slot * C) + pair) : 0u;
+    else if (!ok) vw[n] = 0u;
+  }
+  if (a.new_k && chunk == 0 && fresh_here && tid < kWords) {
+    reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_k) + tid);
+    reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_v) + tid);
+  }
+  const bool scaled = a.window == 0 && a.n_floor > 0;
+  float tau = 1.f;
+  if (scaled) tau = 1.f + a.alpha * logf(fmaxf((float)(position + 1) / (float)a.n_floor, 1.f));
+  for (int i = tid; i < n_heads * C; i += kSmallThreads) {
+    const float x = bf16_to_f32(a.q[((size_t)b * a.heads + head0) * C + i]);
+    s_q[i] = scaled ? round_bf16(x * tau) : x;
+  }
+  for (int i = tid; i < n_heads * a.d_rel; i += kSmallThreads) s_r[i] = a.r[((size_t)b * a.heads + head0) * a.d_rel + i];
+  __syncthreads();
+  // relative bias of this block's slots: (r @ proj)[distance], a BF16 matmul (FP32 sum, rounded once)
+  {
+    const int slot = slot_base + tid % kSmallSlots, d = distance_of(slot);
+    constexpr int kStep = kSmallThreads / kSmallSlots, kMine = kAttnHeads / kStep;   // heads h0, h0 + 4
+    const int h0 = tid / kSmallSlots;
+    float sum[kMine];
+#pragma unroll
+    for (int n = 0; n < kMine; ++n) sum[n] = 0.f;
+    const bool rel = slot < a.slots && d >= 0 && d < a.extent;
+    if (rel) {
+#pragma unroll 8
+      for (int j = 0; j < a.d_rel; ++j) {
+        const float p = bf16_to_f32(__ldg(a.proj + (size_t)j * a.extent + d));
+#pragma unroll
+        for (int n = 0; n < kMine; ++n)
+          if (h0 + n * kStep < n_heads) sum[n] = fmaf(bf16_to_f32(s_r[(h0 + n * kStep) * a.d_rel + j]), p, sum[n]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < kMine; ++n) {
+      float bias = 0.f;
+      if (rel) {
+        bias = round_bf16(sum[n]);
+        if (scaled) bias = round_bf16(bias * tau);
+      }
+      s_scores[(h0 + n * kStep) * kSmallSlots + tid % kSmallSlots] = bias;
+    }
+  }
+  __syncthreads();
+  // ---- scores: warp w holds the key rows of the slots w * 8 .. w * 8 + 7 of the block
+  bool mine_allowed = false;   // of the slot this lane ends up with
+  const int mine = reduced_row<kSmallKeys>(lane);
+#pragma unroll
+  for (int j = 0; j < kSmallKeys; ++j) mine_allowed = j == mine ? k_allowed[j] : mine_allowed;
+#pragma unroll 4
+  for (int h = 0; h < n_heads; ++h) {
+    float dot[kSmallKeys];
+    float2 q2[kPerLane];
+#pragma unroll
+    for (int i = 0; i < kPerLane; ++i) q2[i] = i * 32 + lane < kWords ? reinterpret_cast<const float2*>(s_q + h * C)[i * 32 + lane] : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < kSmallKeys; ++j) {
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < kPerLane; ++i) {
+        if (i * 32 + lane < kWords) {
+          sum = fmaf(q2[i].x, bf16lo(kw[j][i]), sum);
+          sum = fmaf(q2[i].y, bf16hi(kw[j][i]), sum);
+        }
+      }
+      dot[j] = sum;
+    }
+    const float total = multi_reduce<kSmallKeys>(dot, lane);
+    if (reduced_owner<kSmallKeys>(lane)) {
+      float* at = s_scores + h * kSmallSlots + warp * kSmallKeys + mine;
+      *at = mine_allowed ? total * a.scale + *at : -INFINITY;
+    }
+  }
+  __syncthreads();
+  // ---- a warp per head: the maximum of its 64 scores, then the exponentials
+  for (int h = warp; h < n_heads; h += kSmallThreads / 32) {
+    float* sc = s_scores + h * kSmallSlots;
+    const float s0 = sc[lane], s1 = sc[lane + 32];
+    float top = fmaxf(s0, s1);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    sc[lane] = (s0 == -INFINITY) ? 0.f : __expf(s0 - top);
+    sc[lane + 32] = (s1 == -INFINITY) ? 0.f : __expf(s1 - top);
+    if (lane == 0) s_top[h] = top;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int h = 0; h < n_heads; ++h) {
+    float acc0 = 0.f, acc1 = 0.f, sum = 0.f;
+#pragma unroll
+    for (int n = 0; n < kValues; ++n) {
+      const float p = s_scores[h * kSmallSlots + part + n * kParts];
+      acc0 = fmaf(p, bf16lo(vw[n]), acc0);
+      acc1 = fmaf(p, bf16hi(vw[n]), acc1);
+      sum += p;
+    }
+    s_part[h * kSmallThreads + tid] = make_float2(acc0, acc1);
+    if (pair == 0) s_sum[h * kParts + part] = sum;
+  }
+  __syncthreads();
+  const int stride = kAttnPartial + C;
+  for (int i = tid; i < n_heads * kWords; i += kSmallThreads) {
+    const int h = i / kWords, w = i % kWords;
+    float o0 = 0.f, o1 = 0.f, total = 0.f;
+#pragma unroll
+    for (int p = 0; p < kParts; ++p) {
+      const float2 v = s_part[h * kSmallThreads + p * kWords + w];
+      o0 += v.x;
+      o1 += v.y;
+      total += s_sum[h * kParts + p];
+    }
+    const size_t row = (size_t)b * a.heads + head0 + h;
+    if (a.splits == 1) {
+      const float inv = 1.f / total;
+      reinterpret_cast<uint32_t*>(a.out + row * C)[w] = f32_to_bf16_bits(o0 * inv) | (f32_to_bf16_bits(o1 * inv) << 16);
+    } else {
+      float* to = CLUSTER ? s_block + h * (C + 2) + 2 * w : a.partial + (row * a.splits + split) * stride + kAttnPartial + 2 * w;
+      *reinterpret_cast<float2*>(to) = make_float2(o0, o1);
+      if (w == 0) *reinterpret_cast<float2*>(CLUSTER ? s_block + h * (C + 2) + C : a.partial + (row * a.splits + split) * stride) = make_float2(s_top[h], total);
+    }
+  }
+  if (a.splits == 1) return;
+  // ---- join: part p of the sum takes every kParts-th partial, then the parts are added up
+  if constexpr (CLUSTER) {
+    cluster_sync();
+    for (int i = split * kSmallThreads + tid; i < n_heads * kWords; i += a.splits * kSmallThreads) {
+      const int h = i / kWords, w = i % kWords;
+      float2 head[kAttnCluster], val[kAttnCluster];
+      float all_top = -INFINITY;
+#pragma unroll
+      for (int s = 0; s < kAttnCluster; ++s) {
+        head[s] = s < a.splits ? ld_cluster_float2(s_block + h * (C + 2) + C, s) : make_float2(-INFINITY, 0.f);
+        val[s] = s < a.splits ? ld_cluster_float2(s_block + h * (C + 2) + 2 * w, s) : make_float2(0.f, 0.f);
+        all_top = fmaxf(all_top, head[s].x);
+      }
+      float f0 = 0.f, f1 = 0.f, sum_all = 0.f;
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) {
+        float o0 = 0.f, o1 = 0.f, total = 0.f;
+#pragma unroll
+        for (int s = p; s < kAttnCluster; s += kParts) {
+          if (head[s].x == -INFINITY) continue;
+          const float weight = __expf(head[s].x - all_top);
+          total = fmaf(head[s].y, weight, total);
+          o0 = fmaf(val[s].x, weight, o0);
+          o1 = fmaf(val[s].y, weight, o1);
+        }
+        f0 += o0;
+        f1 += o1;
+        sum_all += total;
+      }
+      const float inv = 1.f / sum_all;
+      reinterpret_cast<uint32_t*>(a.out + ((size_t)b * a.heads + head0 + h) * C)[w] = f32_to_bf16_bits(f0 * inv) | (f32_to_bf16_bits(f1 * inv) << 16);
+    }
+    cluster_sync();   // (a block's sums stay until everybody has read them)
+  } else {
+    __threadfence();   // every writer pushes its own stores out before the block is counted
+    __syncthreads();
+    if (tid == 0) {
+      unsigned* arrived = a.arrived + (size_t)b * gridDim.y + blockIdx.y;
+      s_last = atomicAdd(arrived, 1u) + 1u == (unsigned)active;
+      if (s_last) *arrived = 0u;   // left as found, for the next launch
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // a warp per head: every partial's weight (zero beyond the active ones and for empty ones) and their total
+    float* s_weight = s_q;   // [heads][64]
+    for (int h = warp; h < n_heads; h += kSmallThreads / 32) {
+      const float* base = a.partial + ((size_t)b * a.heads + head0 + h) * a.splits * stride;
+      constexpr int kEach = kAttnMaxSplits / 32;
+      float2 head[kEach];
+      float all_top = -INFINITY;
+#pragma unroll
+      for (int n = 0; n < kEach; ++n) {
+        const int s = n * 32 + lane;
+        head[n] = s < active ? __ldcg(reinterpret_cast<const float2*>(base + (size_t)s * stride)) : make_float2(-INFINITY, 0.f);
+        all_top = fmaxf(all_top, head[n].x);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) all_top = fmaxf(all_top, __shfl_xor_sync(0xffffffffu, all_top, o));
+#pragma unroll
+      for (int n = 0; n < kEach; ++n) {
+        s_weight[h * kAttnMaxSplits + n * 32 + lane] = head[n].x == -INFINITY ? 0.f : __expf(head[n].x - all_top);
+        s_scores[h * kAttnMaxSplits + n * 32 + lane] = head[n].y;
+      }
+    }
+    __syncthreads();
+    constexpr int kMost = kAttnMaxSplits / kParts;   // partials per thread and head
+#pragma unroll 1
+    for (int h = 0; h < n_heads; ++h) {
+      const float* base = a.partial + ((size_t)b * a.heads + head0 + h) * a.splits * stride + kAttnPartial + 2 * pair;
+      float2 v[kMost];
+#pragma unroll
+      for (int n = 0; n < kMost; ++n) v[n] = part + n * kParts < active ? __ldcg(reinterpret_cast<const float2*>(base + (size_t)(part + n * kParts) * stride)) : make_float2(0.f, 0.f);
+      float o0 = 0.f, o1 = 0.f, total = 0.f;
+#pragma unroll
+      for (int n = 0; n < kMost; ++n) {   // (an empty partial's weight is zero and its sums are zero: nothing changes)
+        const float weight = s_weight[h * kAttnMaxSplits + part + n * kParts];
+        total = fmaf(s_scores[h * kAttnMaxSplits + part + n * kParts], weight, total);
+        o0 = fmaf(v[n].x, weight, o0);
+        o1 = fmaf(v[n].y, weight, o1);
+      }
+      s_part[h * kSmallThreads + tid] = make_float2(o0, o1);
+      if (pair == 0) s_sum[h * kParts + part] = total;
+    }
+    __syncthreads();
+    for (int i = tid; i < n_heads * kWords; i += kSmallThreads) {
+      const int h = i / kWords, w = i % kWords;
+      float f0 = 0.f, f1 = 0.f, sum_all = 0.f;
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) {
+        const float2 v = s_part[h * kSmallThreads + p * kWords + w];
+        f0 += v.x;
+        f1 += v.y;
+        sum_all += s_sum[h * kParts + p];
+      }
+      const float inv = 1.f / sum_all;
+      reinterpret_cast<uint32_t*>(a.out + ((size_t)b * a.heads + head0 + h) * C)[w] = f32_to_bf16_bits(f0 * inv) | (f32_to_bf16_bits(f1 * inv) << 16);
+    }
+  }
+}
+
 // the new token's key and value into slot `position` (modulo the window in a sliding layer) of both caches
 __global__ void update_kv_kernel(const uint16_t* __restrict__ new_k, const uint16_t* __restrict__ new_v,
                                  uint16_t* __restrict__ k_cache, uint16_t* __restrict__ v_cache,
@@ -437,14 +751,16 @@ extern "C" size_t ink_decode_attention_workspace_bytes(int batch, int heads, int
 }
 
 template <int C>
-static int launch_decode_attention(const AttnArgs& a, dim3 grid, cudaStream_t stream) {
+static int launch_decode_attention(const AttnArgs& a, bool small, dim3 grid, cudaStream_t stream) {
   const size_t sums = sizeof(float) * kAttnWarps * kAttnHeads * (C + 2), rel = sizeof(uint16_t) * kAttnHeads * ((size_t)(a.d_rel + 15) / 16 * 16);
-  const size_t smem = sums > rel ? sums : rel;
   static_assert(kAttnWarps * (C + 2) > kAttnMaxSplits + 1, "the join's weights fit where the warps' sums were");
-  INK_REQUIRE(smem <= 40 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
+  const size_t smem_small = sizeof(float) * kAttnHeads * (2 * kSmallThreads + C + kSmallSlots + kSmallThreads / (C / 2) + C + 2) + rel;
+  const size_t smem = small ? smem_small : sums > rel ? sums : rel;
+  static_assert(kSmallSlots == kAttnMaxSplits && C >= kAttnMaxSplits, "the join's weights fit where queries and scores were");
+  INK_REQUIRE(rel <= 12 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
-  config.blockDim = dim3(kAttnThreads);
+  config.blockDim = dim3(small ? kSmallThreads : kAttnThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute attribute;
@@ -454,8 +770,10 @@ static int launch_decode_attention(const AttnArgs& a, dim3 grid, cudaStream_t st
   config.attrs = &attribute;
   const bool cluster = a.splits > 1 && a.splits <= kAttnCluster;
   config.numAttrs = cluster ? 1 : 0;
-  const cudaError_t e = cluster ? cudaLaunchKernelEx(&config, decode_attention_kernel<C, true>, a)
-                                : cudaLaunchKernelEx(&config, decode_attention_kernel<C, false>, a);
+  void (*kernel)(AttnArgs) = small ? (cluster ? decode_attention_small_kernel<C, true> : decode_attention_small_kernel<C, false>)
+                                   : (cluster ? decode_attention_kernel<C, true> : decode_attention_kernel<C, false>);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, a);
   INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "decode_attention: launch failed: %s", cudaGetErrorString(e));
   return kOk;
 }
@@ -483,22 +801,26 @@ extern "C" int ink_decode_attention(const void* q, const void* r, const void* pr
                   (need == 0 || aligned16(workspace)),
               kMisaligned, "decode_attention: buffers must be 16-byte aligned");
   if (batch == 0) return kOk;
-  // Parts of the cache: two waves of blocks where there is that much to read (three of four warps fit on an SM; two, so that
-  // shorter sequences even out). Short caches are cut no finer than one step per warp while the parts fit a cluster, and no
-  // finer than two steps beyond, where each further part lengthens the join.
   const int pairs = batch * kv_heads * chunks, whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
-  const int short_most = whole <= kAttnCluster ? whole : whole / 2 > kAttnCluster ? whole / 2 : kAttnCluster;
-  const int most = short_most < attention_max_splits(slots) ? short_most : attention_max_splits(slots);
-  const int wanted = (kAttnWaveBlocks * 2 + pairs - 1) / pairs;
-  const int splits = wanted < 1 ? 1 : wanted < most ? wanted : most;
+  // Where all 64-slot parts are resident at once the small form takes them. Else the number of parts that takes the fewest
+  // rounds of (steps a warp makes + what a block costs beside, about four steps' time), over the blocks resident at once.
+  const bool small = whole <= kAttnMaxSplits && (long long)whole * pairs <= kSmallMostBlocks;
+  int splits = whole, best = 0x7fffffff;
+  for (int n = 1, most = attention_max_splits(slots); n <= most && !small; ++n) {
+    const long long rounds = ((long long)pairs * n + kAttnWaveBlocks - 1) / kAttnWaveBlocks, cost = rounds * (4 + (whole + n - 1) / n);
+    if (cost <= best) {   // (of equals the finer: sequences may be shorter than the cache)
+      best = (int)cost;
+      splits = n;
+    }
+  }
   AttnArgs a{(const uint16_t*)q, (const uint16_t*)r, (const uint16_t*)proj, (const uint16_t*)k_cache, (const uint16_t*)v_cache,
              position, pad_counts, (const uint16_t*)new_k, (const uint16_t*)new_v, (uint16_t*)k_cache, (uint16_t*)v_cache,
              (float*)((char*)workspace + attention_counter_bytes(batch, heads)), (unsigned*)workspace, (uint16_t*)out, heads, kv_heads,
              d_rel, rel_extent, slots, window, n_floor, splits, alpha, scale};
   const dim3 grid((unsigned)splits, (unsigned)(kv_heads * chunks), (unsigned)batch);
-  if (head_dim == 64) return launch_decode_attention<64>(a, grid, (cudaStream_t)stream);
-  if (head_dim == 128) return launch_decode_attention<128>(a, grid, (cudaStream_t)stream);
-  return launch_decode_attention<256>(a, grid, (cudaStream_t)stream);
+  if (head_dim == 64) return launch_decode_attention<64>(a, small, grid, (cudaStream_t)stream);
+  if (head_dim == 128) return launch_decode_attention<128>(a, small, grid, (cudaStream_t)stream);
+  return launch_decode_attention<256>(a, small, grid, (cudaStream_t)stream);
 }
 
 extern "C" int ink_update_kv(const void* new_k, const void* new_v, void* k_cache, void* v_cache, const int64_t* position,
