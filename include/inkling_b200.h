@@ -308,7 +308,8 @@ int ink_moe_grouped(const void* x, const int64_t* indices, const void* weights, 
  *  x            BF16 [hidden]: input of the first block (x, residual_io, normed_out, partial_out and every
  *               layer's norm_weight are read and written 16 bytes at a time: 16-byte aligned)
  *  flags        bit 0 = glue, bit 1 = every layer carries bank_maps (run the routed experts on the tensor cores)
- *  glue = 0     n_layers must be 1; partial_out FP32 [hidden] receives the block's output
+ *  glue = 0     n_layers must be 1; partial_out FP32 [hidden] receives the block's output, and normed_out, if not NULL, the
+ *               same rounded to BF16
  *  glue = 1     residual_io BF16 [hidden] is the residual stream (updated in place),
  *               normed_out BF16 [hidden] the normalised output after the last block,
  *               partial_out the last block's FP32 output

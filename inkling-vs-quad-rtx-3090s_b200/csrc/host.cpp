@@ -1,0 +1,255 @@
+// Native host side of the eager calls: argument checks, output and scratch allocation and the launches of one call, without
+// the interpreter in between. A small decode call occupies the GPU for ten to twenty microseconds; the same steps in Python
+// (a dozen attribute reads, checks and conversions per launch) took 25 to 120, so the calls were bound by the host.
+// The functions take positional arguments only and are called by the package's own Python layer.
+#include <Python.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/torch.h>
+
+#include <map>
+#include <mutex>
+#include <string>
+#include <tuple>
+
+#include "../../include/inkling_b200.h"
+
+namespace {
+
+struct Failure {
+  std::string what;
+};
+[[noreturn]] void fail(const std::string& what) { throw Failure{what}; }
+void check(int code) {
+  if (code != 0) fail("inkling_b200: " + std::string(ink_last_error()) + " (code " + std::to_string(code) + ")");
+}
+
+const at::Tensor& tensor_at(PyObject* const* args, Py_ssize_t i) {
+  if (!THPVariable_Check(args[i])) fail("argument " + std::to_string(i) + " is not a tensor");
+  return THPVariable_Unpack(args[i]);
+}
+bool given(PyObject* const* args, Py_ssize_t i) { return args[i] != Py_None; }
+long long int_at(PyObject* const* args, Py_ssize_t i) {
+  const long long v = PyLong_AsLongLong(args[i]);
+  if (v == -1 && PyErr_Occurred()) throw Failure{""};
+  return v;
+}
+double float_at(PyObject* const* args, Py_ssize_t i) {
+  const double v = PyFloat_AsDouble(args[i]);
+  if (v == -1.0 && PyErr_Occurred()) throw Failure{""};
+  return v;
+}
+void require(bool ok, const char* what) {
+  if (!ok) fail(what);
+}
+// a contiguous BF16 tensor on the GPU, its data on a 16-byte boundary
+at::Tensor bf16_rows(const at::Tensor& t, const char* what) {
+  require(t.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+  require(t.scalar_type() == at::kBFloat16, what);
+  at::Tensor c = t.is_contiguous() ? t : t.contiguous();
+  return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
+}
+at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
+  return at::empty(sizes, at::TensorOptions().dtype(type).device(device));
+}
+
+// ------------------------------------------------------------------------------------------------ attention
+// The join's workspace starts with counters that are zero between launches, so it is made once for each (device, stream,
+// size) and kept; calls on different streams do not share one.
+at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, size_t bytes) {
+  static std::mutex mutex;
+  static auto* kept = new std::map<std::tuple<int, cudaStream_t, size_t>, at::Tensor>();   // (not destroyed at exit: the CUDA context may be gone)
+  const std::lock_guard<std::mutex> lock(mutex);
+  at::Tensor& t = (*kept)[{device.index(), stream, bytes}];
+  if (!t.defined()) t = at::zeros({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(device));
+  return t;
+}
+
+// (query, relative_states, proj, k_cache, v_cache, position, pad_counts, window, n_floor, alpha, scale, out, new_key, new_value)
+PyObject* decode_attention(PyObject* const* args) {
+  const at::Tensor &query = tensor_at(args, 0), &proj = tensor_at(args, 2), &k = tensor_at(args, 3), &v = tensor_at(args, 4), &position = tensor_at(args, 5);
+  require(k.is_cuda() && v.is_cuda() && proj.is_cuda() && position.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+  require(query.dim() >= 3 && k.dim() == 4 && proj.dim() == 2, "decode_attention: query [bs, h, (1,) c], caches [bs, hk, slots, c], proj [d_rel, extent]");
+  const int64_t bs = query.size(0), h = query.size(1), c = query.size(-1), hk = k.size(1), slots = k.size(2), d_rel = proj.size(0);
+  const at::Tensor q = bf16_rows(query, "decode_attention: BF16 query");
+  const at::Tensor& states = tensor_at(args, 1);
+  require(states.is_cuda() && states.scalar_type() == at::kBFloat16, "decode_attention: BF16 relative states on the GPU");
+  const at::Tensor r = states.is_contiguous() ? states : states.contiguous();
+  require(q.numel() == bs * h * c && r.numel() == bs * h * d_rel, "decode_attention: one query and one relative state per sequence and head");
+  require(proj.is_contiguous() && k.is_contiguous() && v.is_contiguous() && k.sizes() == v.sizes(), "decode_attention: contiguous proj and caches of one shape");
+  require(proj.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16, "decode_attention: BF16 proj and caches");
+  require(k.size(0) == bs && k.size(3) == c, "decode_attention: caches of the query's batch and head width");
+  require(position.scalar_type() == at::kLong, "decode_attention: int64 position");
+  const void* pads = nullptr;
+  if (given(args, 6)) {
+    const at::Tensor& p = tensor_at(args, 6);
+    require(p.is_cuda() && p.scalar_type() == at::kLong && p.numel() == bs && p.is_contiguous(), "decode_attention: int64 pad_counts [bs]");
+    pads = p.data_ptr();
+  }
+  at::Tensor new_k, new_v;
+  if (given(args, 12)) {
+    require(given(args, 13), "decode_attention: new_key and new_value come together");
+    new_k = bf16_rows(tensor_at(args, 12), "decode_attention: BF16 new_key");
+    new_v = bf16_rows(tensor_at(args, 13), "decode_attention: BF16 new_value");
+    require(new_k.numel() == bs * hk * c && new_v.numel() == bs * hk * c, "decode_attention: one new key and value per sequence and key/value head");
+  }
+  const c10::cuda::CUDAGuard guard(q.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  at::Tensor out;
+  if (given(args, 11)) {
+    out = tensor_at(args, 11);
+    require(out.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+  } else {
+    out = new_tensor({bs, h, 1, c}, at::kBFloat16, q.device());
+  }
+  const size_t need = ink_decode_attention_workspace_bytes((int)bs, (int)h, (int)c, (int)slots);
+  at::Tensor workspace;
+  if (need) workspace = attention_workspace(q.device(), stream, need);
+  check(ink_decode_attention(q.data_ptr(), r.data_ptr(), proj.data_ptr(), k.data_ptr(), v.data_ptr(), (const int64_t*)position.data_ptr(), (const int64_t*)pads,
+                             out.data_ptr(), (int)bs, (int)h, (int)hk, (int)c, (int)d_rel, (int)proj.size(1), (int)slots, (int)int_at(args, 7), (int)int_at(args, 8),
+                             (float)float_at(args, 9), (float)float_at(args, 10), new_k.defined() ? new_k.data_ptr() : nullptr,
+                             new_v.defined() ? new_v.data_ptr() : nullptr, need ? workspace.data_ptr() : nullptr, need, stream));
+  return THPVariable_Wrap(out);
+}
+
+// ------------------------------------------------------------------------------------------------ blocks
+// Addresses and sizes of a module, taken down once (the module keeps the tensors alive and makes a new record when one of
+// them is replaced).
+struct Block {
+  long long v[48];
+};
+enum Field {
+  kHidden, kWidth, kTopK, kShared, kStart, kLocal, kStride, kCapacity, kMaxExpert, kQuantized, kTokens, kRouted,
+  kSources, kPointers, kExperts, kCounts, kRows, kActivated, kDown, kStatus, kBankMaps,
+  kRouterWeight, kRouterBias, kGlobalScale, kSharedMaps, kTopkWeights, kTopkIndices, kGammas, kWorkspace, kWorkspaceBytes, kPartial,
+  kTable, kScratch, kScratchBytes, kStackFlags, kStackStatus, kRouteScaleBits, kFields
+};
+const char* const kFieldNames[kFields] = {
+    "hidden", "width", "top_k", "shared", "start", "local", "stride", "capacity", "max_expert", "quantized", "tokens", "routed",
+    "sources", "pointers", "experts", "counts", "rows", "activated", "down", "status", "bank_maps",
+    "router_weight", "router_bias", "global_scale", "shared_maps", "topk_weights", "topk_indices", "gammas", "workspace", "workspace_bytes", "partial",
+    "table", "scratch", "scratch_bytes", "stack_flags", "stack_status", "route_scale_bits"};
+template <typename T>
+T* at_field(const Block& b, Field f) {
+  return reinterpret_cast<T*>((uintptr_t)b.v[f]);
+}
+
+PyObject* make_block(PyObject* const* args) {
+  auto* block = new Block();
+  for (int f = 0; f < kFields; ++f) {
+    PyObject* item = PyDict_GetItemString(args[0], kFieldNames[f]);
+    if (!item) continue;
+    block->v[f] = PyLong_AsLongLong(item);
+    if (block->v[f] == -1 && PyErr_Occurred()) {
+      delete block;
+      throw Failure{""};
+    }
+  }
+  return PyCapsule_New(block, "inkling_block", [](PyObject* c) { delete (Block*)PyCapsule_GetPointer(c, "inkling_block"); });
+}
+const Block& block_at(PyObject* const* args) {
+  auto* block = (const Block*)PyCapsule_GetPointer(args[0], "inkling_block");
+  if (!block) throw Failure{""};
+  return *block;
+}
+struct Rows {   // the block's input as [tokens, hidden]
+  at::Tensor x;
+  int tokens;
+};
+Rows rows_of(const Block& b, const at::Tensor& t) {
+  require(t.dim() >= 1 && t.size(-1) == b.v[kHidden], "input of another width than the block's");
+  Rows r{bf16_rows(t, "BF16 input expected"), 0};
+  r.tokens = (int)(t.numel() / b.v[kHidden]);
+  return r;
+}
+
+void grouped(const Block& b, const Rows& r, const int64_t* indices, const void* weights, float* partial, void* out, int n_shared, cudaStream_t stream) {
+  const int routes = r.tokens * (int)b.v[kTopK], groups = routes < b.v[kLocal] ? routes : (int)b.v[kLocal];
+  const size_t need = ink_moe_grouped_scratch_bytes(r.tokens, (int)b.v[kTopK], n_shared, (int)b.v[kHidden], (int)b.v[kWidth], groups, (int)b.v[kQuantized]);
+  const at::Tensor scratch = new_tensor({(int64_t)need}, at::kByte, r.x.device());   // (of this stream, or of the graph being captured)
+  check(ink_moe_grouped(r.x.data_ptr(), indices, weights, at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kRows),
+                        at_field<int32_t>(b, kCounts), at_field<void>(b, kBankMaps), n_shared ? at_field<void>(b, kSharedMaps) : nullptr,
+                        n_shared ? at_field<void>(b, kGammas) : nullptr, at_field<void>(b, kActivated), at_field<void>(b, kDown), partial, out, r.tokens,
+                        (int)b.v[kTopK], n_shared, (int)b.v[kHidden], (int)b.v[kWidth], groups, (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kCapacity],
+                        (int)b.v[kMaxExpert], (int)b.v[kQuantized], scratch.data_ptr(), need, at_field<int32_t>(b, kStatus), stream));
+}
+
+// (block, x, want_partial) -> BF16 like x; with want_partial the FP32 output goes to the block's own buffer, None is returned
+PyObject* run_block(PyObject* const* args) {
+  const Block& b = block_at(args);
+  const at::Tensor& input = tensor_at(args, 1);
+  const Rows r = rows_of(b, input);
+  require(r.tokens <= b.v[kTokens], "more tokens than the block's buffers hold");
+  const bool want_partial = args[2] == Py_True;
+  const c10::cuda::CUDAGuard guard(r.x.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();
+  at::Tensor out;
+  if (!want_partial) out = new_tensor(input.sizes(), at::kBFloat16, r.x.device());
+  if (r.tokens == 1 && b.v[kTable]) {
+    check(ink_moe_stack_decode(at_field<void>(b, kTable), 1, r.x.data_ptr(), nullptr, want_partial ? nullptr : out.data_ptr(), at_field<float>(b, kPartial),
+                               (int)b.v[kStackFlags], 1e-6f, (int)b.v[kHidden], (int)b.v[kWidth], (int)b.v[kRouted], (int)b.v[kShared], (int)b.v[kTopK],
+                               at_field<void>(b, kScratch), (size_t)b.v[kScratchBytes], at_field<int32_t>(b, kStackStatus), stream));
+  } else if (r.tokens > 0) {
+    float route_scale;
+    const uint32_t bits = (uint32_t)b.v[kRouteScaleBits];
+    memcpy(&route_scale, &bits, sizeof(route_scale));
+    check(ink_router_plan_forward(r.x.data_ptr(), at_field<void>(b, kRouterWeight), at_field<float>(b, kRouterBias), at_field<void>(b, kGlobalScale), route_scale,
+                                  r.tokens, (int)b.v[kHidden], (int)b.v[kRouted], (int)b.v[kShared], (int)b.v[kTopK], nullptr, at_field<void>(b, kTopkWeights),
+                                  at_field<int64_t>(b, kTopkIndices), at_field<void>(b, kGammas), at_field<void>(b, kWorkspace), (size_t)b.v[kWorkspaceBytes],
+                                  at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kCounts),
+                                  at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], (int)b.v[kCapacity], stream));
+    grouped(b, r, at_field<int64_t>(b, kTopkIndices), at_field<void>(b, kTopkWeights), want_partial ? at_field<float>(b, kPartial) : nullptr,
+            want_partial ? nullptr : out.data_ptr(), (int)b.v[kShared], stream);
+  }
+  if (want_partial) Py_RETURN_NONE;
+  return THPVariable_Wrap(out);
+}
+
+// (block, x, indices, weights) -> BF16 like x: the routed experts alone, plan and projections
+PyObject* run_experts(PyObject* const* args) {
+  const Block& b = block_at(args);
+  const at::Tensor& input = tensor_at(args, 1);
+  const Rows r = rows_of(b, input);
+  const at::Tensor &i = tensor_at(args, 2), weights = bf16_rows(tensor_at(args, 3), "BF16 router weights expected");
+  require(i.is_cuda() && i.scalar_type() == at::kLong && i.numel() == r.tokens * b.v[kTopK] && weights.numel() == i.numel(), "int64 indices and BF16 weights [tokens, top_k]");
+  const at::Tensor indices = i.is_contiguous() ? i : i.contiguous();
+  const int routes = (int)indices.numel();
+  require(routes <= b.v[kCapacity], "more routes than the module's buffers hold");
+  const c10::cuda::CUDAGuard guard(r.x.device());
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();
+  const at::Tensor out = new_tensor(input.sizes(), at::kBFloat16, r.x.device());
+  check(ink_expert_plan((const int64_t*)indices.data_ptr(), at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts),
+                        at_field<int32_t>(b, kCounts), at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], routes,
+                        (int)b.v[kCapacity], stream));
+  grouped(b, r, (const int64_t*)indices.data_ptr(), weights.data_ptr(), nullptr, out.data_ptr(), 0, stream);
+  return THPVariable_Wrap(out);
+}
+
+template <PyObject* (*F)(PyObject* const*), Py_ssize_t N>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != N) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", N, n);
+    return nullptr;
+  }
+  try {
+    return F(args);
+  } catch (const Failure& f) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, f.what.c_str());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+
+PyMethodDef kMethods[] = {
+    {"decode_attention", (PyCFunction)(void*)&entry<decode_attention, 14>, METH_FASTCALL, nullptr},
+    {"make_block", (PyCFunction)(void*)&entry<make_block, 1>, METH_FASTCALL, nullptr},
+    {"run_block", (PyCFunction)(void*)&entry<run_block, 3>, METH_FASTCALL, nullptr},
+    {"run_experts", (PyCFunction)(void*)&entry<run_experts, 4>, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "inkling_b200_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_inkling_b200_host() { return PyModule_Create(&kModule); }

@@ -131,7 +131,7 @@ struct StackArgs {
   float eps;
   const uint16_t* x;               // [hidden] BF16 input (already normalised for the first block)
   uint16_t* residual;              // [2][hidden] BF16: slot 0 holds the incoming residual stream (glue mode)
-  uint16_t* normed_out;            // [hidden] BF16 output of the last norm (glue mode)
+  uint16_t* normed_out;            // [hidden] BF16 output of the last norm (glue mode); else the block's output in BF16, or null
   float* partial;                  // [hidden] FP32 output of the (last) block
   unsigned long long* scores;      // scratch [2][experts + n_shared] router words {selection score, BF16 logit, 16-bit tag}
   uint16_t* activated;             // scratch [2][top_k][f]
@@ -1827,7 +1827,9 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         // one block only: each block writes its own rows, summed over the ranks, as they arrive
         for (int row = ct; row < plan.n_g * S::RT; row += kSC * 32) {
           const size_t i = (size_t)plan.g0 * S::RT + row;
-          a.partial[i] = wait_tagged(summed + i, tag, &sh);
+          const float v = wait_tagged(summed + i, tag, &sh);
+          a.partial[i] = v;
+          if (a.normed_out) a.normed_out[i] = (uint16_t)f32_to_bf16_bits(v);
         }
         break;
       }

@@ -14,12 +14,15 @@ a given token count, and a forward issues a fixed sequence of launches.
 """
 from __future__ import annotations
 
+import struct
+
 import torch
 from torch import nn
 
 from .kernels import (StackDescriptor, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
                       expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode,
                       router_plan_forward, router_workspace, stack_supported)
+from .kernels._host import host
 from .kernels.paired_all_reduce import all_reduce
 
 # Up to this many tokens each route runs its own matrix-vector product
@@ -102,6 +105,24 @@ class ResidentExperts(nn.Module):
         self.status = torch.zeros(1, **i32)
         self.capacity = 0
 
+    # What the native calls know of this module is taken down once (`_record`); replacing a tensor it points to, or growing
+    # the buffers, makes a new one.
+    _native = None
+    generation = 0
+
+    def __setattr__(self, name, value):
+        if isinstance(value, torch.Tensor) or name in ("weights", "capacity"):
+            self.__dict__["_native"] = None
+            self.__dict__["generation"] = self.generation + 1
+        super().__setattr__(name, value)
+
+    def record_fields(self) -> dict:
+        at = lambda t: t.data_ptr()  # noqa: E731
+        return dict(hidden=self.hidden_dim, width=self.intermediate_dim, start=self.start, local=self.local, stride=self.stride,
+                    capacity=self.capacity, max_expert=self.max_expert, quantized=int(self.quantized), sources=at(self.sources),
+                    pointers=at(self.pointers), experts=at(self.experts), counts=at(self.counts), rows=at(self.rows),
+                    activated=at(self.activated), down=at(self.down), status=at(self.status), bank_maps=at(self.bank_maps))
+
     @staticmethod
     def _even_spacing(addresses: list[list[int]], sizes: list[int]):
         layout = []
@@ -176,6 +197,14 @@ class ResidentExperts(nn.Module):
             self.max_expert, 256)
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
+        if self.device_mesh is None and self.bank_maps is not None and hidden_states.shape[0] > 1:
+            routes = top_k_index.numel()
+            if routes > self.capacity:
+                self._reserve(routes)
+            top_k = top_k_index.shape[1]
+            if self._native is None or self._native[0] != top_k:
+                self.__dict__["_native"] = (top_k, host().make_block(dict(self.record_fields(), top_k=top_k)))
+            return host().run_experts(self._native[1], hidden_states, top_k_index, top_k_weights)
         final = torch.zeros_like(hidden_states, dtype=torch.float32)
         self._reserve(top_k_index.numel())
         self._plan(top_k_index)
@@ -220,6 +249,51 @@ class FusedMoE(nn.Module):
         self._tokens = 0
         self._fused = None   # one-launch descriptor for a single token, built on first use
         self._maps_of = None
+
+    _native = None   # what the native calls know of this block, and the experts' generation it was taken down at
+
+    def __setattr__(self, name, value):
+        if isinstance(value, (torch.Tensor, StackDescriptor)) or name in ("experts", "top_k", "route_scale", "_fused"):
+            self.__dict__["_native"] = None
+        super().__setattr__(name, value)
+
+    def _record(self):
+        ex = self.experts
+        at = lambda t: t.data_ptr()  # noqa: E731
+        fields = dict(ex.record_fields() if ex.bank_maps is not None else dict(hidden=ex.hidden_dim, width=ex.intermediate_dim),
+                      tokens=self._tokens if ex.bank_maps is not None else 1, routed=self.router_weight.shape[0] - self.n_shared,
+                      shared=self.n_shared, top_k=self.top_k, router_weight=at(self.router_weight), router_bias=at(self.router_bias),
+                      global_scale=at(self.global_scale), topk_weights=at(self.topk_weights), topk_indices=at(self.topk_indices),
+                      gammas=at(self.gammas), workspace=at(self.workspace), workspace_bytes=self.workspace.numel(), partial=at(self.partial),
+                      route_scale_bits=struct.unpack("<I", struct.pack("<f", self.route_scale))[0])
+        if ex.bank_maps is not None and self.n_shared:
+            fields["shared_maps"] = at(self._shared_maps())
+        if self.one_launch_supported():
+            if self._fused is None:
+                self._fused = self._one_launch()
+            f = self._fused
+            fields.update(table=at(f.table), scratch=at(f.scratch), scratch_bytes=f.scratch.numel(), stack_status=at(f.status),
+                          stack_flags=2 if f.bank_maps is not None else 0)
+        return host().make_block(fields)
+
+    def _one_launch(self) -> StackDescriptor:
+        # across ranks the kernel delivers and sums the partials itself: no separate collective
+        ex = self.experts
+        return StackDescriptor([self.block_descriptor()], ex.hidden_dim, ex.intermediate_dim, ex.local, self.n_shared, self.top_k,
+                               self.router_weight.device, group=_group_of(self.device_mesh))
+
+    def _native_for(self, tokens: int):
+        """The record for the native call with this many tokens, or None where the launches are put together here: several
+        ranks, banks that are not evenly spaced, one token without the one-launch kernel."""
+        if self.device_mesh is not None or (tokens == 1 and self.separate_launches):
+            return None
+        ex = self.experts
+        if tokens > self._tokens:
+            self._reserve(tokens)
+        if self._native is None or self._native[0] != ex.generation:
+            record = self._record()
+            self.__dict__["_native"] = (ex.generation, record, self.one_launch_supported(), ex.bank_maps is not None)
+        return self._native[1] if self._native[2 if tokens == 1 else 3] else None
 
     def block_descriptor(self, norm_weight=None) -> dict:
         """This block as the one-launch kernel takes it (addresses of the module's tensors)."""
@@ -277,6 +351,9 @@ class FusedMoE(nn.Module):
 
     def forward(self, hidden_states):
         shape = hidden_states.shape
+        native = self._native_for(hidden_states.numel() // shape[-1])
+        if native is not None:
+            return host().run_block(native, hidden_states, False)
         flat = hidden_states.reshape(-1, shape[-1]).contiguous()
         return self.forward_partial(flat).to(hidden_states.dtype).view(shape)
 
@@ -286,12 +363,13 @@ class FusedMoE(nn.Module):
         t = flat.shape[0]
         self._reserve(t)
         ex = self.experts
+        native = self._native_for(t)
+        if native is not None:
+            host().run_block(native, flat, True)
+            return self.partial[:t]
         if t == 1 and self.one_launch_supported() and not self.separate_launches:
             if self._fused is None:
-                # across ranks the kernel delivers and sums the partials itself: no separate collective
-                self._fused = StackDescriptor([self.block_descriptor()], ex.hidden_dim, ex.intermediate_dim,
-                                              ex.local, self.n_shared, self.top_k, flat.device,
-                                              group=_group_of(self.device_mesh))
+                self._fused = self._one_launch()
             self._fused.decode(flat, self.partial[:1])
             return self.partial[:1]
         self.route(flat)
