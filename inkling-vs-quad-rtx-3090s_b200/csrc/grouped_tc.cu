@@ -10,14 +10,15 @@
 // (Gathering the digit rows in the main kernel, eight tokens a pass, stalled its MMAs at the head of every pass, and every
 // expert's bank was read once per eight of its tokens: 64 tokens of one block 0.42 ms, 1 024 tokens 2.8 ms.)
 //
-// A ring stage is two weight units of 128 rows x 128 bytes (plus their block scales) and the N operand that goes with
-// them. TALL: the units are the two halves of a 256-row tile, so that each fetch of the N operand serves 256 rows -- for
-// prompts, where L2 traffic counts. Else (a few tokens per expert, everything waits for HBM) they are two consecutive
-// chunks of the contraction of a 128-row tile: smaller work items, which even out better over the SMs.
+// A ring stage is a chunk of the contraction (128 bytes of every row) of a weight tile and the N operand that goes with it.
+// TALL: a tile has 256 rows, so that each fetch of the N operand serves as many -- for prompts, where L2 traffic counts.
+// Else (a few tokens per expert, everything waits for HBM) 128 rows and stages half as large: items even out better over
+// the SMs, and less of the ring is held by stages whose scales are on the way to tensor memory or whose MMAs are running.
 //
 // Persistent blocks, one per SM. The shared experts' items (long) are dealt evenly, the routed items by cost in what is
-// left of each block's share. Warp 0 produces (its lanes issue a stage's copies side by side), warp 1 issues the MMAs,
-// warps 2..5 move block scales to tensor memory, warps 6..9 read accumulators and write outputs. The kernel is launched
+// left of each block's share. Two warps produce, a stage each in turn (a copy takes the
+// issuing warp 200 ns whatever its size: with one producer a stage of 18 KB took 1 us and 64 tokens of one block 0.64 ms),
+// one thread issues the MMAs, four warps move block scales to tensor memory, four read accumulators and write outputs. The kernel is launched
 // while its predecessor runs (programmatic dependent launch): until that is done it only streams weights, whose
 // addresses depend on nothing but the plan. Every wait is bounded; one that gives up sets kFlagWaitTimedOut.
 #include "../../include/inkling_b200.h"
@@ -29,14 +30,19 @@
 
 namespace ink {
 
-constexpr int kGgStages = 4;
-constexpr int kGgUnitBytes = kTcUnitBytes;                       // 128 rows x 128 B of codes, 2 KB of block scales: 18 KB
-constexpr int kGgRowsBytes = 18 * 1024;                          // the stage's N operand: up to 16 KB, and its block scales
-constexpr int kGgStageBytes = 2 * kGgUnitBytes + kGgRowsBytes;   // 54 KB
-constexpr int kGgThreads = 320;
+// A stage: one (TALL: two) tiles of 128 rows x 128 B of weights, their block scales, the N operand, its block scales.
+template <bool TALL>
+struct GgStage {
+  static constexpr int kUnits = TALL ? 2 : 1, kCount = TALL ? 4 : 8;
+  static constexpr int kScalesAt = kUnits * kTcCodeBytes, kRowsAt = kScalesAt + kUnits * kTcScaleBytes;
+  static constexpr int kRowScalesAt = kRowsAt + kUnits * 8192, kBytes = kRowScalesAt + kUnits * 1024;   // 54 KB or 27 KB
+  static constexpr int kSf = kUnits * 16 + 16;   // tensor-memory columns of its scales
+};
+constexpr int kGgProducers = 2;   // (eleven warps: three on a scheduler, 168 registers a thread)
+constexpr int kGgThreads = 320 + (kGgProducers - 1) * 32;
 constexpr int kGgMaxGroups = 1024;
-constexpr int kGgSharedBox = 16;                                 // gate and up rows of a shared expert alternate by so many
-constexpr int kGgColD = 0, kGgColSf = 256, kGgSfPerStage = 64;   // tensor memory: accumulators, then each stage's scales
+constexpr int kGgSharedBox = 64;                                 // rows of one copy of a shared expert's gate or up matrix
+constexpr int kGgColD = 0, kGgColSf = 256;                       // tensor memory: accumulators, then each stage's scales
 
 // tokens in a tile
 __host__ __device__ constexpr int gg_tile(bool fp4, bool tall) { return fp4 ? (tall ? 32 : 16) : (tall ? 128 : 64); }
@@ -45,7 +51,7 @@ __host__ __device__ constexpr int gg_pad(bool fp4) { return fp4 ? 2 : 8; }
 
 struct GgArgs {
   // routed experts
-  const unsigned char* maps;    // descriptors of this projection: codes and scales (NVFP4), or one (BF16)
+  const unsigned char* maps;    // descriptors of this projection: codes and scales (NVFP4; `wide`: TALL has 256-row boxes), or one (BF16)
   const int64_t* pointers;      // [(max_expert + 1) * stride]: a zero row is an inactive expert; scale2 is read through it
   const int32_t* experts;       // [groups]
   const int32_t* counts;        // [groups]
@@ -54,7 +60,7 @@ struct GgArgs {
   const unsigned char* image_scales;
   const float* slot_scale;      // [slots] (NVFP4)
   uint16_t* y;                  // BF16 [route][n / 2] (gate/up) or [route][n]
-  int groups, start, capacity, stride, bank, k, n;
+  int groups, start, capacity, stride, bank, k, n, wide;
   // shared experts
   const unsigned char* shared_maps;    // gate and up, or down
   const unsigned char* shared_image;   // [tile][k / 64][tokens of the tile, padded to 8][128 B]; down: the same per expert
@@ -65,14 +71,13 @@ struct GgArgs {
 };
 
 struct GgShared {
-  uint64_t full[kGgStages], empty[kGgStages], sf_full[kGgStages];
+  uint64_t full[8], empty[8], sf_full[8];
   uint64_t d_full[2], d_empty[2];
   uint32_t tmem_base;
   volatile int failed;
 };
 
 __device__ __forceinline__ bool gg_wait(uint64_t* bar, uint32_t parity, GgShared* sh) {
-  if (sh->failed) return false;
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity)) {
@@ -155,8 +160,7 @@ struct GgWalk {
   int count;                     // routes of `group`
 
   __device__ __forceinline__ int stages_of(bool shared) const {
-    const int chunks = a->k / ((FP4 && !shared) ? kTcChunkK : 64);
-    return TALL ? chunks : (chunks + 1) / 2;
+    return a->k / ((FP4 && !shared) ? kTcChunkK : 64);
   }
   // cost of one item with n tokens: its bytes, the streamed weights weighing most
   __device__ static __forceinline__ int tile_cost(int n, int stages) { return stages * (64 + (TALL ? n : 2 * n) / (FP4 ? 1 : 4)); }
@@ -224,17 +228,48 @@ struct GgWalk {
   }
 };
 
-// E2M1 (block-scaled) items use tc_idesc / tc_mma; BF16 x BF16 -> FP32, M = 128:
+// E2M1 (block-scaled) items use tc_idesc; BF16 x BF16 -> FP32, M = 128:
 __device__ __forceinline__ uint32_t gg_idesc_bf16(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24); }
-__device__ __forceinline__ void gg_mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(ad),
-               "l"(bd), "r"(idesc), "r"(accumulate)
-               : "memory");
+// The four MMAs of a 128-byte chunk, from the low words of the operands' descriptors (tc_desc_sw128; the high word is the
+// same for all, a step of 32 bytes adds 2). One block of instructions: the issuing thread is what a stage of few tokens waits
+// for, and with descriptors put together one by one it took 80 (BF16) to 150 (block-scaled) clocks per MMA.
+__device__ __forceinline__ uint32_t gg_desc_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3fffu) | (1u << 16); }
+constexpr uint32_t kGgDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void gg_mma4_bf16(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n"
+      " setp.ne.b32 p, %4, 0;\n setp.eq.b32 q, 0, 0;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n add.s64 a, a, 2;\n add.s64 b, b, 2;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n add.s64 a, a, 2;\n add.s64 b, b, 2;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n add.s64 a, a, 2;\n add.s64 b, b, 2;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, q;\n}\n" ::"r"(d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kGgDescHi)
+      : "memory");
+}
+__device__ __forceinline__ void gg_mma4_fp4(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n .reg .b32 s, t;\n"
+      " setp.ne.b32 p, %4, 0;\n setp.eq.b32 q, 0, 0;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n mov.b32 s, %6;\n mov.b32 t, %7;\n"
+      " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], a, b, %3, [s], [t], p;\n"
+      " add.s64 a, a, 2;\n add.s64 b, b, 2;\n add.s32 s, s, 4;\n add.s32 t, t, 4;\n"
+      " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], a, b, %3, [s], [t], q;\n"
+      " add.s64 a, a, 2;\n add.s64 b, b, 2;\n add.s32 s, s, 4;\n add.s32 t, t, 4;\n"
+      " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], a, b, %3, [s], [t], q;\n"
+      " add.s64 a, a, 2;\n add.s64 b, b, 2;\n add.s32 s, s, 4;\n add.s32 t, t, 4;\n"
+      " tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], a, b, %3, [s], [t], q;\n}\n" ::"r"(d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kGgDescHi), "r"(sfa), "r"(sfb)
+      : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t chosen;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(chosen));
+  return chosen != 0;
 }
 
 template <bool FP4, int PROJ, bool TALL>
 __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __grid_constant__ GgArgs a) {
   using Walk = GgWalk<FP4, TALL>;
+  using St = GgStage<TALL>;
   constexpr int kAccs = TALL ? 1 : 2;            // accumulators in turn: the next item's MMAs run while one is read
   constexpr int kAccCols = TALL ? 256 : 128;     // columns of one (TALL: 128 per half)
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -242,7 +277,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
   GgTables tables;
-  tables.slot0 = reinterpret_cast<int*>(ring + (size_t)kGgStages * kGgStageBytes);
+  tables.slot0 = reinterpret_cast<int*>(ring + (size_t)St::kCount * St::kBytes);
   tables.cost = tables.slot0 + a.groups + 1;
   Walk walk;
   walk.a = &a;
@@ -252,7 +287,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
 
   for (int g = threadIdx.x; g < a.groups; g += kGgThreads) tables.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kGgStages; ++s) {
+    for (int s = 0; s < St::kCount; ++s) {
       mbar_init(&sh.full[s], 1);
       mbar_init(&sh.empty[s], 1);
       mbar_init(&sh.sf_full[s], 4);
@@ -299,135 +334,158 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   }
   const uint32_t tmem = sh.tmem_base;
 
-  if (warp == 0) {
-    // =========================================================== producer: every lane issues one of the stage's copies
-    const int k_routed = FP4 ? kTcChunkK : 64;
+  if (warp == 0 || warp >= 10) {
+    // =========================================================== producers: every lane issues one of the stage's copies
+    const int producer = warp == 0 ? 0 : warp - 9;
     auto rows_bytes = [&](const GgItem& it) -> uint32_t {   // one chunk of the tile's N operand
       return (FP4 && !it.shared) ? (uint32_t)((it.n + 1) / 2 * 2) * 512u : (uint32_t)((it.n + 7) / 8 * 8) * 128u;
     };
-    auto chunks_of = [&](const GgItem& it) -> int { return a.k / (it.shared ? 64 : k_routed); };
-    auto units_of = [&](const GgItem& it, int s) -> int { return TALL ? 2 : min(2, chunks_of(it) - 2 * s); };
-    auto expect = [&](const GgItem& it, int s, int u) {
+    auto expect = [&](const GgItem& it, int u) {
       if (lane == 0) {
-        const int units = units_of(it, s), b_chunks = TALL ? 1 : units;
-        uint32_t bytes = (uint32_t)units * ((FP4 && !it.shared) ? kTcUnitBytes : kTcCodeBytes) + (uint32_t)b_chunks * rows_bytes(it);
-        if (FP4 && !it.shared) bytes += (uint32_t)b_chunks * (uint32_t)((it.n + 1) / 2 * 2) * 64u;
+        uint32_t bytes = St::kUnits * kTcCodeBytes + rows_bytes(it);
+        if (FP4 && !it.shared) bytes += St::kUnits * kTcScaleBytes + rows_bytes(it) / 8u;
         mbar_expect_tx(&sh.full[u], bytes);
       }
       __syncwarp();
     };
     auto issue_weights = [&](const GgItem& it, int s, int u) {
-      unsigned char* dst = ring + (size_t)u * kGgStageBytes;
-      const int units = units_of(it, s);
-      if (PROJ == 0 && it.shared) {
-        // 16 gate rows, 16 up rows, ... : lane = (unit, box)
-        constexpr int kBoxes = kTcRows / kGgSharedBox;
-        const int unit = lane / kBoxes, box = lane % kBoxes;
-        if (unit < units)
-          tc_tma_3d(dst + unit * kGgUnitBytes + box * (kGgSharedBox * 128), a.shared_maps + (box & 1) * 128, (TALL ? s : 2 * s + unit) * 64,
-                    it.m0 / 2 + (TALL ? unit * (kTcRows / 2) : 0) + (box >> 1) * kGgSharedBox, it.group, &sh.full[u]);
-        return;
-      }
-      const int unit = lane & 1, chunk = TALL ? s : 2 * s + unit, row = it.m0 + (TALL ? unit * kTcRows : 0);
-      if (unit >= units) return;
-      const int z = it.shared ? it.group : a.experts[it.group] - a.start;
+      const int unit = lane & 1;
       const unsigned char* map = it.shared ? a.shared_maps : a.maps;
-      if (FP4 && !it.shared) {
-        if (lane < 2) tc_tma_3d(dst + unit * kGgUnitBytes, map, chunk * 128, row, z, &sh.full[u]);
-        else if (lane < 4) tc_tma_3d(dst + unit * kGgUnitBytes + kTcCodeBytes, map + 128, chunk * 16, row, z, &sh.full[u]);
-      } else if (lane < 2) {
-        tc_tma_3d(dst + unit * kGgUnitBytes, map, chunk * 64, row, z, &sh.full[u]);
+      const int z = it.shared ? it.group : a.experts[it.group] - a.start;
+      int x = s * 64, y = it.m0, at = 0;
+      bool mine = false;
+      if (PROJ == 0 && it.shared) {
+        // 64 rows of gate and of up (TALL: twice that)
+        const int half = lane >> 1;
+        mine = lane < 2 * St::kUnits;
+        map += unit * 128;
+        y = it.m0 / 2 + half * kGgSharedBox;
+        at = TALL ? unit * kTcCodeBytes + half * (kTcCodeBytes / 2) : unit * (kTcCodeBytes / 2);
+      } else if (!FP4 || it.shared) {
+        mine = lane < St::kUnits;
+        y += unit * kTcRows;
+        at = unit * kTcCodeBytes;
+      } else if (lane < 2) {   // codes
+        mine = unit == 0 || (TALL && !a.wide);
+        x = s * 128;
+        y += unit * kTcRows;
+        at = unit * kTcCodeBytes;
+      } else if (lane < 4) {   // block scales
+        mine = unit == 0 || (TALL && !a.wide);
+        map += 128;
+        x = s * 16;
+        y += unit * kTcRows;
+        at = St::kScalesAt + unit * kTcScaleBytes;
       }
+      if (mine) tc_tma_3d(ring + (size_t)u * St::kBytes + at, map, x, y, z, &sh.full[u]);
     };
     auto issue_rows = [&](const GgItem& it, int s, int u) {
-      unsigned char* dst = ring + (size_t)u * kGgStageBytes + 2 * kGgUnitBytes;
-      const int c = lane & 1, chunk = TALL ? s : 2 * s + c;
-      if (c >= (TALL ? 1 : units_of(it, s))) return;
-      const uint32_t bytes = rows_bytes(it);
+      const bool fp4 = FP4 && !it.shared;
+      uint32_t bytes = rows_bytes(it);
+      const unsigned char* from;
+      int at = St::kRowsAt;
       if (it.shared) {
-        const int padded = (a.tokens + 7) / 8 * 8, chunks = a.k / 64;
-        const unsigned char* from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2;
-        if (lane < 2) bulk_g2s(dst + c * 8192, from + (size_t)chunk * bytes, bytes, &sh.full[u]);
-        (void)chunks;
-      } else if (FP4) {
-        if (lane < 2) bulk_g2s(dst + c * 8192, a.image + (size_t)it.slot * a.k * 2 + (size_t)chunk * bytes, bytes, &sh.full[u]);
-        else if (lane < 4) bulk_g2s(dst + 16384 + c * 1024, a.image_scales + (size_t)it.slot * (a.k / 4) + (size_t)chunk * (bytes / 8), bytes / 8, &sh.full[u]);
+        const int padded = (a.tokens + 7) / 8 * 8;
+        from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2 + (size_t)s * bytes;
       } else {
-        if (lane < 2) bulk_g2s(dst + c * 8192, a.image + (size_t)it.slot * a.k * 2 + (size_t)chunk * bytes, bytes, &sh.full[u]);
+        from = a.image + (size_t)it.slot * a.k * 2 + (size_t)s * bytes;
       }
+      if (fp4 && lane == 1) {
+        bytes /= 8;
+        from = a.image_scales + (size_t)it.slot * (a.k / 4) + (size_t)s * bytes;
+        at = St::kRowScalesAt;
+      }
+      if (lane < (fp4 ? 2 : 1)) bulk_g2s(ring + (size_t)u * St::kBytes + at, from, bytes, &sh.full[u]);
     };
-    auto stages = [&](const GgItem& it) -> int { return walk.stages_of(it.shared); };
-    // The first stages' weights are asked for before the kernel in front has finished; their N operand after.
-    Walk ahead = walk;
+    // Stage i of the block's sequence is producer i % 2's. The first round's weights are asked for before the kernel in
+    // front has finished; their N operand after.
+    static_assert(St::kCount % kGgProducers == 0, "a ring slot has one producer");
+    constexpr int kFirst = St::kCount / kGgProducers;   // stages of the first round per producer
+    GgItem early_item[kFirst];
+    int early_stage[kFirst], early = 0;
     GgItem it;
-    bool have = ahead.next(it);
-    int s = 0, early = 0;
-    for (; early < kGgStages && have; ++early) {
-      expect(it, s, early);
-      issue_weights(it, s, early);
-      if (++s == stages(it)) {
-        s = 0;
-        have = ahead.next(it);
+    long long first = 0;   // the block's stages before this item
+    bool waited = false;
+    while (walk.next(it)) {
+      const int stages = walk.stages_of(it.shared);
+      int s = (int)((producer - first % kGgProducers + kGgProducers) % kGgProducers);
+      for (; s < stages; s += kGgProducers) {
+        const long long seq = first + s;
+        const int u = (int)(seq % St::kCount);
+        if (early < kFirst) {
+          expect(it, u);
+          issue_weights(it, s, u);
+#pragma unroll
+          for (int i = 0; i < kFirst; ++i) {
+            if (i == early) {
+              early_item[i] = it;
+              early_stage[i] = s;
+            }
+          }
+          ++early;
+          continue;
+        }
+        if (!waited) {
+          pdl_wait();
+          waited = true;
+#pragma unroll
+          for (int i = 0; i < kFirst; ++i) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+        }
+        if (!__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / St::kCount) - 1) & 1u, &sh))) break;
+        expect(it, u);
+        issue_weights(it, s, u);
+        issue_rows(it, s, u);
       }
+      first += stages;
+      if (sh.failed) break;
     }
-    pdl_wait();
-    GgItem late;
-    int ls = 0;
-    bool more = walk.next(late);
-    for (int i = 0; i < early && more; ++i) {
-      issue_rows(late, ls, i);
-      if (++ls == stages(late)) {
-        ls = 0;
-        more = walk.next(late);
-      }
-    }
-    for (long long seq = early; have; ++seq) {
-      const int u = (int)(seq % kGgStages);
-      if (!__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / kGgStages) - 1) & 1u, &sh))) break;
-      expect(it, s, u);
-      issue_weights(it, s, u);
-      issue_rows(it, s, u);
-      if (++s == stages(it)) {
-        s = 0;
-        have = ahead.next(it);
-      }
+    if (!waited) {
+      pdl_wait();
+#pragma unroll
+      for (int i = 0; i < kFirst; ++i)
+        if (i < early) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
     }
   } else if (warp == 1) {
     // =========================================================== MMA issue
-    if (lane == 0) {
-      GgItem it;
-      long long seq = 0;
-      for (int item = 0; walk.next(it) && !sh.failed; ++item) {
-        const bool fp4 = FP4 && !it.shared;
-        const int buf = kAccs == 2 ? item & 1 : 0;
-        const int columns = fp4 ? (it.n + 1) / 2 * 8 : (it.n + 15) / 16 * 16;
-        const uint32_t idesc = fp4 ? tc_idesc(columns) : gg_idesc_bf16(columns);
-        const int chunks = a.k / (fp4 ? kTcChunkK : 64), stages = walk.stages_of(it.shared);
-        if (!gg_wait(&sh.d_empty[buf], (uint32_t)((item / kAccs) & 1) ^ 1u, &sh)) break;   // this accumulator's previous item has been read
+    // The whole warp walks the stages together (operands of the issue instructions are per-warp registers), one lane issues.
+    GgItem it;
+    uint32_t seq = 0;
+    const uint32_t ring_lo = gg_desc_lo(smem_u32(ring));
+    bool ok = true;
+    for (int item = 0; ok && walk.next(it); ++item) {
+      const bool fp4 = FP4 && !it.shared;
+      const int buf = kAccs == 2 ? item & 1 : 0;
+      const int columns = __shfl_sync(0xffffffffu, fp4 ? (it.n + 1) / 2 * 8 : (it.n + 15) / 16 * 16, 0);
+      const uint32_t idesc = fp4 ? tc_idesc(columns) : gg_idesc_bf16(columns);
+      const int stages = walk.stages_of(it.shared);
+      const uint32_t d = tmem + kGgColD + buf * kAccCols;
+      // Shared gate / up: two accumulators side by side. (!TALL: tiles of 64 rows; what the MMA reads as rows 64.. of one lies
+      // behind it in the stage, and its results go to lanes that nobody reads.)
+      const bool pair = PROJ == 0 && it.shared;
+      const int units = pair ? 2 : St::kUnits;
+      const uint32_t unit_lo = (pair && !TALL ? kTcCodeBytes / 2 : kTcCodeBytes) >> 4;
+      ok = gg_wait(&sh.d_empty[buf], (uint32_t)((item / kAccs) & 1) ^ 1u, &sh);   // this accumulator's previous item has been read
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int s = 0; s < stages; ++s, ++seq) {
+        const uint32_t u = seq % St::kCount, parity = (seq / St::kCount) & 1u;
+        ok = FP4 ? gg_wait(&sh.sf_full[u], parity, &sh) : gg_wait(&sh.full[u], parity, &sh);   // (the scales' warps have seen it full)
+        if (FP4) ok = ok && gg_wait(&sh.full[u], parity, &sh);
+        if (!ok) break;
         tc_fence_after();
-        for (int s = 0; s < stages; ++s, ++seq) {
-          const int u = (int)(seq % kGgStages);
-          const uint32_t parity = (uint32_t)(seq / kGgStages) & 1u;
-          if (!gg_wait(&sh.full[u], parity, &sh)) break;
-          if (FP4 && !gg_wait(&sh.sf_full[u], parity, &sh)) break;
-          tc_fence_after();
-          const uint32_t base = smem_u32(ring + (size_t)u * kGgStageBytes), sf = tmem + kGgColSf + u * kGgSfPerStage;
-          const int units = TALL ? 2 : min(2, chunks - 2 * s);
-          for (int unit = 0; unit < units; ++unit) {
-            const uint64_t ad = tc_desc_sw128(base + unit * kGgUnitBytes);
-            const uint64_t bd = tc_desc_sw128(base + 2 * kGgUnitBytes + (TALL ? 0 : unit * 8192));
-            const uint32_t d = tmem + kGgColD + buf * kAccCols + (TALL ? unit * 128 : 0);
-            const bool fresh = s == 0 && (TALL || unit == 0);
+        const uint32_t lo = ring_lo + u * (St::kBytes >> 4), sf = tmem + kGgColSf + u * St::kSf;
+        if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint32_t accumulate = (fresh && k == 0) ? 0u : 1u;
-              if (fp4) tc_mma(d, ad + 2 * k, bd + 2 * k, idesc, accumulate, sf + unit * 16 + k * 4, sf + 32 + (TALL ? 0 : unit * 16) + k * 4);
-              else gg_mma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, accumulate);
-            }
+          for (int unit = 0; unit < 2; ++unit) {
+            if (unit == 1 && units == 1) break;
+            if (fp4) gg_mma4_fp4(d + unit * (kAccCols / 2), lo + unit * unit_lo, lo + (St::kRowsAt >> 4), idesc, s != 0, sf + unit * 16, sf + St::kUnits * 16);
+            else gg_mma4_bf16(d + unit * (kAccCols / 2), lo + unit * unit_lo, lo + (St::kRowsAt >> 4), idesc, s != 0);
           }
           tc_commit(&sh.empty[u]);
+          if (s + 1 == stages) tc_commit(&sh.d_full[buf]);
         }
-        tc_commit(&sh.d_full[buf]);
+        __syncwarp();
       }
     }
   } else if (warp < 6) {
@@ -438,28 +496,28 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       long long seq = 0;
       bool ok = true;
       while (ok && walk.next(it)) {
-        const int chunks = a.k / (it.shared ? 64 : kTcChunkK), stages = walk.stages_of(it.shared);
+        const int stages = walk.stages_of(it.shared);
         for (int s = 0; s < stages; ++s, ++seq) {
-          const int u = (int)(seq % kGgStages);
-          ok = __all_sync(0xffffffffu, gg_wait(&sh.full[u], (uint32_t)(seq / kGgStages) & 1u, &sh));
+          const int u = (int)(seq % St::kCount);
+          ok = __all_sync(0xffffffffu, gg_wait(&sh.full[u], (uint32_t)(seq / St::kCount) & 1u, &sh));
           if (!ok) break;
           if (!it.shared) {
-            const unsigned char* stage = ring + (size_t)u * kGgStageBytes;
-            const int units = TALL ? 2 : min(2, chunks - 2 * s);
-            // a unit's scales lie as 128 rows of 16 bytes; row r belongs to lane r % 32, column r / 32, four bytes a 64-column step
-            auto upload = [&](const unsigned char* sc, int column) {
+            const unsigned char* stage = ring + (size_t)u * St::kBytes;
+            // row r's scales of a unit, 16 bytes, belong to lane r % 32, column r / 32, four bytes a 64-column step
+            auto upload = [&](const unsigned char* sc, bool all, int column) {
               const uint4 r0 = *reinterpret_cast<const uint4*>(sc + lane * 16), r1 = *reinterpret_cast<const uint4*>(sc + (lane + 32) * 16);
               uint4 r2 = make_uint4(0, 0, 0, 0), r3 = r2;
-              if (TALL || column < 32) {
+              if (all) {
                 r2 = *reinterpret_cast<const uint4*>(sc + (lane + 64) * 16);
                 r3 = *reinterpret_cast<const uint4*>(sc + (lane + 96) * 16);
               }
               const uint32_t w[16] = {r0.x, r1.x, r2.x, r3.x, r0.y, r1.y, r2.y, r3.y, r0.z, r1.z, r2.z, r3.z, r0.w, r1.w, r2.w, r3.w};
-              tc_st16(tmem + lane_base + kGgColSf + u * kGgSfPerStage + column, w);
+              tc_st16(tmem + lane_base + kGgColSf + u * St::kSf + column, w);
             };
             tc_fence_after();
-            for (int unit = 0; unit < units; ++unit) upload(stage + unit * kGgUnitBytes + kTcCodeBytes, unit * 16);
-            for (int c = 0; c < (TALL ? 1 : units); ++c) upload(stage + 2 * kGgUnitBytes + 16384 + c * 1024, 32 + c * 16);
+#pragma unroll
+            for (int unit = 0; unit < St::kUnits; ++unit) upload(stage + St::kScalesAt + unit * kTcScaleBytes, true, unit * 16);
+            upload(stage + St::kRowScalesAt, TALL, St::kUnits * 16);
             tc_wait_st();
             tc_fence_before();
           }
@@ -494,56 +552,107 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       const bool ok = __all_sync(0xffffffffu, gg_wait(&sh.d_full[buf], (uint32_t)((item / kAccs) & 1), &sh));
       if (!ok) break;
       tc_fence_after();
+      if (PROJ == 0 && it.shared) {
+        // a lane has a pair's gate in one accumulator and its up in the other
+        const int row = sub * 32 + lane, pair = it.m0 / 2 + row;
+        if (TALL || sub < 2) {
 #pragma unroll 1
-      for (int half = 0; half < (TALL ? 2 : 1); ++half) {
-        const int r = it.m0 + half * kTcRows + sub * 32 + lane;   // this thread's weight row
-#pragma unroll 1
-        for (int chunk = 0; chunk < token_chunks; ++chunk) {
-          if (token_chunks > 1) my_token = token_of(chunk, my_scale);
-          float v[32];
-          tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, v);
-          if (fp4) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = ((v[4 * j] + v[4 * j + 1]) + (v[4 * j + 2] + v[4 * j + 3])) * __shfl_sync(0xffffffffu, my_scale, j);
-          }
-          const int here = min(per_chunk, it.n - chunk * per_chunk);
-          if (PROJ == 0) {
-            // gate and up rows sit in lanes that differ in one bit (routed banks interleave single rows, the shared experts'
-            // boxes sixteen): of two tokens each of the two lanes finishes one
-            const int bit = it.shared ? kGgSharedBox : 1;
-            const bool second = (lane & bit) != 0;
-            const int pair = it.shared ? it.m0 / 2 + half * (kTcRows / 2) + sub * kGgSharedBox + (lane & (kGgSharedBox - 1)) : r >> 1;
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              if (j >= here) break;
-              const float other = __shfl_xor_sync(0xffffffffu, second ? v[j] : v[j + 1], bit);
-              const float gate = second ? other : v[j], up = second ? v[j + 1] : other;
-              const int token = __shfl_sync(0xffffffffu, my_token, second ? j + 1 : j);
-              if (token >= 0 && 2 * pair < a.n) {
-                if (!it.shared) {
-                  a.y[(size_t)token * (a.n / 2) + pair] = (uint16_t)f32_to_bf16_bits(silu_mul(gate, up));
-                } else {
-                  // the reference's BF16 tensor ops: both bmm outputs, silu, the product and the product with gamma round
-                  const float g = round_bf16(gate), u = round_bf16(up);
-                  const float act = round_bf16(round_bf16(g / (1.f + expf(-g))) * u);
-                  const float gamma = bf16_to_f32(a.gammas[(size_t)token * a.n_shared + it.group]);
-                  const int padded = (a.tokens + 7) / 8 * 8, f = a.n / 2, row = token - it.tile * Walk::kSharedTile;
-                  unsigned char* at = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
-                                      (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + row * 128 + ((((pair & 63) >> 3) ^ (row & 7)) << 4) + (pair & 7) * 2;
-                  *reinterpret_cast<uint16_t*>(at) = (uint16_t)f32_to_bf16_bits(act * gamma);
-                }
-              }
-            }
-          } else {
+          for (int chunk = 0; chunk < token_chunks; ++chunk) {
+            float gate[32], up[32];
+            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + chunk * 32, gate);
+            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + kAccCols / 2 + chunk * 32, up);
+            const int here = min(32, it.n - chunk * 32), padded = (a.tokens + 7) / 8 * 8, f = a.n / 2;
+            unsigned char* tile = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
+                                  (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + (pair & 7) * 2;
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
               if (j >= here) break;
-              const int token = __shfl_sync(0xffffffffu, my_token, j);
-              if (r < a.n) {
-                uint16_t* y = it.shared ? a.shared_y + ((size_t)token * a.n_shared + it.group) * a.n : a.y + (size_t)token * a.n;
-                y[r] = (uint16_t)f32_to_bf16_bits(v[j]);
-              }
+              // the reference's BF16 tensor ops: both bmm outputs, silu, the product and the product with gamma round
+              const int at = chunk * 32 + j, token = it.tile * Walk::kSharedTile + at;
+              const float g = round_bf16(gate[j]), u = round_bf16(up[j]);
+              const float act = round_bf16(round_bf16(g / (1.f + expf(-g))) * u);
+              const float gamma = bf16_to_f32(a.gammas[(size_t)token * a.n_shared + it.group]);
+              if (pair < f) *reinterpret_cast<uint16_t*>(tile + at * 128 + ((((pair & 63) >> 3) ^ (at & 7)) << 4)) = (uint16_t)f32_to_bf16_bits(act * gamma);
             }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
+        continue;
+      }
+      // this thread's weight row for the tokens of a chunk (lane j holds token j's route, or number)
+      auto write = [&](auto& v, int half, int chunk, int tokens) {
+        constexpr int kChunk = sizeof(v) / sizeof(float);
+        const int r = it.m0 + half * kTcRows + sub * 32 + lane;
+        const int here = min(kChunk, it.n - chunk * kChunk);
+        if (PROJ == 0) {
+          // gate and up rows alternate, so neighbouring lanes hold a pair: of two tokens each lane finishes one
+          const bool second = (lane & 1) != 0;
+          const int pair = r >> 1;
+#pragma unroll
+          for (int j = 0; j < kChunk; j += 2) {
+            if (j >= here) break;
+            const float other = __shfl_xor_sync(0xffffffffu, second ? v[j] : v[j + 1], 1);
+            const float gate = second ? other : v[j], up = second ? v[j + 1] : other;
+            const int token = __shfl_sync(0xffffffffu, tokens, second ? j + 1 : j);
+            if (token >= 0 && 2 * pair < a.n) a.y[(size_t)token * (a.n / 2) + pair] = (uint16_t)f32_to_bf16_bits(silu_mul(gate, up));
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < kChunk; ++j) {
+            if (j >= here) break;
+            const int token = __shfl_sync(0xffffffffu, tokens, j);
+            uint16_t* y = it.shared ? a.shared_y + ((size_t)token * a.n_shared + it.group) * a.n : a.y + (size_t)token * a.n;
+            if (r < a.n) y[r] = (uint16_t)f32_to_bf16_bits(v[j]);
+          }
+        }
+      };
+      if constexpr (FP4) {
+        if (!it.shared) {
+          // Everything into registers first (four digit columns add up to a token), so that the accumulator is free for the
+          // next item before the outputs are written: with one accumulator (TALL) its MMAs wait for that.
+          constexpr int kHalves = TALL ? 2 : 1, kChunks = gg_tile(true, TALL) / 8;
+          float v[kHalves][kChunks][8];
+#pragma unroll
+          for (int half = 0; half < kHalves; ++half) {
+#pragma unroll
+            for (int chunk = 0; chunk < kChunks; ++chunk) {
+              if (chunk * 8 >= it.n) break;
+              float w[32];
+              tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, w);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[half][chunk][j] = (w[4 * j] + w[4 * j + 1]) + (w[4 * j + 2] + w[4 * j + 3]);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
+#pragma unroll
+          for (int chunk = 0; chunk < kChunks; ++chunk) {
+            if (chunk * 8 >= it.n) break;
+            if (chunk > 0) my_token = token_of(chunk, my_scale);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float scale = __shfl_sync(0xffffffffu, my_scale, j);
+#pragma unroll
+              for (int half = 0; half < kHalves; ++half) v[half][chunk][j] *= scale;
+            }
+#pragma unroll
+            for (int half = 0; half < kHalves; ++half) write(v[half][chunk], half, chunk, my_token);
+          }
+          continue;
+        }
+      }
+      if constexpr (!FP4 || PROJ == 1) {
+#pragma unroll 1
+        for (int half = 0; half < (TALL ? 2 : 1); ++half) {
+#pragma unroll 1
+          for (int chunk = 0; chunk < token_chunks; ++chunk) {
+            const int tokens = token_chunks > 1 ? token_of(chunk, my_scale) : my_token;
+            float v[32];
+            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, v);
+            write(v, half, chunk, tokens);
           }
         }
       }
@@ -570,6 +679,7 @@ struct StageArgs {
   float* slot_scale;
   unsigned char* shared_image;  // the tokens themselves for the shared experts, or null
   int groups, capacity, stride, bank, k, div;   // div: routes per row of x
+  int plan_ready;               // the plan was complete before the kernel in front started
   int tokens, tile, shared_tile;
 };
 
@@ -591,13 +701,19 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) 
   constexpr int kPad = gg_pad(FP4);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   GgTables t{s_tables, s_tables + a.groups + 1};
-  pdl_wait();
-  pdl_trigger();   // the main kernel may read the plan now
+  if (!a.plan_ready) {
+    pdl_wait();
+    pdl_trigger();   // the main kernel may read the plan now
+  }
   for (int g = threadIdx.x; g < a.groups; g += kStageThreads) t.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
   __syncthreads();
   if (warp == 0) gg_scan(t, a.groups, kPad, lane, [](int count) { return count; });
   __syncthreads();
   const int routed = t.cost[a.groups], total = routed + (a.shared_image ? a.tokens : 0);
+  if (a.plan_ready) {
+    pdl_wait();
+    pdl_trigger();
+  }
   for (int i = blockIdx.x; i < total; i += gridDim.x) {
     if (i >= routed) {
       const int token = i - routed, tile = token / a.shared_tile, row = token % a.shared_tile;
@@ -753,7 +869,7 @@ static cudaError_t launch_dependent(void (*kernel)(Args), dim3 grid, int threads
 
 template <bool FP4, int PROJ, bool TALL>
 static int launch_grouped(const GgArgs& a, cudaStream_t stream) {
-  constexpr size_t kRing = (size_t)kGgStages * kGgStageBytes + 1024;
+  constexpr size_t kRing = (size_t)GgStage<TALL>::kCount * GgStage<TALL>::kBytes + 1024;
   constexpr int kMaxDevices = 64;
   static bool configured[kMaxDevices] = {};
   int device = 0;
@@ -812,6 +928,25 @@ extern "C" int ink_encode_shared(void* out_host_384, const void* gate, const voi
   if (rc == kOk) rc = encode_rows(&maps[1], up, 2, stride, n_shared, intermediate, hidden, 64, kGgSharedBox, true);
   if (rc == kOk) rc = encode_rows(&maps[2], down, 2, stride, n_shared, hidden, intermediate, 64, kTcRows, true);
   if (rc == kOk) memcpy(out_host_384, maps, sizeof(maps));
+  return rc;
+}
+
+// The boxes of both forms of the kernel: 128 rows of codes and scales (the 512 bytes of ink_moe_stack_encode_banks), 256 rows.
+extern "C" int ink_encode_grouped_banks(void* out_host_1024, const void* gate_up_codes, uint64_t gate_up_codes_stride, const void* gate_up_scales,
+                                        uint64_t gate_up_scales_stride, const void* down_codes, uint64_t down_codes_stride, const void* down_scales,
+                                        uint64_t down_scales_stride, int experts, int hidden, int intermediate) {
+  INK_REQUIRE(out_host_1024 != nullptr && experts >= 1, kBadArgument, "encode_grouped_banks: null output or no experts");
+  INK_REQUIRE(hidden % kTcChunkK == 0 && intermediate % kTcChunkK == 0, kUnsupportedShape, "encode_grouped_banks: hidden=%d intermediate=%d", hidden, intermediate);
+  CUtensorMap maps[8];
+  int rc = kOk;
+  for (int i = 0; i < 4 && rc == kOk; ++i) {
+    const int rows = kTcRows << (i >> 1);   // forms; then projections
+    const bool down = i & 1;
+    const int n = down ? hidden : 2 * intermediate, k = down ? intermediate : hidden;
+    rc = encode_rows(&maps[2 * i], down ? down_codes : gate_up_codes, 1, down ? down_codes_stride : gate_up_codes_stride, experts, n, k / 2, 128, rows, true);
+    if (rc == kOk) rc = encode_rows(&maps[2 * i + 1], down ? down_scales : gate_up_scales, 1, down ? down_scales_stride : gate_up_scales_stride, experts, n, k / 16, 16, rows, false);
+  }
+  if (rc == kOk) memcpy(out_host_1024, maps, sizeof(maps));
   return rc;
 }
 
@@ -883,7 +1018,8 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   if (int rc = launch_stage(fp4, st, routes + (n_shared ? tokens : 0), s)) return rc;
 
   GgArgs g = {};
-  g.maps = (const unsigned char*)bank_maps;
+  g.maps = (const unsigned char*)bank_maps + (fp4 && tall ? 512 : 0);
+  g.wide = 1;
   g.pointers = pointers;
   g.experts = experts;
   g.counts = counts;
@@ -916,6 +1052,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   st.bank = bank;
   st.k = intermediate;
   st.div = 1;
+  st.plan_ready = 1;
   if (int rc = launch_stage(fp4, st, routes, s)) return rc;
 
   g.maps += fp4 ? 256 : 128;
