@@ -197,14 +197,16 @@ int ink_short_conv(const void* x, int x_is_fp32, const float* taps, float* histo
  *  k_cache / v_cache BF16 [batch, kv_heads, slots, head_dim]: either the current token is already stored
  *  (ink_update_kv; new_k = new_v = NULL), or its key and value are given as new_k / new_v BF16 [batch, kv_heads,
  *  head_dim] and this call stores them at slot `position` (modulo the window) as well, saving the launch, position: device int64 scalar = tokens stored before this one (a CUDA graph advances it),
- *  pad_counts int64 [batch] or NULL, out BF16 [batch, heads, head_dim]. head_dim 64, 128 or 256. q, caches, new_k, new_v and
- *  out 16-byte aligned.
+ *  pad_counts int64 [batch] or NULL, out BF16 [batch, heads, head_dim]. head_dim 64, 128 or 256. q, caches and out
+ *  16-byte aligned.
  *  The slots in use are cut into parts, one block per (up to eight heads of one key/value head, sequence, part); with more
- *  than one part the partial results pass through `workspace` (ink_decode_attention_workspace_bytes, 16-byte aligned) and
- *  the block that stores the last partial of its heads joins them. The workspace must be ZERO before its first
- *  use (it starts with the arrival counters); every launch leaves the counters zero again, so the
- *  same workspace serves call after call on one stream. */
+ *  than eight parts the partial results pass through `workspace` (ink_decode_attention_workspace_bytes, 16-byte aligned) and
+ *  the block that stores the last partial of its heads joins them. The arrival counters at the start of the workspace
+ *  (ink_decode_attention_counter_bytes) must be ZERO before its first use; every launch leaves them zero again, so the
+ *  same workspace serves call after call of the same sizes on one stream. */
 size_t ink_decode_attention_workspace_bytes(int batch, int heads, int head_dim, int slots);
+/* how many bytes at its start are the arrival counters, the only part that must be zero */
+size_t ink_decode_attention_counter_bytes(int batch, int heads);
 int ink_decode_attention(const void* q, const void* r, const void* proj, void* k_cache, void* v_cache,
                          const int64_t* position, const int64_t* pad_counts, void* out, int batch, int heads,
                          int kv_heads, int head_dim, int d_rel, int rel_extent, int slots, int window, int n_floor,

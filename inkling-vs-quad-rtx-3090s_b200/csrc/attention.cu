@@ -738,8 +738,10 @@ __global__ void update_kv_kernel(const uint16_t* __restrict__ new_k, const uint1
 using namespace ink;
 
 static size_t attention_counter_bytes(int batch, int heads) { return ((size_t)batch * heads * sizeof(unsigned) + 255) / 256 * 256; }
+extern "C" size_t ink_decode_attention_counter_bytes(int batch, int heads) { return attention_counter_bytes(batch, heads); }
 
-// Splits along the cache at most: what the workspace is sized for, whatever the number of key/value heads.
+// Splits along the cache at most: what the workspace is sized for, whatever the number of key/value heads. (Up to
+// kAttnCluster parts always meet in a cluster and need none.)
 static int attention_max_splits(int slots) {
   const int whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
   return whole < kAttnMaxSplits ? whole : kAttnMaxSplits;
@@ -747,7 +749,7 @@ static int attention_max_splits(int slots) {
 
 extern "C" size_t ink_decode_attention_workspace_bytes(int batch, int heads, int head_dim, int slots) {
   const size_t splits = (size_t)attention_max_splits(slots);
-  return splits <= 1 ? 0 : attention_counter_bytes(batch, heads) + sizeof(float) * (size_t)batch * heads * splits * (kAttnPartial + head_dim);
+  return splits <= kAttnCluster ? 0 : attention_counter_bytes(batch, heads) + sizeof(float) * (size_t)batch * heads * splits * (kAttnPartial + head_dim);
 }
 
 template <int C>
@@ -757,7 +759,7 @@ static int launch_decode_attention(const AttnArgs& a, bool small, dim3 grid, cud
   const size_t smem_small = sizeof(float) * kAttnHeads * (2 * kSmallThreads + C + kSmallSlots + kSmallThreads / (C / 2) + C + 2) + rel;
   const size_t smem = small ? smem_small : sums > rel ? sums : rel;
   static_assert(kSmallSlots == kAttnMaxSplits && C >= kAttnMaxSplits, "the join's weights fit where queries and scores were");
-  INK_REQUIRE(rel <= 12 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
+  INK_REQUIRE(rel <= 160 * 1024, kUnsupportedShape, "decode_attention: d_rel=%d is too wide", a.d_rel);
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = dim3(small ? kSmallThreads : kAttnThreads);
@@ -772,7 +774,7 @@ static int launch_decode_attention(const AttnArgs& a, bool small, dim3 grid, cud
   config.numAttrs = cluster ? 1 : 0;
   void (*kernel)(AttnArgs) = small ? (cluster ? decode_attention_small_kernel<C, true> : decode_attention_small_kernel<C, false>)
                                    : (cluster ? decode_attention_kernel<C, true> : decode_attention_kernel<C, false>);
-  if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const cudaError_t e = cudaLaunchKernelEx(&config, kernel, a);
   INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "decode_attention: launch failed: %s", cudaGetErrorString(e));
   return kOk;
@@ -797,10 +799,14 @@ extern "C" int ink_decode_attention(const void* q, const void* r, const void* pr
   const size_t need = ink_decode_attention_workspace_bytes(batch, heads, head_dim, slots);
   INK_REQUIRE(need == 0 || (workspace && workspace_bytes >= need), kBadArgument,
               "decode_attention: workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-  INK_REQUIRE(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out) && aligned16(new_k) && aligned16(new_v) &&
+  INK_REQUIRE(aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && aligned16(out) &&
                   (need == 0 || aligned16(workspace)),
               kMisaligned, "decode_attention: buffers must be 16-byte aligned");
   if (batch == 0) return kOk;
+  if (!aligned16(new_k) || !aligned16(new_v)) {   // (the kernels read these rows 16 bytes at a time: stored first instead)
+    if (int rc = ink_update_kv(new_k, new_v, k_cache, v_cache, position, batch, kv_heads, head_dim, slots, window, stream)) return rc;
+    new_k = new_v = nullptr;
+  }
   const int pairs = batch * kv_heads * chunks, whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
   // Where all 64-slot parts are resident at once the small form takes them. Else the number of parts that takes the fewest
   // rounds of (steps a warp makes + what a block costs beside, about four steps' time), over the blocks resident at once.

@@ -9,9 +9,11 @@
 #include <torch/torch.h>
 
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
-#include <tuple>
+#include <utility>
+#include <vector>
 
 #include "../../include/inkling_b200.h"
 
@@ -55,15 +57,34 @@ at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const at::Devi
 }
 
 // ------------------------------------------------------------------------------------------------ attention
-// The join's workspace starts with counters that are zero between launches, so it is made once for each (device, stream,
-// size) and kept; calls on different streams do not share one.
-at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, size_t bytes) {
+// The join's workspace starts with counters that are zero between launches. An eager call keeps one for its stream (made
+// again, zeroed, when the sizes change; at most kMostWorkspaces, then the pool starts anew -- the memory goes back to the
+// allocator, which hands it out on the same stream only). A call under capture gets its own from the graph's pool, its
+// counters cleared by the graph: graphs may be replayed in any order, on any stream.
+at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, size_t bytes, size_t counters) {
+  const auto options = at::TensorOptions().dtype(at::kByte).device(device);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    const at::Tensor t = at::empty({(int64_t)bytes}, options);
+    if (cudaMemsetAsync(t.data_ptr(), 0, counters, stream) != cudaSuccess) fail("decode_attention: the workspace could not be cleared");
+    return t;
+  }
+  struct Kept {
+    size_t counters = 0;
+    at::Tensor t;
+  };
+  constexpr size_t kMostWorkspaces = 64;
   static std::mutex mutex;
-  static auto* kept = new std::map<std::tuple<int, cudaStream_t, size_t>, at::Tensor>();   // (not destroyed at exit: the CUDA context may be gone)
+  static auto* pool = new std::map<std::pair<int, cudaStream_t>, Kept>();   // (not destroyed at exit: the CUDA context may be gone)
   const std::lock_guard<std::mutex> lock(mutex);
-  at::Tensor& t = (*kept)[{device.index(), stream, bytes}];
-  if (!t.defined()) t = at::zeros({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(device));
-  return t;
+  if (pool->size() >= kMostWorkspaces && !pool->count({device.index(), stream})) pool->clear();
+  Kept& kept = (*pool)[{device.index(), stream}];
+  if (!kept.t.defined() || kept.counters != counters || (size_t)kept.t.numel() < bytes) {
+    kept.t = at::Tensor();
+    kept.t = at::zeros({(int64_t)bytes}, options);
+    kept.counters = counters;
+  }
+  return kept.t;
 }
 
 // (query, relative_states, proj, k_cache, v_cache, position, pad_counts, window, n_floor, alpha, scale, out, new_key, new_value)
@@ -105,7 +126,7 @@ PyObject* decode_attention(PyObject* const* args) {
   }
   const size_t need = ink_decode_attention_workspace_bytes((int)bs, (int)h, (int)c, (int)slots);
   at::Tensor workspace;
-  if (need) workspace = attention_workspace(q.device(), stream, need);
+  if (need) workspace = attention_workspace(q.device(), stream, need, ink_decode_attention_counter_bytes((int)bs, (int)h));
   check(ink_decode_attention(q.data_ptr(), r.data_ptr(), proj.data_ptr(), k.data_ptr(), v.data_ptr(), (const int64_t*)position.data_ptr(), (const int64_t*)pads,
                              out.data_ptr(), (int)bs, (int)h, (int)hk, (int)c, (int)d_rel, (int)proj.size(1), (int)slots, (int)int_at(args, 7), (int)int_at(args, 8),
                              (float)float_at(args, 9), (float)float_at(args, 10), new_k.defined() ? new_k.data_ptr() : nullptr,
@@ -114,39 +135,51 @@ PyObject* decode_attention(PyObject* const* args) {
 }
 
 // ------------------------------------------------------------------------------------------------ blocks
-// Addresses and sizes of a module, taken down once (the module keeps the tensors alive and makes a new record when one of
-// them is replaced).
+// What the calls need of a module, taken down once (the module makes a new record when one of its tensors is replaced).
+// The record holds the tensors themselves beside their addresses: storage that was exchanged underneath a tensor shows as
+// another address, and the call then returns NotImplemented for the module to make a new record.
 struct Block {
-  long long v[48];
+  long long v[48] = {};
+  std::vector<std::pair<int, at::Tensor>> kept;
+  bool current() const {
+    for (const auto& [f, t] : kept)
+      if ((long long)(uintptr_t)t.data_ptr() != v[f]) return false;
+    return true;
+  }
 };
 enum Field {
   kHidden, kWidth, kTopK, kShared, kStart, kLocal, kStride, kCapacity, kMaxExpert, kQuantized, kTokens, kRouted,
   kSources, kPointers, kExperts, kCounts, kRows, kActivated, kDown, kStatus, kBankMaps,
   kRouterWeight, kRouterBias, kGlobalScale, kSharedMaps, kTopkWeights, kTopkIndices, kGammas, kWorkspace, kWorkspaceBytes, kPartial,
-  kTable, kScratch, kScratchBytes, kStackFlags, kStackStatus, kRouteScaleBits, kFields
+  kTable, kScratch, kScratchBytes, kStackFlags, kStackStatus, kRouteScaleBits, kSharedGate, kSharedUp, kSharedDown, kFields
 };
 const char* const kFieldNames[kFields] = {
     "hidden", "width", "top_k", "shared", "start", "local", "stride", "capacity", "max_expert", "quantized", "tokens", "routed",
     "sources", "pointers", "experts", "counts", "rows", "activated", "down", "status", "bank_maps",
     "router_weight", "router_bias", "global_scale", "shared_maps", "topk_weights", "topk_indices", "gammas", "workspace", "workspace_bytes", "partial",
-    "table", "scratch", "scratch_bytes", "stack_flags", "stack_status", "route_scale_bits"};
+    "table", "scratch", "scratch_bytes", "stack_flags", "stack_status", "route_scale_bits", "shared_gate", "shared_up", "shared_down"};
 template <typename T>
 T* at_field(const Block& b, Field f) {
   return reinterpret_cast<T*>((uintptr_t)b.v[f]);
 }
 
 PyObject* make_block(PyObject* const* args) {
-  auto* block = new Block();
+  auto block = std::make_unique<Block>();
   for (int f = 0; f < kFields; ++f) {
     PyObject* item = PyDict_GetItemString(args[0], kFieldNames[f]);
     if (!item) continue;
-    block->v[f] = PyLong_AsLongLong(item);
-    if (block->v[f] == -1 && PyErr_Occurred()) {
-      delete block;
-      throw Failure{""};
+    if (THPVariable_Check(item)) {
+      const at::Tensor& t = THPVariable_Unpack(item);
+      block->v[f] = (long long)(uintptr_t)t.data_ptr();
+      block->kept.emplace_back(f, t);
+      continue;
     }
+    block->v[f] = PyLong_AsLongLong(item);
+    if (block->v[f] == -1 && PyErr_Occurred()) throw Failure{""};
   }
-  return PyCapsule_New(block, "inkling_block", [](PyObject* c) { delete (Block*)PyCapsule_GetPointer(c, "inkling_block"); });
+  PyObject* capsule = PyCapsule_New(block.get(), "inkling_block", [](PyObject* c) { delete (Block*)PyCapsule_GetPointer(c, "inkling_block"); });
+  if (capsule) (void)block.release();
+  return capsule;
 }
 const Block& block_at(PyObject* const* args) {
   auto* block = (const Block*)PyCapsule_GetPointer(args[0], "inkling_block");
@@ -164,20 +197,29 @@ Rows rows_of(const Block& b, const at::Tensor& t) {
   return r;
 }
 
-void grouped(const Block& b, const Rows& r, const int64_t* indices, const void* weights, float* partial, void* out, int n_shared, cudaStream_t stream) {
-  const int routes = r.tokens * (int)b.v[kTopK], groups = routes < b.v[kLocal] ? routes : (int)b.v[kLocal];
-  const size_t need = ink_moe_grouped_scratch_bytes(r.tokens, (int)b.v[kTopK], n_shared, (int)b.v[kHidden], (int)b.v[kWidth], groups, (int)b.v[kQuantized]);
+// Tokens of a many-token call that are planned and projected at a time: the images of the tokens take about 85 KB a token
+// at full width (2.7 GB), the banks are read once per 32 768 tokens (0.5 of about 20 ms), and the kernels' work counters
+// stay far inside 32 bits.
+constexpr int kMostTokens = 32768;
+void grouped(const Block& b, const Rows& r, int t0, int tokens, const int64_t* indices, const char* weights, const char* gammas, float* partial, void* out,
+             int n_shared, cudaStream_t stream) {
+  const int top_k = (int)b.v[kTopK], hidden = (int)b.v[kHidden];
+  const int routes = tokens * top_k, groups = routes < b.v[kLocal] ? routes : (int)b.v[kLocal];
+  const size_t need = ink_moe_grouped_scratch_bytes(tokens, top_k, n_shared, hidden, (int)b.v[kWidth], groups, (int)b.v[kQuantized]);
   const at::Tensor scratch = new_tensor({(int64_t)need}, at::kByte, r.x.device());   // (of this stream, or of the graph being captured)
-  check(ink_moe_grouped(r.x.data_ptr(), indices, weights, at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kRows),
-                        at_field<int32_t>(b, kCounts), at_field<void>(b, kBankMaps), n_shared ? at_field<void>(b, kSharedMaps) : nullptr,
-                        n_shared ? at_field<void>(b, kGammas) : nullptr, at_field<void>(b, kActivated), at_field<void>(b, kDown), partial, out, r.tokens,
-                        (int)b.v[kTopK], n_shared, (int)b.v[kHidden], (int)b.v[kWidth], groups, (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kCapacity],
-                        (int)b.v[kMaxExpert], (int)b.v[kQuantized], scratch.data_ptr(), need, at_field<int32_t>(b, kStatus), stream));
+  const size_t before = (size_t)t0 * hidden;
+  check(ink_moe_grouped((const char*)r.x.data_ptr() + 2 * before, indices, weights, at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts),
+                        at_field<int32_t>(b, kRows), at_field<int32_t>(b, kCounts), at_field<void>(b, kBankMaps),
+                        n_shared ? at_field<void>(b, kSharedMaps) : nullptr, n_shared ? gammas : nullptr, at_field<void>(b, kActivated), at_field<void>(b, kDown),
+                        partial ? partial + before : nullptr, out ? (char*)out + 2 * before : nullptr, tokens, top_k, n_shared, hidden, (int)b.v[kWidth], groups,
+                        (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kCapacity], (int)b.v[kMaxExpert], (int)b.v[kQuantized], scratch.data_ptr(), need,
+                        at_field<int32_t>(b, kStatus), stream));
 }
 
 // (block, x, want_partial) -> BF16 like x; with want_partial the FP32 output goes to the block's own buffer, None is returned
 PyObject* run_block(PyObject* const* args) {
   const Block& b = block_at(args);
+  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
   const at::Tensor& input = tensor_at(args, 1);
   const Rows r = rows_of(b, input);
   require(r.tokens <= b.v[kTokens], "more tokens than the block's buffers hold");
@@ -191,16 +233,23 @@ PyObject* run_block(PyObject* const* args) {
                                (int)b.v[kStackFlags], 1e-6f, (int)b.v[kHidden], (int)b.v[kWidth], (int)b.v[kRouted], (int)b.v[kShared], (int)b.v[kTopK],
                                at_field<void>(b, kScratch), (size_t)b.v[kScratchBytes], at_field<int32_t>(b, kStackStatus), stream));
   } else if (r.tokens > 0) {
+    require(b.v[kBankMaps] != 0, "a record for one token only");
     float route_scale;
     const uint32_t bits = (uint32_t)b.v[kRouteScaleBits];
     memcpy(&route_scale, &bits, sizeof(route_scale));
-    check(ink_router_plan_forward(r.x.data_ptr(), at_field<void>(b, kRouterWeight), at_field<float>(b, kRouterBias), at_field<void>(b, kGlobalScale), route_scale,
-                                  r.tokens, (int)b.v[kHidden], (int)b.v[kRouted], (int)b.v[kShared], (int)b.v[kTopK], nullptr, at_field<void>(b, kTopkWeights),
-                                  at_field<int64_t>(b, kTopkIndices), at_field<void>(b, kGammas), at_field<void>(b, kWorkspace), (size_t)b.v[kWorkspaceBytes],
-                                  at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kCounts),
-                                  at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], (int)b.v[kCapacity], stream));
-    grouped(b, r, at_field<int64_t>(b, kTopkIndices), at_field<void>(b, kTopkWeights), want_partial ? at_field<float>(b, kPartial) : nullptr,
-            want_partial ? nullptr : out.data_ptr(), (int)b.v[kShared], stream);
+    for (int t0 = 0; t0 < r.tokens; t0 += kMostTokens) {
+      const int tokens = std::min(kMostTokens, r.tokens - t0);
+      const size_t routes0 = (size_t)t0 * b.v[kTopK];
+      char *weights = at_field<char>(b, kTopkWeights) + 2 * routes0, *gammas = at_field<char>(b, kGammas) + 2 * (size_t)t0 * b.v[kShared];
+      int64_t* indices = at_field<int64_t>(b, kTopkIndices) + routes0;
+      check(ink_router_plan_forward((const char*)r.x.data_ptr() + 2 * (size_t)t0 * b.v[kHidden], at_field<void>(b, kRouterWeight), at_field<float>(b, kRouterBias),
+                                    at_field<void>(b, kGlobalScale), route_scale, tokens, (int)b.v[kHidden], (int)b.v[kRouted], (int)b.v[kShared], (int)b.v[kTopK],
+                                    nullptr, weights, indices, gammas, at_field<void>(b, kWorkspace), (size_t)b.v[kWorkspaceBytes], at_field<int64_t>(b, kSources),
+                                    at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kCounts), at_field<int32_t>(b, kRows),
+                                    (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], (int)b.v[kCapacity], stream));
+      grouped(b, r, t0, tokens, indices, weights, gammas, want_partial ? at_field<float>(b, kPartial) : nullptr, want_partial ? nullptr : out.data_ptr(),
+              (int)b.v[kShared], stream);
+    }
   }
   if (want_partial) Py_RETURN_NONE;
   return THPVariable_Wrap(out);
@@ -209,20 +258,24 @@ PyObject* run_block(PyObject* const* args) {
 // (block, x, indices, weights) -> BF16 like x: the routed experts alone, plan and projections
 PyObject* run_experts(PyObject* const* args) {
   const Block& b = block_at(args);
+  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
   const at::Tensor& input = tensor_at(args, 1);
   const Rows r = rows_of(b, input);
   const at::Tensor &i = tensor_at(args, 2), weights = bf16_rows(tensor_at(args, 3), "BF16 router weights expected");
   require(i.is_cuda() && i.scalar_type() == at::kLong && i.numel() == r.tokens * b.v[kTopK] && weights.numel() == i.numel(), "int64 indices and BF16 weights [tokens, top_k]");
   const at::Tensor indices = i.is_contiguous() ? i : i.contiguous();
-  const int routes = (int)indices.numel();
-  require(routes <= b.v[kCapacity], "more routes than the module's buffers hold");
+  require(indices.numel() <= b.v[kCapacity], "more routes than the module's buffers hold");
   const c10::cuda::CUDAGuard guard(r.x.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();
   const at::Tensor out = new_tensor(input.sizes(), at::kBFloat16, r.x.device());
-  check(ink_expert_plan((const int64_t*)indices.data_ptr(), at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts),
-                        at_field<int32_t>(b, kCounts), at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], routes,
-                        (int)b.v[kCapacity], stream));
-  grouped(b, r, (const int64_t*)indices.data_ptr(), weights.data_ptr(), nullptr, out.data_ptr(), 0, stream);
+  for (int t0 = 0; t0 < r.tokens; t0 += kMostTokens) {
+    const int tokens = std::min(kMostTokens, r.tokens - t0);
+    const size_t routes0 = (size_t)t0 * b.v[kTopK];
+    const int64_t* here = (const int64_t*)indices.data_ptr() + routes0;
+    check(ink_expert_plan(here, at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kCounts),
+                          at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], tokens * (int)b.v[kTopK], (int)b.v[kCapacity], stream));
+    grouped(b, r, t0, tokens, here, (const char*)weights.data_ptr() + 2 * routes0, nullptr, nullptr, out.data_ptr(), 0, stream);
+  }
   return THPVariable_Wrap(out);
 }
 

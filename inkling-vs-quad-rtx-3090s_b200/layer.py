@@ -28,6 +28,8 @@ from .kernels.paired_all_reduce import all_reduce
 # Up to this many tokens each route runs its own matrix-vector product
 # (my_inkling/offloaded_experts.py:22).
 MATVEC_TOKENS = 8
+# Up to this many tokens are planned and projected together (the native calls' kMostTokens, see there).
+GROUPED_TOKENS = 32768
 
 
 def _group_of(device_mesh):
@@ -105,8 +107,8 @@ class ResidentExperts(nn.Module):
         self.status = torch.zeros(1, **i32)
         self.capacity = 0
 
-    # What the native calls know of this module is taken down once (`_record`); replacing a tensor it points to, or growing
-    # the buffers, makes a new one.
+    # What the native calls need of this module is taken down once (`record_fields`); replacing a tensor, or growing the
+    # buffers, makes a new one, and so does a call that finds a tensor's storage exchanged.
     _native = None
     generation = 0
 
@@ -116,12 +118,14 @@ class ResidentExperts(nn.Module):
             self.__dict__["generation"] = self.generation + 1
         super().__setattr__(name, value)
 
+    def __getstate__(self):   # copies and pickles make their own record
+        return {k: v for k, v in self.__dict__.items() if k != "_native"}
+
     def record_fields(self) -> dict:
-        at = lambda t: t.data_ptr()  # noqa: E731
         return dict(hidden=self.hidden_dim, width=self.intermediate_dim, start=self.start, local=self.local, stride=self.stride,
-                    capacity=self.capacity, max_expert=self.max_expert, quantized=int(self.quantized), sources=at(self.sources),
-                    pointers=at(self.pointers), experts=at(self.experts), counts=at(self.counts), rows=at(self.rows),
-                    activated=at(self.activated), down=at(self.down), status=at(self.status), bank_maps=at(self.bank_maps))
+                    capacity=self.capacity, max_expert=self.max_expert, quantized=int(self.quantized), sources=self.sources,
+                    pointers=self.pointers, experts=self.experts, counts=self.counts, rows=self.rows,
+                    activated=self.activated, down=self.down, status=self.status, bank_maps=self.bank_maps)
 
     @staticmethod
     def _even_spacing(addresses: list[list[int]], sizes: list[int]):
@@ -197,18 +201,26 @@ class ResidentExperts(nn.Module):
             self.max_expert, 256)
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
-        if self.device_mesh is None and self.bank_maps is not None and hidden_states.shape[0] > 1:
+        if self.device_mesh is None and self.bank_maps is not None and hidden_states.shape[0] > 1 and hidden_states.dim() == 2:
             routes = top_k_index.numel()
             if routes > self.capacity:
                 self._reserve(routes)
             top_k = top_k_index.shape[1]
-            if self._native is None or self._native[0] != top_k:
-                self.__dict__["_native"] = (top_k, host().make_block(dict(self.record_fields(), top_k=top_k)))
-            return host().run_experts(self._native[1], hidden_states, top_k_index, top_k_weights)
+            out = NotImplemented
+            while out is NotImplemented:
+                if self._native is None or self._native[0] != top_k:
+                    self.__dict__["_native"] = (top_k, host().make_block(dict(self.record_fields(), top_k=top_k)))
+                out = host().run_experts(self._native[1], hidden_states, top_k_index, top_k_weights)
+                if out is NotImplemented:
+                    self.__dict__["_native"] = None
+            return out
         final = torch.zeros_like(hidden_states, dtype=torch.float32)
         self._reserve(top_k_index.numel())
-        self._plan(top_k_index)
-        self._project(hidden_states.contiguous(), top_k_index.contiguous(), top_k_weights.contiguous(), final)
+        x, index, weights = hidden_states.contiguous(), top_k_index.contiguous(), top_k_weights.contiguous()
+        for t0 in range(0, max(1, x.shape[0]), GROUPED_TOKENS):
+            part = slice(t0, t0 + GROUPED_TOKENS)
+            self._plan(index[part])
+            self._project(x[part], index[part], weights[part], final[part])
         final = all_reduce(final, _group_of(self.device_mesh))
         return final.to(hidden_states.dtype)
 
@@ -249,30 +261,37 @@ class FusedMoE(nn.Module):
         self._tokens = 0
         self._fused = None   # one-launch descriptor for a single token, built on first use
         self._maps_of = None
+        if experts.bank_maps is not None and self.n_shared and all(
+                w.is_cuda and w.is_contiguous() and w.dtype == torch.bfloat16 for w in (shared_gate, shared_up, shared_down)):
+            self._shared_maps()   # here, so that a first call may be one under graph capture
 
     _native = None   # what the native calls know of this block, and the experts' generation it was taken down at
 
     def __setattr__(self, name, value):
-        if isinstance(value, (torch.Tensor, StackDescriptor)) or name in ("experts", "top_k", "route_scale", "_fused"):
+        if isinstance(value, (torch.Tensor, StackDescriptor)) or name in ("experts", "top_k", "n_shared", "route_scale", "_fused"):
             self.__dict__["_native"] = None
         super().__setattr__(name, value)
 
-    def _record(self):
+    def __getstate__(self):   # copies and pickles make their own record and table
+        return dict({k: v for k, v in self.__dict__.items() if k != "_native"}, _fused=None)
+
+    def _record(self, one_token: bool):
+        """The record for several tokens, with `one_token` also the one-launch kernel's table (made on the first such call only)."""
         ex = self.experts
-        at = lambda t: t.data_ptr()  # noqa: E731
         fields = dict(ex.record_fields() if ex.bank_maps is not None else dict(hidden=ex.hidden_dim, width=ex.intermediate_dim),
                       tokens=self._tokens if ex.bank_maps is not None else 1, routed=self.router_weight.shape[0] - self.n_shared,
-                      shared=self.n_shared, top_k=self.top_k, router_weight=at(self.router_weight), router_bias=at(self.router_bias),
-                      global_scale=at(self.global_scale), topk_weights=at(self.topk_weights), topk_indices=at(self.topk_indices),
-                      gammas=at(self.gammas), workspace=at(self.workspace), workspace_bytes=self.workspace.numel(), partial=at(self.partial),
+                      shared=self.n_shared, top_k=self.top_k, router_weight=self.router_weight, router_bias=self.router_bias,
+                      global_scale=self.global_scale, topk_weights=self.topk_weights, topk_indices=self.topk_indices,
+                      gammas=self.gammas, workspace=self.workspace, workspace_bytes=self.workspace.numel(), partial=self.partial,
+                      shared_gate=self.shared_gate, shared_up=self.shared_up, shared_down=self.shared_down,
                       route_scale_bits=struct.unpack("<I", struct.pack("<f", self.route_scale))[0])
         if ex.bank_maps is not None and self.n_shared:
-            fields["shared_maps"] = at(self._shared_maps())
-        if self.one_launch_supported():
+            fields["shared_maps"] = self._shared_maps()
+        if one_token:
             if self._fused is None:
                 self._fused = self._one_launch()
             f = self._fused
-            fields.update(table=at(f.table), scratch=at(f.scratch), scratch_bytes=f.scratch.numel(), stack_status=at(f.status),
+            fields.update(table=f.table, scratch=f.scratch, scratch_bytes=f.scratch.numel(), stack_status=f.status,
                           stack_flags=2 if f.bank_maps is not None else 0)
         return host().make_block(fields)
 
@@ -282,18 +301,27 @@ class FusedMoE(nn.Module):
         return StackDescriptor([self.block_descriptor()], ex.hidden_dim, ex.intermediate_dim, ex.local, self.n_shared, self.top_k,
                                self.router_weight.device, group=_group_of(self.device_mesh))
 
-    def _native_for(self, tokens: int):
-        """The record for the native call with this many tokens, or None where the launches are put together here: several
-        ranks, banks that are not evenly spaced, one token without the one-launch kernel."""
+    def _call_native(self, tokens: int, x, want_partial: bool):
+        """The block in one native call, or NotImplemented where the launches are put together here: several ranks, banks that
+        are not evenly spaced, one token without the one-launch kernel."""
         if self.device_mesh is not None or (tokens == 1 and self.separate_launches):
-            return None
+            return NotImplemented
         ex = self.experts
         if tokens > self._tokens:
             self._reserve(tokens)
-        if self._native is None or self._native[0] != ex.generation:
-            record = self._record()
-            self.__dict__["_native"] = (ex.generation, record, self.one_launch_supported(), ex.bank_maps is not None)
-        return self._native[1] if self._native[2 if tokens == 1 else 3] else None
+        one = tokens == 1
+        for _ in range(2):   # (again where the record turns out to be of storage that has been exchanged)
+            native = self._native
+            if native is None or native[0] != ex.generation or not native[2 if one else 3]:
+                if not (self.one_launch_supported() if one else ex.bank_maps is not None):
+                    return NotImplemented
+                record = self._record(one)
+                native = self.__dict__["_native"] = (ex.generation, record, one, ex.bank_maps is not None)
+            out = host().run_block(native[1], x, want_partial)
+            if out is not NotImplemented:
+                return out
+            self._fused = None   # (drops the record too)
+        raise RuntimeError("FusedMoE: a tensor's storage was exchanged during the call")
 
     def block_descriptor(self, norm_weight=None) -> dict:
         """This block as the one-launch kernel takes it (addresses of the module's tensors)."""
@@ -340,20 +368,20 @@ class FusedMoE(nn.Module):
             self._maps, self._maps_of = encode_shared_maps(self.shared_gate, self.shared_up, self.shared_down), at
         return self._maps
 
-    def route(self, flat):
-        """Router and plan for `flat` [t, d]; fills the module's routing buffers."""
-        t = flat.shape[0]
+    def route(self, flat, t0: int = 0):
+        """Router and plan for `flat` [t, d]; fills the module's routing buffers from token t0 on."""
+        t1 = t0 + flat.shape[0]
         ex = self.experts
         args = (flat, self.router_weight, self.router_bias, self.global_scale, self.route_scale, self.top_k,
-                self.n_shared, self.topk_weights[:t], self.topk_indices[:t], self.gammas[:t], self.workspace)
+                self.n_shared, self.topk_weights[t0:t1], self.topk_indices[t0:t1], self.gammas[t0:t1], self.workspace)
         router_plan_forward(*args, ex.sources, ex.pointers, ex.experts, ex.counts, ex.rows, ex.start,
                             ex.local, ex.stride, ex.capacity)
 
     def forward(self, hidden_states):
         shape = hidden_states.shape
-        native = self._native_for(hidden_states.numel() // shape[-1])
-        if native is not None:
-            return host().run_block(native, hidden_states, False)
+        out = self._call_native(hidden_states.numel() // shape[-1], hidden_states, False)
+        if out is not NotImplemented:
+            return out
         flat = hidden_states.reshape(-1, shape[-1]).contiguous()
         return self.forward_partial(flat).to(hidden_states.dtype).view(shape)
 
@@ -363,20 +391,21 @@ class FusedMoE(nn.Module):
         t = flat.shape[0]
         self._reserve(t)
         ex = self.experts
-        native = self._native_for(t)
-        if native is not None:
-            host().run_block(native, flat, True)
+        if self._call_native(t, flat, True) is not NotImplemented:
             return self.partial[:t]
         if t == 1 and self.one_launch_supported() and not self.separate_launches:
             if self._fused is None:
                 self._fused = self._one_launch()
             self._fused.decode(flat, self.partial[:1])
             return self.partial[:1]
-        self.route(flat)
         if t > 1 and ex.bank_maps is not None:
-            ex.grouped(flat, self.topk_indices[:t], self.topk_weights[:t], self.partial[:t], shared_maps=self._shared_maps() if self.n_shared else None,
-                       gammas=self.gammas[:t], n_shared=self.n_shared)
+            for t0 in range(0, t, GROUPED_TOKENS):
+                t1 = min(t, t0 + GROUPED_TOKENS)
+                self.route(flat[t0:t1], t0)
+                ex.grouped(flat[t0:t1], self.topk_indices[t0:t1], self.topk_weights[t0:t1], self.partial[t0:t1],
+                           shared_maps=self._shared_maps() if self.n_shared else None, gammas=self.gammas[t0:t1], n_shared=self.n_shared)
             return all_reduce(self.partial[:t], _group_of(self.device_mesh))
+        self.route(flat)
         for t0 in range(0, t, MATVEC_TOKENS):
             t1 = min(t, t0 + MATVEC_TOKENS)
             moe_decode(flat[t0:t1], self.topk_indices[t0:t1], self.topk_weights[t0:t1], ex.pointers,

@@ -387,3 +387,52 @@ def test_decode_attention_at_the_edges_of_its_parts(ib, c, h, hk, slots, window,
     torch.cuda.synchronize()
     assert (got[:, :, 0].float().cpu() - want).abs().max() <= TOL * want.abs().max()
     assert torch.equal(before[0].cpu(), k) and torch.equal(before[1].cpu(), v)
+
+
+def _many_part_inputs(device, bs=1, slots=1100, seed=3, misaligned=False):
+    gen = torch.Generator(device).manual_seed(seed)
+    draw = lambda *shape: torch.randn(*shape, generator=gen, device=device).bfloat16()  # noqa: E731
+    h, hk, c = 8, 2, 64
+    new = [draw(bs * hk * c + 1)[int(misaligned):][:bs * hk * c].view(bs, hk, 1, c) for _ in range(2)]
+    return dict(query=draw(bs, h, c), relative_states=draw(bs, h, 16), proj=draw(16, 512), k_cache=draw(bs, hk, slots, c),
+                v_cache=draw(bs, hk, slots, c), position=torch.tensor(slots - 5, device=device), new_key=new[0], new_value=new[1])
+
+
+def test_graphs_with_many_parts_replay_in_any_order(ib):
+    """Two graphs captured on one stream, the second replayed first, eager calls of other sizes in between: each finds its
+    arrival counters as it needs them. The same kernel on the same inputs gives the same bits."""
+    device = torch.device("cuda", 0)
+    sizes = [dict(bs=1), dict(bs=3, slots=1500), dict(bs=1)]
+    inputs = [_many_part_inputs(device, seed=i, **s) for i, s in enumerate(sizes)]
+    want = [ib.kernels.decode_attention(**i).clone() for i in inputs]
+    stream, graphs, outs = torch.cuda.Stream(), [], []
+    torch.cuda.synchronize()
+    for i in inputs:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            outs.append(ib.kernels.decode_attention(**i))
+        graphs.append(graph)
+    for _ in range(2):
+        for n in (2, 0, 1, 0):
+            outs[n].zero_()
+            graphs[n].replay()
+            assert torch.equal(outs[n], want[n])
+            assert torch.equal(ib.kernels.decode_attention(**inputs[1 - n % 2]), want[1 - n % 2])
+
+
+def test_a_new_token_at_any_address_through_the_c_entry(ib):
+    """Key and value rows that do not start on 16 bytes are stored first and read from the caches: the same bits."""
+    from inkling_b200.kernels import _abi
+
+    device = torch.device("cuda", 0)
+    i = _many_part_inputs(device, slots=100, misaligned=True)
+    caches = [i["k_cache"].clone(), i["v_cache"].clone()]
+    want = ib.kernels.decode_attention(**i)
+    assert i["new_key"].data_ptr() % 16 == 2
+    out = torch.empty_like(want)
+    _abi.check(_abi.lib().ink_decode_attention(
+        i["query"].data_ptr(), i["relative_states"].data_ptr(), i["proj"].data_ptr(), caches[0].data_ptr(), caches[1].data_ptr(),
+        i["position"].data_ptr(), None, out.data_ptr(), 1, 8, 2, 64, 16, 512, 100, 0, 0, 0.0, 1 / 64, i["new_key"].data_ptr(),
+        i["new_value"].data_ptr(), None, 0, _abi.stream()))
+    assert torch.equal(out, want)
+    assert torch.equal(caches[0], i["k_cache"]) and torch.equal(caches[1], i["v_cache"])

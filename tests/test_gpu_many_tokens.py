@@ -122,3 +122,59 @@ def test_the_plan_is_a_stable_sort_at_any_size(ib, device, local, start, routes)
     for got, name in ((experts, "experts"), (counts, "counts"), (rows, "rows")):
         assert torch.equal(got.cpu(), torch.as_tensor(want[name]).to(torch.int32)), name
     assert torch.equal(pointers.cpu(), torch.as_tensor(want["pointers"]))
+
+
+def _block(ib, device, tokens, seed=5, d=256, f=256, experts=8):
+    p, banks, x = cases.make_layer(d, f, experts, 2, 3, tokens, seed=seed, bias="randn")
+    dp = layer_on_device(p, device)
+    return ib.FusedMoE(dp["router_weight"], dp["router_bias"], dp["global_scale"], p["route_scale"], p["top_k"], dp["shared_gate"],
+                       dp["shared_up"], dp["shared_down"], ib.ResidentExperts(d, f, None, one_allocation_per_kind(banks, device)), None), x.to(device)
+
+
+def test_more_tokens_than_are_planned_at_a_time(ib, device):
+    """A call of 32 768 tokens and a rest: the rest comes out as in a call of its own. Tokens do not mix, so only the order
+    of FP32 sums could differ, if at all: one rounding of the BF16 result."""
+    layer, x = _block(ib, device, 64)
+    many = x.repeat(32768 // 64 + 1, 1)[:32768 + 37].contiguous()
+    whole = layer(many)
+    idx, w = layer.topk_indices[:len(many)].clone(), layer.topk_weights[:len(many)].clone()
+    rest = layer(many[32768:])
+    assert max_rel(whole[32768:].float().cpu(), rest.float().cpu()) <= 2 ** -8
+    assert max_rel(whole[:64].float().cpu(), layer(x).float().cpu()) <= 2 ** -8
+    routed = layer.experts(many, idx, w)
+    assert max_rel(routed[32768:].float().cpu(), layer.experts(many[32768:], idx[32768:], w[32768:]).float().cpu()) <= 2 ** -8
+    layer.experts.check_status()
+
+
+@pytest.mark.parametrize("tokens", [1, 9])
+def test_a_block_sees_weights_exchanged_underneath(ib, device, tokens):
+    """`tensor.data = ...` keeps the tensor and changes its storage; a copy of the module makes its own record."""
+    import copy
+
+    d, f = (1024, 512)
+    layer, x = _block(ib, device, tokens, d=d, f=f, experts=32)
+    other, _ = _block(ib, device, tokens, seed=8, d=d, f=f, experts=32)
+    first = layer(x).clone()
+    other.experts = layer.experts
+    want = other(x).clone()
+    old = [getattr(layer, n).clone() for n in ("router_weight", "router_bias", "shared_gate", "shared_up", "shared_down")]
+    keep = [getattr(layer, n).data for n in ("router_weight", "router_bias", "shared_gate", "shared_up", "shared_down")]
+    twin = copy.deepcopy(layer)
+    for n in ("router_weight", "router_bias", "shared_gate", "shared_up", "shared_down"):
+        getattr(layer, n).data = getattr(other, n).clone()
+    assert torch.equal(layer(x), want) and not torch.equal(first, want)
+    assert torch.equal(twin(x), first)
+    del old, keep
+
+
+@pytest.mark.parametrize("tokens", [2, 12])
+def test_a_first_call_may_be_one_under_capture(ib, device, tokens):
+    layer, x = _block(ib, device, tokens)
+    twin, _ = _block(ib, device, tokens)
+    want = twin(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = layer(x)
+    graph.replay()
+    assert torch.equal(out, want)
