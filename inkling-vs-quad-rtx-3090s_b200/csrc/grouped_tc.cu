@@ -146,6 +146,7 @@ struct GgItem {
   int m0;         // first weight row
   int tile, n;    // tile of tokens, and how many
   int slot;       // first slot of the tile (routed)
+  int bank;       // index of the expert's matrix (set by the producers)
 };
 
 template <bool FP4, bool TALL>
@@ -335,67 +336,53 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   const uint32_t tmem = sh.tmem_base;
 
   if (warp == 0 || warp >= 10) {
-    // =========================================================== producers: every lane issues one of the stage's copies
+    // =========================================================== producers
     const int producer = warp == 0 ? 0 : warp - 9;
     auto rows_bytes = [&](const GgItem& it) -> uint32_t {   // one chunk of the tile's N operand
       return (FP4 && !it.shared) ? (uint32_t)((it.n + 1) / 2 * 2) * 512u : (uint32_t)((it.n + 7) / 8 * 8) * 128u;
     };
+    // (one elected lane issues a stage's copies one after the other: copies issued by several lanes of a warp at once were
+    // taken apart lane by lane, 270 to 340 clocks each, 1 000 to 1 270 a stage)
     auto expect = [&](const GgItem& it, int u) {
-      if (lane == 0) {
-        uint32_t bytes = St::kUnits * kTcCodeBytes + rows_bytes(it);
-        if (FP4 && !it.shared) bytes += St::kUnits * kTcScaleBytes + rows_bytes(it) / 8u;
-        mbar_expect_tx(&sh.full[u], bytes);
-      }
-      __syncwarp();
+      uint32_t bytes = St::kUnits * kTcCodeBytes + rows_bytes(it);
+      if (FP4 && !it.shared) bytes += St::kUnits * kTcScaleBytes + rows_bytes(it) / 8u;
+      mbar_expect_tx(&sh.full[u], bytes);
     };
     auto issue_weights = [&](const GgItem& it, int s, int u) {
-      const int unit = lane & 1;
-      const unsigned char* map = it.shared ? a.shared_maps : a.maps;
-      const int z = it.shared ? it.group : a.experts[it.group] - a.start;
-      int x = s * 64, y = it.m0, at = 0;
-      bool mine = false;
-      if (PROJ == 0 && it.shared) {
-        // 64 rows of gate and of up (TALL: twice that)
-        const int half = lane >> 1;
-        mine = lane < 2 * St::kUnits;
-        map += unit * 128;
-        y = it.m0 / 2 + half * kGgSharedBox;
-        at = TALL ? unit * kTcCodeBytes + half * (kTcCodeBytes / 2) : unit * (kTcCodeBytes / 2);
+      unsigned char* stage = ring + (size_t)u * St::kBytes;
+      uint64_t* bar = &sh.full[u];
+      if (PROJ == 0 && it.shared) {   // 64 rows of gate and of up (TALL: twice that)
+        constexpr int kUp = TALL ? kTcCodeBytes : kTcCodeBytes / 2;
+#pragma unroll
+        for (int half = 0; half < St::kUnits; ++half) {
+          tc_tma_3d(stage + half * (kTcCodeBytes / 2), a.shared_maps, s * 64, it.m0 / 2 + half * kGgSharedBox, it.bank, bar);
+          tc_tma_3d(stage + kUp + half * (kTcCodeBytes / 2), a.shared_maps + 128, s * 64, it.m0 / 2 + half * kGgSharedBox, it.bank, bar);
+        }
       } else if (!FP4 || it.shared) {
-        mine = lane < St::kUnits;
-        y += unit * kTcRows;
-        at = unit * kTcCodeBytes;
-      } else if (lane < 2) {   // codes
-        mine = unit == 0 || (TALL && !a.wide);
-        x = s * 128;
-        y += unit * kTcRows;
-        at = unit * kTcCodeBytes;
-      } else if (lane < 4) {   // block scales
-        mine = unit == 0 || (TALL && !a.wide);
-        map += 128;
-        x = s * 16;
-        y += unit * kTcRows;
-        at = St::kScalesAt + unit * kTcScaleBytes;
+        const unsigned char* map = it.shared ? a.shared_maps : a.maps;
+#pragma unroll
+        for (int unit = 0; unit < St::kUnits; ++unit) tc_tma_3d(stage + unit * kTcCodeBytes, map, s * 64, it.m0 + unit * kTcRows, it.bank, bar);
+      } else {
+#pragma unroll
+        for (int unit = 0; unit < St::kUnits; ++unit) {
+          if (unit > 0 && a.wide) break;
+          tc_tma_3d(stage + unit * kTcCodeBytes, a.maps, s * 128, it.m0 + unit * kTcRows, it.bank, bar);
+          tc_tma_3d(stage + St::kScalesAt + unit * kTcScaleBytes, a.maps + 128, s * 16, it.m0 + unit * kTcRows, it.bank, bar);
+        }
       }
-      if (mine) tc_tma_3d(ring + (size_t)u * St::kBytes + at, map, x, y, z, &sh.full[u]);
     };
     auto issue_rows = [&](const GgItem& it, int s, int u) {
-      const bool fp4 = FP4 && !it.shared;
-      uint32_t bytes = rows_bytes(it);
+      unsigned char* stage = ring + (size_t)u * St::kBytes;
+      const uint32_t bytes = rows_bytes(it);
       const unsigned char* from;
-      int at = St::kRowsAt;
       if (it.shared) {
         const int padded = (a.tokens + 7) / 8 * 8;
-        from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2 + (size_t)s * bytes;
+        from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2;
       } else {
-        from = a.image + (size_t)it.slot * a.k * 2 + (size_t)s * bytes;
+        from = a.image + (size_t)it.slot * a.k * 2;
       }
-      if (fp4 && lane == 1) {
-        bytes /= 8;
-        from = a.image_scales + (size_t)it.slot * (a.k / 4) + (size_t)s * bytes;
-        at = St::kRowScalesAt;
-      }
-      if (lane < (fp4 ? 2 : 1)) bulk_g2s(ring + (size_t)u * St::kBytes + at, from, bytes, &sh.full[u]);
+      bulk_g2s(stage + St::kRowsAt, from + (size_t)s * bytes, bytes, &sh.full[u]);
+      if (FP4 && !it.shared) bulk_g2s(stage + St::kRowScalesAt, a.image_scales + (size_t)it.slot * (a.k / 4) + (size_t)s * (bytes / 8), bytes / 8, &sh.full[u]);
     };
     // Stage i of the block's sequence is producer i % 2's. The first round's weights are asked for before the kernel in
     // front has finished; their N operand after.
@@ -407,14 +394,18 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     long long first = 0;   // the block's stages before this item
     bool waited = false;
     while (walk.next(it)) {
+      it.bank = it.shared ? it.group : a.experts[it.group] - a.start;
       const int stages = walk.stages_of(it.shared);
       int s = (int)((producer - first % kGgProducers + kGgProducers) % kGgProducers);
       for (; s < stages; s += kGgProducers) {
         const long long seq = first + s;
         const int u = (int)(seq % St::kCount);
         if (early < kFirst) {
-          expect(it, u);
-          issue_weights(it, s, u);
+          if (elect_one()) {
+            expect(it, u);
+            issue_weights(it, s, u);
+          }
+          __syncwarp();
 #pragma unroll
           for (int i = 0; i < kFirst; ++i) {
             if (i == early) {
@@ -429,12 +420,17 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
           pdl_wait();
           waited = true;
 #pragma unroll
-          for (int i = 0; i < kFirst; ++i) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+          for (int i = 0; i < kFirst; ++i)
+            if (elect_one()) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+          __syncwarp();
         }
         if (!__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / St::kCount) - 1) & 1u, &sh))) break;
-        expect(it, u);
-        issue_weights(it, s, u);
-        issue_rows(it, s, u);
+        if (elect_one()) {
+          expect(it, u);
+          issue_weights(it, s, u);
+          issue_rows(it, s, u);
+        }
+        __syncwarp();
       }
       first += stages;
       if (sh.failed) break;
@@ -443,7 +439,8 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       pdl_wait();
 #pragma unroll
       for (int i = 0; i < kFirst; ++i)
-        if (i < early) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+        if (i < early && elect_one()) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+      __syncwarp();
     }
   } else if (warp == 1) {
     // =========================================================== MMA issue
