@@ -267,7 +267,7 @@ int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, con
  * my_inkling/model.py:192-226): both routed projections and the weighted sum, and -- with n_shared > 0 -- the shared
  * experts as further tiles of the same launches. Each active expert's bytes cross HBM once.
  *  indices, weights, experts, rows, counts, pointers   as for ink_expert_gemm / ink_expert_reduce, of ink_expert_plan
- *  quantized   1: NVFP4 banks, bank_maps of ink_encode_grouped_banks (1024 bytes, arguments as ink_moe_stack_encode_banks); 0: BF16 banks (pointer stride 2),
+ *  quantized   1: NVFP4 banks, bank_maps of ink_moe_stack_encode_banks (512 bytes); 0: BF16 banks (pointer stride 2),
  *              bank_maps of ink_encode_bf16_banks (256 bytes); device copies, 128-byte aligned
  *  shared_maps device copy of ink_encode_shared's 384 bytes, gammas BF16 [tokens, n_shared] (both unused for n_shared = 0)
  *  activated   scratch BF16 [tokens * top_k, intermediate]: left holding the routes' gate/up results; down likewise BF16
@@ -276,10 +276,6 @@ int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, con
  *  groups      entries of experts / counts to visit; start, local: first expert and number of experts of this rank
  *  status      bit 0: a route named an expert outside [0, max_expert] (it is skipped); bit 1: a bounded wait gave up
  * Constraints: hidden and intermediate up to 4096, multiples of 256 (BF16 banks: of 64, hidden of 128); groups <= 1024. */
-int ink_encode_grouped_banks(void* out_host_1024, const void* gate_up_codes, uint64_t gate_up_codes_stride,
-                             const void* gate_up_scales, uint64_t gate_up_scales_stride, const void* down_codes,
-                             uint64_t down_codes_stride, const void* down_scales, uint64_t down_scales_stride, int experts,
-                             int hidden, int intermediate);
 int ink_encode_bf16_banks(void* out_host_256, const void* gate_up, uint64_t gate_up_stride, const void* down,
                           uint64_t down_stride, int experts, int hidden, int intermediate);
 int ink_encode_shared(void* out_host_384, const void* gate, const void* up, const void* down, int n_shared, int hidden,

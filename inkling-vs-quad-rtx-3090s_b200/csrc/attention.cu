@@ -66,8 +66,7 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 // the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
 // deliver at HBM speed, so scores, bias and weighted values go through warp-level matrix instructions (M = heads: the
 // contraction is far too flat for the 128-row tcgen05 tiles). Measured on B200, batch 8, 64 heads on 8 key/value
-// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, see the table of the design notes for
-// this one.
+// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, 173 us with this one (5.0 TB/s).
 //
 // A warp takes 16 slots a step and keeps everything in registers; nothing of the cache passes through shared memory,
 // because the sums over channels may run in any order as long as both operands agree:

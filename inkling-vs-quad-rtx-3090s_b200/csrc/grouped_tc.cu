@@ -5,20 +5,20 @@
 //
 // The N operand is laid out by a small kernel in front (`stage_rows_kernel`) exactly as the main kernel's ring wants it,
 // tile by tile, so that the main kernel fetches it with one bulk copy per stage next to the weights and never gathers:
-//   NVFP4  a token is four E2M1 digit rows with power-of-two block scales (tc_path.cuh); a tile is up to 32 tokens;
-//   BF16   a token is a row of 64-column pieces; a tile is up to 128 tokens.
+//   NVFP4  a token is four E2M1 digit rows with power-of-two block scales (tc_path.cuh); a tile is T = 16, 32 or 64 tokens;
+//   BF16   a token is a row of 64-column pieces; a tile is 4 T tokens.
 // (Gathering the digit rows in the main kernel, eight tokens a pass, stalled its MMAs at the head of every pass, and every
 // expert's bank was read once per eight of its tokens: 64 tokens of one block 0.42 ms, 1 024 tokens 2.8 ms.)
 //
-// A ring stage is a chunk of the contraction (128 bytes of every row) of a weight tile and the N operand that goes with it.
-// TALL: a tile has 256 rows, so that each fetch of the N operand serves as many -- for prompts, where L2 traffic counts.
-// Else (a few tokens per expert, everything waits for HBM) 128 rows and stages half as large: items even out better over
-// the SMs, and less of the ring is held by stages whose scales are on the way to tensor memory or whose MMAs are running.
+// A ring stage is a chunk of the contraction (128 bytes of every row) of a tile of 128 weight rows and the N operand that goes
+// with it: 8 stages of 27 KB, 6 of 36 KB or 4 of 54 KB. Whatever T, a weight tile meets one tile of tokens after the other in
+// one block, so its next reads follow within some 300 KB of the block's stream (44 MB over the chip: they hit L2; with tiles of
+// 256 weight rows, tried before, they came from HBM again). A larger T saves these reads, a smaller one leaves more of
+// the ring to the weights: see gg_tokens.
 //
 // Persistent blocks, one per SM. The shared experts' items (long) are dealt evenly, the routed items by cost in what is
-// left of each block's share. Two warps produce, a stage each in turn (a copy takes the
-// issuing warp 200 ns whatever its size: with one producer a stage of 18 KB took 1 us and 64 tokens of one block 0.64 ms),
-// one thread issues the MMAs, four warps move block scales to tensor memory, four read accumulators and write outputs. The kernel is launched
+// left of each block's share. Two warps produce, a stage each in turn (a stage's copies
+// take the issuing lane 300 clocks), one thread issues the MMAs, four warps move block scales to tensor memory, four read accumulators and write outputs. The kernel is launched
 // while its predecessor runs (programmatic dependent launch): until that is done it only streams weights, whose
 // addresses depend on nothing but the plan. Every wait is bounded; one that gives up sets kFlagWaitTimedOut.
 #include "../../include/inkling_b200.h"
@@ -30,28 +30,29 @@
 
 namespace ink {
 
-// A stage: one (TALL: two) tiles of 128 rows x 128 B of weights, their block scales, the N operand, its block scales.
-template <bool TALL>
+// A stage: a tile of 128 rows x 128 B of weights, its block scales, the N operand, its block scales.
+template <int T>
 struct GgStage {
-  static constexpr int kUnits = TALL ? 2 : 1, kCount = TALL ? 4 : 8;
-  static constexpr int kScalesAt = kUnits * kTcCodeBytes, kRowsAt = kScalesAt + kUnits * kTcScaleBytes;
-  static constexpr int kRowScalesAt = kRowsAt + kUnits * 8192, kBytes = kRowScalesAt + kUnits * 1024;   // 54 KB or 27 KB
-  static constexpr int kSf = kUnits * 16 + 16;   // tensor-memory columns of its scales
+  static constexpr int kCount = T == 16 ? 8 : T == 32 ? 6 : 4;
+  static constexpr int kScalesAt = kTcCodeBytes, kRowsAt = kScalesAt + kTcScaleBytes;
+  static constexpr int kRowScalesAt = kRowsAt + T * 512, kBytes = (kRowScalesAt + T * 64 + 1023) / 1024 * 1024;
+  static constexpr int kSf = T == 64 ? 48 : 32;   // tensor-memory columns of its scales
 };
 constexpr int kGgProducers = 2;   // (eleven warps: three on a scheduler, 168 registers a thread)
 constexpr int kGgThreads = 320 + (kGgProducers - 1) * 32;
 constexpr int kGgMaxGroups = 1024;
-constexpr int kGgSharedBox = 64;                                 // rows of one copy of a shared expert's gate or up matrix
-constexpr int kGgColD = 0, kGgColSf = 256;                       // tensor memory: accumulators, then each stage's scales
+constexpr int kGgPairRows = 16;                                  // shared experts: rows of gate and of up in turn
+constexpr int kGgColD = 0, kGgColSf = 256;                       // tensor memory: two accumulators, then each stage's scales
+constexpr int kGgAccCols = 128;                                  // of one: 32 tokens of digit rows or 128 BF16 tokens
 
 // tokens in a tile
-__host__ __device__ constexpr int gg_tile(bool fp4, bool tall) { return fp4 ? (tall ? 32 : 16) : (tall ? 128 : 64); }
+__host__ __device__ constexpr int gg_tile(bool fp4, int t) { return fp4 ? t : 4 * t; }
 // slots of a group are padded to whole 1024-byte swizzle atoms of its tiles
 __host__ __device__ constexpr int gg_pad(bool fp4) { return fp4 ? 2 : 8; }
 
 struct GgArgs {
   // routed experts
-  const unsigned char* maps;    // descriptors of this projection: codes and scales (NVFP4; `wide`: TALL has 256-row boxes), or one (BF16)
+  const unsigned char* maps;    // descriptors of this projection: codes and scales (NVFP4), or one (BF16)
   const int64_t* pointers;      // [(max_expert + 1) * stride]: a zero row is an inactive expert; scale2 is read through it
   const int32_t* experts;       // [groups]
   const int32_t* counts;        // [groups]
@@ -60,9 +61,9 @@ struct GgArgs {
   const unsigned char* image_scales;
   const float* slot_scale;      // [slots] (NVFP4)
   uint16_t* y;                  // BF16 [route][n / 2] (gate/up) or [route][n]
-  int groups, start, capacity, stride, bank, k, n, wide;
+  int groups, start, capacity, stride, bank, k, n;
   // shared experts
-  const unsigned char* shared_maps;    // gate and up, or down
+  const unsigned char* shared_maps;    // gate and up in one, with a word behind it that says which comes first; or down
   const unsigned char* shared_image;   // [tile][k / 64][tokens of the tile, padded to 8][128 B]; down: the same per expert
   uint16_t* shared_y;           // gate/up: the image of the down projection; down: BF16 [tokens][n_shared][n]
   const uint16_t* gammas;       // [tokens, n_shared]
@@ -139,7 +140,7 @@ __device__ __forceinline__ int gg_group_count(const int* slot0, int g, int pad) 
   return gg_first_slot(slot0, g + 1, pad) - gg_first_slot(slot0, g, pad) - (slot0[g] & (pad - 1));
 }
 
-// One work item: a 128 (256) row tile of one expert's matrix against one tile of its tokens.
+// One work item: a 128-row tile of one expert's matrix against one tile of its tokens.
 struct GgItem {
   bool shared;
   int group;      // group of routes, or shared expert
@@ -149,10 +150,10 @@ struct GgItem {
   int bank;       // index of the expert's matrix (set by the producers)
 };
 
-template <bool FP4, bool TALL>
+template <bool FP4, int T>
 struct GgWalk {
-  static constexpr int kM = TALL ? 256 : 128;
-  static constexpr int kTile = gg_tile(FP4, TALL), kPad = gg_pad(FP4), kSharedTile = gg_tile(false, TALL);
+  static constexpr int kM = kTcRows;
+  static constexpr int kTile = gg_tile(FP4, T), kPad = gg_pad(FP4), kSharedTile = gg_tile(false, T);
   const GgArgs* a;
   GgTables t;
   int m_tiles, shared_tiles;
@@ -164,7 +165,7 @@ struct GgWalk {
     return a->k / ((FP4 && !shared) ? kTcChunkK : 64);
   }
   // cost of one item with n tokens: its bytes, the streamed weights weighing most
-  __device__ static __forceinline__ int tile_cost(int n, int stages) { return stages * (64 + (TALL ? n : 2 * n) / (FP4 ? 1 : 4)); }
+  __device__ static __forceinline__ int tile_cost(int n, int stages) { return stages * (64 + (T == 16 ? 2 * n : T == 32 ? n / 4 : n) / (FP4 ? 1 : 4)); }
   __device__ __forceinline__ int cost_per_mt(int c, int stages) const {
     return c / kTile * tile_cost(kTile, stages) + (c % kTile ? tile_cost(c % kTile, stages) : 0);
   }
@@ -267,12 +268,13 @@ __device__ __forceinline__ bool elect_one() {
   return chosen != 0;
 }
 
-template <bool FP4, int PROJ, bool TALL>
+template <bool FP4, int PROJ, int T>
 __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __grid_constant__ GgArgs a) {
-  using Walk = GgWalk<FP4, TALL>;
-  using St = GgStage<TALL>;
-  constexpr int kAccs = TALL ? 1 : 2;            // accumulators in turn: the next item's MMAs run while one is read
-  constexpr int kAccCols = TALL ? 256 : 128;     // columns of one (TALL: 128 per half)
+  using Walk = GgWalk<FP4, T>;
+  using St = GgStage<T>;
+  // Two accumulators in turn: the next item's MMAs run while one is read. A tile of more than kGgAccCols columns (T = 64)
+  // takes both. `acc` counts those a role has passed: number acc & 1, for the (acc >> 1)-th time.
+  auto accs_of = [](const GgItem& it) -> int { return T < 64 ? 1 : it.n > (FP4 && !it.shared ? 32 : 128) ? 2 : 1; };
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ GgShared sh;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -344,31 +346,20 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     // (one elected lane issues a stage's copies one after the other: copies issued by several lanes of a warp at once were
     // taken apart lane by lane, 270 to 340 clocks each, 1 000 to 1 270 a stage)
     auto expect = [&](const GgItem& it, int u) {
-      uint32_t bytes = St::kUnits * kTcCodeBytes + rows_bytes(it);
-      if (FP4 && !it.shared) bytes += St::kUnits * kTcScaleBytes + rows_bytes(it) / 8u;
+      uint32_t bytes = kTcCodeBytes + rows_bytes(it);
+      if (FP4 && !it.shared) bytes += kTcScaleBytes + rows_bytes(it) / 8u;
       mbar_expect_tx(&sh.full[u], bytes);
     };
     auto issue_weights = [&](const GgItem& it, int s, int u) {
       unsigned char* stage = ring + (size_t)u * St::kBytes;
       uint64_t* bar = &sh.full[u];
-      if (PROJ == 0 && it.shared) {   // 64 rows of gate and of up (TALL: twice that)
-        constexpr int kUp = TALL ? kTcCodeBytes : kTcCodeBytes / 2;
-#pragma unroll
-        for (int half = 0; half < St::kUnits; ++half) {
-          tc_tma_3d(stage + half * (kTcCodeBytes / 2), a.shared_maps, s * 64, it.m0 / 2 + half * kGgSharedBox, it.bank, bar);
-          tc_tma_3d(stage + kUp + half * (kTcCodeBytes / 2), a.shared_maps + 128, s * 64, it.m0 / 2 + half * kGgSharedBox, it.bank, bar);
-        }
+      if (PROJ == 0 && it.shared) {   // gate and up rows, sixteen in turn: {column, row, which, block of rows, expert}
+        tc_tma_5d(stage, a.shared_maps, s * 64, 0, 0, it.m0 / (2 * kGgPairRows), it.bank, bar);
       } else if (!FP4 || it.shared) {
-        const unsigned char* map = it.shared ? a.shared_maps : a.maps;
-#pragma unroll
-        for (int unit = 0; unit < St::kUnits; ++unit) tc_tma_3d(stage + unit * kTcCodeBytes, map, s * 64, it.m0 + unit * kTcRows, it.bank, bar);
+        tc_tma_3d(stage, it.shared ? a.shared_maps : a.maps, s * 64, it.m0, it.bank, bar);
       } else {
-#pragma unroll
-        for (int unit = 0; unit < St::kUnits; ++unit) {
-          if (unit > 0 && a.wide) break;
-          tc_tma_3d(stage + unit * kTcCodeBytes, a.maps, s * 128, it.m0 + unit * kTcRows, it.bank, bar);
-          tc_tma_3d(stage + St::kScalesAt + unit * kTcScaleBytes, a.maps + 128, s * 16, it.m0 + unit * kTcRows, it.bank, bar);
-        }
+        tc_tma_3d(stage, a.maps, s * 128, it.m0, it.bank, bar);
+        tc_tma_3d(stage + St::kScalesAt, a.maps + 128, s * 16, it.m0, it.bank, bar);
       }
     };
     auto issue_rows = [&](const GgItem& it, int s, int u) {
@@ -449,19 +440,15 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     uint32_t seq = 0;
     const uint32_t ring_lo = gg_desc_lo(smem_u32(ring));
     bool ok = true;
-    for (int item = 0; ok && walk.next(it); ++item) {
+    for (uint32_t acc = 0; ok && walk.next(it);) {
       const bool fp4 = FP4 && !it.shared;
-      const int buf = kAccs == 2 ? item & 1 : 0;
-      const int columns = __shfl_sync(0xffffffffu, fp4 ? (it.n + 1) / 2 * 8 : (it.n + 15) / 16 * 16, 0);
-      const uint32_t idesc = fp4 ? tc_idesc(columns) : gg_idesc_bf16(columns);
+      const int accs = __shfl_sync(0xffffffffu, accs_of(it), 0), n = __shfl_sync(0xffffffffu, it.n, 0);
+      const int per_acc = fp4 ? 32 : 128, n_last = n - (accs - 1) * per_acc;
+      auto idesc_of = [&](int tokens) { return fp4 ? tc_idesc((tokens + 1) / 2 * 8) : gg_idesc_bf16((tokens + 15) / 16 * 16); };
+      const uint32_t idesc_last = idesc_of(n_last), idesc_first = accs > 1 ? idesc_of(per_acc) : idesc_last;
       const int stages = walk.stages_of(it.shared);
-      const uint32_t d = tmem + kGgColD + buf * kAccCols;
-      // Shared gate / up: two accumulators side by side. (!TALL: tiles of 64 rows; what the MMA reads as rows 64.. of one lies
-      // behind it in the stage, and its results go to lanes that nobody reads.)
-      const bool pair = PROJ == 0 && it.shared;
-      const int units = pair ? 2 : St::kUnits;
-      const uint32_t unit_lo = (pair && !TALL ? kTcCodeBytes / 2 : kTcCodeBytes) >> 4;
-      ok = gg_wait(&sh.d_empty[buf], (uint32_t)((item / kAccs) & 1) ^ 1u, &sh);   // this accumulator's previous item has been read
+      const uint32_t d_first = tmem + kGgColD + (acc & 1) * kGgAccCols, d_second = tmem + kGgColD + ((acc + 1) & 1) * kGgAccCols;
+      for (int i = 0; ok && i < accs; ++i) ok = gg_wait(&sh.d_empty[(acc + i) & 1], ((acc + i) >> 1 & 1u) ^ 1u, &sh);   // their previous items have been read
       if (!ok) break;
       tc_fence_after();
 #pragma unroll 1
@@ -471,19 +458,23 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
         if (FP4) ok = ok && gg_wait(&sh.full[u], parity, &sh);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t lo = ring_lo + u * (St::kBytes >> 4), sf = tmem + kGgColSf + u * St::kSf;
+        const uint32_t lo = ring_lo + u * (St::kBytes >> 4), rows = lo + (St::kRowsAt >> 4), sf = tmem + kGgColSf + u * St::kSf;
         if (elect_one()) {
-#pragma unroll
-          for (int unit = 0; unit < 2; ++unit) {
-            if (unit == 1 && units == 1) break;
-            if (fp4) gg_mma4_fp4(d + unit * (kAccCols / 2), lo + unit * unit_lo, lo + (St::kRowsAt >> 4), idesc, s != 0, sf + unit * 16, sf + St::kUnits * 16);
-            else gg_mma4_bf16(d + unit * (kAccCols / 2), lo + unit * unit_lo, lo + (St::kRowsAt >> 4), idesc, s != 0);
+          if (fp4) gg_mma4_fp4(d_first, lo, rows, idesc_first, s != 0, sf, sf + 16);
+          else gg_mma4_bf16(d_first, lo, rows, idesc_first, s != 0);
+          if (T == 64 && accs > 1) {   // the tile's upper half: 16 KB further in the N operand, whichever its type
+            if (fp4) gg_mma4_fp4(d_second, lo, rows + (16384 >> 4), idesc_last, s != 0, sf, sf + 32);
+            else gg_mma4_bf16(d_second, lo, rows + (16384 >> 4), idesc_last, s != 0);
           }
           tc_commit(&sh.empty[u]);
-          if (s + 1 == stages) tc_commit(&sh.d_full[buf]);
+          if (s + 1 == stages) {
+            tc_commit(&sh.d_full[acc & 1]);
+            if (T == 64 && accs > 1) tc_commit(&sh.d_full[(acc + 1) & 1]);
+          }
         }
         __syncwarp();
       }
+      acc += accs;
     }
   } else if (warp < 6) {
     // =========================================================== block scales: shared -> tensor memory
@@ -512,9 +503,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
               tc_st16(tmem + lane_base + kGgColSf + u * St::kSf + column, w);
             };
             tc_fence_after();
-#pragma unroll
-            for (int unit = 0; unit < St::kUnits; ++unit) upload(stage + St::kScalesAt + unit * kTcScaleBytes, true, unit * 16);
-            upload(stage + St::kRowScalesAt, TALL, St::kUnits * 16);
+            upload(stage + St::kScalesAt, true, 0);
+            upload(stage + St::kRowScalesAt, T > 16, 16);
+            if (T == 64 && it.n > 32) upload(stage + St::kRowScalesAt + 2048, true, 32);
             tc_wait_st();
             tc_fence_before();
           }
@@ -529,60 +520,26 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     const int sub = warp & 3;
     const uint32_t lane_base = (uint32_t)(sub * 32) << 16;
     GgItem it;
-    for (int item = 0; walk.next(it); ++item) {
+    bool ok = true;
+    for (uint32_t acc = 0; ok && walk.next(it);) {
       const bool fp4 = FP4 && !it.shared;
-      const int buf = kAccs == 2 ? item & 1 : 0;
       const int expert = it.shared ? 0 : a.experts[it.group];
       const float scale2 = fp4 ? *reinterpret_cast<const float*>(a.pointers[(size_t)expert * a.stride + a.bank + 2]) : 1.f;
-      const int per_chunk = fp4 ? 8 : 32, token_chunks = (it.n + per_chunk - 1) / per_chunk;
+      const int per_chunk = fp4 ? 8 : 32, per_acc = fp4 ? 32 : 128;
+      const int r = it.m0 + sub * 32 + lane;   // this thread's weight row
       // lane i holds token i of a chunk: its route (or token number), and its scale
-      auto token_of = [&](int chunk, float& scale) -> int {
-        const int i = chunk * per_chunk + lane;
+      auto token_of = [&](int at, float& scale) -> int {   // `at`: the chunk's first token in the tile
+        const int i = at + lane;
         scale = 0.f;
         if (lane >= per_chunk || i >= it.n) return -1;
         if (it.shared) return it.tile * Walk::kSharedTile + i;
         if (fp4) scale = scale2 * a.slot_scale[it.slot + i];
         return a.rows[(size_t)it.group * a.capacity + it.tile * Walk::kTile + i];
       };
-      float my_scale;
-      int my_token = token_of(0, my_scale);
-      const bool ok = __all_sync(0xffffffffu, gg_wait(&sh.d_full[buf], (uint32_t)((item / kAccs) & 1), &sh));
-      if (!ok) break;
-      tc_fence_after();
-      if (PROJ == 0 && it.shared) {
-        // a lane has a pair's gate in one accumulator and its up in the other
-        const int row = sub * 32 + lane, pair = it.m0 / 2 + row;
-        if (TALL || sub < 2) {
-#pragma unroll 1
-          for (int chunk = 0; chunk < token_chunks; ++chunk) {
-            float gate[32], up[32];
-            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + chunk * 32, gate);
-            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + kAccCols / 2 + chunk * 32, up);
-            const int here = min(32, it.n - chunk * 32), padded = (a.tokens + 7) / 8 * 8, f = a.n / 2;
-            unsigned char* tile = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
-                                  (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + (pair & 7) * 2;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (j >= here) break;
-              // the reference's BF16 tensor ops: both bmm outputs, silu, the product and the product with gamma round
-              const int at = chunk * 32 + j, token = it.tile * Walk::kSharedTile + at;
-              const float g = round_bf16(gate[j]), u = round_bf16(up[j]);
-              const float act = round_bf16(round_bf16(g / (1.f + expf(-g))) * u);
-              const float gamma = bf16_to_f32(a.gammas[(size_t)token * a.n_shared + it.group]);
-              if (pair < f) *reinterpret_cast<uint16_t*>(tile + at * 128 + ((((pair & 63) >> 3) ^ (at & 7)) << 4)) = (uint16_t)f32_to_bf16_bits(act * gamma);
-            }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
-        continue;
-      }
-      // this thread's weight row for the tokens of a chunk (lane j holds token j's route, or number)
-      auto write = [&](auto& v, int half, int chunk, int tokens) {
+      // this thread's weight row for the tokens at .. of a chunk (lane j holds token j's route, or number)
+      auto write = [&](auto& v, int at, int tokens) {
         constexpr int kChunk = sizeof(v) / sizeof(float);
-        const int r = it.m0 + half * kTcRows + sub * 32 + lane;
-        const int here = min(kChunk, it.n - chunk * kChunk);
+        const int here = min(kChunk, it.n - at);
         if (PROJ == 0) {
           // gate and up rows alternate, so neighbouring lanes hold a pair: of two tokens each lane finishes one
           const bool second = (lane & 1) != 0;
@@ -593,7 +550,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
             const float other = __shfl_xor_sync(0xffffffffu, second ? v[j] : v[j + 1], 1);
             const float gate = second ? other : v[j], up = second ? v[j + 1] : other;
             const int token = __shfl_sync(0xffffffffu, tokens, second ? j + 1 : j);
-            if (token >= 0 && 2 * pair < a.n) a.y[(size_t)token * (a.n / 2) + pair] = (uint16_t)f32_to_bf16_bits(silu_mul(gate, up));
+            if (token >= 0) a.y[(size_t)token * (a.n / 2) + pair] = (uint16_t)f32_to_bf16_bits(silu_mul(gate, up));
           }
         } else {
 #pragma unroll
@@ -601,61 +558,103 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
             if (j >= here) break;
             const int token = __shfl_sync(0xffffffffu, tokens, j);
             uint16_t* y = it.shared ? a.shared_y + ((size_t)token * a.n_shared + it.group) * a.n : a.y + (size_t)token * a.n;
-            if (r < a.n) y[r] = (uint16_t)f32_to_bf16_bits(v[j]);
+            y[r] = (uint16_t)f32_to_bf16_bits(v[j]);
           }
         }
       };
       if constexpr (FP4) {
         if (!it.shared) {
-          // Everything into registers first (four digit columns add up to a token), so that the accumulator is free for the
-          // next item before the outputs are written: with one accumulator (TALL) its MMAs wait for that.
-          constexpr int kHalves = TALL ? 2 : 1, kChunks = gg_tile(true, TALL) / 8;
-          float v[kHalves][kChunks][8];
+          // Everything into registers first (four digit columns add up to a token), so that the accumulators are free for the
+          // next items before the outputs are written: written one by one, the second waited for the first one's outputs and
+          // the MMAs for both (a fifth of the gate/up projection of 1 999 tokens).
+          constexpr int kChunks = T / 8;
+          float v[kChunks][8], my_scale;
+          int my_token = token_of(0, my_scale);   // (asked for before the wait)
 #pragma unroll
-          for (int half = 0; half < kHalves; ++half) {
+          for (int i = 0; i < (T == 64 ? 2 : 1); ++i) {
+            if (i * 32 >= it.n) break;
+            const int buf = acc & 1;
+            ok = __all_sync(0xffffffffu, gg_wait(&sh.d_full[buf], (acc >> 1) & 1u, &sh));
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll
-            for (int chunk = 0; chunk < kChunks; ++chunk) {
-              if (chunk * 8 >= it.n) break;
+            for (int c = 0; c < (T < 32 ? T : 32) / 8; ++c) {
+              if (i * 32 + c * 8 >= it.n) break;
               float w[32];
-              tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, w);
+              tc_ld32(tmem + lane_base + kGgColD + buf * kGgAccCols + c * 32, w);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) v[half][chunk][j] = (w[4 * j] + w[4 * j + 1]) + (w[4 * j + 2] + w[4 * j + 3]);
+              for (int j = 0; j < 8; ++j) v[i * 4 + c][j] = (w[4 * j] + w[4 * j + 1]) + (w[4 * j + 2] + w[4 * j + 3]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
+            ++acc;
+          }
+          if (!ok) break;
+#pragma unroll
+          for (int chunk = 0; chunk < kChunks; ++chunk) {
+            if (chunk * 8 >= it.n) break;
+            if (chunk > 0) my_token = token_of(chunk * 8, my_scale);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[chunk][j] *= __shfl_sync(0xffffffffu, my_scale, j);
+            write(v[chunk], chunk * 8, my_token);
+          }
+          continue;
+        }
+      }
+#pragma unroll 1
+      for (int first = 0; first < it.n; first += per_acc, ++acc) {   // (an item's accumulators, one after the other)
+        const int buf = acc & 1, here_n = min(per_acc, it.n - first), token_chunks = (here_n + per_chunk - 1) / per_chunk;
+        const uint32_t d = tmem + lane_base + kGgColD + buf * kGgAccCols;
+        float unused;
+        const int first_token = token_of(first, unused);
+        ok = __all_sync(0xffffffffu, gg_wait(&sh.d_full[buf], (acc >> 1) & 1u, &sh));
+        if (!ok) break;
+        tc_fence_after();
+        if (PROJ == 0 && it.shared) {
+          // lanes 0-15 hold sixteen pairs' gate rows, lanes 16-31 their up rows (or the other way round): of two tokens each
+          // lane finishes one
+          const bool second = (lane & 16) != 0, up_first = *reinterpret_cast<const int*>(a.shared_maps + 128) != 0;
+          const int pair = it.m0 / 2 + sub * kGgPairRows + (lane & 15), padded = (a.tokens + 7) / 8 * 8, f = a.n / 2;
+          unsigned char* tile = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
+                                (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + (pair & 7) * 2;
+#pragma unroll 1
+          for (int chunk = 0; chunk < token_chunks; ++chunk) {
+            float v[32];
+            tc_ld32(d + chunk * 32, v);
+            const int here = min(32, here_n - chunk * 32);
+            const int at0 = first + chunk * 32, mine = min(at0 + lane, it.n - 1);   // (lane j's gamma is that of token j)
+            const float my_gamma = bf16_to_f32(a.gammas[(size_t)(it.tile * Walk::kSharedTile + mine) * a.n_shared + it.group]);
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              if (j >= here) break;
+              // the reference's BF16 tensor ops: both bmm outputs, silu, the product and the product with gamma round
+              const float other = __shfl_xor_sync(0xffffffffu, second ? v[j] : v[j + 1], 16), own = second ? v[j + 1] : v[j];
+              const float gamma = __shfl_sync(0xffffffffu, my_gamma, second ? j + 1 : j);
+              const float g = round_bf16(second != up_first ? other : own), u = round_bf16(second != up_first ? own : other);
+              const float act = round_bf16(round_bf16(g / (1.f + expf(-g))) * u);
+              const int at = at0 + j + (second ? 1 : 0);
+              if (at < it.n) *reinterpret_cast<uint16_t*>(tile + at * 128 + ((((pair & 63) >> 3) ^ (at & 7)) << 4)) = (uint16_t)f32_to_bf16_bits(act * gamma);
             }
           }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
-#pragma unroll
-          for (int chunk = 0; chunk < kChunks; ++chunk) {
-            if (chunk * 8 >= it.n) break;
-            if (chunk > 0) my_token = token_of(chunk, my_scale);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float scale = __shfl_sync(0xffffffffu, my_scale, j);
-#pragma unroll
-              for (int half = 0; half < kHalves; ++half) v[half][chunk][j] *= scale;
-            }
-#pragma unroll
-            for (int half = 0; half < kHalves; ++half) write(v[half][chunk], half, chunk, my_token);
-          }
           continue;
         }
-      }
-      if constexpr (!FP4 || PROJ == 1) {
-#pragma unroll 1
-        for (int half = 0; half < (TALL ? 2 : 1); ++half) {
+        if constexpr (!FP4 || PROJ == 1) {
 #pragma unroll 1
           for (int chunk = 0; chunk < token_chunks; ++chunk) {
-            const int tokens = token_chunks > 1 ? token_of(chunk, my_scale) : my_token;
+            const int tokens = chunk > 0 ? token_of(first + chunk * 32, unused) : first_token;
             float v[32];
-            tc_ld32(tmem + lane_base + kGgColD + buf * kAccCols + half * 128 + chunk * 32, v);
-            write(v, half, chunk, tokens);
+            tc_ld32(d + chunk * 32, v);
+            write(v, first + chunk * 32, tokens);
           }
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.d_empty[buf]);
     }
   }
   __syncwarp();
@@ -864,28 +863,30 @@ static cudaError_t launch_dependent(void (*kernel)(Args), dim3 grid, int threads
   return cudaLaunchKernelEx(&config, kernel, args);
 }
 
-template <bool FP4, int PROJ, bool TALL>
+template <bool FP4, int PROJ, int T>
 static int launch_grouped(const GgArgs& a, cudaStream_t stream) {
-  constexpr size_t kRing = (size_t)GgStage<TALL>::kCount * GgStage<TALL>::kBytes + 1024;
+  constexpr size_t kRing = (size_t)GgStage<T>::kCount * GgStage<T>::kBytes + 1024;
+  static_assert(kGgColSf + GgStage<T>::kCount * GgStage<T>::kSf <= 512, "tensor memory");
   constexpr int kMaxDevices = 64;
   static bool configured[kMaxDevices] = {};
   int device = 0;
   cudaGetDevice(&device);
   INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "grouped projections: device ordinal %d", device);
   if (!configured[device]) {
-    const size_t most = kRing + 2 * sizeof(int) * (kGgMaxGroups + 1);
-    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<FP4, PROJ, TALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    constexpr size_t most = kRing + 2 * sizeof(int) * (kGgMaxGroups + 1);
+    static_assert(most + sizeof(GgShared) <= 227 * 1024, "shared memory");
+    cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel<FP4, PROJ, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "grouped projections: %zu bytes of shared memory refused: %s", most, cudaGetErrorString(e));
     configured[device] = true;
   }
-  const cudaError_t e = launch_dependent(grouped_gemm_kernel<FP4, PROJ, TALL>, dim3(gg_sms()), kGgThreads,
+  const cudaError_t e = launch_dependent(grouped_gemm_kernel<FP4, PROJ, T>, dim3(gg_sms()), kGgThreads,
                                          kRing + 2 * sizeof(int) * (a.groups + 1), stream, a);
   INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "grouped projections: launch failed: %s", cudaGetErrorString(e));
   return kOk;
 }
 template <bool FP4, int PROJ>
-static int launch_grouped(bool tall, const GgArgs& a, cudaStream_t s) {
-  return tall ? launch_grouped<FP4, PROJ, true>(a, s) : launch_grouped<FP4, PROJ, false>(a, s);
+static int launch_grouped(int tokens, const GgArgs& a, cudaStream_t s) {
+  return tokens == 64 ? launch_grouped<FP4, PROJ, 64>(a, s) : tokens == 32 ? launch_grouped<FP4, PROJ, 32>(a, s) : launch_grouped<FP4, PROJ, 16>(a, s);
 }
 
 static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStream_t stream) {
@@ -897,9 +898,10 @@ static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStre
   return kOk;
 }
 
-// Tall tiles pay where an expert has more than a few tokens: below, every weight tile meets one tile of tokens anyway and
-// the smaller items even out better (measured: see the table of the design notes).
-static bool gg_tall(long long routes, int experts) { return routes > 8LL * experts; }
+// Tokens T of a tile, from the mean number of routes per expert. Routed experts of one layer at full width (256 of 4096 x 2048),
+// evenly / unevenly chosen (rank^-0.6), T = 16, 32, 64, us a call:  mean 4: 606 610 655 / 596 598 643;  8: 668 647 707 / 680 653
+// 721;  24: 1114 823 868 / 1145 924 948;  36: 1516 1245 1102 / 1526 1175 1194;  48: 1948 1620 1405 / 2119 1511 1502.
+static int gg_tokens(long long routes, int experts) { return routes > 24LL * experts ? 64 : routes > 8LL * experts ? 32 : 16; }
 
 }  // namespace ink
 
@@ -919,32 +921,30 @@ extern "C" int ink_encode_bf16_banks(void* out_host_256, const void* gate_up, ui
 extern "C" int ink_encode_shared(void* out_host_384, const void* gate, const void* up, const void* down, int n_shared, int hidden, int intermediate) {
   INK_REQUIRE(out_host_384 != nullptr && n_shared >= 1, kBadArgument, "encode_shared: null output or no experts");
   INK_REQUIRE(hidden % 64 == 0 && intermediate % 64 == 0, kUnsupportedShape, "encode_shared: hidden=%d intermediate=%d", hidden, intermediate);
-  CUtensorMap maps[3];
-  const uint64_t stride = 2ull * hidden * intermediate;
-  int rc = encode_rows(&maps[0], gate, 2, stride, n_shared, intermediate, hidden, 64, kGgSharedBox, true);
-  if (rc == kOk) rc = encode_rows(&maps[1], up, 2, stride, n_shared, intermediate, hidden, 64, kGgSharedBox, true);
-  if (rc == kOk) rc = encode_rows(&maps[2], down, 2, stride, n_shared, hidden, intermediate, 64, kTcRows, true);
-  if (rc == kOk) memcpy(out_host_384, maps, sizeof(maps));
-  return rc;
-}
-
-// The boxes of both forms of the kernel: 128 rows of codes and scales (the 512 bytes of ink_moe_stack_encode_banks), 256 rows.
-extern "C" int ink_encode_grouped_banks(void* out_host_1024, const void* gate_up_codes, uint64_t gate_up_codes_stride, const void* gate_up_scales,
-                                        uint64_t gate_up_scales_stride, const void* down_codes, uint64_t down_codes_stride, const void* down_scales,
-                                        uint64_t down_scales_stride, int experts, int hidden, int intermediate) {
-  INK_REQUIRE(out_host_1024 != nullptr && experts >= 1, kBadArgument, "encode_grouped_banks: null output or no experts");
-  INK_REQUIRE(hidden % kTcChunkK == 0 && intermediate % kTcChunkK == 0, kUnsupportedShape, "encode_grouped_banks: hidden=%d intermediate=%d", hidden, intermediate);
-  CUtensorMap maps[8];
-  int rc = kOk;
-  for (int i = 0; i < 4 && rc == kOk; ++i) {
-    const int rows = kTcRows << (i >> 1);   // forms; then projections
-    const bool down = i & 1;
-    const int n = down ? hidden : 2 * intermediate, k = down ? intermediate : hidden;
-    rc = encode_rows(&maps[2 * i], down ? down_codes : gate_up_codes, 1, down ? down_codes_stride : gate_up_codes_stride, experts, n, k / 2, 128, rows, true);
-    if (rc == kOk) rc = encode_rows(&maps[2 * i + 1], down ? down_scales : gate_up_scales, 1, down ? down_scales_stride : gate_up_scales_stride, experts, n, k / 16, 16, rows, false);
-  }
-  if (rc == kOk) memcpy(out_host_1024, maps, sizeof(maps));
-  return rc;
+  // Gate and up in one descriptor, sixteen rows of each in turn, the one at the lower address first; the word
+  // that follows it is not zero if that is `up`.
+  const bool up_first = (uintptr_t)up < (uintptr_t)gate;
+  const uintptr_t low = (uintptr_t)(up_first ? up : gate), high = (uintptr_t)(up_first ? gate : up);
+  const uint64_t stride = 2ull * hidden * intermediate, row_bytes = 2ull * hidden;
+  unsigned char maps[384] = {};
+  TensorMapEncodeFn enc = tensor_map_encoder();
+  INK_REQUIRE(enc != nullptr, kLaunchFailed, "encode_shared: the driver has no cuTensorMapEncodeTiled");
+  INK_REQUIRE(low != 0 && low % 16 == 0 && high % 16 == 0 && high > low && high - low < (1ull << 40), kMisaligned,
+              "encode_shared: gate at %p and up at %p", gate, up);
+  cuuint64_t dims[5] = {(cuuint64_t)hidden, (cuuint64_t)kGgPairRows, 2, (cuuint64_t)(intermediate / kGgPairRows), (cuuint64_t)n_shared};
+  cuuint64_t strides[4] = {row_bytes, high - low, kGgPairRows * row_bytes, stride};
+  cuuint32_t box[5] = {64, (cuuint32_t)kGgPairRows, 2, (cuuint32_t)(kTcRows / 2 / kGgPairRows), 1}, elem[5] = {1, 1, 1, 1, 1};
+  CUtensorMap both;
+  const CUresult r = enc(&both, CU_TENSOR_MAP_DATA_TYPE_UINT16, 5, (void*)low, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  INK_REQUIRE(r == CUDA_SUCCESS, kBadArgument, "encode_shared: cuTensorMapEncodeTiled returned %d", (int)r);
+  memcpy(maps, &both, sizeof(both));
+  maps[128] = up_first ? 1 : 0;
+  CUtensorMap last;
+  if (int rc = encode_rows(&last, down, 2, stride, n_shared, hidden, intermediate, 64, kTcRows, true)) return rc;
+  memcpy(maps + 256, &last, sizeof(last));
+  memcpy(out_host_384, maps, sizeof(maps));
+  return kOk;
 }
 
 static int check_grouped_shape(bool fp4, int n, int k, int groups) {
@@ -990,7 +990,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   unsigned char *act_image = take(act.image), *act_scales = take(act.image_scales), *act_slot = take(act.slot_scale);
   unsigned char *x_image = take(n_shared ? padded * hidden * 2 : 0), *sact_image = take(padded * n_shared * intermediate * 2);
   unsigned char* shared_out = take((size_t)tokens * n_shared * hidden * 2);
-  const bool tall = gg_tall((long long)routes, local);
+  const int t = gg_tokens((long long)routes, local);
   const int bank = fp4 ? 3 : 1, stride = fp4 ? kBank : 2;
 
   StageArgs st = {};
@@ -1010,13 +1010,12 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   st.k = hidden;
   st.div = top_k;
   st.tokens = tokens;
-  st.tile = gg_tile(fp4, tall);
-  st.shared_tile = gg_tile(false, tall);
+  st.tile = gg_tile(fp4, t);
+  st.shared_tile = gg_tile(false, t);
   if (int rc = launch_stage(fp4, st, routes + (n_shared ? tokens : 0), s)) return rc;
 
   GgArgs g = {};
-  g.maps = (const unsigned char*)bank_maps + (fp4 && tall ? 512 : 0);
-  g.wide = 1;
+  g.maps = (const unsigned char*)bank_maps;
   g.pointers = pointers;
   g.experts = experts;
   g.counts = counts;
@@ -1039,7 +1038,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   g.n_shared = n_shared;
   g.tokens = tokens;
   g.status = status;
-  if (int rc = fp4 ? launch_grouped<true, 0>(tall, g, s) : launch_grouped<false, 0>(tall, g, s)) return rc;
+  if (int rc = fp4 ? launch_grouped<true, 0>(t, g, s) : launch_grouped<false, 0>(t, g, s)) return rc;
 
   st.x = (const uint16_t*)activated;
   st.image = act_image;
@@ -1063,7 +1062,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   g.shared_maps = n_shared ? g.shared_maps + 256 : nullptr;
   g.shared_image = sact_image;
   g.shared_y = (uint16_t*)shared_out;
-  if (int rc = fp4 ? launch_grouped<true, 1>(tall, g, s) : launch_grouped<false, 1>(tall, g, s)) return rc;
+  if (int rc = fp4 ? launch_grouped<true, 1>(t, g, s) : launch_grouped<false, 1>(t, g, s)) return rc;
 
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)tokens, (unsigned)((hidden / 8 + 255) / 256));
@@ -1106,7 +1105,7 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   if (groups == 0 || routes == 0) return kOk;
   cudaStream_t s = (cudaStream_t)stream;
   const GgScratch sizes(true, routes, groups, k);
-  const bool tall = gg_tall((long long)routes, groups);
+  const int t = gg_tokens((long long)routes, groups);
   StageArgs st = {};
   st.x = (const uint16_t*)x;
   st.pointers = pointers;
@@ -1122,8 +1121,8 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   st.bank = projection ? 3 : 0;
   st.k = k;
   st.div = projection ? 1 : top_k;
-  st.tile = gg_tile(true, tall);
-  st.shared_tile = gg_tile(false, tall);
+  st.tile = gg_tile(true, t);
+  st.shared_tile = gg_tile(false, t);
   if (int rc = launch_stage(true, st, routes, s)) return rc;
   GgArgs g = {};
   g.maps = (const unsigned char*)bank_maps + (projection ? 256 : 0);
@@ -1143,5 +1142,5 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   g.k = k;
   g.n = n;
   g.status = status;
-  return projection == 0 ? launch_grouped<true, 0>(tall, g, s) : launch_grouped<true, 1>(tall, g, s);
+  return projection == 0 ? launch_grouped<true, 0>(t, g, s) : launch_grouped<true, 1>(t, g, s);
 }

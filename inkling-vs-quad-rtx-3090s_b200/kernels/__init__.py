@@ -1,7 +1,7 @@
 """Drop-in counterpart of the reference's `kernels` package for the NVFP4
 routed-expert path: same names, same call signatures, sm_100a library underneath."""
 from .expert_planner import expert_copy, expert_plan
-from .grouped_experts import (block_scaled_supported, encode_bank_maps, encode_bf16_bank_maps, encode_grouped_bank_maps, encode_shared_maps,
+from .grouped_experts import (block_scaled_supported, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps,
                               expert_bank_names, expert_gemm, expert_reduce, moe_grouped)
 from .attention import decode_attention, update_kv
 from .routed_decode import add_rmsnorm, moe_decode, routed_decode, short_conv
@@ -13,7 +13,6 @@ __all__ = [
     "block_scaled_supported",
     "encode_bank_maps",
     "encode_bf16_bank_maps",
-    "encode_grouped_bank_maps",
     "encode_shared_maps",
     "expert_bank_names",
     "expert_copy",

@@ -40,7 +40,6 @@ _SIGNATURES = {
     "ink_expert_reduce": (I, [P, P, P, P, P, I, I, I, I, I, P]),
     "ink_expert_gemm_tc_scratch_bytes": (Z, [I, I]),
     "ink_expert_gemm_tc": (I, [P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, P, Z, P, P]),
-    "ink_encode_grouped_banks": (I, [P, P, ctypes.c_uint64, P, ctypes.c_uint64, P, ctypes.c_uint64, P, ctypes.c_uint64, I, I, I]),
     "ink_encode_bf16_banks": (I, [P, P, ctypes.c_uint64, P, ctypes.c_uint64, I, I, I]),
     "ink_encode_shared": (I, [P, P, P, P, I, I, I]),
     "ink_moe_grouped_scratch_bytes": (Z, [I, I, I, I, I, I, I]),

@@ -46,14 +46,6 @@ def encode_bank_maps(layout, experts: int, hidden: int, intermediate: int, devic
         out, gc, gcs, gs, gss, dc, dcs, ds, dss, experts, hidden, intermediate))
 
 
-def encode_grouped_bank_maps(layout, experts: int, hidden: int, intermediate: int, device) -> torch.Tensor:
-    """The descriptors `moe_grouped` takes for the same banks (ink_encode_grouped_banks): 1024 bytes, those of
-    `encode_bank_maps` first."""
-    (gc, gcs), (gs, gss), (dc, dcs), (ds, dss) = layout
-    return _maps_to_device(1024, device, lambda out: _abi.lib().ink_encode_grouped_banks(
-        out, gc, gcs, gs, gss, dc, dcs, ds, dss, experts, hidden, intermediate))
-
-
 def encode_bf16_bank_maps(layout, experts: int, hidden: int, intermediate: int, device) -> torch.Tensor:
     """The same for evenly spaced BF16 banks (ink_encode_bf16_banks): `layout` = ((address of expert 0, byte distance
     between experts) for gate_up_proj, down_proj)."""

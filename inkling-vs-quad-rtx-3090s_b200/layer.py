@@ -19,7 +19,7 @@ import struct
 import torch
 from torch import nn
 
-from .kernels import (StackDescriptor, encode_bf16_bank_maps, encode_grouped_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
+from .kernels import (StackDescriptor, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
                       expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode,
                       router_plan_forward, router_workspace, stack_supported)
 from .kernels._host import host
@@ -91,7 +91,7 @@ class ResidentExperts(nn.Module):
         self.bank_maps = None
         step, widest = (256 if self.quantized else 128), max(hidden_dim, intermediate_dim)
         if self.bank_layout is not None and hidden_dim % step == 0 and intermediate_dim % step == 0 and widest <= 4096 and self.local <= 1024:
-            encode = encode_grouped_bank_maps if self.quantized else encode_bf16_bank_maps
+            encode = encode_bank_maps if self.quantized else encode_bf16_bank_maps
             self.bank_maps = encode(self.bank_layout, self.local, hidden_dim, intermediate_dim, self.device)
         self.resident = torch.ones(self.local, **i32)
         self.destinations = torch.zeros((0, self.stride), dtype=torch.int64, device=self.device)

@@ -32,8 +32,9 @@ def one_allocation_per_kind(banks, device):
 
 @pytest.mark.parametrize("d,f,experts,tokens", [
     (1024, 512, 32, 2), (1024, 512, 32, 15), (1024, 512, 32, 17), (1024, 512, 32, 65),   # tiles of 16 and 64 tokens
-    (512, 256, 4, 33), (512, 256, 4, 129),                                                # tall tiles of 32 and 128
-    (512, 768, 4, 31), (256, 256, 16, 9),                                                 # an odd number of chunks; a single one
+    (512, 256, 16, 70), (512, 768, 4, 31),                                                # of 32 and 128; an odd number of chunks
+    (512, 256, 4, 33), (512, 256, 4, 129), (512, 256, 4, 300),                            # of 64 and 256: one or both accumulators
+    (256, 256, 16, 9),                                                                    # a single chunk
 ])
 def test_a_block_of_several_tokens(ib, device, d, f, experts, tokens):
     p, banks, x = cases.make_layer(d, f, experts, 2, 3, tokens, seed=tokens, bias="randn")
@@ -51,7 +52,7 @@ def test_a_block_of_several_tokens(ib, device, d, f, experts, tokens):
     assert max_rel(alone, oracle_moe.routed_experts_fp32(x, idx, w, banks)) <= TOL
 
 
-@pytest.mark.parametrize("d,f,experts,tokens", [(256, 128, 8, 2), (256, 128, 8, 70), (384, 128, 2, 131), (512, 256, 5, 17)])
+@pytest.mark.parametrize("d,f,experts,tokens", [(256, 128, 8, 2), (256, 128, 8, 70), (384, 128, 2, 131), (256, 128, 2, 300), (512, 256, 5, 17)])
 def test_unquantised_banks_of_several_tokens(ib, device, d, f, experts, tokens):
     gen = torch.Generator().manual_seed(tokens)
     banks = {e: dict(gate_up_proj=(torch.randn(2 * f, d, generator=gen) * 0.05).to(BF16), down_proj=(torch.randn(d, f, generator=gen) * 0.05).to(BF16))
