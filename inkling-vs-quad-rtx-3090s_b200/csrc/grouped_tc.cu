@@ -750,7 +750,8 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) 
       for (int w = 0; w < kStageThreads / 32; ++w) amax = max(amax, s_amax[w]);
       float inverse;
       const float scale = pow2_normaliser(amax, &inverse);
-      if (threadIdx.x == 0) a.slot_scale[slot0 + row] = inverse * (1.f / 512.f);
+      // (digits cannot hold a NaN or an infinity: the token's scale carries it into all of its results)
+      if (threadIdx.x == 0) a.slot_scale[slot0 + row] = amax >= 0x7f80u ? __int_as_float(0x7fffffff) : inverse * (1.f / 512.f);
       unsigned char* image = a.image + (size_t)slot0 * a.k * 2 + (size_t)row * 512;
       unsigned char* scales = a.image_scales + (size_t)slot0 * (a.k / 4) + (size_t)row * 64;
 #pragma unroll

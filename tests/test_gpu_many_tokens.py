@@ -179,3 +179,27 @@ def test_a_first_call_may_be_one_under_capture(ib, device, tokens):
         out = layer(x)
     graph.replay()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("tokens", [2, 9, 70])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 2.0 ** 126])
+def test_a_token_that_is_not_finite_stays_its_own(ib, device, tokens, value):
+    """A NaN or an infinity in one token (or, with 2^126, in its gate/up result only) reaches all of its outputs: every row of
+    the second projection has a non-zero weight for a non-finite input. The others keep their bits."""
+    d, f = 512, 256
+    p, banks, x = cases.make_layer(d, f, 8, 2, 3, tokens, seed=4, bias="randn")
+    module = ib.ResidentExperts(d, f, None, one_allocation_per_kind(banks, device))
+    gen = torch.Generator().manual_seed(2)
+    idx = torch.stack([torch.randperm(8, generator=gen)[:3] for _ in range(tokens)]).to(device)
+    w = (0.5 + torch.rand(tokens, 3, generator=gen)).to(BF16).to(device)
+    x = x.to(device)
+    clean = module(x, idx, w)
+    bad = tokens // 2
+    x[bad, 100:200:50] = value
+    got = module(x, idx, w)
+    assert not torch.isfinite(got[bad]).any()
+    rest = [t for t in range(tokens) if t != bad]
+    assert torch.equal(got[rest], clean[rest])
+    block = ib.FusedMoE(p["router_weight"][:8].to(device).contiguous(), p["router_bias"].to(device), p["global_scale"].to(device), p["route_scale"], 3,
+                        *(torch.empty(0, *s, dtype=BF16, device=device) for s in ((f, d), (f, d), (d, f))), module, None)
+    assert not torch.isfinite(block(x)[bad]).any()
