@@ -69,16 +69,16 @@ at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, si
     if (cudaMemsetAsync(t.data_ptr(), 0, counters, stream) != cudaSuccess) fail("decode_attention: the workspace could not be cleared");
     return t;
   }
-  struct Kept {
+  struct Workspace {
     size_t counters = 0;
     at::Tensor t;
   };
   constexpr size_t kMostWorkspaces = 64;
   static std::mutex mutex;
-  static auto* pool = new std::map<std::pair<int, cudaStream_t>, Kept>();   // (not destroyed at exit: the CUDA context may be gone)
+  static auto* pool = new std::map<std::pair<int, cudaStream_t>, Workspace>();   // (not destroyed at exit: the CUDA context may be gone)
   const std::lock_guard<std::mutex> lock(mutex);
   if (pool->size() >= kMostWorkspaces && !pool->count({device.index(), stream})) pool->clear();
-  Kept& kept = (*pool)[{device.index(), stream}];
+  Workspace& kept = (*pool)[{device.index(), stream}];
   if (!kept.t.defined() || kept.counters != counters || (size_t)kept.t.numel() < bytes) {
     kept.t = at::Tensor();
     kept.t = at::zeros({(int64_t)bytes}, options);
@@ -136,14 +136,22 @@ PyObject* decode_attention(PyObject* const* args) {
 
 // ------------------------------------------------------------------------------------------------ blocks
 // What the calls need of a module, taken down once (the module makes a new record when one of its tensors is replaced).
-// The record holds the tensors themselves beside their addresses: storage that was exchanged underneath a tensor shows as
-// another address, and the call then returns NotImplemented for the module to make a new record.
+// The record holds the tensors themselves beside what was found of them: a tensor whose storage, type, sizes or strides were
+// exchanged underneath shows, and the call then returns NotImplemented for the module to check it and make a new record.
+struct Kept {
+  int field;
+  at::Tensor t;
+  at::ScalarType type;
+  at::DimVector sizes, strides;
+};
 struct Block {
   long long v[48] = {};
-  std::vector<std::pair<int, at::Tensor>> kept;
+  std::vector<Kept> kept;
   bool current() const {
-    for (const auto& [f, t] : kept)
-      if ((long long)(uintptr_t)t.data_ptr() != v[f]) return false;
+    for (const Kept& k : kept)
+      if ((long long)(uintptr_t)k.t.data_ptr() != v[k.field] || k.t.scalar_type() != k.type || k.t.sizes() != at::IntArrayRef(k.sizes) ||
+          k.t.strides() != at::IntArrayRef(k.strides))
+        return false;
     return true;
   }
 };
@@ -171,7 +179,7 @@ PyObject* make_block(PyObject* const* args) {
     if (THPVariable_Check(item)) {
       const at::Tensor& t = THPVariable_Unpack(item);
       block->v[f] = (long long)(uintptr_t)t.data_ptr();
-      block->kept.emplace_back(f, t);
+      block->kept.push_back({f, t, t.scalar_type(), at::DimVector(t.sizes()), at::DimVector(t.strides())});
       continue;
     }
     block->v[f] = PyLong_AsLongLong(item);

@@ -22,6 +22,7 @@ from torch import nn
 from .kernels import (StackDescriptor, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps, expert_bank_names, expert_copy,
                       expert_gemm, expert_plan, expert_reduce, moe_decode, moe_grouped, routed_decode,
                       router_plan_forward, router_workspace, stack_supported)
+from .kernels._abi import require_cuda
 from .kernels._host import host
 from .kernels.paired_all_reduce import all_reduce
 
@@ -261,8 +262,8 @@ class FusedMoE(nn.Module):
         self._tokens = 0
         self._fused = None   # one-launch descriptor for a single token, built on first use
         self._maps_of = None
-        if experts.bank_maps is not None and self.n_shared and all(
-                w.is_cuda and w.is_contiguous() and w.dtype == torch.bfloat16 for w in (shared_gate, shared_up, shared_down)):
+        if experts.bank_maps is not None and self.n_shared and self._shared_as_expected() and all(
+                w.is_cuda for w in (shared_gate, shared_up, shared_down)):
             self._shared_maps()   # here, so that a first call may be one under graph capture
 
     _native = None   # what the native calls know of this block, and the experts' generation it was taken down at
@@ -275,8 +276,24 @@ class FusedMoE(nn.Module):
     def __getstate__(self):   # copies and pickles make their own record and table
         return dict({k: v for k, v in self.__dict__.items() if k != "_native"}, _fused=None)
 
+    def _shared_as_expected(self) -> bool:
+        d, f, n = self.experts.hidden_dim, self.experts.intermediate_dim, self.n_shared
+        gate, up, down = self.shared_gate, self.shared_up, self.shared_down
+        return (gate.shape == up.shape == (n, f, d) and down.shape == (n, d, f)
+                and all(t.dtype == torch.bfloat16 and t.is_contiguous() for t in (gate, up, down)))
+
+    def _check(self) -> None:
+        """The block's tensors as the kernels read them, by address alone: made sure of whenever addresses are taken down."""
+        weight, bias, scale = self.router_weight, self.router_bias, self.global_scale
+        assert weight.dtype == scale.dtype == torch.bfloat16 and bias.dtype == torch.float32
+        assert weight.dim() == 2 and weight.shape[1] == self.experts.hidden_dim and bias.shape == (weight.shape[0] - self.n_shared,)
+        assert scale.numel() >= 1 and all(t.is_contiguous() for t in (weight, bias, scale))
+        assert self._shared_as_expected()
+        require_cuda(weight, bias, scale, self.shared_gate, self.shared_up, self.shared_down)
+
     def _record(self, one_token: bool):
         """The record for several tokens, with `one_token` also the one-launch kernel's table (made on the first such call only)."""
+        self._check()
         ex = self.experts
         fields = dict(ex.record_fields() if ex.bank_maps is not None else dict(hidden=ex.hidden_dim, width=ex.intermediate_dim),
                       tokens=self._tokens if ex.bank_maps is not None else 1, routed=self.router_weight.shape[0] - self.n_shared,
@@ -325,6 +342,7 @@ class FusedMoE(nn.Module):
 
     def block_descriptor(self, norm_weight=None) -> dict:
         """This block as the one-launch kernel takes it (addresses of the module's tensors)."""
+        self._check()
         self._reserve(1)
         ex = self.experts
         return dict(router_weight=self.router_weight, router_bias=self.router_bias, global_scale=self.global_scale,
@@ -365,6 +383,7 @@ class FusedMoE(nn.Module):
         """TMA descriptors of the shared experts, made when they are first needed (and again if the tensors are replaced)."""
         at = (self.shared_gate.data_ptr(), self.shared_up.data_ptr(), self.shared_down.data_ptr())
         if self._maps_of != at:
+            assert self._shared_as_expected()
             self._maps, self._maps_of = encode_shared_maps(self.shared_gate, self.shared_up, self.shared_down), at
         return self._maps
 

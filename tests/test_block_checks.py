@@ -1,0 +1,49 @@
+"""What a block refuses before any address of its tensors reaches a kernel (no GPU: the checks come first)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+from torch import nn
+
+D, F, ROUTED, SHARED = 256, 128, 8, 2
+
+
+class _Experts(nn.Module):
+    """What a FusedMoE needs of its experts to take its own tensors down."""
+
+    quantized, bank_maps, generation, hidden_dim, intermediate_dim = True, None, 0, D, F
+
+    def _reserve(self, routes):
+        pass
+
+
+def _block(**other):
+    import inkling_b200 as ib
+
+    bf = dict(dtype=torch.bfloat16)
+    t = dict(router_weight=torch.zeros(ROUTED + SHARED, D, **bf), router_bias=torch.zeros(ROUTED), global_scale=torch.ones(1, **bf),
+             shared_gate=torch.zeros(SHARED, F, D, **bf), shared_up=torch.zeros(SHARED, F, D, **bf), shared_down=torch.zeros(SHARED, D, F, **bf))
+    t.update(other)
+    block = ib.FusedMoE(t["router_weight"], t["router_bias"], t["global_scale"], 1.0, 2, t["shared_gate"], t["shared_up"], t["shared_down"], _Experts())
+    block._reserve(4)
+    return block
+
+
+@pytest.mark.parametrize("name,change", [
+    ("router_weight", lambda t: t.float()), ("router_weight", lambda t: t.half()), ("router_weight", lambda t: t[:, :-8].contiguous()),
+    ("router_weight", lambda t: t.t().contiguous().t()), ("router_bias", lambda t: t[:-1]), ("router_bias", lambda t: t.repeat(2)),
+    ("global_scale", lambda t: t.float()), ("shared_gate", lambda t: t.float()), ("shared_gate", lambda t: t.transpose(1, 2).contiguous()),
+    ("shared_up", lambda t: t[:, :-16].contiguous()), ("shared_up", lambda t: t[:1]), ("shared_down", lambda t: t.transpose(1, 2)),
+    ("shared_down", lambda t: t[:, :, :-16].contiguous()),
+], ids=lambda v: v if isinstance(v, str) else "")
+def test_a_tensor_the_kernels_would_misread_is_refused(name, change):
+    block = _block(**{name: change(getattr(_block(), name))})
+    with pytest.raises(AssertionError):
+        block._record(False)
+    with pytest.raises(AssertionError):
+        block.block_descriptor()
+
+
+def test_tensors_on_the_host_are_refused():
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        _block()._record(False)

@@ -203,3 +203,20 @@ def test_a_token_that_is_not_finite_stays_its_own(ib, device, tokens, value):
     block = ib.FusedMoE(p["router_weight"][:8].to(device).contiguous(), p["router_bias"].to(device), p["global_scale"].to(device), p["route_scale"], 3,
                         *(torch.empty(0, *s, dtype=BF16, device=device) for s in ((f, d), (f, d), (d, f))), module, None)
     assert not torch.isfinite(block(x)[bad]).any()
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 9])
+@pytest.mark.parametrize("name,change", [
+    ("router_weight", lambda t: t.float()), ("router_weight", lambda t: t.view(torch.float16)), ("router_weight", lambda t: t.t()),
+    ("global_scale", lambda t: t.float()), ("shared_down", lambda t: t.transpose(1, 2)), ("shared_up", lambda t: t.view(torch.float16)),
+])
+def test_a_tensor_changed_underneath_is_checked_again(ib, device, tokens, name, change):
+    """Another type, layout or storage after the first call, also at the same address: refused, and right again when taken back."""
+    layer, x = _block(ib, device, tokens, d=1024, f=512, experts=8)
+    want = layer(x).clone()
+    was = getattr(layer, name).data
+    getattr(layer, name).data = change(was)
+    with pytest.raises(AssertionError):
+        layer(x)
+    getattr(layer, name).data = was
+    assert torch.equal(layer(x), want)
