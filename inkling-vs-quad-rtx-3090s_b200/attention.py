@@ -16,9 +16,27 @@ import torch.nn.functional as F
 
 from .kernels import add_rmsnorm, decode_attention, short_conv
 from .kernels.paired_all_reduce import all_reduce
+from .layer import KeepsForGraphs
 
 
-class DecodeAttention(nn.Module):
+class _ZeroRows(KeepsForGraphs):
+    """The FP32 zeros that the norm kernel adds to its rows, kept from call to call."""
+
+    _zeros = None
+
+    def _zero_rows(self, rows: torch.Tensor) -> torch.Tensor:
+        n, width = rows.shape
+        if self._zeros is None or self._zeros.shape[0] < n or self._zeros.shape[1] != width:
+            zeros = torch.zeros(n, width, dtype=torch.float32, device=rows.device)
+            if torch.cuda.is_current_stream_capturing():
+                return zeros   # (filled in by that graph alone, when it is replayed: not for other calls)
+            self._replace(self._zeros)
+            self._zeros = zeros
+        self._note_capture()
+        return self._zeros[:n]
+
+
+class DecodeAttention(_ZeroRows, nn.Module):
     def __init__(self, qkvr_weight, o_weight, q_norm_weight, k_norm_weight, k_taps, v_taps, rel_proj, *, layer_idx: int,
                  heads: int, kv_heads: int, head_dim: int, d_rel: int, window: int = 0, log_scaling_n_floor=None,
                  log_scaling_alpha: float = 0.1, eps: float = 1e-6, group=None):
@@ -34,7 +52,6 @@ class DecodeAttention(nn.Module):
         for name, t in (("qkvr_weight", qkvr_weight), ("o_weight", o_weight), ("q_norm_weight", q_norm_weight),
                         ("k_norm_weight", k_norm_weight), ("k_taps", k_taps), ("v_taps", v_taps), ("rel_proj", rel_proj)):
             self.register_buffer(name, t.contiguous())
-        self._zeros = None
 
     @classmethod
     def from_reference(cls, attention, group=None) -> "DecodeAttention":
@@ -49,10 +66,8 @@ class DecodeAttention(nn.Module):
 
     def _norm(self, rows: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         """RMS norm over the last dimension of BF16 [n, c] with the reference's rounding (kernels/decode.py:36-43)."""
-        if self._zeros is None or self._zeros.shape[0] < rows.shape[0]:
-            self._zeros = torch.zeros(rows.shape[0], rows.shape[1], dtype=torch.float32, device=rows.device)
         normed = torch.empty_like(rows)
-        add_rmsnorm(self._zeros[: rows.shape[0]], rows, weight, self.eps, normed)   # rows + 0, then the norm
+        add_rmsnorm(self._zero_rows(rows), rows, weight, self.eps, normed)   # rows + 0, then the norm
         return normed
 
     def forward(self, hidden_states: torch.Tensor, cache) -> torch.Tensor:
@@ -77,7 +92,7 @@ class DecodeAttention(nn.Module):
         return y
 
 
-class DecodeLayer(nn.Module):
+class DecodeLayer(_ZeroRows, nn.Module):
     """One sparse decoder layer at decode, `MyInklingDecoderLayer.forward` (my_inkling/model.py:661-675):
     h' = attn_sconv(attention(input_norm(h)), residual=h);  out = mlp_sconv(moe(post_norm(h')), residual=h').
     `attention` is a DecodeAttention, `moe` a FusedMoE (a sparse layer) or a DenseMLP (a dense one); the two short
@@ -89,14 +104,11 @@ class DecodeLayer(nn.Module):
         for name, t in (("input_norm_weight", input_norm_weight), ("post_norm_weight", post_norm_weight),
                         ("attn_taps", attn_taps), ("mlp_taps", mlp_taps)):
             self.register_buffer(name, t.contiguous())
-        self._zeros = None
 
     def _norm(self, x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         rows = x.reshape(-1, x.shape[-1]).clone()          # (the norm kernel adds its FP32 input to the rows in place: zero here)
-        if self._zeros is None or self._zeros.shape != rows.shape:
-            self._zeros = torch.zeros(rows.shape, dtype=torch.float32, device=rows.device)
         normed = torch.empty_like(rows)
-        add_rmsnorm(self._zeros, rows, weight, self.eps, normed)
+        add_rmsnorm(self._zero_rows(rows), rows, weight, self.eps, normed)
         return normed.view(x.shape)
 
     def forward(self, hidden_states: torch.Tensor, cache) -> torch.Tensor:

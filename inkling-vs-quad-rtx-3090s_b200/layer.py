@@ -47,7 +47,28 @@ def _next_pow2(n: int) -> int:
     return 1 << (max(n, 1) - 1).bit_length()
 
 
-class ResidentExperts(nn.Module):
+class KeepsForGraphs:
+    """A captured graph holds the addresses of a module's buffers and nothing that keeps them alive: buffers that a captured
+    call has used are not given back when larger ones take their place, they stay as long as the module does."""
+
+    _captured = False   # the present buffers are in a captured graph
+    _kept = ()
+
+    def _note_capture(self) -> None:
+        if torch.cuda.is_current_stream_capturing():
+            self.__dict__["_captured"] = True
+
+    def _keep(self, *old) -> None:
+        self.__dict__["_kept"] = (*self._kept, *(o for o in old if o is not None))
+
+    def _replace(self, *old) -> None:
+        """`old`, all that captured calls may have used, are about to be replaced."""
+        if self._captured:
+            self._keep(*old)
+        self.__dict__["_captured"] = False
+
+
+class ResidentExperts(KeepsForGraphs, nn.Module):
     """Drop-in for the routed-experts module with every expert's banks resident.
 
     `weights` is keyed by global expert id, each value the bank dictionary
@@ -107,6 +128,7 @@ class ResidentExperts(nn.Module):
         self.counts = torch.empty(self.local, **i32)
         self.status = torch.zeros(1, **i32)
         self.capacity = 0
+        self.rows = self.activated = self.down = None
 
     # What the native calls need of this module is taken down once (`record_fields`); replacing a tensor, or growing the
     # buffers, makes a new one, and so does a call that finds a tensor's storage exchanged.
@@ -120,7 +142,7 @@ class ResidentExperts(nn.Module):
         super().__setattr__(name, value)
 
     def __getstate__(self):   # copies and pickles make their own record
-        return {k: v for k, v in self.__dict__.items() if k != "_native"}
+        return {k: v for k, v in self.__dict__.items() if k not in ("_native", "_captured", "_kept")}
 
     def record_fields(self) -> dict:
         return dict(hidden=self.hidden_dim, width=self.intermediate_dim, start=self.start, local=self.local, stride=self.stride,
@@ -141,13 +163,14 @@ class ResidentExperts(nn.Module):
         return layout
 
     def _reserve(self, routes: int) -> None:
-        if routes <= self.capacity:
-            return
-        self.capacity = _next_pow2(routes)
-        self.rows = torch.empty((self.local, self.capacity), dtype=torch.int32, device=self.device)
-        options = dict(dtype=self.dtype, device=self.device)
-        self.activated = torch.empty((self.capacity, self.intermediate_dim), **options)
-        self.down = torch.empty((self.capacity, self.hidden_dim), **options)
+        if routes > self.capacity:
+            self._replace(self.rows, self.activated, self.down)
+            self.capacity = _next_pow2(routes)
+            self.rows = torch.empty((self.local, self.capacity), dtype=torch.int32, device=self.device)
+            options = dict(dtype=self.dtype, device=self.device)
+            self.activated = torch.empty((self.capacity, self.intermediate_dim), **options)
+            self.down = torch.empty((self.capacity, self.hidden_dim), **options)
+        self._note_capture()
 
     def _plan(self, indices) -> None:
         routes = indices.numel()
@@ -203,9 +226,7 @@ class ResidentExperts(nn.Module):
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
         if self.device_mesh is None and self.bank_maps is not None and hidden_states.shape[0] > 1 and hidden_states.dim() == 2:
-            routes = top_k_index.numel()
-            if routes > self.capacity:
-                self._reserve(routes)
+            self._reserve(top_k_index.numel())
             top_k = top_k_index.shape[1]
             out = NotImplemented
             while out is NotImplemented:
@@ -238,7 +259,7 @@ class ResidentExperts(nn.Module):
             raise RuntimeError("ResidentExperts: a route named an expert id outside the pointer table")
 
 
-class FusedMoE(nn.Module):
+class FusedMoE(KeepsForGraphs, nn.Module):
     """Router + routed NVFP4 experts + shared BF16 experts + one all-reduce.
 
     Parameters are this rank's: router replicated, shared experts and routed experts
@@ -260,8 +281,9 @@ class FusedMoE(nn.Module):
         self.experts = experts
         self.device_mesh = device_mesh
         self._tokens = 0
+        self._of_capture = False   # the buffers were made under capture: their zeros are filled in by that graph alone
         self._fused = None   # one-launch descriptor for a single token, built on first use
-        self._maps_of = None
+        self._maps = self._maps_of = None
         if experts.bank_maps is not None and self.n_shared and self._shared_as_expected() and all(
                 w.is_cuda for w in (shared_gate, shared_up, shared_down)):
             self._shared_maps()   # here, so that a first call may be one under graph capture
@@ -274,7 +296,7 @@ class FusedMoE(nn.Module):
         super().__setattr__(name, value)
 
     def __getstate__(self):   # copies and pickles make their own record and table
-        return dict({k: v for k, v in self.__dict__.items() if k != "_native"}, _fused=None)
+        return dict({k: v for k, v in self.__dict__.items() if k not in ("_native", "_captured", "_kept")}, _fused=None)
 
     def _shared_as_expected(self) -> bool:
         d, f, n = self.experts.hidden_dim, self.experts.intermediate_dim, self.n_shared
@@ -324,8 +346,6 @@ class FusedMoE(nn.Module):
         if self.device_mesh is not None or (tokens == 1 and self.separate_launches):
             return NotImplemented
         ex = self.experts
-        if tokens > self._tokens:
-            self._reserve(tokens)
         one = tokens == 1
         for _ in range(2):   # (again where the record turns out to be of storage that has been exchanged)
             native = self._native
@@ -337,13 +357,16 @@ class FusedMoE(nn.Module):
             out = host().run_block(native[1], x, want_partial)
             if out is not NotImplemented:
                 return out
+            if self._captured:
+                self._keep(self._fused)
             self._fused = None   # (drops the record too)
         raise RuntimeError("FusedMoE: a tensor's storage was exchanged during the call")
 
     def block_descriptor(self, norm_weight=None) -> dict:
         """This block as the one-launch kernel takes it (addresses of the module's tensors)."""
         self._check()
-        self._reserve(1)
+        if not self._tokens:
+            self._reserve(1)
         ex = self.experts
         return dict(router_weight=self.router_weight, router_bias=self.router_bias, global_scale=self.global_scale,
                     sources=ex.sources, shared_gate=self.shared_gate, shared_up=self.shared_up,
@@ -365,25 +388,34 @@ class FusedMoE(nn.Module):
                                                  self.top_k)
 
     def _reserve(self, tokens: int) -> None:
-        if tokens <= self._tokens:
+        """Buffers for `tokens` tokens. Those of a first call under capture serve that call alone: the router's counters in them
+        are cleared by that graph, when it is replayed, so the next call, eager or of another graph, has its own."""
+        capturing = torch.cuda.is_current_stream_capturing()
+        if tokens <= self._tokens and not self._of_capture and not capturing:
             return
-        dev, bf = self.router_weight.device, torch.bfloat16
-        self._tokens = tokens
-        self._fused = None          # descriptors hold addresses of the buffers replaced below
-        self.generation = getattr(self, "generation", 0) + 1
-        self.topk_weights = torch.empty(tokens, self.top_k, dtype=bf, device=dev)
-        self.topk_indices = torch.empty(tokens, self.top_k, dtype=torch.int64, device=dev)
-        self.gammas = torch.empty(tokens, self.n_shared, dtype=bf, device=dev)
-        self.shared_activated = torch.empty(tokens * self.n_shared, self.experts.intermediate_dim, dtype=bf, device=dev)
-        self.workspace = router_workspace(tokens, self.router_weight.shape[0], dev)
-        self.partial = torch.empty(tokens, self.experts.hidden_dim, dtype=torch.float32, device=dev)
+        if tokens > self._tokens or self._of_capture:
+            if self._tokens:
+                self._replace(self.topk_weights, self.topk_indices, self.gammas, self.shared_activated, self.workspace, self.partial, self._fused)
+            dev, bf = self.router_weight.device, torch.bfloat16
+            self._tokens = tokens
+            self._of_capture = capturing
+            self._fused = None          # descriptors hold addresses of the buffers replaced below
+            self.generation = getattr(self, "generation", 0) + 1
+            self.topk_weights = torch.empty(tokens, self.top_k, dtype=bf, device=dev)
+            self.topk_indices = torch.empty(tokens, self.top_k, dtype=torch.int64, device=dev)
+            self.gammas = torch.empty(tokens, self.n_shared, dtype=bf, device=dev)
+            self.shared_activated = torch.empty(tokens * self.n_shared, self.experts.intermediate_dim, dtype=bf, device=dev)
+            self.workspace = router_workspace(tokens, self.router_weight.shape[0], dev)
+            self.partial = torch.empty(tokens, self.experts.hidden_dim, dtype=torch.float32, device=dev)
         self.experts._reserve(tokens * self.top_k)
+        self._note_capture()
 
     def _shared_maps(self):
         """TMA descriptors of the shared experts, made when they are first needed (and again if the tensors are replaced)."""
         at = (self.shared_gate.data_ptr(), self.shared_up.data_ptr(), self.shared_down.data_ptr())
         if self._maps_of != at:
             assert self._shared_as_expected()
+            self._keep(self._maps)   # (a graph, or another stream, may still read them: 384 bytes)
             self._maps, self._maps_of = encode_shared_maps(self.shared_gate, self.shared_up, self.shared_down), at
         return self._maps
 
@@ -398,20 +430,25 @@ class FusedMoE(nn.Module):
 
     def forward(self, hidden_states):
         shape = hidden_states.shape
-        out = self._call_native(hidden_states.numel() // shape[-1], hidden_states, False)
+        tokens = hidden_states.numel() // shape[-1]
+        self._reserve(tokens)
+        out = self._call_native(tokens, hidden_states, False)
         if out is not NotImplemented:
             return out
         flat = hidden_states.reshape(-1, shape[-1]).contiguous()
-        return self.forward_partial(flat).to(hidden_states.dtype).view(shape)
+        return self._partial(flat).to(hidden_states.dtype).view(shape)
 
     def forward_partial(self, flat):
         """flat BF16 [t, d] -> the all-reduced FP32 layer output [t, d] (a view of the
         module's own buffer, overwritten by the next call)."""
         t = flat.shape[0]
         self._reserve(t)
-        ex = self.experts
         if self._call_native(t, flat, True) is not NotImplemented:
             return self.partial[:t]
+        return self._partial(flat)
+
+    def _partial(self, flat):
+        t, ex = flat.shape[0], self.experts
         if t == 1 and self.one_launch_supported() and not self.separate_launches:
             if self._fused is None:
                 self._fused = self._one_launch()

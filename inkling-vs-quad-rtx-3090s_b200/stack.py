@@ -8,11 +8,11 @@ import torch
 from torch import nn
 
 from .kernels import StackDescriptor, add_rmsnorm
-from .layer import FusedMoE, ResidentExperts
+from .layer import FusedMoE, KeepsForGraphs, ResidentExperts
 from .synthetic import make_expert_banks, make_layer_params
 
 
-class MoEStack(nn.Module):
+class MoEStack(KeepsForGraphs, nn.Module):
     def __init__(self, layers: list[FusedMoE], hidden: int, eps: float = 1e-6):
         super().__init__()
         self.layers = nn.ModuleList(layers)
@@ -20,6 +20,7 @@ class MoEStack(nn.Module):
         dev = layers[0].router_weight.device
         self.norm_weight = torch.ones(hidden, dtype=torch.bfloat16, device=dev)
         self._tokens = 0
+        self.residual = self.normed = None
         self._fused = None
         # one launch for the whole stack, on one GPU or across tensor-parallel ranks
         self.one_launch = all(layer.one_launch_supported() for layer in layers)
@@ -41,10 +42,12 @@ class MoEStack(nn.Module):
 
     def _reserve(self, tokens: int) -> None:
         if tokens > self._tokens:
+            self._replace(self.residual, self.normed, self._fused)
             dev = self.norm_weight.device
             self._tokens = tokens
             self.residual = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=dev)
             self.normed = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=dev)
+        self._note_capture()
 
     def forward(self, x):
         """x BF16 [t, d] -> BF16 [t, d]: h <- h + moe(norm(h)) per block, final norm."""
@@ -59,9 +62,14 @@ class MoEStack(nn.Module):
                 ex = first.experts
                 blocks = [layer.block_descriptor(self.norm_weight) for layer in self.layers]
                 from .layer import _group_of
+                if self._captured:
+                    self._keep(self._fused)
                 self._fused = StackDescriptor(blocks, ex.hidden_dim, ex.intermediate_dim, ex.local, first.n_shared,
                                               first.top_k, x.device, group=_group_of(first.device_mesh))
                 self._fused_generations = tuple(layer.generation for layer in self.layers)
+            if torch.cuda.is_current_stream_capturing():
+                for layer in self.layers:
+                    layer._note_capture()   # (the launch has their buffers)
             self._fused.decode(x, self.layers[-1].partial[:1], residual, normed, self.eps)
             return normed
         normed.copy_(x)

@@ -17,6 +17,11 @@ class _Experts(nn.Module):
         pass
 
 
+@pytest.fixture(autouse=True)
+def nothing_is_captured(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)   # (the question needs a device)
+
+
 def _block(**other):
     import inkling_b200 as ib
 

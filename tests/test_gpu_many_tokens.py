@@ -220,3 +220,89 @@ def test_a_tensor_changed_underneath_is_checked_again(ib, device, tokens, name, 
         layer(x)
     getattr(layer, name).data = was
     assert torch.equal(layer(x), want)
+
+
+def _fill_what_is_free(device):
+    """Tensors that take whatever the allocator has got back, so that a write to it, or a read of what was there, shows."""
+    return [torch.full((512 << k,), 127, dtype=torch.uint8, device=device) for k in range(15) for _ in range(24)]
+
+
+def _capture(step):
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        out = step()
+    return graph, out
+
+
+@pytest.mark.parametrize("tokens", [1, 4, 12])
+def test_a_graph_outlives_a_larger_call(ib, device, tokens):
+    """A step captured after an eager one; then a prompt through the same modules replaces their buffers."""
+    layer, x = _block(ib, device, tokens, d=1024, f=512, experts=8)
+    stack = ib.MoEStack([_block(ib, device, 1, seed=s, d=1024, f=512, experts=8)[0] for s in (6, 7)], 1024)
+    decode = ib.DecodeStackGraph(stack, x[:1])
+    alone = decode.replay().clone()
+    idx, w = torch.arange(tokens * 3, device=device).view(tokens, 3) % 8, torch.ones(tokens, 3, dtype=BF16, device=device)
+
+    def step():
+        return layer(x), layer.experts(x, idx, w), layer.forward_partial(x)
+
+    want = [t.clone() for t in step()]
+    graph, out = _capture(step)
+    prompt = x.repeat(-(-700 // tokens), 1)
+    layer(prompt), layer.experts(prompt, idx.repeat(len(prompt) // tokens, 1), w.repeat(len(prompt) // tokens, 1))
+    stack(prompt), stack.layers[-1](prompt)
+    fill = _fill_what_is_free(device)
+    for t in out:
+        t.zero_()
+    graph.replay()
+    assert all(torch.equal(got, t) for got, t in zip(out, want))
+    decode.out.zero_()
+    assert torch.equal(decode.replay(), alone)
+    assert all(bool((t == 127).all()) for t in fill)
+
+
+@pytest.mark.parametrize("tokens", [2, 8, 12])
+def test_buffers_made_under_capture_are_the_graphs_alone(ib, device, tokens):
+    """First calls under capture; then an eager call and the second graph, both before the first graph's first replay (which is
+    what clears the router's counters in its buffers)."""
+    layer, x = _block(ib, device, tokens)
+    want = _block(ib, device, tokens)[0](x)
+    fill = _fill_what_is_free(device)
+    del fill
+    graphs = [_capture(lambda: (layer(x), layer(x))) for _ in range(2)]
+    assert torch.equal(layer(x), want)
+    for graph, out in reversed(graphs):
+        graph.replay()
+        assert torch.equal(out[0], want) and torch.equal(out[1], want)
+    assert torch.equal(layer(x), want)
+
+
+@pytest.mark.parametrize("kind", ["heads", "rows"])
+def test_the_zeros_of_a_norm_under_capture(ib, device, kind):
+    """The norm's zero rows, used by a graph and replaced by a larger call; first made under capture, then needed eagerly."""
+    draw = lambda *shape: torch.randn(*shape, device=device).to(BF16)  # noqa: E731
+    taps = torch.zeros(128, 1, 4, device=device)
+
+    def make():
+        attention = ib.DecodeAttention(draw(640, 128), draw(128, 256), draw(64), draw(64), taps, taps, draw(16, 8), layer_idx=0, heads=4, kv_heads=2,
+                                       head_dim=64, d_rel=32)
+        return attention if kind == "heads" else ib.DecodeLayer(attention, None, draw(64), draw(64), taps, taps)
+
+    x, weight = draw(5, 64), draw(64)
+    want = make()._norm(x.clone(), weight)
+    module = make()
+    module._norm(x.clone(), weight)
+    graph, out = _capture(lambda: module._norm(x, weight))
+    module._norm(draw(3000, 64), weight)
+    fill = _fill_what_is_free(device)
+    graph.replay()
+    assert torch.equal(out, want)
+    del fill
+    module = make()
+    graph, out = _capture(lambda: module._norm(x, weight))
+    assert torch.equal(module._norm(x.clone(), weight), want)
+    graph.replay()
+    assert torch.equal(out, want)
