@@ -1097,8 +1097,7 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   if (int rc = check_grouped_shape(true, n, k, groups)) return rc;
   INK_REQUIRE(capacity >= 1 && top_k >= 1 && input_rows >= 0 && start >= 0, kBadArgument, "expert_gemm_tc: bad sizes (capacity=%d top_k=%d rows=%d)",
               capacity, top_k, input_rows);
-  const long long all = projection == 0 ? (long long)input_rows * top_k : input_rows;
-  const size_t routes = (size_t)(all < capacity ? all : capacity);
+  const size_t routes = (size_t)input_rows * (projection == 0 ? top_k : 1);   // (`capacity` bounds one group's, not all of them)
   INK_REQUIRE(scratch_bytes >= expert_gemm_tc_bytes(routes, groups, k), kBadArgument,
               "expert_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, expert_gemm_tc_bytes(routes, groups, k));
   INK_REQUIRE(aligned16(x) && aligned16(y) && aligned16(scratch) && (reinterpret_cast<uintptr_t>(bank_maps) & 127u) == 0,

@@ -99,7 +99,7 @@ def _expert_gemm(X, Pointers, Experts, Rows, Counts, Y, CAPACITY, N, K, TOP_K, P
     _abi.require_cuda(X, Pointers, Experts, Rows, Counts, Y)
     groups = Experts.numel() if groups is None else groups
     if bank_maps is not None and QUANTIZED and block_scaled_supported(N, K, groups):
-        routes = min(X.shape[0] * (TOP_K if PROJECTION == 0 else 1), CAPACITY)
+        routes = X.shape[0] * (TOP_K if PROJECTION == 0 else 1)   # (CAPACITY bounds one group's, not all of them)
         scratch = _scratch(_abi.lib().ink_expert_gemm_tc_scratch_bytes((routes + 7) // 8, K), X.device)
         _abi.check(_abi.lib().ink_expert_gemm_tc(
             X.data_ptr(), X.shape[0], bank_maps.data_ptr(), Pointers.data_ptr(), Experts.data_ptr(), Rows.data_ptr(),

@@ -44,6 +44,17 @@ def test_argument_errors_are_reported_without_a_gpu():
     assert rc < 0
 
 
+def test_scratch_of_a_projection_holds_every_route_whatever_the_capacity():
+    """`capacity` is the row pitch of one expert's list. 32 tokens of six choices over 16 experts, capacity 32 (as the plan
+    accepts it): the staging kernel writes 192 rows, so scratch for 32 of them is refused (before anything is launched)."""
+    from inkling_b200.kernels import _abi
+
+    handle, at = _abi.lib(), 1 << 20   # (addresses are not followed on the host)
+    for_32 = handle.ink_expert_gemm_tc_scratch_bytes(4, 512)   # eight choices a row
+    rc = handle.ink_expert_gemm_tc(at, 32, at, at, at, at, at, at, 32, 512, 512, 6, 0, 16, 0, at, for_32, None, None)
+    assert rc == -1 and b"scratch" in handle.ink_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from inkling_b200.kernels import _abi
     import pytest

@@ -193,3 +193,26 @@ def test_block_scaled_projections_against_oracle(ib, device, d, f, E, tokens):
     assert max_rel(down.float(), want_down.float()) <= 1.6e-2
     assert max_rel(out, oracle_moe.routed_experts_fp32(x, idx, w, cpu_banks)) <= TOL
     assert max_rel(out, outs["fp16"][2]) <= TOL
+
+
+def test_block_scaled_projection_with_the_smallest_capacity(ib, device):
+    """`capacity` bounds one expert's routes (here: one per token), not all of them: the same bits as with room for every route."""
+    d, f, E, k, tokens = 512, 256, 16, 6, 32
+    banks = ib.make_expert_banks(E, d, f, device, seed=3)
+    module = ib.ResidentExperts(d, f, None, banks.weights)
+    gen = torch.Generator().manual_seed(1)
+    x = torch.randn(tokens, d, generator=gen).to(BF16).to(device)
+    idx = torch.stack([torch.randperm(E, generator=gen)[:k] for _ in range(tokens)]).to(device)
+    i32 = dict(dtype=torch.int32, device=device)
+    outs = []
+    for capacity in (tokens, tokens * k):
+        pointers = torch.zeros(E * 6, dtype=torch.int64, device=device)
+        experts, counts, rows = torch.empty(E, **i32), torch.empty(E, **i32), torch.full((E, capacity), -1, **i32)
+        ib.kernels.expert_plan[(1,)](idx, module.sources, None, None, None, None, None, torch.empty(0, **i32), pointers, experts, counts, rows,
+                                     0, E, 0, 6, tokens * k, capacity)
+        activated, down = torch.zeros(tokens * k, f, dtype=BF16, device=device), torch.zeros(tokens * k, d, dtype=BF16, device=device)
+        for args in ((x, pointers, experts, rows, counts, activated, capacity, 2 * f, d, k, 0), (activated, pointers, experts, rows, counts, down, capacity, d, f, k, 1)):
+            ib.kernels.expert_gemm[(1, 1, E)](*args, True, 6, 16, 64, 64, status=module.status, bank_maps=module.bank_maps)
+        outs.append((activated, down))
+    module.check_status()
+    assert all(torch.equal(a, b) and bool(a.any(1).all()) for a, b in zip(*outs))
