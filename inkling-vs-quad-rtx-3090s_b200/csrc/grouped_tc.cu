@@ -47,6 +47,8 @@ constexpr int kGgAccCols = 128;                                  // of one: 32 t
 
 // tokens in a tile
 __host__ __device__ constexpr int gg_tile(bool fp4, int t) { return fp4 ? t : 4 * t; }
+// no tile costs more (GgWalk::tile_cost)
+constexpr int gg_most_cost = 128;
 // slots of a group are padded to whole 1024-byte swizzle atoms of its tiles
 __host__ __device__ constexpr int gg_pad(bool fp4) { return fp4 ? 2 : 8; }
 
@@ -164,13 +166,13 @@ struct GgWalk {
   __device__ __forceinline__ int stages_of(bool shared) const {
     return a->k / ((FP4 && !shared) ? kTcChunkK : 64);
   }
-  // cost of one item with n tokens: its bytes, the streamed weights weighing most
-  __device__ static __forceinline__ int tile_cost(int n, int stages) { return stages * (64 + (T == 16 ? 2 * n : T == 32 ? n / 4 : n) / (FP4 ? 1 : 4)); }
-  __device__ __forceinline__ int cost_per_mt(int c, int stages) const {
-    return c / kTile * tile_cost(kTile, stages) + (c % kTile ? tile_cost(c % kTile, stages) : 0);
+  // cost of one item with n tokens, per ring stage (they have equally many): its bytes, the streamed weights weighing most.
+  // At most gg_most_cost, and all of them together fit an int (gg_costs_fit).
+  __device__ static __forceinline__ int tile_cost(int n) { return 64 + (T == 16 ? 2 * n : T == 32 ? n / 4 : n) / (FP4 ? 1 : 4); }
+  __device__ __forceinline__ int cost_per_mt(int c) const {
+    return c / kTile * tile_cost(kTile) + (c % kTile ? tile_cost(c % kTile) : 0);
   }
   __device__ __forceinline__ void find(int from) {   // the first routed item whose cost offset is at least `from`
-    const int stages = stages_of(false);
     int lo = 0, hi = a->groups;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
@@ -180,9 +182,9 @@ struct GgWalk {
     group = lo;
     mt = tile = 0;
     count = a->groups > 0 ? gg_group_count(t.slot0, group, kPad) : 0;
-    const int cm = cost_per_mt(count, stages);
+    const int cm = cost_per_mt(count);
     if (cm > 0) {
-      const int off = from - t.cost[group], ct = tile_cost(kTile, stages);
+      const int off = from - t.cost[group], ct = tile_cost(kTile);
       mt = off / cm;
       tile = (off % cm + ct - 1) / ct;
       if (tile * kTile >= count) {
@@ -213,8 +215,7 @@ struct GgWalk {
       return true;
     }
     if (group >= a->groups) return false;
-    const int stages = stages_of(false);
-    if (t.cost[group] + mt * cost_per_mt(count, stages) + tile * tile_cost(kTile, stages) >= limit) return false;
+    if (t.cost[group] + mt * cost_per_mt(count) + tile * tile_cost(kTile) >= limit) return false;
     it.shared = false;
     it.group = group;
     it.m0 = mt * kM;
@@ -306,8 +307,8 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   tc_fence_before();
   __syncthreads();
   if (warp == 0) {
-    const int stages = walk.stages_of(false), m_tiles = walk.m_tiles;
-    gg_scan(tables, a.groups, Walk::kPad, lane, [&](int count) { return m_tiles * walk.cost_per_mt(count, stages); });
+    const int m_tiles = walk.m_tiles;
+    gg_scan(tables, a.groups, Walk::kPad, lane, [&](int count) { return m_tiles * walk.cost_per_mt(count); });
   }
   __syncthreads();
   tc_fence_after();
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   // ---- this block's share: its shared items, and the routed items in what remains of total / blocks
   {
     const int shared_items = a.n_shared * walk.m_tiles * walk.shared_tiles, G = gridDim.x, b = blockIdx.x;
-    const long long shared_cost = a.n_shared > 0 ? (long long)walk.stages_of(true) * (64 + min(a.tokens, Walk::kSharedTile) / 4) : 0;
+    const long long shared_cost = a.n_shared > 0 ? (long long)(walk.stages_of(true) / walk.stages_of(false)) * (64 + min(a.tokens, Walk::kSharedTile) / 4) : 0;
     const long long routed = tables.cost[a.groups], total = routed + shared_cost * shared_items;
     // routed cost taken by the blocks before block x (a block whose shared items exceed its share takes none)
     auto before = [&](int x) -> long long { return total * x / G - shared_cost * ((long long)shared_items * x / G); };
@@ -948,6 +949,14 @@ extern "C" int ink_encode_shared(void* out_host_384, const void* gate, const voi
   return kOk;
 }
 
+// The items' costs are added up in 32 bits: 16 million routes at the greatest widths.
+static int check_costs_fit(bool fp4, size_t routes, int groups, int n, int t) {
+  const size_t tiles = routes / gg_tile(fp4, t) + (size_t)groups;
+  INK_REQUIRE(tiles * (n / kTcRows) * gg_most_cost <= 0x7fffffff && routes <= 0x40000000, kUnsupportedShape,
+              "grouped projections: %zu routes in one call", routes);
+  return kOk;
+}
+
 static int check_grouped_shape(bool fp4, int n, int k, int groups) {
   const int step = fp4 ? kTcChunkK : 64;
   INK_REQUIRE(k % step == 0 && k >= step && k <= kTcMaxK && n % kTcRows == 0 && n > 0, kUnsupportedShape,
@@ -976,6 +985,9 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   const bool fp4 = quantized != 0;
   if (int rc = check_grouped_shape(fp4, 2 * intermediate, hidden, groups)) return rc;
   if (int rc = check_grouped_shape(fp4, hidden, intermediate, groups)) return rc;
+  const size_t routes = (size_t)tokens * top_k, padded = ((size_t)tokens + 7) / 8 * 8;
+  const int t = gg_tokens((long long)routes, local);
+  if (int rc = check_costs_fit(fp4, routes, groups, 2 * intermediate > hidden ? 2 * intermediate : hidden, t)) return rc;
   INK_REQUIRE(scratch_bytes >= ink_moe_grouped_scratch_bytes(tokens, top_k, n_shared, hidden, intermediate, groups, quantized), kBadArgument,
               "moe_grouped: scratch of %zu bytes is too small", scratch_bytes);
   INK_REQUIRE(aligned16(x) && aligned16(activated) && aligned16(down) && aligned16(output) && aligned16(output_bf16) && (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0 &&
@@ -983,7 +995,6 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
               kMisaligned, "moe_grouped: misaligned buffer (scratch 256 bytes, descriptors 128, x and outputs 16)");
   if (tokens == 0) return kOk;
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t routes = (size_t)tokens * top_k, padded = ((size_t)tokens + 7) / 8 * 8;
   const GgScratch in(fp4, routes, groups, hidden), act(fp4, routes, groups, intermediate);
   unsigned char* p = (unsigned char*)scratch;
   auto take = [&](size_t n) { unsigned char* q = p; p += gg_pad256(n); return q; };
@@ -991,7 +1002,6 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   unsigned char *act_image = take(act.image), *act_scales = take(act.image_scales), *act_slot = take(act.slot_scale);
   unsigned char *x_image = take(n_shared ? padded * hidden * 2 : 0), *sact_image = take(padded * n_shared * intermediate * 2);
   unsigned char* shared_out = take((size_t)tokens * n_shared * hidden * 2);
-  const int t = gg_tokens((long long)routes, local);
   const int bank = fp4 ? 3 : 1, stride = fp4 ? kBank : 2;
 
   StageArgs st = {};
@@ -1098,6 +1108,8 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   INK_REQUIRE(capacity >= 1 && top_k >= 1 && input_rows >= 0 && start >= 0, kBadArgument, "expert_gemm_tc: bad sizes (capacity=%d top_k=%d rows=%d)",
               capacity, top_k, input_rows);
   const size_t routes = (size_t)input_rows * (projection == 0 ? top_k : 1);   // (`capacity` bounds one group's, not all of them)
+  const int t = gg_tokens((long long)routes, groups);
+  if (int rc = check_costs_fit(true, routes, groups, n, t)) return rc;
   INK_REQUIRE(scratch_bytes >= expert_gemm_tc_bytes(routes, groups, k), kBadArgument,
               "expert_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, expert_gemm_tc_bytes(routes, groups, k));
   INK_REQUIRE(aligned16(x) && aligned16(y) && aligned16(scratch) && (reinterpret_cast<uintptr_t>(bank_maps) & 127u) == 0,
@@ -1105,7 +1117,6 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   if (groups == 0 || routes == 0) return kOk;
   cudaStream_t s = (cudaStream_t)stream;
   const GgScratch sizes(true, routes, groups, k);
-  const int t = gg_tokens((long long)routes, groups);
   StageArgs st = {};
   st.x = (const uint16_t*)x;
   st.pointers = pointers;

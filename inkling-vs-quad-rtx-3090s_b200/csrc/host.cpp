@@ -206,8 +206,8 @@ Rows rows_of(const Block& b, const at::Tensor& t) {
 }
 
 // Tokens of a many-token call that are planned and projected at a time: the images of the tokens take about 85 KB a token
-// at full width (2.7 GB), the banks are read once per 32 768 tokens (0.5 of about 20 ms), and the kernels' work counters
-// stay far inside 32 bits.
+// at full width (2.7 GB), the banks are read once per 32 768 tokens (0.5 of about 20 ms), and the kernels' 32-bit work
+// counters hold sixteen times as many with the router's most choices (32).
 constexpr int kMostTokens = 32768;
 void grouped(const Block& b, const Rows& r, int t0, int tokens, const int64_t* indices, const char* weights, const char* gammas, float* partial, void* out,
              int n_shared, cudaStream_t stream) {

@@ -55,6 +55,18 @@ def test_scratch_of_a_projection_holds_every_route_whatever_the_capacity():
     assert rc == -1 and b"scratch" in handle.ink_last_error()
 
 
+def test_more_routes_than_the_grouped_kernels_counters_hold_are_refused():
+    """32-bit cost counters: 2^25 routes at 4096 x 4096 do not fit (a tile of 64 counts up to 128 for each of 64 weight tiles)."""
+    from inkling_b200.kernels import _abi
+
+    handle, at, enough = _abi.lib(), 1 << 20, 1 << 60
+    rc = handle.ink_moe_grouped(at, at, at, at, at, at, at, at, None, None, at, at, at, None, 1 << 22, 8, 0, 4096, 4096, 256, 0, 256, 1 << 22,
+                                255, 1, at, enough, None, None)
+    assert rc == -2 and b"routes" in handle.ink_last_error()
+    rc = handle.ink_expert_gemm_tc(at, 1 << 22, at, at, at, at, at, at, 1 << 22, 8192, 4096, 8, 0, 256, 0, at, enough, None, None)
+    assert rc == -2 and b"routes" in handle.ink_last_error()
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from inkling_b200.kernels import _abi
     import pytest
