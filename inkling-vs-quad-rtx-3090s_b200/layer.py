@@ -164,12 +164,13 @@ class ResidentExperts(KeepsForGraphs, nn.Module):
 
     def _reserve(self, routes: int) -> None:
         if routes > self.capacity:
+            capacity, options = _next_pow2(routes), dict(dtype=self.dtype, device=self.device)
             self._replace(self.rows, self.activated, self.down)
-            self.capacity = _next_pow2(routes)
-            self.rows = torch.empty((self.local, self.capacity), dtype=torch.int32, device=self.device)
-            options = dict(dtype=self.dtype, device=self.device)
-            self.activated = torch.empty((self.capacity, self.intermediate_dim), **options)
-            self.down = torch.empty((self.capacity, self.hidden_dim), **options)
+            self.capacity, self.rows, self.activated, self.down = 0, None, None, None   # (so it stays if memory runs out here)
+            self.rows = torch.empty((self.local, capacity), dtype=torch.int32, device=self.device)
+            self.activated = torch.empty((capacity, self.intermediate_dim), **options)
+            self.down = torch.empty((capacity, self.hidden_dim), **options)
+            self.capacity = capacity
         self._note_capture()
 
     def _plan(self, indices) -> None:
@@ -396,10 +397,11 @@ class FusedMoE(KeepsForGraphs, nn.Module):
         if tokens > self._tokens or self._of_capture:
             if self._tokens:
                 self._replace(self.topk_weights, self.topk_indices, self.gammas, self.shared_activated, self.workspace, self.partial, self._fused)
+            self._tokens = 0            # (so it stays if memory runs out here)
+            self._fused = None          # descriptors hold addresses of the buffers replaced here
+            self.topk_weights = self.topk_indices = self.gammas = self.shared_activated = self.workspace = self.partial = None
+            self.experts._reserve(tokens * self.top_k)
             dev, bf = self.router_weight.device, torch.bfloat16
-            self._tokens = tokens
-            self._of_capture = capturing
-            self._fused = None          # descriptors hold addresses of the buffers replaced below
             self.generation = getattr(self, "generation", 0) + 1
             self.topk_weights = torch.empty(tokens, self.top_k, dtype=bf, device=dev)
             self.topk_indices = torch.empty(tokens, self.top_k, dtype=torch.int64, device=dev)
@@ -407,7 +409,9 @@ class FusedMoE(KeepsForGraphs, nn.Module):
             self.shared_activated = torch.empty(tokens * self.n_shared, self.experts.intermediate_dim, dtype=bf, device=dev)
             self.workspace = router_workspace(tokens, self.router_weight.shape[0], dev)
             self.partial = torch.empty(tokens, self.experts.hidden_dim, dtype=torch.float32, device=dev)
-        self.experts._reserve(tokens * self.top_k)
+            self._of_capture = capturing
+            self._tokens = tokens
+        self.experts._note_capture()
         self._note_capture()
 
     def _shared_maps(self):

@@ -43,10 +43,10 @@ class MoEStack(KeepsForGraphs, nn.Module):
     def _reserve(self, tokens: int) -> None:
         if tokens > self._tokens:
             self._replace(self.residual, self.normed, self._fused)
-            dev = self.norm_weight.device
+            self._tokens, self.residual, self.normed = 0, None, None   # (so it stays if memory runs out here)
+            self.residual = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=self.norm_weight.device)
+            self.normed = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=self.norm_weight.device)
             self._tokens = tokens
-            self.residual = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=dev)
-            self.normed = torch.empty(tokens, self.hidden, dtype=torch.bfloat16, device=dev)
         self._note_capture()
 
     def forward(self, x):

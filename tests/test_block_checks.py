@@ -16,6 +16,9 @@ class _Experts(nn.Module):
     def _reserve(self, routes):
         pass
 
+    def _note_capture(self):
+        pass
+
 
 @pytest.fixture(autouse=True)
 def nothing_is_captured(monkeypatch):
@@ -52,3 +55,49 @@ def test_a_tensor_the_kernels_would_misread_is_refused(name, change):
 def test_tensors_on_the_host_are_refused():
     with pytest.raises(RuntimeError, match="CUDA tensors only"):
         _block()._record(False)
+
+
+def _out_of_memory_at(monkeypatch, nth):
+    """torch.empty and torch.zeros as usual, the nth call of both together out of memory."""
+    calls = []
+
+    def wrap(make):
+        def allocate(*args, **kwargs):
+            calls.append(1)
+            if len(calls) == nth:
+                raise torch.OutOfMemoryError("planted")
+            return make(*args, **kwargs)
+        return allocate
+
+    for name in ("empty", "zeros"):
+        monkeypatch.setattr(torch, name, wrap(getattr(torch, name)))
+
+
+@pytest.mark.parametrize("nth", range(1, 7))
+def test_a_block_that_ran_out_of_memory_counts_on_no_buffers(monkeypatch, nth):
+    block = _block()
+    with monkeypatch.context() as m:
+        _out_of_memory_at(m, nth)
+        with pytest.raises(torch.OutOfMemoryError):
+            block._reserve(9)
+    assert block._tokens == 0
+    block._reserve(2)
+    assert block._tokens == 2 and all(getattr(block, n).shape[0] == 2 for n in ("topk_weights", "topk_indices", "gammas", "partial"))
+
+
+@pytest.mark.parametrize("nth", range(1, 4))
+def test_experts_that_ran_out_of_memory_count_on_no_buffers(monkeypatch, nth):
+    import inkling_b200 as ib
+
+    experts = ib.ResidentExperts.__new__(ib.ResidentExperts)
+    nn.Module.__init__(experts)
+    experts.local, experts.device, experts.dtype, experts.hidden_dim, experts.intermediate_dim, experts.capacity = 3, "cpu", torch.bfloat16, D, F, 0
+    experts.rows = experts.activated = experts.down = None
+    experts._reserve(4)
+    with monkeypatch.context() as m:
+        _out_of_memory_at(m, nth)
+        with pytest.raises(torch.OutOfMemoryError):
+            experts._reserve(9)
+    assert experts.capacity == 0
+    experts._reserve(2)
+    assert experts.capacity == 2 and experts.rows.shape == (3, 2) and experts.activated.shape == (2, F) and experts.down.shape == (2, D)
