@@ -230,7 +230,7 @@ PyObject* run_block(PyObject* const* args) {
   if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
   const at::Tensor& input = tensor_at(args, 1);
   const Rows r = rows_of(b, input);
-  require(r.tokens <= b.v[kTokens], "more tokens than the block's buffers hold");
+  require(r.tokens <= b.v[kTokens] && (r.tokens == 1 || std::min(r.tokens, kMostTokens) * b.v[kTopK] <= b.v[kCapacity]), "more tokens than the block's buffers hold");
   const bool want_partial = args[2] == Py_True;
   const c10::cuda::CUDAGuard guard(r.x.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();

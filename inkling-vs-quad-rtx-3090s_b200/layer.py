@@ -318,6 +318,7 @@ class FusedMoE(KeepsForGraphs, nn.Module):
         """The record for several tokens, with `one_token` also the one-launch kernel's table (made on the first such call only)."""
         self._check()
         ex = self.experts
+        ex._reserve(self._tokens * self.top_k)   # (experts that were put in the place of others may have less room)
         fields = dict(ex.record_fields() if ex.bank_maps is not None else dict(hidden=ex.hidden_dim, width=ex.intermediate_dim),
                       tokens=self._tokens if ex.bank_maps is not None else 1, routed=self.router_weight.shape[0] - self.n_shared,
                       shared=self.n_shared, top_k=self.top_k, router_weight=self.router_weight, router_bias=self.router_bias,

@@ -306,3 +306,14 @@ def test_the_zeros_of_a_norm_under_capture(ib, device, kind):
     assert torch.equal(module._norm(x.clone(), weight), want)
     graph.replay()
     assert torch.equal(out, want)
+
+
+def test_experts_put_in_place_of_others_get_the_room_they_need(ib, device):
+    """A block that has seen 40 tokens is given experts that have seen two (room for eight routes)."""
+    layer, x = _block(ib, device, 40)
+    want = layer(x).clone()
+    fresh = _block(ib, device, 2)[0].experts
+    fresh(x[:2], layer.topk_indices[:2], layer.topk_weights[:2])
+    assert fresh.capacity == 8
+    layer.experts = fresh
+    assert torch.equal(layer(x), want)
