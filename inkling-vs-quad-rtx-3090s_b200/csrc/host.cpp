@@ -5,6 +5,7 @@
 #include <Python.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
 
@@ -19,36 +20,45 @@
 
 namespace {
 
+// Errors keep the types that the Python layer's calls have: AssertionError for an argument of the wrong form, RuntimeError for
+// what the library refuses and for tensors that are not on the GPU, torch's own (out of memory, say) for what torch throws.
 struct Failure {
   std::string what;
+  PyObject* type = nullptr;   // null: the interpreter's error is set already
 };
-[[noreturn]] void fail(const std::string& what) { throw Failure{what}; }
+[[noreturn]] void fail(const std::string& what) { throw Failure{what, PyExc_RuntimeError}; }
 void check(int code) {
   if (code != 0) fail("inkling_b200: " + std::string(ink_last_error()) + " (code " + std::to_string(code) + ")");
 }
 
 const at::Tensor& tensor_at(PyObject* const* args, Py_ssize_t i) {
-  if (!THPVariable_Check(args[i])) fail("argument " + std::to_string(i) + " is not a tensor");
+  if (!THPVariable_Check(args[i])) throw Failure{"argument " + std::to_string(i) + " is not a tensor", PyExc_TypeError};
   return THPVariable_Unpack(args[i]);
 }
 bool given(PyObject* const* args, Py_ssize_t i) { return args[i] != Py_None; }
 long long int_at(PyObject* const* args, Py_ssize_t i) {
   const long long v = PyLong_AsLongLong(args[i]);
-  if (v == -1 && PyErr_Occurred()) throw Failure{""};
+  if (v == -1 && PyErr_Occurred()) throw Failure{};
   return v;
 }
 double float_at(PyObject* const* args, Py_ssize_t i) {
   const double v = PyFloat_AsDouble(args[i]);
-  if (v == -1.0 && PyErr_Occurred()) throw Failure{""};
+  if (v == -1.0 && PyErr_Occurred()) throw Failure{};
   return v;
 }
 void require(bool ok, const char* what) {
+  if (!ok) throw Failure{what, PyExc_AssertionError};
+}
+void require_cuda(const at::Tensor& t) {
+  if (!t.is_cuda()) fail("inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+}
+void require_reshape(bool ok, const char* what) {   // (what torch's reshape refuses, and with its type)
   if (!ok) fail(what);
 }
 // a contiguous BF16 tensor on the GPU, its data on a 16-byte boundary
 at::Tensor bf16_rows(const at::Tensor& t, const char* what) {
-  require(t.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
   require(t.scalar_type() == at::kBFloat16, what);
+  require_cuda(t);
   at::Tensor c = t.is_contiguous() ? t : t.contiguous();
   return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
 }
@@ -89,38 +99,39 @@ at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, si
 
 // (query, relative_states, proj, k_cache, v_cache, position, pad_counts, window, n_floor, alpha, scale, out, new_key, new_value)
 PyObject* decode_attention(PyObject* const* args) {
-  const at::Tensor &query = tensor_at(args, 0), &proj = tensor_at(args, 2), &k = tensor_at(args, 3), &v = tensor_at(args, 4), &position = tensor_at(args, 5);
-  require(k.is_cuda() && v.is_cuda() && proj.is_cuda() && position.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+  const at::Tensor &query = tensor_at(args, 0), &states = tensor_at(args, 1), &proj = tensor_at(args, 2), &k = tensor_at(args, 3), &v = tensor_at(args, 4);
+  require(THPVariable_Check(args[5]) && tensor_at(args, 5).scalar_type() == at::kLong, "decode_attention: int64 position on the device");
+  const at::Tensor& position = tensor_at(args, 5);
+  for (const at::Tensor* t : {&query, &states, &proj, &k, &v}) require(t->scalar_type() == at::kBFloat16, "decode_attention: BF16 query, relative states, proj and caches");
   require(query.dim() >= 3 && k.dim() == 4 && proj.dim() == 2, "decode_attention: query [bs, h, (1,) c], caches [bs, hk, slots, c], proj [d_rel, extent]");
   const int64_t bs = query.size(0), h = query.size(1), c = query.size(-1), hk = k.size(1), slots = k.size(2), d_rel = proj.size(0);
-  const at::Tensor q = bf16_rows(query, "decode_attention: BF16 query");
-  const at::Tensor& states = tensor_at(args, 1);
-  require(states.is_cuda() && states.scalar_type() == at::kBFloat16, "decode_attention: BF16 relative states on the GPU");
-  const at::Tensor r = states.is_contiguous() ? states : states.contiguous();
-  require(q.numel() == bs * h * c && r.numel() == bs * h * d_rel, "decode_attention: one query and one relative state per sequence and head");
   require(proj.is_contiguous() && k.is_contiguous() && v.is_contiguous() && k.sizes() == v.sizes(), "decode_attention: contiguous proj and caches of one shape");
-  require(proj.scalar_type() == at::kBFloat16 && k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16, "decode_attention: BF16 proj and caches");
   require(k.size(0) == bs && k.size(3) == c, "decode_attention: caches of the query's batch and head width");
-  require(position.scalar_type() == at::kLong, "decode_attention: int64 position");
+  require_reshape(query.numel() == bs * h * c, "decode_attention: one query per sequence and head");
+  require(states.numel() == bs * h * d_rel, "decode_attention: one relative state per sequence and head");
   const void* pads = nullptr;
   if (given(args, 6)) {
     const at::Tensor& p = tensor_at(args, 6);
-    require(p.is_cuda() && p.scalar_type() == at::kLong && p.numel() == bs && p.is_contiguous(), "decode_attention: int64 pad_counts [bs]");
+    require(p.scalar_type() == at::kLong && p.numel() == bs && p.is_contiguous(), "decode_attention: int64 pad_counts [bs]");
+    require_cuda(p);
     pads = p.data_ptr();
   }
+  for (const at::Tensor* t : {&states, &proj, &k, &v, &position}) require_cuda(*t);
+  const at::Tensor q = bf16_rows(query, "decode_attention: BF16 query");
+  const at::Tensor r = states.is_contiguous() ? states : states.contiguous();
   at::Tensor new_k, new_v;
   if (given(args, 12)) {
     require(given(args, 13), "decode_attention: new_key and new_value come together");
     new_k = bf16_rows(tensor_at(args, 12), "decode_attention: BF16 new_key");
     new_v = bf16_rows(tensor_at(args, 13), "decode_attention: BF16 new_value");
-    require(new_k.numel() == bs * hk * c && new_v.numel() == bs * hk * c, "decode_attention: one new key and value per sequence and key/value head");
+    require_reshape(new_k.numel() == bs * hk * c && new_v.numel() == bs * hk * c, "decode_attention: one new key and value per sequence and key/value head");
   }
   const c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
   at::Tensor out;
   if (given(args, 11)) {
     out = tensor_at(args, 11);
-    require(out.is_cuda(), "inkling_b200 kernels run on CUDA tensors only (no CPU path)");
+    require_cuda(out);
   } else {
     out = new_tensor({bs, h, 1, c}, at::kBFloat16, q.device());
   }
@@ -183,7 +194,7 @@ PyObject* make_block(PyObject* const* args) {
       continue;
     }
     block->v[f] = PyLong_AsLongLong(item);
-    if (block->v[f] == -1 && PyErr_Occurred()) throw Failure{""};
+    if (block->v[f] == -1 && PyErr_Occurred()) throw Failure{};
   }
   PyObject* capsule = PyCapsule_New(block.get(), "inkling_block", [](PyObject* c) { delete (Block*)PyCapsule_GetPointer(c, "inkling_block"); });
   if (capsule) (void)block.release();
@@ -191,7 +202,7 @@ PyObject* make_block(PyObject* const* args) {
 }
 const Block& block_at(PyObject* const* args) {
   auto* block = (const Block*)PyCapsule_GetPointer(args[0], "inkling_block");
-  if (!block) throw Failure{""};
+  if (!block) throw Failure{};
   return *block;
 }
 struct Rows {   // the block's input as [tokens, hidden]
@@ -270,7 +281,8 @@ PyObject* run_experts(PyObject* const* args) {
   const at::Tensor& input = tensor_at(args, 1);
   const Rows r = rows_of(b, input);
   const at::Tensor &i = tensor_at(args, 2), weights = bf16_rows(tensor_at(args, 3), "BF16 router weights expected");
-  require(i.is_cuda() && i.scalar_type() == at::kLong && i.numel() == r.tokens * b.v[kTopK] && weights.numel() == i.numel(), "int64 indices and BF16 weights [tokens, top_k]");
+  require(i.scalar_type() == at::kLong && i.numel() == r.tokens * b.v[kTopK] && weights.numel() == i.numel(), "int64 indices and BF16 weights [tokens, top_k]");
+  require_cuda(i);
   const at::Tensor indices = i.is_contiguous() ? i : i.contiguous();
   require(indices.numel() <= b.v[kCapacity], "more routes than the module's buffers hold");
   const c10::cuda::CUDAGuard guard(r.x.device());
@@ -296,9 +308,9 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   try {
     return F(args);
   } catch (const Failure& f) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, f.what.c_str());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+    if (f.type) PyErr_SetString(f.type, f.what.c_str());
+  } catch (...) {
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }

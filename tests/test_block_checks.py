@@ -101,3 +101,23 @@ def test_experts_that_ran_out_of_memory_count_on_no_buffers(monkeypatch, nth):
     assert experts.capacity == 0
     experts._reserve(2)
     assert experts.capacity == 2 and experts.rows.shape == (3, 2) and experts.activated.shape == (2, F) and experts.down.shape == (2, D)
+
+
+@pytest.mark.parametrize("error,change", [
+    (AssertionError, dict(query=lambda t: t.float())), (AssertionError, dict(k_cache=lambda t: t.transpose(2, 3))),
+    (AssertionError, dict(position=lambda t: 3)), (AssertionError, dict(position=lambda t: t.int())), (AssertionError, dict(proj=lambda t: t.t())),
+    (AssertionError, dict(pad_counts=lambda t: t.int())), (AssertionError, dict(pad_counts=lambda t: t[:1])), (AssertionError, dict(v_cache=lambda t: t[:, :, :-1])),
+    (AssertionError, dict(relative_states=lambda t: t[..., :-1].contiguous())), (RuntimeError, dict(query=lambda t: torch.cat([t, t], 2))), (RuntimeError, {}),
+    (TypeError, dict(k_cache=lambda t: None)),
+], ids=lambda v: v.__name__ if isinstance(v, type) else "-".join(v) or "on the host")
+def test_what_attention_refuses_and_with_which_error(error, change):
+    """Arguments of the wrong form are assertions, whichever device they are on; then come the tensors that are not on a GPU."""
+    import inkling_b200 as ib
+
+    zeros = lambda *s: torch.zeros(*s, dtype=torch.bfloat16)  # noqa: E731
+    args = dict(query=zeros(2, 4, 1, 64), relative_states=zeros(2, 1, 4, 16), proj=zeros(16, 8), k_cache=zeros(2, 2, 20, 64), v_cache=zeros(2, 2, 20, 64),
+                position=torch.tensor(3), pad_counts=torch.zeros(2, dtype=torch.int64))
+    args.update({n: f(args[n]) for n, f in change.items()})
+    with pytest.raises(error) as caught:
+        ib.kernels.decode_attention(**args)
+    assert caught.type is error

@@ -317,3 +317,36 @@ def test_experts_put_in_place_of_others_get_the_room_they_need(ib, device):
     assert fresh.capacity == 8
     layer.experts = fresh
     assert torch.equal(layer(x), want)
+
+
+@pytest.mark.parametrize("tokens", [1, 9])
+def test_errors_of_the_native_calls_keep_their_types(ib, device, tokens):
+    layer, x = _block(ib, device, tokens, d=1024, f=512, experts=8)
+    idx, w = torch.zeros(tokens, 3, dtype=torch.int64, device=device), torch.ones(tokens, 3, dtype=BF16, device=device)
+    for wrong in (x.float(), x[:, :-8], x.cpu().float()):
+        with pytest.raises(AssertionError):
+            layer(wrong)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        layer(x.cpu())
+    if tokens > 1:
+        for args in ((x, idx.int(), w), (x, idx, w.float()), (x, idx, w[:, :-1])):
+            with pytest.raises(AssertionError):
+                layer.experts(*args)
+
+
+def test_out_of_memory_in_a_native_call_is_torchs_error(ib, device):
+    """The scratch of a call finds no room: the allocator's limit is set to what is reserved, and the
+    scratch of the next call comes on top."""
+    layer, x = _block(ib, device, 64)
+    prompt = x.repeat(64, 1)
+    want = layer(prompt).clone()   # (buffers of the module, and the scratch, which goes back)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(device).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(device) + (1 << 20)) / total, device)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            layer(prompt)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, device)
+    assert torch.equal(layer(prompt), want)
