@@ -62,6 +62,13 @@ at::Tensor bf16_rows(const at::Tensor& t, const char* what) {
   at::Tensor c = t.is_contiguous() ? t : t.contiguous();
   return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 15) ? c.clone() : c;
 }
+// Allocation and launches run without the interpreter's lock: a launch waits while the stream's queue is full, and the other
+// threads, or a host function that a stream is waiting for, may need the interpreter meanwhile. (The caller's frame holds the
+// arguments.)
+struct WithoutGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
 at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
   return at::empty(sizes, at::TensorOptions().dtype(type).device(device));
 }
@@ -117,31 +124,37 @@ PyObject* decode_attention(PyObject* const* args) {
     pads = p.data_ptr();
   }
   for (const at::Tensor* t : {&states, &proj, &k, &v, &position}) require_cuda(*t);
-  const at::Tensor q = bf16_rows(query, "decode_attention: BF16 query");
-  const at::Tensor r = states.is_contiguous() ? states : states.contiguous();
-  at::Tensor new_k, new_v;
-  if (given(args, 12)) {
-    require(given(args, 13), "decode_attention: new_key and new_value come together");
-    new_k = bf16_rows(tensor_at(args, 12), "decode_attention: BF16 new_key");
-    new_v = bf16_rows(tensor_at(args, 13), "decode_attention: BF16 new_value");
-    require_reshape(new_k.numel() == bs * hk * c && new_v.numel() == bs * hk * c, "decode_attention: one new key and value per sequence and key/value head");
-  }
-  const c10::cuda::CUDAGuard guard(q.device());
-  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  at::Tensor out;
+  at::Tensor out, new_k, new_v;
   if (given(args, 11)) {
     out = tensor_at(args, 11);
     require_cuda(out);
-  } else {
-    out = new_tensor({bs, h, 1, c}, at::kBFloat16, q.device());
   }
-  const size_t need = ink_decode_attention_workspace_bytes((int)bs, (int)h, (int)c, (int)slots);
-  at::Tensor workspace;
-  if (need) workspace = attention_workspace(q.device(), stream, need, ink_decode_attention_counter_bytes((int)bs, (int)h));
-  check(ink_decode_attention(q.data_ptr(), r.data_ptr(), proj.data_ptr(), k.data_ptr(), v.data_ptr(), (const int64_t*)position.data_ptr(), (const int64_t*)pads,
-                             out.data_ptr(), (int)bs, (int)h, (int)hk, (int)c, (int)d_rel, (int)proj.size(1), (int)slots, (int)int_at(args, 7), (int)int_at(args, 8),
-                             (float)float_at(args, 9), (float)float_at(args, 10), new_k.defined() ? new_k.data_ptr() : nullptr,
-                             new_v.defined() ? new_v.data_ptr() : nullptr, need ? workspace.data_ptr() : nullptr, need, stream));
+  if (given(args, 12)) {
+    require(given(args, 13), "decode_attention: new_key and new_value come together");
+    new_k = tensor_at(args, 12);
+    new_v = tensor_at(args, 13);
+    require_reshape(new_k.numel() == bs * hk * c && new_v.numel() == bs * hk * c, "decode_attention: one new key and value per sequence and key/value head");
+  }
+  const int window = (int)int_at(args, 7), n_floor = (int)int_at(args, 8);
+  const float alpha = (float)float_at(args, 9), scale = (float)float_at(args, 10);
+  {
+    const WithoutGil unlocked;
+    const at::Tensor q = bf16_rows(query, "decode_attention: BF16 query");
+    const at::Tensor r = states.is_contiguous() ? states : states.contiguous();
+    if (new_k.defined()) {
+      new_k = bf16_rows(new_k, "decode_attention: BF16 new_key");
+      new_v = bf16_rows(new_v, "decode_attention: BF16 new_value");
+    }
+    const c10::cuda::CUDAGuard guard(q.device());
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+    if (!out.defined()) out = new_tensor({bs, h, 1, c}, at::kBFloat16, q.device());
+    const size_t need = ink_decode_attention_workspace_bytes((int)bs, (int)h, (int)c, (int)slots);
+    at::Tensor workspace;
+    if (need) workspace = attention_workspace(q.device(), stream, need, ink_decode_attention_counter_bytes((int)bs, (int)h));
+    check(ink_decode_attention(q.data_ptr(), r.data_ptr(), proj.data_ptr(), k.data_ptr(), v.data_ptr(), (const int64_t*)position.data_ptr(), (const int64_t*)pads,
+                               out.data_ptr(), (int)bs, (int)h, (int)hk, (int)c, (int)d_rel, (int)proj.size(1), (int)slots, window, n_floor, alpha, scale, new_k.defined() ? new_k.data_ptr() : nullptr,
+                               new_v.defined() ? new_v.data_ptr() : nullptr, need ? workspace.data_ptr() : nullptr, need, stream));
+  }
   return THPVariable_Wrap(out);
 }
 
@@ -158,6 +171,7 @@ struct Kept {
 struct Block {
   long long v[48] = {};
   std::vector<Kept> kept;
+  std::shared_ptr<std::mutex> launching;   // see launch_lock
   bool current() const {
     for (const Kept& k : kept)
       if ((long long)(uintptr_t)k.t.data_ptr() != v[k.field] || k.t.scalar_type() != k.type || k.t.sizes() != at::IntArrayRef(k.sizes) ||
@@ -182,6 +196,18 @@ T* at_field(const Block& b, Field f) {
   return reinterpret_cast<T*>((uintptr_t)b.v[f]);
 }
 
+// The launches of a call hand buffers of the module from one to the next, so they go to their stream as one sequence although
+// the interpreter is free meanwhile: one lock per pointer table, i.e. for a module of experts and every block that uses it.
+std::shared_ptr<std::mutex> launch_lock(long long pointers) {
+  static std::mutex mutex;
+  static auto* locks = new std::map<long long, std::weak_ptr<std::mutex>>();
+  const std::lock_guard<std::mutex> lock(mutex);
+  for (auto it = locks->begin(); it != locks->end();) it = it->second.expired() ? locks->erase(it) : std::next(it);
+  std::shared_ptr<std::mutex> found = (*locks)[pointers].lock();
+  if (!found) (*locks)[pointers] = found = std::make_shared<std::mutex>();
+  return found;
+}
+
 PyObject* make_block(PyObject* const* args) {
   auto block = std::make_unique<Block>();
   for (int f = 0; f < kFields; ++f) {
@@ -196,6 +222,7 @@ PyObject* make_block(PyObject* const* args) {
     block->v[f] = PyLong_AsLongLong(item);
     if (block->v[f] == -1 && PyErr_Occurred()) throw Failure{};
   }
+  block->launching = launch_lock(block->v[kPointers]);
   PyObject* capsule = PyCapsule_New(block.get(), "inkling_block", [](PyObject* c) { delete (Block*)PyCapsule_GetPointer(c, "inkling_block"); });
   if (capsule) (void)block.release();
   return capsule;
@@ -235,16 +262,12 @@ void grouped(const Block& b, const Rows& r, int t0, int tokens, const int64_t* i
                         at_field<int32_t>(b, kStatus), stream));
 }
 
-// (block, x, want_partial) -> BF16 like x; with want_partial the FP32 output goes to the block's own buffer, None is returned
-PyObject* run_block(PyObject* const* args) {
-  const Block& b = block_at(args);
-  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
-  const at::Tensor& input = tensor_at(args, 1);
+at::Tensor block_forward(const Block& b, const at::Tensor& input, bool want_partial) {
   const Rows r = rows_of(b, input);
   require(r.tokens <= b.v[kTokens] && (r.tokens == 1 || std::min(r.tokens, kMostTokens) * b.v[kTopK] <= b.v[kCapacity]), "more tokens than the block's buffers hold");
-  const bool want_partial = args[2] == Py_True;
   const c10::cuda::CUDAGuard guard(r.x.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();
+  const std::lock_guard<std::mutex> one_call(*b.launching);
   at::Tensor out;
   if (!want_partial) out = new_tensor(input.sizes(), at::kBFloat16, r.x.device());
   if (r.tokens == 1 && b.v[kTable]) {
@@ -270,23 +293,33 @@ PyObject* run_block(PyObject* const* args) {
               (int)b.v[kShared], stream);
     }
   }
+  return out;
+}
+// (block, x, want_partial) -> BF16 like x; with want_partial the FP32 output goes to the block's own buffer, None is returned
+PyObject* run_block(PyObject* const* args) {
+  const Block& b = block_at(args);
+  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
+  const at::Tensor& input = tensor_at(args, 1);
+  const bool want_partial = args[2] == Py_True;
+  at::Tensor out;
+  {
+    const WithoutGil unlocked;
+    out = block_forward(b, input, want_partial);
+  }
   if (want_partial) Py_RETURN_NONE;
   return THPVariable_Wrap(out);
 }
 
-// (block, x, indices, weights) -> BF16 like x: the routed experts alone, plan and projections
-PyObject* run_experts(PyObject* const* args) {
-  const Block& b = block_at(args);
-  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
-  const at::Tensor& input = tensor_at(args, 1);
+at::Tensor experts_forward(const Block& b, const at::Tensor& input, const at::Tensor& i, const at::Tensor& w) {
   const Rows r = rows_of(b, input);
-  const at::Tensor &i = tensor_at(args, 2), weights = bf16_rows(tensor_at(args, 3), "BF16 router weights expected");
+  const at::Tensor weights = bf16_rows(w, "BF16 router weights expected");
   require(i.scalar_type() == at::kLong && i.numel() == r.tokens * b.v[kTopK] && weights.numel() == i.numel(), "int64 indices and BF16 weights [tokens, top_k]");
   require_cuda(i);
   const at::Tensor indices = i.is_contiguous() ? i : i.contiguous();
   require(indices.numel() <= b.v[kCapacity], "more routes than the module's buffers hold");
   const c10::cuda::CUDAGuard guard(r.x.device());
   const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(r.x.device().index()).stream();
+  const std::lock_guard<std::mutex> one_call(*b.launching);
   const at::Tensor out = new_tensor(input.sizes(), at::kBFloat16, r.x.device());
   for (int t0 = 0; t0 < r.tokens; t0 += kMostTokens) {
     const int tokens = std::min(kMostTokens, r.tokens - t0);
@@ -295,6 +328,18 @@ PyObject* run_experts(PyObject* const* args) {
     check(ink_expert_plan(here, at_field<int64_t>(b, kSources), at_field<int64_t>(b, kPointers), at_field<int32_t>(b, kExperts), at_field<int32_t>(b, kCounts),
                           at_field<int32_t>(b, kRows), (int)b.v[kStart], (int)b.v[kLocal], (int)b.v[kStride], tokens * (int)b.v[kTopK], (int)b.v[kCapacity], stream));
     grouped(b, r, t0, tokens, here, (const char*)weights.data_ptr() + 2 * routes0, nullptr, nullptr, out.data_ptr(), 0, stream);
+  }
+  return out;
+}
+// (block, x, indices, weights) -> BF16 like x: the routed experts alone, plan and projections
+PyObject* run_experts(PyObject* const* args) {
+  const Block& b = block_at(args);
+  if (!b.current()) Py_RETURN_NOTIMPLEMENTED;
+  const at::Tensor &input = tensor_at(args, 1), &indices = tensor_at(args, 2), &weights = tensor_at(args, 3);
+  at::Tensor out;
+  {
+    const WithoutGil unlocked;
+    out = experts_forward(b, input, indices, weights);
   }
   return THPVariable_Wrap(out);
 }

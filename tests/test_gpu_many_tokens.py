@@ -350,3 +350,59 @@ def test_out_of_memory_in_a_native_call_is_torchs_error(ib, device):
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0, device)
     assert torch.equal(layer(prompt), want)
+
+
+def test_other_threads_run_while_a_call_waits_for_its_stream(ib, device):
+    """More launches than a stream's queue holds, behind 0.3 s of other work: the call that finds the queue full waits, but not
+    with the interpreter."""
+    import threading
+    import time
+
+    layer, x = _block(ib, device, 9)
+    layer(x)
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), []
+
+    def ticks():
+        last = time.monotonic()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.monotonic()
+            gaps.append(now - last)
+            last = now
+
+    thread = threading.Thread(target=ticks)
+    thread.start()
+    torch.cuda._sleep(int(0.3 * 1.9e9))
+    start = time.monotonic()
+    for _ in range(600):
+        layer(x)
+    waited = time.monotonic() - start
+    stop.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.15, "the queue took everything: the call never waited"
+    assert max(gaps) < 0.1
+
+
+def test_calls_of_several_threads_do_not_mix(ib, device):
+    """One module on one stream from four threads: a call's launches follow one another."""
+    import threading
+
+    layer, x = _block(ib, device, 48)
+    inputs = [x[12 * i:12 * i + 12].contiguous() for i in range(4)]
+    want = [layer(t).clone() for t in inputs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def run(i):
+        for n in range(150):
+            if not torch.equal(layer(inputs[i]), want[i]):
+                wrong.append((i, n))
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
