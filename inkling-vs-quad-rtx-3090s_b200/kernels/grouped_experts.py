@@ -31,8 +31,7 @@ def _maps_to_device(size: int, device, encode) -> torch.Tensor:
     _abi.check(encode((ctypes.c_char * size).from_buffer(host)))
     if torch.cuda.is_current_stream_capturing():
         raise RuntimeError("descriptors are made before graph capture")   # (a recorded copy would read this buffer at replay)
-    # a copy from pageable memory has read its source when it returns, but does not wait for the work in front of it
-    maps = torch.frombuffer(host, dtype=torch.uint8).to(device, non_blocking=True)
+    maps = torch.frombuffer(host, dtype=torch.uint8).to(device)   # (waits: the descriptors may be used on any stream from here on)
     assert maps.data_ptr() % 128 == 0
     return maps
 

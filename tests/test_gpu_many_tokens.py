@@ -406,3 +406,19 @@ def test_calls_of_several_threads_do_not_mix(ib, device):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_descriptors_are_there_for_every_stream(ib, device):
+    """Made on a stream that has other work in front; a stream that does not wait for it finds them whole."""
+    gate, up, down = torch.zeros(2, 256, 512, dtype=BF16, device=device), torch.zeros(2, 256, 512, dtype=BF16, device=device), torch.zeros(2, 512, 256, dtype=BF16, device=device)
+    want = ib.kernels.encode_shared_maps(gate, up, down).cpu()
+    torch.cuda.synchronize()
+    busy, other = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        used = torch.full((1 << 14,), 127, dtype=torch.uint8, device=device)   # (what the allocator may hand out next)
+        del used
+        torch.cuda._sleep(int(0.1 * 1.9e9))
+        maps = ib.kernels.encode_shared_maps(gate, up, down)
+    with torch.cuda.stream(other):
+        assert torch.equal(maps.cpu(), want)
+    torch.cuda.synchronize()
