@@ -66,7 +66,7 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 // the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
 // deliver at HBM speed, so scores, bias and weighted values go through warp-level matrix instructions (M = heads: the
 // contraction is far too flat for the 128-row tcgen05 tiles). Measured on B200, batch 8, 64 heads on 8 key/value
-// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, 173 us with this one (5.0 TB/s).
+// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, 172 us with this one (5.0 TB/s).
 //
 // A warp takes 16 slots a step and keeps everything in registers; nothing of the cache passes through shared memory,
 // because the sums over channels may run in any order as long as both operands agree:
@@ -74,8 +74,8 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 //           of slot g; the four words of a piece are two k-steps' worth of B.
 //   values  A = the exponentials, which the score accumulators already hold in A's layout; B = the values: lane (g, t)
 //           loads the piece g (and g + 8) of the rows 2t, 2t+1, 2t+8, 2t+9, and word pairs of neighbouring rows are
-//           interleaved into B. The unused upper eight rows of A carry what BF16 cuts off the exponentials (p = hi + lo),
-//           so the weights keep 16 bits at no further instruction.
+//           interleaved into B. An exponential's 24 bits are three BF16 values, p = hi + mid + lo exactly: hi in the rows of
+//           the heads, mid in the eight rows below, which nobody needs, lo by a second instruction (4 of the 172 us).
 //
 // The parts of a group of heads are joined in one of two ways. Up to eight of them form a thread-block cluster (CLUSTER)
 // and read one another's sums through distributed shared memory; more leave their sums in global memory and the block that
@@ -245,13 +245,15 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
         acc[i][3] *= factor;
       }
     }
-    uint32_t p_hi[2], p_lo[2];
+    uint32_t p_hi[2], p_mid[2], p_lo[2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const float p0 = s[n][0] == -INFINITY ? 0.f : __expf(s[n][0] - top), p1 = s[n][1] == -INFINITY ? 0.f : __expf(s[n][1] - top);
       total += p0 + p1;
       p_hi[n] = pack_bf16(p0, p1);
-      p_lo[n] = pack_bf16(p0 - bf16lo(p_hi[n]), p1 - bf16hi(p_hi[n]));
+      const float r0 = p0 - bf16lo(p_hi[n]), r1 = p1 - bf16hi(p_hi[n]);
+      p_mid[n] = pack_bf16(r0, r1);
+      p_lo[n] = pack_bf16(r0 - bf16lo(p_mid[n]), r1 - bf16hi(p_mid[n]));
     }
     // ---- weighted values: 8 channels of the lane's piece, one instruction each
 #pragma unroll
@@ -262,8 +264,12 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
       const uint32_t w2[4] = {v4[2].x, v4[2].y, v4[2].z, v4[2].w}, w3[4] = {v4[3].x, v4[3].y, v4[3].z, v4[3].w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        mma_bf16(acc[h * 8 + 2 * j], p_hi[0], p_lo[0], p_hi[1], p_lo[1], __byte_perm(w0[j], w1[j], 0x5410), __byte_perm(w2[j], w3[j], 0x5410));
-        mma_bf16(acc[h * 8 + 2 * j + 1], p_hi[0], p_lo[0], p_hi[1], p_lo[1], __byte_perm(w0[j], w1[j], 0x7632), __byte_perm(w2[j], w3[j], 0x7632));
+#pragma unroll
+        for (int odd = 0; odd < 2; ++odd) {
+          const uint32_t b0 = __byte_perm(w0[j], w1[j], odd ? 0x7632 : 0x5410), b1 = __byte_perm(w2[j], w3[j], odd ? 0x7632 : 0x5410);
+          mma_bf16(acc[h * 8 + 2 * j + odd], p_hi[0], p_mid[0], p_hi[1], p_mid[1], b0, b1);
+          mma_bf16(acc[h * 8 + 2 * j + odd], p_lo[0], 0u, p_lo[1], 0u, b0, b1);
+        }
       }
     }
   }

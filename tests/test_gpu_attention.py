@@ -436,3 +436,29 @@ def test_a_new_token_at_any_address_through_the_c_entry(ib):
         i["new_value"].data_ptr(), None, 0, _abi.stream()))
     assert torch.equal(out, want)
     assert torch.equal(caches[0], i["k_cache"]) and torch.equal(caches[1], i["v_cache"])
+
+
+def test_the_exponentials_keep_their_bits(ib):
+    """Slots of three kinds in equal numbers: exponential p with value 1, exponential 1 with values -c and -r, where c is p in
+    BF16 and r what that leaves, in BF16. The result is what 16 bits of p do not hold (some 2^-18) over p + 2; the hardware
+    exponential is good to about 2^-22, a sixteenth of it, so a quarter is asked for."""
+    device = torch.device("cuda", 0)
+    scores = -torch.arange(128, 256).double() / 512
+    p = scores.exp()
+    c = p.bfloat16().double()
+    r = (p - c).bfloat16().double()
+    left = p - c - r
+    pick = int(left.abs().argmax())
+    bs, hk, group, width, slots, used = 8, 8, 8, 64, 1024, 1023
+    kind = torch.arange(slots) % 3
+    k, v = torch.zeros(bs, hk, slots, width), torch.zeros(bs, hk, slots, width)
+    k[..., 0] = torch.tensor([float(scores[pick]), 0.0, 0.0])[kind]
+    v[:] = torch.tensor([1.0, -float(c[pick]), -float(r[pick])])[kind][:, None]
+    q = torch.zeros(bs, hk * group, width)
+    q[..., 0] = 1.0
+    to = lambda t: t.bfloat16().to(device)  # noqa: E731
+    assert torch.equal(to(k).cpu().float(), k) and torch.equal(to(v).cpu().float(), v)
+    got = ib.kernels.decode_attention(to(q), to(torch.zeros(bs, hk * group, 16)), to(torch.zeros(16, 8)), to(k), to(v),
+                                      torch.tensor(used - 1, device=device), scale=1.0).double().cpu()
+    want = float(left[pick] / (p[pick] + 2))
+    assert abs(want) > 2.0 ** -21 and (got - want).abs().max() <= abs(want) / 4
