@@ -49,6 +49,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return r;
 }
 
+// the two floats cut off to BF16
+__device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -66,7 +69,7 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 // the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
 // deliver at HBM speed, so scores, bias and weighted values go through warp-level matrix instructions (M = heads: the
 // contraction is far too flat for the 128-row tcgen05 tiles). Measured on B200, batch 8, 64 heads on 8 key/value
-// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, 172 us with this one (5.0 TB/s).
+// heads, 30 000 of 32 768 slots: 2 586 us with one block per head and 64 slots, 171 us with this one (5.1 TB/s).
 //
 // A warp takes 16 slots a step and keeps everything in registers; nothing of the cache passes through shared memory,
 // because the sums over channels may run in any order as long as both operands agree:
@@ -75,7 +78,10 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 //   values  A = the exponentials, which the score accumulators already hold in A's layout; B = the values: lane (g, t)
 //           loads the piece g (and g + 8) of the rows 2t, 2t+1, 2t+8, 2t+9, and word pairs of neighbouring rows are
 //           interleaved into B. An exponential's 24 bits are three BF16 values, p = hi + mid + lo exactly: hi in the rows of
-//           the heads, mid in the eight rows below, which nobody needs, lo by a second instruction (4 of the 172 us).
+//           the heads, mid in the eight rows below, which nobody needs, lo by a second instruction, half of it in either
+//           row (165 us without it; in any order of the instructions). The parts are cut off, not rounded, and never zero
+//           beside a p that is not (2^-40 p instead, which p does not feel), so that each of them takes an infinite value
+//           to the same infinity.
 //
 // The parts of a group of heads are joined in one of two ways. Up to eight of them form a thread-block cluster (CLUSTER)
 // and read one another's sums through distributed shared memory; more leave their sums in global memory and the block that
@@ -250,10 +256,12 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
     for (int n = 0; n < 2; ++n) {
       const float p0 = s[n][0] == -INFINITY ? 0.f : __expf(s[n][0] - top), p1 = s[n][1] == -INFINITY ? 0.f : __expf(s[n][1] - top);
       total += p0 + p1;
-      p_hi[n] = pack_bf16(p0, p1);
-      const float r0 = p0 - bf16lo(p_hi[n]), r1 = p1 - bf16hi(p_hi[n]);
-      p_mid[n] = pack_bf16(r0, r1);
-      p_lo[n] = pack_bf16(r0 - bf16lo(p_mid[n]), r1 - bf16hi(p_mid[n]));
+      const float mid0 = p0 - bf16hi(__float_as_uint(p0)), mid1 = p1 - bf16hi(__float_as_uint(p1));
+      const float lo0 = mid0 - bf16hi(__float_as_uint(mid0)), lo1 = mid1 - bf16hi(__float_as_uint(mid1));
+      constexpr float kNext = 0x1p-40f;
+      p_hi[n] = high_halves(p0, p1);
+      p_mid[n] = high_halves(fmaxf(mid0, p0 * kNext), fmaxf(mid1, p1 * kNext));
+      p_lo[n] = high_halves(0.5f * fmaxf(lo0, p0 * kNext), 0.5f * fmaxf(lo1, p1 * kNext));
     }
     // ---- weighted values: 8 channels of the lane's piece, one instruction each
 #pragma unroll
@@ -268,7 +276,7 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
         for (int odd = 0; odd < 2; ++odd) {
           const uint32_t b0 = __byte_perm(w0[j], w1[j], odd ? 0x7632 : 0x5410), b1 = __byte_perm(w2[j], w3[j], odd ? 0x7632 : 0x5410);
           mma_bf16(acc[h * 8 + 2 * j + odd], p_hi[0], p_mid[0], p_hi[1], p_mid[1], b0, b1);
-          mma_bf16(acc[h * 8 + 2 * j + odd], p_lo[0], 0u, p_lo[1], 0u, b0, b1);
+          mma_bf16(acc[h * 8 + 2 * j + odd], p_lo[0], p_lo[0], p_lo[1], p_lo[1], b0, b1);   // (a half of lo in either row)
         }
       }
     }

@@ -462,3 +462,23 @@ def test_the_exponentials_keep_their_bits(ib):
                                       torch.tensor(used - 1, device=device), scale=1.0).double().cpu()
     want = float(left[pick] / (p[pick] + 2))
     assert abs(want) > 2.0 ** -21 and (got - want).abs().max() <= abs(want) / 4
+
+
+@pytest.mark.parametrize("bs,hk,slots", [(1, 2, 40), (8, 8, 1000), (16, 16, 200), (2, 2, 5000)])   # small form, then parts joined in memory, in a cluster
+def test_values_that_are_not_finite(ib, bs, hk, slots):
+    """An infinite cached value is an infinite result, of its sign and in its channel only, whatever its weight's bits (the top
+    slots' weight is 1); NaN and both infinities together are NaN; slots that do not count may hold anything."""
+    device = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(slots)
+    draw = lambda *shape: (torch.randn(*shape, generator=gen) * 0.3).bfloat16()  # noqa: E731
+    q, r, proj, k, v = draw(bs, 4 * hk, 64), draw(bs, 4 * hk, 16), draw(16, 8), draw(bs, hk, slots, 64), draw(bs, hk, slots, 64)
+    inf, nan, used = float("inf"), float("nan"), slots - 9
+    v[..., 0], v[:, :, 3, 1], v[:, :, 5, 2], v[:, :, 6, 3], v[:, :, 7, 3], v[:, :, used - 1, 4] = inf, -inf, nan, inf, -inf, inf
+    k[:, :, used:], v[:, :, used:] = nan, nan
+    pad = torch.zeros(bs, dtype=torch.int64)
+    got = ib.kernels.decode_attention(*(t.to(device) for t in (q, r, proj, k, v)), torch.tensor(used - 1, device=device), pad.to(device))[:, :, 0].float().cpu()
+    keep = (k[:, :, :used], v[:, :, :used])
+    want = oa.decode_attention(q, r, proj, *keep, used - 1, pad, 0, None, 0.1, 1.0 / 64).float()
+    finite = torch.isfinite(want)
+    assert torch.equal(got[~finite].nan_to_num(7.0, 1.0, -1.0), want[~finite].nan_to_num(7.0, 1.0, -1.0)) and int((~finite).sum()) == bs * 4 * hk * 5
+    assert torch.isfinite(got[finite]).all() and (got[finite] - want[finite]).abs().max() <= TOL * want[finite].abs().max()
