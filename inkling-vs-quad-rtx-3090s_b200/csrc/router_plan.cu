@@ -466,10 +466,18 @@ static int launch_router(const RouterArgs& a, const PlanArgs* p, cudaStream_t st
     INK_CHECK_LAUNCH("ink_router_forward");
     return kOk;
   }
-  const dim3 grid((unsigned)((rows + kManyRows - 1) / kManyRows), (unsigned)((a.tokens + kManyTokens - 1) / kManyTokens));
-  INK_REQUIRE(grid.y <= 65535, kUnsupportedShape, "router: %d tokens in one call", a.tokens);
-  router_logits_kernel<<<grid, kManyThreads, 0, stream>>>(a);
-  INK_CHECK_LAUNCH("ink_router_forward (logits)");
+  constexpr int kMost = 65535 * kManyTokens;   // (what a grid's second dimension holds)
+  for (int t0 = 0; t0 < a.tokens; t0 += kMost) {
+    RouterArgs part = a;
+    part.tokens = a.tokens - t0 < kMost ? a.tokens - t0 : kMost;
+    part.x += (size_t)t0 * a.hidden;
+    part.logits += (size_t)t0 * rows;
+    part.scores += (size_t)t0 * a.n_routed;
+    const dim3 grid((unsigned)((rows + kManyRows - 1) / kManyRows), (unsigned)((part.tokens + kManyTokens - 1) / kManyTokens));
+    router_logits_kernel<<<grid, kManyThreads, 0, stream>>>(part);
+    INK_CHECK_LAUNCH("ink_router_forward (logits)");
+    if (a.tokens - t0 <= kMost) break;   // (t0 stays inside an int)
+  }
   const unsigned selects = (unsigned)((a.tokens + 31) / 32);
   if (!p) {
     router_select_kernel<false><<<selects, 1024, 0, stream>>>(a, PlanArgs{}, 0);

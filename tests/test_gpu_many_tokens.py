@@ -422,3 +422,20 @@ def test_descriptors_are_there_for_every_stream(ib, device):
     with torch.cuda.stream(other):
         assert torch.equal(maps.cpu(), want)
     torch.cuda.synchronize()
+
+
+def test_a_router_call_of_more_tokens_than_a_grid_is_high(ib, device):
+    """65 535 tiles of sixteen tokens and a few more: the last tokens as in a call of their own."""
+    tokens, hidden, routed, top_k = 65535 * 16 + 21, 8, 4, 2
+    gen = torch.Generator(device).manual_seed(1)
+    draw = lambda *s: torch.randn(*s, generator=gen, device=device)  # noqa: E731
+    x, weight, bias, scale = draw(tokens, hidden).to(BF16), draw(routed, hidden).to(BF16), draw(routed) * 0.1, torch.ones(1, dtype=BF16, device=device)
+
+    def route(x):
+        t = x.shape[0]
+        out = (torch.empty(t, top_k, dtype=BF16, device=device), torch.empty(t, top_k, dtype=torch.int64, device=device), torch.empty(t, 0, dtype=BF16, device=device))
+        ib.kernels.router_forward(x, weight, bias, scale, 8.0, top_k, 0, *out, ib.kernels.router_workspace(t, routed, device))
+        return out
+
+    whole, last = route(x), route(x[-40:].contiguous())
+    assert all(torch.equal(a[-40:], b) for a, b in zip(whole, last))
