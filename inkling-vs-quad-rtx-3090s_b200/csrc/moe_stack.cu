@@ -1253,9 +1253,11 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       // every block resolves the routing for itself (same inputs, same arithmetic, same result): the
       // code stays warm in this SM's instruction cache and nothing has to be published between blocks
       if (!stack_router_tail(a, a.layers[layer], layer, &sh)) break;
-      // the constants of this layer are in the route table now; fetch the next layer's while this one streams.
+      // The constants of this layer are in the route table now; the next layer's are fetched while this one streams: on
+      // the CUDA-core path after the counters below, which blocks are waiting for (the loads in front of them held every
+      // narrow layer up by some 3 us); nobody needs the constants before the next layer starts.
       // (The consumers read this layer's biases only before they publish its scores, i.e. before this point.)
-      if (layer + 1 < a.n_layers) load_route_consts(a, layer + 1, &sh);
+      if (tc && layer + 1 < a.n_layers) load_route_consts(a, layer + 1, &sh);
       if (!tc && lane == 0) {
         // One lane polls the layer's grid-wide counters for the whole block and raises a flag in shared memory
         // for each: eight polling warps per block crowd the counter's L2 line and hold up its increments.
@@ -1267,6 +1269,8 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         __threadfence_block();
         sh.seen[1] = layer + 1;
       }
+      __syncwarp();
+      if (!tc && layer + 1 < a.n_layers) load_route_consts(a, layer + 1, &sh);
       if (tc && lane == 0 && !sh.failed) {
         // ---- the routed projections on the tensor cores: one thread issues. A unit is 128 weight rows x
         // 256 columns in two ring slots; four MMAs of 64 columns each accumulate it into the tile's accumulator.
