@@ -367,26 +367,72 @@ def test_a_decode_step_of_the_whole_model(ib, step):
     (64, 8, 2, 48, 48, 1000, 16),         # a ring that is not a multiple of a step, wrapped
 ])
 def test_decode_attention_at_the_edges_of_its_parts(ib, c, h, hk, slots, window, position, d_rel):
-    """Steps of 16 slots, groups of eight heads, parts along the cache: remainders of each, against the oracle with
-    the module's roundings (bar: BF16 results of a softmax-weighted sum, as above)."""
+    """Two sequences: parts of 64 slots on the CUDA cores, groups of eight heads, remainders of each (5 000 slots: the form with
+    matrix instructions, 55 parts)."""
+    _against_the_oracle(ib, 2, c, h, hk, slots, window, position, d_rel)
+
+
+def _against_the_oracle(ib, bs, c, h, hk, slots, window, position, d_rel):
+    """Against the oracle with the module's roundings (bar: BF16 results of a softmax-weighted sum, as above), twice; returns
+    the call."""
     device = torch.device("cuda", 0)
     gen = torch.Generator().manual_seed(17)
-    bs, extent = 2, max(8, slots // 2)
+    extent = max(8, slots // 2)
     draw = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()  # noqa: E731
     q, r, proj = draw(bs, h, c), draw(bs, h, d_rel), draw(d_rel, extent)
     k, v, new_k, new_v = draw(bs, hk, slots, c), draw(bs, hk, slots, c), draw(bs, hk, c), draw(bs, hk, c)
     slot = position % window if window else position
     before = [t.clone().to(device) for t in (k, v)]
     k[:, :, slot], v[:, :, slot] = new_k, new_v
-    pad = torch.tensor([0, min(position, 19)])
+    pad = torch.tensor([0, min(position, 19)] + [min(position, 3)] * (bs - 2))[:bs]
     want = oa.decode_attention(q, r, proj, k, v, position, pad, window, 40, 0.1, 1.0 / c).float()
+    args = (q.to(device), r.to(device), proj.to(device), *before, torch.tensor(position, device=device), pad.to(device))
+    new = dict(new_key=new_k.to(device).unsqueeze(2), new_value=new_v.to(device).unsqueeze(2))
+
+    def call():
+        return ib.kernels.decode_attention(*args, window=window, log_scaling_n_floor=40, **new)
+
     for _ in range(2):   # the second call finds the arrival counters as the first left them
-        got = ib.kernels.decode_attention(q.to(device), r.to(device), proj.to(device), *before, torch.tensor(position, device=device),
-                                          pad.to(device), window=window, log_scaling_n_floor=40, new_key=new_k.to(device).unsqueeze(2),
-                                          new_value=new_v.to(device).unsqueeze(2))
+        got = call()
     torch.cuda.synchronize()
     assert (got[:, :, 0].float().cpu() - want).abs().max() <= TOL * want.abs().max()
     assert torch.equal(before[0].cpu(), k) and torch.equal(before[1].cpu(), v)
+    return call
+
+
+def _launched(call, tmp_path):
+    """Name and grid of the attention kernel that a call launches."""
+    import json
+
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        call()
+        torch.cuda.synchronize()
+    profile.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    (kernel,) = [e for e in events if e.get("cat") == "kernel" and "decode_attention" in e["name"]]
+    return kernel["name"], kernel["args"]["grid"]
+
+
+@pytest.mark.parametrize("parts,bs,c,h,hk,slots,window,position,d_rel", [
+    (1, 40, 64, 16, 16, 41, 0, 40, 16),          # one part: a step and a piece of one
+    (1, 40, 128, 72, 8, 100, 100, 1234, 20),     # nine heads on one key/value head; a ring that has wrapped, of a length between steps
+    (1, 40, 256, 16, 16, 100, 0, 99, 7),         # 256 channels (half of a value row at a time); relative states shorter than a step
+    ("cluster", 9, 64, 32, 16, 777, 0, 700, 20),
+    ("cluster", 8, 128, 36, 4, 1000, 1000, 600, 7),       # a ring that is not full yet
+    ("cluster", 8, 128, 64, 16, 512, 512, 5000, 16),      # the model's sliding layers at eight sequences
+    ("cluster", 7, 256, 16, 16, 600, 0, 599, 16),
+    ("memory", 3, 64, 64, 8, 3001, 0, 2990, 16),
+    ("memory", 3, 128, 72, 8, 3000, 3000, 10007, 20),
+    ("memory", 2, 128, 27, 3, 5003, 0, 3000, 7),          # a cache that is in use for three fifths
+    ("memory", 3, 256, 8, 8, 2555, 0, 2554, 20),
+])
+def test_the_form_with_matrix_instructions_at_the_edges_of_its_parts(ib, tmp_path, parts, bs, c, h, hk, slots, window, position, d_rel):
+    """Steps of 16 slots, groups of eight heads, parts along the cache: remainders of each, for every way in which parts are
+    joined; that a case runs the kernel it is meant for is read off its launch."""
+    call = _against_the_oracle(ib, bs, c, h, hk, slots, window, position, d_rel)
+    name, grid = _launched(call, tmp_path)
+    assert f"decode_attention_kernel<{c}, {'true' if parts == 'cluster' else 'false'}>" in name
+    assert grid[0] == 1 if parts == 1 else 2 <= grid[0] <= 8 if parts == "cluster" else grid[0] > 8
 
 
 def _many_part_inputs(device, bs=1, slots=1100, seed=3, misaligned=False):
