@@ -255,7 +255,7 @@ int ink_expert_reduce(const void* down, const int64_t* indices, const void* weig
  *             the first bank the descriptors cover (experts[g] - start indexes them)
  *  pointers   as for ink_expert_gemm: the FP32 scale2 is read through it, a zero row skips the expert
  *  scratch    ink_expert_gemm_tc_scratch_bytes(input_rows, k) bytes (of up to eight choices a row; more choices: as if
- *             for proportionally more rows): a kernel in front writes the N operand there
+ *             for proportionally more rows), whatever `capacity`: a kernel in front writes the N operand there
  * Constraints: n a multiple of 128, k a multiple of 256 up to 4096, groups <= 1024. */
 size_t ink_expert_gemm_tc_scratch_bytes(int input_rows, int k);
 int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, const int64_t* pointers,
@@ -265,7 +265,8 @@ int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, con
 
 /* The whole layer after the routing for several tokens, on the same kernels (my_inkling/offloaded_experts.py:249-310 and
  * my_inkling/model.py:192-226): both routed projections and the weighted sum, and -- with n_shared > 0 -- the shared
- * experts as further tiles of the same launches. Each active expert's bytes cross HBM once.
+ * experts as further tiles of the same launches. Each active expert's bytes cross HBM once per tile of its tokens (16 to 64).
+ * A token with a NaN or an infinity comes out as NaN (quantized = 1: all of it).
  *  indices, weights, experts, rows, counts, pointers   as for ink_expert_gemm / ink_expert_reduce, of ink_expert_plan
  *  quantized   1: NVFP4 banks, bank_maps of ink_moe_stack_encode_banks (512 bytes); 0: BF16 banks (pointer stride 2),
  *              bank_maps of ink_encode_bf16_banks (256 bytes); device copies, 128-byte aligned
@@ -275,7 +276,8 @@ int ink_expert_gemm_tc(const void* x, int input_rows, const void* bank_maps, con
  *  output      FP32 [tokens, hidden], fully overwritten, or NULL; output_bf16 the same rounded to BF16, or NULL
  *  groups      entries of experts / counts to visit; start, local: first expert and number of experts of this rank
  *  status      bit 0: a route named an expert outside [0, max_expert] (it is skipped); bit 1: a bounded wait gave up
- * Constraints: hidden and intermediate up to 4096, multiples of 256 (BF16 banks: of 64, hidden of 128); groups <= 1024. */
+ * Constraints: hidden and intermediate up to 4096, multiples of 256 (BF16 banks: of 64, hidden of 128); groups <= 1024; 16
+ * million routes at the greatest widths. */
 int ink_encode_bf16_banks(void* out_host_256, const void* gate_up, uint64_t gate_up_stride, const void* down,
                           uint64_t down_stride, int experts, int hidden, int intermediate);
 int ink_encode_shared(void* out_host_384, const void* gate, const void* up, const void* down, int n_shared, int hidden,

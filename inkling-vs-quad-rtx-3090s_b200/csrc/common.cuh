@@ -43,9 +43,10 @@ enum DeviceFlag : int {
     }                                                                       \
   } while (0)
 
-// Every kernel of the library asks for the largest shared-memory carve-out, so that the
-// SMs are not re-partitioned between L1 and shared memory from one launch to the next
-// (the streaming kernels need almost all of it).
+// The kernels that run between the streaming kernels (which need almost all of it) ask for the
+// largest shared-memory carve-out too, so that the SMs are not re-partitioned between L1 and shared
+// memory from one launch to the next. (The router, the plan, attention and the kernels around the
+// grouped one read through L1 and leave it to the runtime.)
 #define INK_PREFER_MAX_SMEM(kernel)                                                             \
   do {                                                                                          \
     static bool done_ = false;                                                                  \

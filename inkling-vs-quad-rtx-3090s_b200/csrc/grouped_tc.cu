@@ -12,9 +12,9 @@
 //
 // A ring stage is a chunk of the contraction (128 bytes of every row) of a tile of 128 weight rows and the N operand that goes
 // with it: 8 stages of 27 KB, 6 of 36 KB or 4 of 54 KB. Whatever T, a weight tile meets one tile of tokens after the other in
-// one block, so its next reads follow within some 300 KB of the block's stream (44 MB over the chip: they hit L2; with tiles of
-// 256 weight rows, tried before, they came from HBM again). A larger T saves these reads, a smaller one leaves more of
-// the ring to the weights: see gg_tokens.
+// one block, so its next reads follow within some 300 KB of the block's stream (44 MB over the chip). Not all of them hit L2:
+// gate/up of 1 999 tokens at full width reads 5.1 GB from DRAM where the banks are 2.5 GB (36 % of its sectors hit). A larger T saves these reads, a smaller one leaves more of the ring
+// to the weights: see gg_tokens.
 //
 // Persistent blocks, one per SM. The shared experts' items (long) are dealt evenly, the routed items by cost in what is
 // left of each block's share. Two warps produce, a stage each in turn (a stage's copies
@@ -166,8 +166,11 @@ struct GgWalk {
   __device__ __forceinline__ int stages_of(bool shared) const {
     return a->k / ((FP4 && !shared) ? kTcChunkK : 64);
   }
-  // cost of one item with n tokens, per ring stage (they have equally many): its bytes, the streamed weights weighing most.
-  // At most gg_most_cost, and all of them together fit an int (gg_costs_fit).
+  // cost of one item with n tokens, per ring stage (they have equally many): its weights' bytes, and its tokens' as they weigh
+  // beside them. The weights 2 n, n / 4 and n are a fit to 256 experts of 4096 x 2048. Against the bytes alone (2 n at every T),
+  // us a call: there 735 for 767 (400 tokens of eight choices), 1 010 for 1 070 (1 024 of six); 4096 x 512, 500 tokens: 360 for
+  // 343; 128 experts of 2048 x 1024, 1 500 tokens: 396 for 388; few tokens and whole blocks within 1.5 % either way.
+  // At most gg_most_cost, and all of them together fit an int (check_costs_fit).
   __device__ static __forceinline__ int tile_cost(int n) { return 64 + (T == 16 ? 2 * n : T == 32 ? n / 4 : n) / (FP4 ? 1 : 4); }
   __device__ __forceinline__ int cost_per_mt(int c) const {
     return c / kTile * tile_cost(kTile) + (c % kTile ? tile_cost(c % kTile) : 0);
@@ -900,9 +903,13 @@ static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStre
   return kOk;
 }
 
-// Tokens T of a tile, from the mean number of routes per expert. Routed experts of one layer at full width (256 of 4096 x 2048),
-// evenly / unevenly chosen (rank^-0.6), T = 16, 32, 64, us a call:  mean 4: 606 610 655 / 596 598 643;  8: 668 647 707 / 680 653
-// 721;  24: 1114 823 868 / 1145 924 948;  36: 1516 1245 1102 / 1526 1175 1194;  48: 1948 1620 1405 / 2119 1511 1502.
+// Tokens T of a tile, from the mean number of routes per expert. T = 16, 32, 64, us a call, experts evenly / unevenly chosen
+// (rank^-0.6):
+//   256 of 4096 x 2048   mean 8: 676 701 761 / 759 710 770;  24: 1226 905 977 / 1277 1030 1060;  36: 1736 1407 1215 / 1738 1333 1323
+//   256 of 4096 x 512         8: 239 252 260 / 249 299 316;  24:  438 392 408 /  451  450  484;  36:  610  587  534 /  630  585  611
+//   128 of 2048 x 1024        8: 124 121 131 / 128 136 157;  24:  203 167 175 /  203  188  213;  36:  267  236  221 /  271  235  254
+//    64 of 1024 x 512         8:  50  52  52 /  51  58  64;  24:   69  70  71 /   70   74   81;  36:   84   87   88 /   86   87   90
+// so at a mean of 8 the smallest is right on the whole, and for the smallest layers it stays so (up to 10 % at mean 16).
 static int gg_tokens(long long routes, int experts) { return routes > 24LL * experts ? 64 : routes > 8LL * experts ? 32 : 16; }
 
 }  // namespace ink

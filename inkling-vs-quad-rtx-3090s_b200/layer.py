@@ -4,13 +4,18 @@ stands.
 * `ResidentExperts`  -- same constructor shape, tables and `forward(hidden, top_k_index,
   top_k_weights)` as the reference's OffloadedExperts (my_inkling/offloaded_experts.py:
   25-314), with every expert resident in HBM: no cache slots, no LRU, no copy kernel.
-* `FusedMoE`         -- the whole of MyInklingMoE.forward (my_inkling/model.py:361-374)
-  in two or three launches plus one all-reduce: router+plan, gate/up, down+combine.
+* `FusedMoE`         -- the whole of MyInklingMoE.forward (my_inkling/model.py:361-374): one token in
+  one launch, several in the router, the plan and five launches around the grouped kernel (or, with banks
+  that are not evenly spaced, router+plan, gate/up, down+combine), plus one all-reduce.
 * `apply_resident_plan` / `apply_fused_moe_plan` install them into a model the way
   apply_offload_plan does (my_inkling/offloaded_experts.py:317-340).
 
-Everything here is capture-safe: buffers are allocated in __init__ or on first use for
-a given token count, and a forward issues a fixed sequence of launches.
+Everything here is capture-safe: a module's buffers are made on first use for a given
+token count and kept, a call's scratch comes from the caching allocator (under capture,
+from the graph's pool), and a forward issues a fixed sequence of launches. One token and
+several run different arithmetic (FP16 products on the CUDA cores; E2M1 digits on the
+tensor cores), so a token's result may differ in its last bits with its company; its
+routing does not.
 """
 from __future__ import annotations
 
@@ -78,7 +83,7 @@ class ResidentExperts(KeepsForGraphs, nn.Module):
     banks are the unquantised layer's {gate_up_proj BF16 [2f, d] (rows interleave gate and
     up), down_proj BF16 [d, f]} and the pointer table has stride 2
     (kernels/grouped_experts.py:9-22); that layer runs one matrix-vector product per route
-    at every token count.
+    for one token, and at every token count where the banks are not evenly spaced in memory.
     """
 
     def __init__(self, hidden_dim: int, intermediate_dim: int, device_mesh, weights: dict, quantized: bool = True,
