@@ -517,9 +517,14 @@ def batched_numbers(ib, layers, steps: int, token_counts=(64,)) -> dict:
             ex._plan(idx)
             ex._project_grouped(x, idx, w, final)
 
-        def gemv(layer):
+        def gemv(layer):   # eight tokens at a time, as the reference's switch has it
+            ex = layer.experts
+            final = torch.zeros(tokens, HIDDEN, dtype=torch.float32, device=device)
+            ex._reserve(idx.numel())
             for i in range(0, tokens, 8):
-                layer.experts(x[i:i + 8], idx[i:i + 8], w[i:i + 8])
+                part = slice(i, i + 8)
+                ex._plan(idx[part])
+                ib.kernels.routed_decode(x[part], idx[part], w[part], ex.pointers, ex.activated, final[part], ex.max_expert, True, status=ex.status)
 
         grouped_ms, gemv_ms = timed(grouped), timed(gemv)
         out[str(tokens)] = {
