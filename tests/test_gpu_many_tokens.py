@@ -439,3 +439,11 @@ def test_a_router_call_of_more_tokens_than_a_grid_is_high(ib, device):
 
     whole, last = route(x), route(x[-40:].contiguous())
     assert all(torch.equal(a[-40:], b) for a, b in zip(whole, last))
+
+
+def test_a_token_comes_out_the_same_in_any_larger_company(ib, device):
+    """From two tokens on, tiles of 16, 32 and 64 tokens: a token is a column of its own, its sums run in the same order."""
+    layer, x = _block(ib, device, 300, d=512, f=256, experts=8)
+    whole = layer(x)
+    for tokens in (2, 9, 17, 40, 70, 131):   # means of 0.75 to 49 routes an expert (whole: 113)
+        assert torch.equal(layer(x[:tokens].contiguous()), whole[:tokens]), tokens
