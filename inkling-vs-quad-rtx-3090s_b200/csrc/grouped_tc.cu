@@ -754,15 +754,16 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) 
       for (int w = 0; w < kStageThreads / 32; ++w) amax = max(amax, s_amax[w]);
       float inverse;
       const float scale = pow2_normaliser(amax, &inverse);
+      const float below = amax >= 0x7f00u ? 256.f : 512.f;   // brings the largest below 1024 (2^127 and more: normalised to [2, 4))
       // (digits cannot hold a NaN or an infinity: the token's scale carries it into all of its results)
-      if (threadIdx.x == 0) a.slot_scale[slot0 + row] = amax >= 0x7f80u ? __int_as_float(0x7fffffff) : inverse * (1.f / 512.f);
+      if (threadIdx.x == 0) a.slot_scale[slot0 + row] = amax >= 0x7f80u ? __int_as_float(0x7fffffff) : inverse / below;
       unsigned char* image = a.image + (size_t)slot0 * a.k * 2 + (size_t)row * 512;
       unsigned char* scales = a.image_scales + (size_t)slot0 * (a.k / 4) + (size_t)row * 64;
 #pragma unroll
       for (int n = 0; n < kMost; ++n) {
         const int p = n * kStageThreads + threadIdx.x, chunk = p >> 5;   // a warp holds a chunk of 256 elements
         if (chunk * kTcChunkK < a.k)
-          tc_stage8_row(v[n], 512.f * scale, image + (size_t)chunk * padded * 512, 4 * (row & 1), scales + (size_t)chunk * padded * 64, lane);
+          tc_stage8_row(v[n], below * scale, image + (size_t)chunk * padded * 512, 4 * (row & 1), scales + (size_t)chunk * padded * 64, lane);
       }
     }
   }

@@ -216,3 +216,26 @@ def test_block_scaled_projection_with_the_smallest_capacity(ib, device):
         outs.append((activated, down))
     module.check_status()
     assert all(torch.equal(a, b) and bool(a.any(1).all()) for a, b in zip(*outs))
+
+
+def test_the_largest_finite_inputs_of_a_block_scaled_projection(ib, device):
+    """Down projection of rows whose largest element is in BF16's last binade: as the kernel that expands to FP16 has it."""
+    d, f, E, tokens = 256, 256, 4, 9
+    banks = ib.make_expert_banks(E, d, f, device, seed=3)
+    module = ib.ResidentExperts(d, f, None, banks.weights)
+    gen = torch.Generator().manual_seed(1)
+    x = torch.randn(tokens, f, generator=gen) * 0.1
+    x[:, 7] = torch.linspace(0.9, 1.99, tokens) * 2.0 ** 127
+    x = x.to(BF16).to(device)
+    idx = (torch.arange(tokens, device=device) % E).view(-1, 1)
+    i32 = dict(dtype=torch.int32, device=device)
+    pointers = torch.zeros(E * 6, dtype=torch.int64, device=device)
+    experts, counts, rows = torch.empty(E, **i32), torch.empty(E, **i32), torch.full((E, tokens), -1, **i32)
+    ib.kernels.expert_plan[(1,)](idx, module.sources, None, None, None, None, None, torch.empty(0, **i32), pointers, experts, counts, rows,
+                                 0, E, 0, 6, tokens, tokens)
+    outs = []
+    for maps in (module.bank_maps, None):
+        outs.append(torch.zeros(tokens, d, dtype=BF16, device=device))
+        ib.kernels.expert_gemm[(1, 1, E)](x, pointers, experts, rows, counts, outs[-1], tokens, d, f, 1, 1, True, 6, 16, 64, 64, bank_maps=maps)
+    assert torch.isfinite(x).all() and torch.isfinite(outs[1]).all()
+    assert all(max_rel(a, b) <= 1.6e-2 for a, b in zip(*outs))
