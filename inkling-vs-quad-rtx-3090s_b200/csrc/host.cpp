@@ -199,6 +199,7 @@ T* at_field(const Block& b, Field f) {
 // The launches of a call hand buffers of the module from one to the next, so they go to their stream as one sequence although
 // the interpreter is free meanwhile: one lock per pointer table, i.e. for a module of experts and every block that uses it.
 std::shared_ptr<std::mutex> launch_lock(long long pointers) {
+  if (!pointers) return std::make_shared<std::mutex>();   // (a record for one token: a single launch)
   static std::mutex mutex;
   static auto* locks = new std::map<long long, std::weak_ptr<std::mutex>>();
   const std::lock_guard<std::mutex> lock(mutex);
