@@ -59,6 +59,9 @@ class KeepsForGraphs:
     _captured = False   # the present buffers are in a captured graph
     _kept = ()
 
+    def __getstate__(self):   # (no graph has the addresses of a copy's buffers)
+        return {k: v for k, v in self.__dict__.items() if k not in ("_captured", "_kept")}
+
     def _note_capture(self) -> None:
         if torch.cuda.is_current_stream_capturing():
             self.__dict__["_captured"] = True
@@ -147,7 +150,7 @@ class ResidentExperts(KeepsForGraphs, nn.Module):
         super().__setattr__(name, value)
 
     def __getstate__(self):   # copies and pickles make their own record
-        return {k: v for k, v in self.__dict__.items() if k not in ("_native", "_captured", "_kept")}
+        return {k: v for k, v in super().__getstate__().items() if k != "_native"}
 
     def record_fields(self) -> dict:
         return dict(hidden=self.hidden_dim, width=self.intermediate_dim, start=self.start, local=self.local, stride=self.stride,
@@ -302,7 +305,7 @@ class FusedMoE(KeepsForGraphs, nn.Module):
         super().__setattr__(name, value)
 
     def __getstate__(self):   # copies and pickles make their own record and table
-        return dict({k: v for k, v in self.__dict__.items() if k not in ("_native", "_captured", "_kept")}, _fused=None)
+        return dict({k: v for k, v in super().__getstate__().items() if k != "_native"}, _fused=None)
 
     def _shared_as_expected(self) -> bool:
         d, f, n = self.experts.hidden_dim, self.experts.intermediate_dim, self.n_shared

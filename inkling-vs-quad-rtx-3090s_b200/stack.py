@@ -25,6 +25,9 @@ class MoEStack(KeepsForGraphs, nn.Module):
         # one launch for the whole stack, on one GPU or across tensor-parallel ranks
         self.one_launch = all(layer.one_launch_supported() for layer in layers)
 
+    def __getstate__(self):   # copies make their own table (it holds addresses)
+        return dict(super().__getstate__(), _fused=None)
+
     @classmethod
     def synthetic(cls, n_layers: int, hidden: int, intermediate: int, experts: int, n_shared: int, top_k: int,
                   device, seed: int = 0, device_mesh=None, rank: int = 0, world: int = 1,

@@ -447,3 +447,22 @@ def test_a_token_comes_out_the_same_in_any_larger_company(ib, device):
     whole = layer(x)
     for tokens in (2, 9, 17, 40, 70, 131):   # means of 0.75 to 49 routes an expert (whole: 113)
         assert torch.equal(layer(x[:tokens].contiguous()), whole[:tokens]), tokens
+
+
+def test_a_copy_of_a_stack_is_its_own(ib, device):
+    """The copy's launch reads the copy's tensors, and takes nothing over that was kept for the original's graphs."""
+    import copy
+
+    stack = ib.MoEStack([_block(ib, device, 1, seed=s, d=1024, f=512, experts=8)[0] for s in (6, 7)], 1024)
+    x = _block(ib, device, 1, d=1024, f=512, experts=8)[1]
+    decode = ib.DecodeStackGraph(stack, x)
+    stack.layers[0](x.repeat(40, 1))   # (replaces buffers that the graph has)
+    want = stack(x).clone()
+    twin = copy.deepcopy(stack)
+    assert not twin._kept and not twin.layers[0]._kept and stack.layers[0]._kept
+    for block in stack.layers:
+        for t in (block.router_weight, block.shared_down, block.shared_gate):
+            t.zero_()
+    assert not torch.equal(stack(x), want)
+    assert torch.equal(twin(x), want)
+    del decode
