@@ -353,7 +353,7 @@ def test_out_of_memory_in_a_native_call_is_torchs_error(ib, device):
 
 
 def test_other_threads_run_while_a_call_waits_for_its_stream(ib, device):
-    """More launches than a stream's queue holds, behind 0.3 s of other work: the call that finds the queue full waits, but not
+    """More launches than a stream's queue holds, behind 0.5 s of other work: the call that finds the queue full waits, but not
     with the interpreter."""
     import threading
     import time
@@ -373,7 +373,7 @@ def test_other_threads_run_while_a_call_waits_for_its_stream(ib, device):
 
     thread = threading.Thread(target=ticks)
     thread.start()
-    torch.cuda._sleep(int(0.3 * 1.9e9))
+    torch.cuda._sleep(int(0.5 * 1.9e9))
     start = time.monotonic()
     for _ in range(600):
         layer(x)
@@ -381,8 +381,8 @@ def test_other_threads_run_while_a_call_waits_for_its_stream(ib, device):
     stop.set()
     thread.join()
     torch.cuda.synchronize()
-    assert waited > 0.15, "the queue took everything: the call never waited"
-    assert max(gaps) < 0.1
+    assert waited > 0.25, "the queue took everything: the call never waited"
+    assert max(gaps) < waited / 2   # (nearly all of it with the interpreter's lock held, a millisecond on an idle host)
 
 
 def test_calls_of_several_threads_do_not_mix(ib, device):
