@@ -201,6 +201,9 @@ class ResidentExperts(KeepsForGraphs, nn.Module):
         if tokens > (1 if self.bank_maps is not None else MATVEC_TOKENS) and self.grouped_supported():
             self._project_grouped(x, indices, weights, output)
             return
+        if tokens <= MATVEC_TOKENS:
+            routed_decode(x, indices, weights, self.pointers, self.activated, output, self.max_expert, self.quantized, status=self.status)
+            return
         for t0 in range(0, tokens, MATVEC_TOKENS):
             t1 = min(tokens, t0 + MATVEC_TOKENS)
             routed_decode(x[t0:t1], indices[t0:t1], weights[t0:t1], self.pointers,
@@ -248,10 +251,14 @@ class ResidentExperts(KeepsForGraphs, nn.Module):
         final = torch.zeros_like(hidden_states, dtype=torch.float32)
         self._reserve(top_k_index.numel())
         x, index, weights = hidden_states.contiguous(), top_k_index.contiguous(), top_k_weights.contiguous()
-        for t0 in range(0, max(1, x.shape[0]), GROUPED_TOKENS):
-            part = slice(t0, t0 + GROUPED_TOKENS)
-            self._plan(index[part])
-            self._project(x[part], index[part], weights[part], final[part])
+        if x.shape[0] <= GROUPED_TOKENS:   # (a decode call is bound by the host: views of all of it would cost a fifth)
+            self._plan(index)
+            self._project(x, index, weights, final)
+        else:
+            for t0 in range(0, x.shape[0], GROUPED_TOKENS):
+                part = slice(t0, t0 + GROUPED_TOKENS)
+                self._plan(index[part])
+                self._project(x[part], index[part], weights[part], final[part])
         final = all_reduce(final, _group_of(self.device_mesh))
         return final.to(hidden_states.dtype)
 

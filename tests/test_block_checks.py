@@ -121,3 +121,26 @@ def test_what_attention_refuses_and_with_which_error(error, change):
     with pytest.raises(error) as caught:
         ib.kernels.decode_attention(**args)
     assert caught.type is error
+
+
+@pytest.mark.parametrize("tokens,pieces", [(1, [1]), (8, [8]), (20, [8, 8, 4])])
+def test_a_decode_call_of_the_experts_makes_no_views(monkeypatch, tokens, pieces):
+    """Banks that are not evenly spaced, recorded launches: a call that fits one launch hands its own tensors over (each view
+    is a microsecond of a host-bound call), a larger one pieces of eight tokens in order."""
+    import inkling_b200 as ib
+
+    layer = __import__("sys").modules[ib.ResidentExperts.__module__]
+    experts = ib.ResidentExperts.__new__(ib.ResidentExperts)
+    nn.Module.__init__(experts)
+    experts.local, experts.device, experts.dtype, experts.hidden_dim, experts.intermediate_dim, experts.capacity = 3, "cpu", torch.bfloat16, 32, 32, 0
+    experts.rows = experts.activated = experts.down = experts.bank_maps = experts.device_mesh = None
+    experts.quantized, experts.pointers, experts.max_expert, experts.status = True, None, 2, None
+    planned, launched = [], []
+    monkeypatch.setattr(ib.ResidentExperts, "_plan", lambda self, indices: planned.append(indices))
+    monkeypatch.setattr(layer, "routed_decode", lambda x, i, w, p, a, out, *_, **__: (launched.append((x, i, w)), out.copy_(x.float() + 1)))
+    x, indices, weights = torch.randn(tokens, 32).to(torch.bfloat16), torch.zeros(tokens, 2, dtype=torch.int64), torch.ones(tokens, 2, dtype=torch.bfloat16)
+    got = experts(x, indices, weights)
+    assert torch.equal(got, (x.float() + 1).to(torch.bfloat16)) and planned[0] is indices and len(planned) == 1
+    assert [len(t[0]) for t in launched] == pieces
+    if len(pieces) == 1:
+        assert launched[0][0] is x and launched[0][1] is indices and launched[0][2] is weights
