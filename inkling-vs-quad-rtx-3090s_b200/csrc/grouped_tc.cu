@@ -11,13 +11,11 @@
 // expert's bank was read once per eight of its tokens: 64 tokens of one block 0.42 ms, 1 024 tokens 2.8 ms.)
 //
 // A ring stage is a chunk of the contraction (128 bytes of every row) of a tile of 128 weight rows and the N operand that goes
-// with it: 8 stages of 27 KB, 6 of 36 KB or 4 of 54 KB. Whatever T, a weight tile meets one tile of tokens after the other in
-// one block, so its next reads follow within some 300 KB of the block's stream (44 MB over the chip). Not all of them hit L2:
-// gate/up of 1 999 tokens at full width reads 5.1 GB from DRAM where the banks are 2.5 GB (36 % of its sectors hit). A larger T saves these reads, a smaller one leaves more of the ring
-// to the weights: see gg_tokens.
+// with it: 8 stages of 27 KB, 6 of 36 KB or 4 of 54 KB. Prompts are bound by what crosses from L2 to the SMs: an image of 64 tokens is
+// twice its weight tile's bytes, 8 GB in all for gate/up of 1 999 tokens at full width, 734 us = 10.9 TB/s (bulk copies alone reach 13.9).
+// A larger T moves the weights less often, a smaller one leaves more of the ring to them: see gg_tokens.
 //
-// Persistent blocks, one per SM. The shared experts' items (long) are dealt evenly, the routed items by cost in what is
-// left of each block's share. Two warps produce, a stage each in turn (a stage's copies
+// Persistent blocks, one per SM, that take the items from a counter (GgDeal). One warp deals, two produce, a stage each in turn (a stage's copies
 // take the issuing lane 300 clocks), one thread issues the MMAs, four warps move block scales to tensor memory, four read accumulators and write outputs. The kernel is launched
 // while its predecessor runs (programmatic dependent launch): until that is done it only streams weights, whose
 // addresses depend on nothing but the plan. Every wait is bounded; one that gives up sets kFlagWaitTimedOut.
@@ -38,8 +36,11 @@ struct GgStage {
   static constexpr int kRowScalesAt = kRowsAt + T * 512, kBytes = (kRowScalesAt + T * 64 + 1023) / 1024 * 1024;
   static constexpr int kSf = T == 64 ? 48 : 32;   // tensor-memory columns of its scales
 };
-constexpr int kGgProducers = 2;   // (eleven warps: three on a scheduler, 168 registers a thread)
-constexpr int kGgThreads = 320 + (kGgProducers - 1) * 32;
+constexpr int kGgProducers = 2;
+constexpr int kGgDealer = 10 + kGgProducers - 1;                  // the warp that deals the items out
+constexpr int kGgThreads = (kGgDealer + 1) * 32;                 // (twelve warps: three on a scheduler, 168 registers a thread)
+constexpr int kGgQueue = 8;                                      // items a block knows at once
+constexpr int kGgDealStages = 16;                                // ring stages worth one step of the counter
 constexpr int kGgMaxGroups = 1024;
 constexpr int kGgPairRows = 16;                                  // shared experts: rows of gate and of up in turn
 constexpr int kGgColD = 0, kGgColSf = 256;                       // tensor memory: two accumulators, then each stage's scales
@@ -47,8 +48,6 @@ constexpr int kGgAccCols = 128;                                  // of one: 32 t
 
 // tokens in a tile
 __host__ __device__ constexpr int gg_tile(bool fp4, int t) { return fp4 ? t : 4 * t; }
-// no tile costs more (GgWalk::tile_cost)
-constexpr int gg_most_cost = 128;
 // slots of a group are padded to whole 1024-byte swizzle atoms of its tiles
 __host__ __device__ constexpr int gg_pad(bool fp4) { return fp4 ? 2 : 8; }
 
@@ -70,13 +69,26 @@ struct GgArgs {
   uint16_t* shared_y;           // gate/up: the image of the down projection; down: BF16 [tokens][n_shared][n]
   const uint16_t* gammas;       // [tokens, n_shared]
   int n_shared, tokens;
+  unsigned* next;               // deals taken beyond the blocks' first ones; zero when this kernel's predecessor is done
   int32_t* status;
+};
+
+// One work item: a 128-row tile of one expert's matrix against one tile of its tokens.
+struct GgItem {
+  int shared;     // 1: of a shared expert; -1: no more items
+  int group;      // group of routes, or shared expert
+  int m0;         // first weight row
+  int tile, n;    // tile of tokens, and how many
+  int slot;       // first slot of the tile (routed)
 };
 
 struct GgShared {
   uint64_t full[8], empty[8], sf_full[8];
   uint64_t d_full[2], d_empty[2];
+  uint64_t item_full[kGgQueue], item_empty[kGgQueue];
+  GgItem items[kGgQueue];
   uint32_t tmem_base;
+  volatile int taken;           // items the first producer has taken
   volatile int failed;
 };
 
@@ -114,123 +126,100 @@ __device__ __forceinline__ int warp_before(int mine, int lane, int* total) {
   return up_to - mine;
 }
 
-// The groups' tables in shared memory: slot0[g] = first slot | padding slots of the group, cost[g] = cost of all groups
-// before. `slot0[g]` holds the group's count on entry.
-struct GgTables { int* slot0; int* cost; };
-template <typename CostOf>
-__device__ __forceinline__ void gg_scan(const GgTables& t, int groups, int pad, int lane, CostOf cost_of) {
-  int slots = 0, cost = 0;
+// The groups' tables in shared memory: slot0[g] = first slot | padding slots of the group, before[g] = tiles (or routes) of
+// all groups before. `slot0[g]` holds the group's count on entry.
+struct GgTables { int* slot0; int* before; };
+template <typename Of>
+__device__ __forceinline__ void gg_scan(const GgTables& t, int groups, int pad, int lane, Of of) {
+  int slots = 0, sum = 0;
   for (int g0 = 0; g0 < groups; g0 += 32) {
     const int g = g0 + lane, count = g < groups ? t.slot0[g] : 0;
-    const int padded = (count + pad - 1) / pad * pad, c = cost_of(count);
-    int all_slots, all_cost;
-    const int s = slots + warp_before(padded, lane, &all_slots), w = cost + warp_before(c, lane, &all_cost);
+    const int padded = (count + pad - 1) / pad * pad, c = of(count);
+    int all_slots, all;
+    const int s = slots + warp_before(padded, lane, &all_slots), w = sum + warp_before(c, lane, &all);
     if (g < groups) {
       t.slot0[g] = s | (padded - count);
-      t.cost[g] = w;
+      t.before[g] = w;
     }
     slots += all_slots;
-    cost += all_cost;
+    sum += all;
   }
   if (lane == 0) {
     t.slot0[groups] = slots;
-    t.cost[groups] = cost;
+    t.before[groups] = sum;
   }
+}
+// the group that holds number i of what `before` counts
+__device__ __forceinline__ int gg_group_of(const int* before, int groups, int i) {
+  int lo = 0, hi = groups;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (before[mid] <= i) lo = mid;
+    else hi = mid;
+  }
+  return lo;
 }
 __device__ __forceinline__ int gg_first_slot(const int* slot0, int g, int pad) { return slot0[g] & ~(pad - 1); }
 __device__ __forceinline__ int gg_group_count(const int* slot0, int g, int pad) {
   return gg_first_slot(slot0, g + 1, pad) - gg_first_slot(slot0, g, pad) - (slot0[g] & (pad - 1));
 }
 
-// One work item: a 128-row tile of one expert's matrix against one tile of its tokens.
-struct GgItem {
-  bool shared;
-  int group;      // group of routes, or shared expert
-  int m0;         // first weight row
-  int tile, n;    // tile of tokens, and how many
-  int slot;       // first slot of the tile (routed)
-  int bank;       // index of the expert's matrix (set by the producers)
-};
-
+// The items in the order in which they are dealt: the shared experts' (the longest) first, then expert by expert the routed
+// ones, all tiles of tokens of a tile of weight rows in a row. The blocks take them from one counter, a few ring stages'
+// worth at a time, so that what runs at one time over the chip are the tiles of about five experts: the second tile of tokens of a weight
+// tile finds the weights in L2, and so do the weight tiles of an expert the images of its tokens. (Dealt in contiguous shares
+// by cost, each block read the weights again 0.8 MB later in its own stream, 120 MB over the chip, and two thirds of those
+// reads went to DRAM: gate/up of 1 999 tokens at full width 985 us, now 734; down 490, now 410. No share is longer than another's:
+// 61 tokens, gate/up 176 us, now 166, down 102, now 90; four tokens of a whole block 112, now 107.)
 template <bool FP4, int T>
-struct GgWalk {
-  static constexpr int kM = kTcRows;
+struct GgDeal {
   static constexpr int kTile = gg_tile(FP4, T), kPad = gg_pad(FP4), kSharedTile = gg_tile(false, T);
   const GgArgs* a;
   GgTables t;
   int m_tiles, shared_tiles;
-  int shared_next, shared_end;   // shared items left
-  int group, mt, tile, limit;    // next routed item; it is this block's while its cost offset is below `limit`
-  int count;                     // routes of `group`
 
-  __device__ __forceinline__ int stages_of(bool shared) const {
-    return a->k / ((FP4 && !shared) ? kTcChunkK : 64);
+  __device__ __forceinline__ int stages_of(bool shared) const { return a->k / ((FP4 && !shared) ? kTcChunkK : 64); }
+  __device__ __forceinline__ int per_deal(bool shared) const { return max(1, kGgDealStages / stages_of(shared)); }
+  __device__ __forceinline__ int shared_items() const { return a->n_shared * m_tiles * shared_tiles; }
+  __device__ __forceinline__ int routed_items() const { return t.before[a->groups] * m_tiles; }
+  __device__ __forceinline__ GgItem shared_item(int i) const {
+    GgItem it;
+    const int per_e = m_tiles * shared_tiles;
+    it.shared = 1;
+    it.group = i / per_e;
+    it.m0 = i % per_e / shared_tiles * kTcRows;
+    it.tile = i % shared_tiles;
+    it.n = min(kSharedTile, a->tokens - it.tile * kSharedTile);
+    it.slot = 0;
+    return it;
   }
-  // cost of one item with n tokens, per ring stage (they have equally many): its weights' bytes, and its tokens' as they weigh
-  // beside them. The weights 2 n, n / 4 and n are a fit to 256 experts of 4096 x 2048. Against the bytes alone (2 n at every T),
-  // us a call: there 735 for 767 (400 tokens of eight choices), 1 010 for 1 070 (1 024 of six); 4096 x 512, 500 tokens: 360 for
-  // 343; 128 experts of 2048 x 1024, 1 500 tokens: 396 for 388; few tokens and whole blocks within 1.5 % either way.
-  // At most gg_most_cost, and all of them together fit an int (check_costs_fit).
-  __device__ static __forceinline__ int tile_cost(int n) { return 64 + (T == 16 ? 2 * n : T == 32 ? n / 4 : n) / (FP4 ? 1 : 4); }
-  __device__ __forceinline__ int cost_per_mt(int c) const {
-    return c / kTile * tile_cost(kTile) + (c % kTile ? tile_cost(c % kTile) : 0);
-  }
-  __device__ __forceinline__ void find(int from) {   // the first routed item whose cost offset is at least `from`
-    int lo = 0, hi = a->groups;
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (t.cost[mid] <= from) lo = mid;
-      else hi = mid;
-    }
-    group = lo;
-    mt = tile = 0;
-    count = a->groups > 0 ? gg_group_count(t.slot0, group, kPad) : 0;
-    const int cm = cost_per_mt(count);
-    if (cm > 0) {
-      const int off = from - t.cost[group], ct = tile_cost(kTile);
-      mt = off / cm;
-      tile = (off % cm + ct - 1) / ct;
-      if (tile * kTile >= count) {
-        tile = 0;
-        ++mt;
-      }
-    } else {
-      mt = m_tiles;
-    }
-    skip();
-  }
-  __device__ __forceinline__ void skip() {
-    while (group < a->groups && (mt >= m_tiles || count == 0)) {
-      ++group;
-      mt = 0;
-      count = group < a->groups ? gg_group_count(t.slot0, group, kPad) : 0;
-    }
-  }
-  __device__ __forceinline__ bool next(GgItem& it) {
-    if (shared_next < shared_end) {
-      const int s = shared_next++, per_e = (a->n + kM - 1) / kM * shared_tiles;
-      it.shared = true;
-      it.group = s / per_e;
-      it.m0 = s % per_e / shared_tiles * kM;
-      it.tile = s % shared_tiles;
-      it.n = min(kSharedTile, a->tokens - it.tile * kSharedTile);
-      it.slot = 0;
-      return true;
-    }
-    if (group >= a->groups) return false;
-    if (t.cost[group] + mt * cost_per_mt(count) + tile * tile_cost(kTile) >= limit) return false;
-    it.shared = false;
+  // routed item i; `group` is the group that holds it
+  __device__ __forceinline__ GgItem routed_item(int i, int group) const {
+    GgItem it;
+    const int tiles = t.before[group + 1] - t.before[group], at = i - t.before[group] * m_tiles;
+    const int first = gg_first_slot(t.slot0, group, kPad), count = gg_group_count(t.slot0, group, kPad);
+    it.shared = 0;
     it.group = group;
-    it.m0 = mt * kM;
-    it.tile = tile;
-    it.n = min(kTile, count - tile * kTile);
-    it.slot = gg_first_slot(t.slot0, group, kPad) + tile * kTile;
-    if (++tile * kTile >= count) {
-      tile = 0;
-      ++mt;
-      skip();
-    }
-    return true;
+    it.m0 = at / tiles * kTcRows;
+    it.tile = at % tiles;
+    it.n = min(kTile, count - it.tile * kTile);
+    it.slot = first + it.tile * kTile;
+    return it;
+  }
+};
+
+// A role's way through the block's items: waits for the next one and takes it (whole warps call it).
+struct GgTaker {
+  uint32_t n = 0;
+  __device__ __forceinline__ bool next(GgItem& it, GgShared* sh, int lane) {
+    const uint32_t at = n % kGgQueue;
+    const bool ok = __all_sync(0xffffffffu, gg_wait(&sh->item_full[at], n / kGgQueue & 1u, sh));
+    if (!ok) return false;
+    it = sh->items[at];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->item_empty[at]);
+    ++n;
+    return it.shared >= 0;
   }
 };
 
@@ -274,7 +263,7 @@ __device__ __forceinline__ bool elect_one() {
 
 template <bool FP4, int PROJ, int T>
 __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __grid_constant__ GgArgs a) {
-  using Walk = GgWalk<FP4, T>;
+  using Deal = GgDeal<FP4, T>;
   using St = GgStage<T>;
   // Two accumulators in turn: the next item's MMAs run while one is read. A tile of more than kGgAccCols columns (T = 64)
   // takes both. `acc` counts those a role has passed: number acc & 1, for the (acc >> 1)-th time.
@@ -285,12 +274,12 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
   unsigned char* ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // swizzled tiles: 1024-byte aligned
   GgTables tables;
   tables.slot0 = reinterpret_cast<int*>(ring + (size_t)St::kCount * St::kBytes);
-  tables.cost = tables.slot0 + a.groups + 1;
-  Walk walk;
-  walk.a = &a;
-  walk.t = tables;
-  walk.m_tiles = (a.n + Walk::kM - 1) / Walk::kM;
-  walk.shared_tiles = a.n_shared > 0 ? (a.tokens + Walk::kSharedTile - 1) / Walk::kSharedTile : 0;
+  tables.before = tables.slot0 + a.groups + 1;
+  Deal deal;
+  deal.a = &a;
+  deal.t = tables;
+  deal.m_tiles = (a.n + kTcRows - 1) / kTcRows;
+  deal.shared_tiles = a.n_shared > 0 ? (a.tokens + Deal::kSharedTile - 1) / Deal::kSharedTile : 0;
 
   for (int g = threadIdx.x; g < a.groups; g += kGgThreads) tables.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
   if (threadIdx.x == 0) {
@@ -303,45 +292,76 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       mbar_init(&sh.d_full[s], 1);
       mbar_init(&sh.d_empty[s], 4);
     }
+    for (int s = 0; s < kGgQueue; ++s) {
+      mbar_init(&sh.item_full[s], 1);
+      mbar_init(&sh.item_empty[s], kGgProducers + 1 + (FP4 ? 4 : 0) + 4);   // every warp that takes items
+    }
+    sh.taken = 0;
     sh.failed = 0;
     mbar_init_fence();
   }
   if (warp == 1) tc_alloc(&sh.tmem_base, 512);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) {
-    const int m_tiles = walk.m_tiles;
-    gg_scan(tables, a.groups, Walk::kPad, lane, [&](int count) { return m_tiles * walk.cost_per_mt(count); });
-  }
+  if (warp == 0) gg_scan(tables, a.groups, Deal::kPad, lane, [](int count) { return (count + Deal::kTile - 1) / Deal::kTile; });
   __syncthreads();
   tc_fence_after();
   pdl_trigger();
-  // ---- this block's share: its shared items, and the routed items in what remains of total / blocks
-  {
-    const int shared_items = a.n_shared * walk.m_tiles * walk.shared_tiles, G = gridDim.x, b = blockIdx.x;
-    const long long shared_cost = a.n_shared > 0 ? (long long)(walk.stages_of(true) / walk.stages_of(false)) * (64 + min(a.tokens, Walk::kSharedTile) / 4) : 0;
-    const long long routed = tables.cost[a.groups], total = routed + shared_cost * shared_items;
-    // routed cost taken by the blocks before block x (a block whose shared items exceed its share takes none)
-    auto before = [&](int x) -> long long { return total * x / G - shared_cost * ((long long)shared_items * x / G); };
-    long long from = 0, to = 0;
-    for (int x = lane; x <= b + 1; x += 32) {
-      const long long v = before(x) < 0 ? 0 : before(x);
-      if (x <= b && v > from) from = v;
-      if (v > to) to = v;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      from = max(from, __shfl_xor_sync(0xffffffffu, from, o));
-      to = max(to, __shfl_xor_sync(0xffffffffu, to, o));
-    }
-    walk.shared_next = (int)((long long)shared_items * b / G);
-    walk.shared_end = (int)((long long)shared_items * (b + 1) / G);
-    walk.limit = (int)(b + 1 == G ? routed : min(to, routed));
-    walk.find((int)min(from, routed));
-  }
   const uint32_t tmem = sh.tmem_base;
 
-  if (warp == 0 || warp >= 10) {
+  if (warp == kGgDealer) {
+    // =========================================================== the dealer
+    // One lane. The first deal is the block's own number; the others come from the counter, which the kernel in front has
+    // cleared, one deal ahead of the first producer: far enough to hide the counter's round trip (a deal lasts 2 us and
+    // more), and no further, so that no block is left with items that others could have taken.
+    if (lane == 0) {
+      const int shared = deal.shared_items(), routed = deal.routed_items();
+      const int per_s = deal.per_deal(true), per_r = deal.per_deal(false);
+      const int deals_s = (shared + per_s - 1) / per_s, deals = deals_s + (routed + per_r - 1) / per_r;
+      int dealt = 0;   // items dealt to this block
+      auto put = [&](const GgItem& it) -> bool {
+        const uint32_t at = (uint32_t)dealt % kGgQueue;
+        if (dealt >= kGgQueue && !gg_wait(&sh.item_empty[at], (uint32_t)(dealt / kGgQueue - 1) & 1u, &sh)) return false;
+        sh.items[at] = it;
+        mbar_arrive(&sh.item_full[at]);
+        ++dealt;
+        return true;
+      };
+      bool ok = true, waited = false;
+      for (int d = blockIdx.x; ok && d < deals;) {
+        const int before = dealt;
+        if (d < deals_s) {
+          for (int i = d * per_s; ok && i < min(shared, (d + 1) * per_s); ++i) ok = put(deal.shared_item(i));
+        } else {
+          const int first = (d - deals_s) * per_r;
+          int group = gg_group_of(tables.before, a.groups, first / deal.m_tiles);
+          for (int i = first; ok && i < min(routed, first + per_r); ++i) {
+            while (tables.before[group + 1] * deal.m_tiles <= i) ++group;
+            ok = put(deal.routed_item(i, group));
+          }
+        }
+        if (!waited) {
+          pdl_wait();
+          waited = true;
+        }
+        const long long t0 = clock64();
+        while (ok && sh.taken <= before) {   // this deal's first item has not been taken
+          if (sh.failed || clock64() - t0 > kWaitLimitCycles) {
+            sh.failed = 1;
+            ok = false;
+          }
+          __nanosleep(50);
+        }
+        d = (int)gridDim.x + (int)atomicAdd(a.next, 1u);
+      }
+      if (ok) {
+        GgItem end = {};
+        end.shared = -1;
+        put(end);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 0 || warp >= 10) {
     // =========================================================== producers
     const int producer = warp == 0 ? 0 : warp - 9;
     auto rows_bytes = [&](const GgItem& it) -> uint32_t {   // one chunk of the tile's N operand
@@ -354,16 +374,17 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       if (FP4 && !it.shared) bytes += kTcScaleBytes + rows_bytes(it) / 8u;
       mbar_expect_tx(&sh.full[u], bytes);
     };
+    int bank = 0;   // index of the item's matrix
     auto issue_weights = [&](const GgItem& it, int s, int u) {
       unsigned char* stage = ring + (size_t)u * St::kBytes;
       uint64_t* bar = &sh.full[u];
       if (PROJ == 0 && it.shared) {   // gate and up rows, sixteen in turn: {column, row, which, block of rows, expert}
-        tc_tma_5d(stage, a.shared_maps, s * 64, 0, 0, it.m0 / (2 * kGgPairRows), it.bank, bar);
+        tc_tma_5d(stage, a.shared_maps, s * 64, 0, 0, it.m0 / (2 * kGgPairRows), bank, bar);
       } else if (!FP4 || it.shared) {
-        tc_tma_3d(stage, it.shared ? a.shared_maps : a.maps, s * 64, it.m0, it.bank, bar);
+        tc_tma_3d(stage, it.shared ? a.shared_maps : a.maps, s * 64, it.m0, bank, bar);
       } else {
-        tc_tma_3d(stage, a.maps, s * 128, it.m0, it.bank, bar);
-        tc_tma_3d(stage + St::kScalesAt, a.maps + 128, s * 16, it.m0, it.bank, bar);
+        tc_tma_3d(stage, a.maps, s * 128, it.m0, bank, bar);
+        tc_tma_3d(stage + St::kScalesAt, a.maps + 128, s * 16, it.m0, bank, bar);
       }
     };
     auto issue_rows = [&](const GgItem& it, int s, int u) {
@@ -372,7 +393,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       const unsigned char* from;
       if (it.shared) {
         const int padded = (a.tokens + 7) / 8 * 8;
-        from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Walk::kSharedTile) * a.k * 2;
+        from = a.shared_image + ((size_t)(PROJ ? it.group : 0) * padded + (size_t)it.tile * Deal::kSharedTile) * a.k * 2;
       } else {
         from = a.image + (size_t)it.slot * a.k * 2;
       }
@@ -388,14 +409,27 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     GgItem it;
     long long first = 0;   // the block's stages before this item
     bool waited = false;
-    while (walk.next(it)) {
-      it.bank = it.shared ? it.group : a.experts[it.group] - a.start;
-      const int stages = walk.stages_of(it.shared);
+    auto rows_of_first_round = [&]() {
+      pdl_wait();
+      waited = true;
+#pragma unroll
+      for (int i = 0; i < kFirst; ++i)
+        if (i < early && elect_one()) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
+      __syncwarp();
+    };
+    GgTaker taker;
+    while (true) {
+      // (items beyond the queue's length arrive when others have taken theirs, which may wait for these rows)
+      if (!waited && taker.n == kGgQueue) rows_of_first_round();
+      if (!taker.next(it, &sh, lane)) break;
+      if (producer == 0 && lane == 0) sh.taken = (int)taker.n;
+      bank = it.shared ? it.group : a.experts[it.group] - a.start;
+      const int stages = deal.stages_of(it.shared);
       int s = (int)((producer - first % kGgProducers + kGgProducers) % kGgProducers);
       for (; s < stages; s += kGgProducers) {
         const long long seq = first + s;
         const int u = (int)(seq % St::kCount);
-        if (early < kFirst) {
+        if (!waited && early < kFirst) {
           if (elect_one()) {
             expect(it, u);
             issue_weights(it, s, u);
@@ -411,15 +445,8 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
           ++early;
           continue;
         }
-        if (!waited) {
-          pdl_wait();
-          waited = true;
-#pragma unroll
-          for (int i = 0; i < kFirst; ++i)
-            if (elect_one()) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
-          __syncwarp();
-        }
-        if (!__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / St::kCount) - 1) & 1u, &sh))) break;
+        if (!waited) rows_of_first_round();
+        if (seq >= St::kCount && !__all_sync(0xffffffffu, gg_wait(&sh.empty[u], (uint32_t)((seq / St::kCount) - 1) & 1u, &sh))) break;
         if (elect_one()) {
           expect(it, u);
           issue_weights(it, s, u);
@@ -430,13 +457,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       first += stages;
       if (sh.failed) break;
     }
-    if (!waited) {
-      pdl_wait();
-#pragma unroll
-      for (int i = 0; i < kFirst; ++i)
-        if (i < early && elect_one()) issue_rows(early_item[i], early_stage[i], producer + i * kGgProducers);
-      __syncwarp();
-    }
+    if (!waited) rows_of_first_round();
   } else if (warp == 1) {
     // =========================================================== MMA issue
     // The whole warp walks the stages together (operands of the issue instructions are per-warp registers), one lane issues.
@@ -444,13 +465,14 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     uint32_t seq = 0;
     const uint32_t ring_lo = gg_desc_lo(smem_u32(ring));
     bool ok = true;
-    for (uint32_t acc = 0; ok && walk.next(it);) {
+    GgTaker taker;
+    for (uint32_t acc = 0; ok && taker.next(it, &sh, lane);) {
       const bool fp4 = FP4 && !it.shared;
       const int accs = __shfl_sync(0xffffffffu, accs_of(it), 0), n = __shfl_sync(0xffffffffu, it.n, 0);
       const int per_acc = fp4 ? 32 : 128, n_last = n - (accs - 1) * per_acc;
       auto idesc_of = [&](int tokens) { return fp4 ? tc_idesc((tokens + 1) / 2 * 8) : gg_idesc_bf16((tokens + 15) / 16 * 16); };
       const uint32_t idesc_last = idesc_of(n_last), idesc_first = accs > 1 ? idesc_of(per_acc) : idesc_last;
-      const int stages = walk.stages_of(it.shared);
+      const int stages = deal.stages_of(it.shared);
       const uint32_t d_first = tmem + kGgColD + (acc & 1) * kGgAccCols, d_second = tmem + kGgColD + ((acc + 1) & 1) * kGgAccCols;
       for (int i = 0; ok && i < accs; ++i) ok = gg_wait(&sh.d_empty[(acc + i) & 1], ((acc + i) >> 1 & 1u) ^ 1u, &sh);   // their previous items have been read
       if (!ok) break;
@@ -487,8 +509,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
       GgItem it;
       long long seq = 0;
       bool ok = true;
-      while (ok && walk.next(it)) {
-        const int stages = walk.stages_of(it.shared);
+      GgTaker taker;
+      while (ok && taker.next(it, &sh, lane)) {
+        const int stages = deal.stages_of(it.shared);
         for (int s = 0; s < stages; ++s, ++seq) {
           const int u = (int)(seq % St::kCount);
           ok = __all_sync(0xffffffffu, gg_wait(&sh.full[u], (uint32_t)(seq / St::kCount) & 1u, &sh));
@@ -525,7 +548,8 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
     const uint32_t lane_base = (uint32_t)(sub * 32) << 16;
     GgItem it;
     bool ok = true;
-    for (uint32_t acc = 0; ok && walk.next(it);) {
+    GgTaker taker;
+    for (uint32_t acc = 0; ok && taker.next(it, &sh, lane);) {
       const bool fp4 = FP4 && !it.shared;
       const int expert = it.shared ? 0 : a.experts[it.group];
       const float scale2 = fp4 ? *reinterpret_cast<const float*>(a.pointers[(size_t)expert * a.stride + a.bank + 2]) : 1.f;
@@ -536,9 +560,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
         const int i = at + lane;
         scale = 0.f;
         if (lane >= per_chunk || i >= it.n) return -1;
-        if (it.shared) return it.tile * Walk::kSharedTile + i;
+        if (it.shared) return it.tile * Deal::kSharedTile + i;
         if (fp4) scale = scale2 * a.slot_scale[it.slot + i];
-        return a.rows[(size_t)it.group * a.capacity + it.tile * Walk::kTile + i];
+        return a.rows[(size_t)it.group * a.capacity + it.tile * Deal::kTile + i];
       };
       // this thread's weight row for the tokens at .. of a chunk (lane j holds token j's route, or number)
       auto write = [&](auto& v, int at, int tokens) {
@@ -620,7 +644,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
           // lane finishes one
           const bool second = (lane & 16) != 0, up_first = *reinterpret_cast<const int*>(a.shared_maps + 128) != 0;
           const int pair = it.m0 / 2 + sub * kGgPairRows + (lane & 15), padded = (a.tokens + 7) / 8 * 8, f = a.n / 2;
-          unsigned char* tile = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Walk::kSharedTile) * f * 2 +
+          unsigned char* tile = reinterpret_cast<unsigned char*>(a.shared_y) + ((size_t)it.group * padded + (size_t)it.tile * Deal::kSharedTile) * f * 2 +
                                 (size_t)(pair >> 6) * ((it.n + 7) / 8 * 8) * 128 + (pair & 7) * 2;
 #pragma unroll 1
           for (int chunk = 0; chunk < token_chunks; ++chunk) {
@@ -628,7 +652,7 @@ __global__ void __launch_bounds__(kGgThreads, 1) grouped_gemm_kernel(const __gri
             tc_ld32(d + chunk * 32, v);
             const int here = min(32, here_n - chunk * 32);
             const int at0 = first + chunk * 32, mine = min(at0 + lane, it.n - 1);   // (lane j's gamma is that of token j)
-            const float my_gamma = bf16_to_f32(a.gammas[(size_t)(it.tile * Walk::kSharedTile + mine) * a.n_shared + it.group]);
+            const float my_gamma = bf16_to_f32(a.gammas[(size_t)(it.tile * Deal::kSharedTile + mine) * a.n_shared + it.group]);
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
               if (j >= here) break;
@@ -680,6 +704,7 @@ struct StageArgs {
   unsigned char* shared_image;  // the tokens themselves for the shared experts, or null
   int groups, capacity, stride, bank, k, div;   // div: routes per row of x
   int plan_ready;               // the plan was complete before the kernel in front started
+  unsigned* next;               // the main kernel's counter of deals, cleared here
   int tokens, tile, shared_tile;
 };
 
@@ -705,11 +730,12 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) 
     pdl_wait();
     pdl_trigger();   // the main kernel may read the plan now
   }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.next = 0;   // (nothing in flight uses it: each projection of a call has its own)
   for (int g = threadIdx.x; g < a.groups; g += kStageThreads) t.slot0[g] = gg_count(a.counts, a.experts, a.pointers, a.stride, a.bank, g);
   __syncthreads();
   if (warp == 0) gg_scan(t, a.groups, kPad, lane, [](int count) { return count; });
   __syncthreads();
-  const int routed = t.cost[a.groups], total = routed + (a.shared_image ? a.tokens : 0);
+  const int routed = t.before[a.groups], total = routed + (a.shared_image ? a.tokens : 0);
   if (a.plan_ready) {
     pdl_wait();
     pdl_trigger();
@@ -721,13 +747,8 @@ __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) 
       stage_bf16_row(a.x + (size_t)token * a.k, a.shared_image + (size_t)tile * a.shared_tile * a.k * 2, row, padded, a.k);
       continue;
     }
-    int lo = 0, hi = a.groups;   // the group of active route i
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (t.cost[mid] <= i) lo = mid;
-      else hi = mid;
-    }
-    const int pos = i - t.cost[lo], count = t.cost[lo + 1] - t.cost[lo];
+    const int lo = gg_group_of(t.before, a.groups, i);   // the group of active route i
+    const int pos = i - t.before[lo], count = t.before[lo + 1] - t.before[lo];
     const int tile = pos / a.tile, row = pos % a.tile, slot0 = gg_first_slot(t.slot0, lo, kPad) + tile * a.tile;
     const int padded = (min(a.tile, count - tile * a.tile) + kPad - 1) / kPad * kPad;
     const uint16_t* from = a.x + (size_t)(a.rows[(size_t)lo * a.capacity + pos] / a.div) * a.k;
@@ -828,14 +849,15 @@ static size_t gg_pad256(size_t n) { return (n + 255) / 256 * 256; }
 
 // what one projection's N operand takes: images of the routed slots, of the tokens for the shared experts
 struct GgScratch {
-  size_t slots, image, image_scales, slot_scale, total;
+  size_t slots, image, image_scales, slot_scale, next, total;
   GgScratch(bool fp4, size_t routes, size_t groups, int k) {
     const size_t active = routes < groups ? routes : groups;
     slots = routes + active * (gg_pad(fp4) - 1);
     image = gg_pad256(slots * (size_t)k * 2);
     image_scales = fp4 ? gg_pad256(slots * (size_t)k / 4) : 0;
     slot_scale = fp4 ? gg_pad256(slots * sizeof(float)) : 0;
-    total = image + image_scales + slot_scale;
+    next = 256;   // the counter of deals
+    total = image + image_scales + slot_scale + next;
   }
 };
 
@@ -904,14 +926,13 @@ static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStre
   return kOk;
 }
 
-// Tokens T of a tile, from the mean number of routes per expert. T = 16, 32, 64, us a call, experts evenly / unevenly chosen
-// (rank^-0.6):
-//   256 of 4096 x 2048   mean 8: 676 701 761 / 759 710 770;  24: 1226 905 977 / 1277 1030 1060;  36: 1736 1407 1215 / 1738 1333 1323
-//   256 of 4096 x 512         8: 239 252 260 / 249 299 316;  24:  438 392 408 /  451  450  484;  36:  610  587  534 /  630  585  611
-//   128 of 2048 x 1024        8: 124 121 131 / 128 136 157;  24:  203 167 175 /  203  188  213;  36:  267  236  221 /  271  235  254
-//    64 of 1024 x 512         8:  50  52  52 /  51  58  64;  24:   69  70  71 /   70   74   81;  36:   84   87   88 /   86   87   90
-// so at a mean of 8 the smallest is right on the whole, and for the smallest layers it stays so (up to 10 % at mean 16).
-static int gg_tokens(long long routes, int experts) { return routes > 24LL * experts ? 64 : routes > 8LL * experts ? 32 : 16; }
+// Tokens T of a tile, from the mean number of routes per expert. T = 16, 32, 64, us a call, experts chosen evenly / as rank^-0.6:
+//   256 of 4096 x 2048   mean 8: 600 621 713 / 629 633 716;  16:  825 690 784 /  874  742  812;  32: 1283  981  971 / 1347  969 1059;  46: 1713 1308 1201 / 1895 1246 1252
+//   256 of 4096 x 512         8: 227 229 239 / 239 253 283;  16:  308 293 303 /  313  306  327;  32:  514  451  440 /  518  454  481;  46:  717  616  590 /  721  606  602
+//   128 of 2048 x 1024        8: 120 117 123 / 117 120 134;  16:  144 140 142 /  144  145  164;  32:  232  205  198 /  232  199  215;  48:  311  275  271 /  313  268  279
+//    64 of 1024 x 512         8:  51  54  53 /  52  60  75;  16:   62  64  63 /   63   67   94;  32:   87   88   98 /   87   89  104;  48:  105   99  114 /  101  100  125
+// T = 16 and 32 meet between means of 10 (615 629 / 661 647 for the largest layers) and 12 (646 650 / 699 676).
+static int gg_tokens(long long routes, int experts) { return routes > 32LL * experts ? 64 : routes > 10LL * experts ? 32 : 16; }
 
 }  // namespace ink
 
@@ -957,10 +978,10 @@ extern "C" int ink_encode_shared(void* out_host_384, const void* gate, const voi
   return kOk;
 }
 
-// The items' costs are added up in 32 bits: 16 million routes at the greatest widths.
-static int check_costs_fit(bool fp4, size_t routes, int groups, int n, int t) {
+// The items are counted in 32 bits, with room to spare: 16 million routes at the greatest widths.
+static int check_items_fit(bool fp4, size_t routes, int groups, int n, int t) {
   const size_t tiles = routes / gg_tile(fp4, t) + (size_t)groups;
-  INK_REQUIRE(tiles * (n / kTcRows) * gg_most_cost <= 0x7fffffff && routes <= 0x40000000, kUnsupportedShape,
+  INK_REQUIRE(tiles * (n / kTcRows) * 128 <= 0x7fffffff && routes <= 0x40000000, kUnsupportedShape,
               "grouped projections: %zu routes in one call", routes);
   return kOk;
 }
@@ -995,7 +1016,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   if (int rc = check_grouped_shape(fp4, hidden, intermediate, groups)) return rc;
   const size_t routes = (size_t)tokens * top_k, padded = ((size_t)tokens + 7) / 8 * 8;
   const int t = gg_tokens((long long)routes, local);
-  if (int rc = check_costs_fit(fp4, routes, groups, 2 * intermediate > hidden ? 2 * intermediate : hidden, t)) return rc;
+  if (int rc = check_items_fit(fp4, routes, groups, 2 * intermediate > hidden ? 2 * intermediate : hidden, t)) return rc;
   INK_REQUIRE(scratch_bytes >= ink_moe_grouped_scratch_bytes(tokens, top_k, n_shared, hidden, intermediate, groups, quantized), kBadArgument,
               "moe_grouped: scratch of %zu bytes is too small", scratch_bytes);
   INK_REQUIRE(aligned16(x) && aligned16(activated) && aligned16(down) && aligned16(output) && aligned16(output_bf16) && (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0 &&
@@ -1006,8 +1027,8 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   const GgScratch in(fp4, routes, groups, hidden), act(fp4, routes, groups, intermediate);
   unsigned char* p = (unsigned char*)scratch;
   auto take = [&](size_t n) { unsigned char* q = p; p += gg_pad256(n); return q; };
-  unsigned char *in_image = take(in.image), *in_scales = take(in.image_scales), *in_slot = take(in.slot_scale);
-  unsigned char *act_image = take(act.image), *act_scales = take(act.image_scales), *act_slot = take(act.slot_scale);
+  unsigned char *in_image = take(in.image), *in_scales = take(in.image_scales), *in_slot = take(in.slot_scale), *in_next = take(in.next);
+  unsigned char *act_image = take(act.image), *act_scales = take(act.image_scales), *act_slot = take(act.slot_scale), *act_next = take(act.next);
   unsigned char *x_image = take(n_shared ? padded * hidden * 2 : 0), *sact_image = take(padded * n_shared * intermediate * 2);
   unsigned char* shared_out = take((size_t)tokens * n_shared * hidden * 2);
   const int bank = fp4 ? 3 : 1, stride = fp4 ? kBank : 2;
@@ -1021,6 +1042,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   st.image = in_image;
   st.image_scales = in_scales;
   st.slot_scale = (float*)in_slot;
+  st.next = (unsigned*)in_next;
   st.shared_image = n_shared ? x_image : nullptr;
   st.groups = groups;
   st.capacity = capacity;
@@ -1042,6 +1064,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   g.image = in_image;
   g.image_scales = in_scales;
   g.slot_scale = (const float*)in_slot;
+  g.next = (unsigned*)in_next;
   g.y = (uint16_t*)activated;
   g.groups = groups;
   g.start = start;
@@ -1063,6 +1086,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   st.image = act_image;
   st.image_scales = act_scales;
   st.slot_scale = (float*)act_slot;
+  st.next = (unsigned*)act_next;
   st.shared_image = nullptr;
   st.bank = bank;
   st.k = intermediate;
@@ -1074,6 +1098,7 @@ extern "C" int ink_moe_grouped(const void* x, const int64_t* indices, const void
   g.image = act_image;
   g.image_scales = act_scales;
   g.slot_scale = (const float*)act_slot;
+  g.next = (unsigned*)act_next;
   g.y = (uint16_t*)down;
   g.bank = bank;
   g.k = intermediate;
@@ -1117,7 +1142,7 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
               capacity, top_k, input_rows);
   const size_t routes = (size_t)input_rows * (projection == 0 ? top_k : 1);   // (`capacity` bounds one group's, not all of them)
   const int t = gg_tokens((long long)routes, groups);
-  if (int rc = check_costs_fit(true, routes, groups, n, t)) return rc;
+  if (int rc = check_items_fit(true, routes, groups, n, t)) return rc;
   INK_REQUIRE(scratch_bytes >= expert_gemm_tc_bytes(routes, groups, k), kBadArgument,
               "expert_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, expert_gemm_tc_bytes(routes, groups, k));
   INK_REQUIRE(aligned16(x) && aligned16(y) && aligned16(scratch) && (reinterpret_cast<uintptr_t>(bank_maps) & 127u) == 0,
@@ -1134,6 +1159,7 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   st.image = (unsigned char*)scratch;
   st.image_scales = st.image + sizes.image;
   st.slot_scale = (float*)(st.image_scales + sizes.image_scales);
+  st.next = (unsigned*)(st.image_scales + sizes.image_scales + sizes.slot_scale);
   st.groups = groups;
   st.capacity = capacity;
   st.stride = kBank;
@@ -1152,6 +1178,7 @@ extern "C" int ink_expert_gemm_tc(const void* x, int input_rows, const void* ban
   g.image = st.image;
   g.image_scales = st.image_scales;
   g.slot_scale = st.slot_scale;
+  g.next = st.next;
   g.y = (uint16_t*)y;
   g.groups = groups;
   g.start = start;

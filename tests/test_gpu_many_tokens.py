@@ -67,6 +67,32 @@ def test_unquantised_banks_of_several_tokens(ib, device, d, f, experts, tokens):
     assert max_rel(got, oracle_moe.routed_experts_bf16_fp32(x, idx, w, banks)) <= TOL
 
 
+@pytest.mark.parametrize("d,f,experts,tokens", [
+    (256, 2048, 100, 100), (256, 2048, 100, 500),   # one ring stage an item, more deals than blocks, more items a deal than the queue holds
+    (512, 1024, 60, 290),                            # deals that end inside an expert; gate/up and down of different lengths
+    (4096, 128, 3, 5), (256, 256, 1, 2),             # one item a deal; fewer items than blocks
+])
+def test_every_item_is_dealt_whatever_their_number(ib, device, d, f, experts, tokens):
+    if f % 256:   # (packed banks need a multiple of 256 columns: BF16 ones)
+        gen = torch.Generator().manual_seed(tokens)
+        banks = {e: dict(gate_up_proj=(torch.randn(2 * f, d, generator=gen) * 0.05).to(BF16), down_proj=(torch.randn(d, f, generator=gen) * 0.05).to(BF16))
+                 for e in range(experts)}
+        x = torch.randn(tokens, d, generator=gen).to(BF16)
+        want = oracle_moe.routed_experts_bf16_fp32
+    else:
+        _, banks, x = cases.make_layer(d, f, experts, 1, 1, tokens, seed=tokens, bias="randn")
+        gen, want = torch.Generator().manual_seed(tokens), oracle_moe.routed_experts_fp32
+    k = min(3, experts)
+    idx = torch.stack([torch.randperm(experts, generator=gen)[:k] for _ in range(tokens)])
+    w = torch.rand(tokens, k, generator=gen).to(BF16)
+    module = ib.ResidentExperts(d, f, None, one_allocation_per_kind(banks, device), quantized=f % 256 == 0)
+    assert module.bank_maps is not None
+    for _ in range(2):   # (the counter starts over)
+        got = module(x.to(device), idx.to(device), w.to(device)).float().cpu()
+        module.check_status()
+        assert max_rel(got, want(x, idx, w, banks)) <= TOL
+
+
 def test_experts_that_are_not_there_are_skipped_and_reported(ib, device):
     """A rank that holds the experts 2..5 of 8: routes to the others add nothing; an id beyond the table sets the status."""
     d, f, tokens = 512, 256, 20
