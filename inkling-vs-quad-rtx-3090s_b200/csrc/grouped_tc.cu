@@ -716,8 +716,8 @@ __device__ __forceinline__ void stage_bf16_row(const uint16_t* from, unsigned ch
     *reinterpret_cast<uint4*>(tile + (size_t)(p >> 3) * padded * 128 + row * 128 + (((p & 7) ^ (row & 7)) << 4)) = reinterpret_cast<const uint4*>(from)[p];
 }
 
-// Blocks take routed slots in turn, then the tokens for the shared experts. Bound by the digit arithmetic (about a hundred
-// instructions per eight elements) and, for prompts, by the image's bytes; a token is converted once per route, which
+// Blocks take routed slots in turn, then the tokens for the shared experts. Bound by the digit arithmetic (tc_digits8; more
+// blocks an SM, 12 or 16 for 8, changed nothing) and, for prompts, by the image's bytes; a token is converted once per route, which
 // costs less than gathering it from one copy sixteen times per expert in the main kernel.
 template <bool FP4>
 __global__ void __launch_bounds__(kStageThreads) stage_rows_kernel(StageArgs a) {
