@@ -169,6 +169,9 @@ int ink_moe_down(const void* x, const int64_t* indices, const void* weights, con
 int ink_add_rmsnorm(const float* partial, void* residual, const void* weight, float eps, void* normed,
                     int tokens, int hidden, ink_stream_t stream);
 
+/* The norm alone (MyInklingRMSNorm, my_inkling/model.py:140-150): x BF16 [tokens, hidden] is only read. Constraints as above. */
+int ink_rmsnorm(const void* x, const void* weight, float eps, void* normed, int tokens, int hidden, ink_stream_t stream);
+
 /* The decode step of MyInklingShortConv (my_inkling/model.py:400-409), i.e. the Triton kernel
  * _short_conv (kernels/decode.py:65-146), which follows the MoE block as mlp_sconv with the
  * decoder residual (my_inkling/model.py:674-675): per channel c
@@ -183,6 +186,28 @@ int ink_add_rmsnorm(const float* partial, void* residual, const void* weight, fl
  * kernel_size 2..4 (the model uses 4). */
 int ink_short_conv(const void* x, int x_is_fp32, const float* taps, float* history, const void* residual,
                    void* y, int batch, int hidden, int kernel_size, ink_stream_t stream);
+
+/* ink_short_conv with BF16 x and a residual, and the norm of its result as ink_rmsnorm gives it, in one launch (attn_sconv,
+ * residual and post-attention norm of MyInklingDecoderLayer.forward, my_inkling/model.py:664-671): the same bits in y, history and normed.
+ * taps and history 16-byte aligned, hidden % 8 == 0, hidden <= 16384, batch <= 65535. */
+int ink_short_conv_norm(const void* x, const float* taps, float* history, const void* residual, const void* weight, float eps, void* y,
+                        void* normed, int batch, int hidden, int kernel_size, ink_stream_t stream);
+
+/* What MyInklingAttention.forward does between the fused projection and the cache update at decode (my_inkling/model.py:504-531):
+ * q = norm(q heads), k = norm(short_conv(k heads)), v = short_conv(v heads), r = the relative states, in the bits of ink_short_conv and ink_rmsnorm.
+ *  qkvr BF16 [batch, (heads + 2 kv_heads) head_dim + heads d_rel]; q BF16 [batch, heads, head_dim], k, v BF16 [batch, kv_heads, head_dim],
+ *  r BF16 [batch, heads, d_rel]; taps FP32 [kv_heads head_dim, kernel_size], histories FP32 [batch, kv_heads head_dim, kernel_size], moved on in place.
+ * head_dim % 8 == 0 up to 256, heads d_rel % 8 == 0, everything 16-byte aligned. */
+int ink_attention_heads(const void* qkvr, const void* q_weight, const void* k_weight, const float* k_taps, const float* v_taps, float* k_history,
+                        float* v_history, float eps, void* q, void* k, void* v, void* r, int batch, int heads, int kv_heads, int head_dim,
+                        int d_rel, int kernel_size, ink_stream_t stream);
+
+/* Dense BF16 projections of up to eight tokens (the layer's fused QKVR, output and dense-MLP projections and the LM head at decode):
+ * y = bf16(x . weight^T), x BF16 [tokens, k], weight BF16 [n, k], y BF16 [tokens, n], sums in FP32 over
+ * the columns in order, sixteen at a time. With `up` BF16 [n, k]:
+ * y = bf16(bf16(silu(bf16(x . weight^T))) * bf16(x . up^T)). With `scale` BF16 [1]: y is multiplied by it and rounded once more.
+ * k a multiple of 32 up to 8192; x, weight and up 16-byte aligned. */
+int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k, ink_stream_t stream);
 
 /* Decode attention with the learned relative-position bias, one query token per sequence: the static_decode
  * branch of MyInklingAttention.forward (my_inkling/model.py:533-612) from the normed query to the output of
@@ -207,6 +232,8 @@ int ink_short_conv(const void* x, int x_is_fp32, const float* taps, float* histo
 size_t ink_decode_attention_workspace_bytes(int batch, int heads, int head_dim, int slots);
 /* how many bytes at its start are the arrival counters, the only part that must be zero */
 size_t ink_decode_attention_counter_bytes(int batch, int heads);
+/* 1: a call of these sizes joins its parts through the workspace; 0: it does not touch it (its contents may be anything) */
+int ink_decode_attention_joins(int batch, int heads, int kv_heads, int head_dim, int slots);
 int ink_decode_attention(const void* q, const void* r, const void* proj, void* k_cache, void* v_cache,
                          const int64_t* position, const int64_t* pad_counts, void* out, int batch, int heads,
                          int kv_heads, int head_dim, int d_rel, int rel_extent, int slots, int window, int n_floor,

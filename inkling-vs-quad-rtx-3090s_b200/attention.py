@@ -3,9 +3,8 @@
 `MyInklingAttention.forward` with a decoding cache (my_inkling/model.py:504-622) is: the fused QKVR projection,
 RMS norm of the query heads, short convolution + RMS norm of the key, short convolution of the value, `update_kv`,
 relative-position bias + mask + `scaled_dot_product_attention`, the output projection (and its all-reduce under
-tensor parallelism). Here the two dense projections stay library GEMVs (`torch.nn.functional.linear`), everything
-between them runs in this library: `ink_short_conv`, `ink_add_rmsnorm`, `ink_decode_attention` (which also stores
-the token in the caches). The cache object is the reference's `MyInklingCache` (or anything with the same fields:
+tensor parallelism). Here that is `ink_linear` (up to eight sequences; library GEMMs above), `ink_attention_heads`,
+`ink_decode_attention` (which also stores the token in the caches) and `ink_linear` again. The cache object is the reference's `MyInklingCache` (or anything with the same fields:
 `layers[i].k_cache / v_cache / conv_caches[0 | 1].cache`, `position`, `pad_counts`).
 """
 from __future__ import annotations
@@ -14,29 +13,20 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .kernels import add_rmsnorm, decode_attention, short_conv
+from .kernels import attention_heads, decode_attention, gated, linear, rmsnorm, short_conv, short_conv_norm
 from .kernels.paired_all_reduce import all_reduce
-from .layer import KeepsForGraphs
 
 
-class _ZeroRows(KeepsForGraphs):
-    """The FP32 zeros that the norm kernel adds to its rows, kept from call to call."""
-
-    _zeros = None
-
-    def _zero_rows(self, rows: torch.Tensor) -> torch.Tensor:
-        n, width = rows.shape
-        if self._zeros is None or self._zeros.shape[0] < n or self._zeros.shape[1] != width:
-            zeros = torch.zeros(n, width, dtype=torch.float32, device=rows.device)
-            if torch.cuda.is_current_stream_capturing():
-                return zeros   # (filled in by that graph alone, when it is replayed: not for other calls)
-            self._replace(self._zeros)
-            self._zeros = zeros
-        self._note_capture()
-        return self._zeros[:n]
+def _norm_rows(rows: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """RMS norm over the last dimension of BF16 [n, c] with the reference's rounding (kernels/decode.py:36-43)."""
+    return rmsnorm(rows if rows.data_ptr() % 16 == 0 else rows.clone(), weight, eps)
 
 
-class DecodeAttention(_ZeroRows, nn.Module):
+def _aligned(*tensors: torch.Tensor) -> bool:
+    return all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
+class DecodeAttention(nn.Module):
     def __init__(self, qkvr_weight, o_weight, q_norm_weight, k_norm_weight, k_taps, v_taps, rel_proj, *, layer_idx: int,
                  heads: int, kv_heads: int, head_dim: int, d_rel: int, window: int = 0, log_scaling_n_floor=None,
                  log_scaling_alpha: float = 0.1, eps: float = 1e-6, group=None):
@@ -65,10 +55,7 @@ class DecodeAttention(_ZeroRows, nn.Module):
                    eps=attention.q_norm.variance_epsilon, group=group)
 
     def _norm(self, rows: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-        """RMS norm over the last dimension of BF16 [n, c] with the reference's rounding (kernels/decode.py:36-43)."""
-        normed = torch.empty_like(rows)
-        add_rmsnorm(self._zero_rows(rows), rows, weight, self.eps, normed)   # rows + 0, then the norm
-        return normed
+        return _norm_rows(rows, weight, self.eps)
 
     def forward(self, hidden_states: torch.Tensor, cache) -> torch.Tensor:
         """hidden_states BF16 [bs, 1, d], cache in decode mode -> BF16 [bs, 1, d]; the caches and the convolution
@@ -77,22 +64,28 @@ class DecodeAttention(_ZeroRows, nn.Module):
         assert s == 1, "one token per sequence"
         layer = cache.layers[self.layer_idx]
         h, hk, c = self.heads, self.kv_heads, self.head_dim
-        q, k, v, r = F.linear(hidden_states, self.qkvr_weight).split(self.sizes, dim=-1)
-        q = self._norm(q.reshape(bs * h, c).contiguous(), self.q_norm_weight)
-        k = short_conv(k.contiguous(), self.k_taps, layer.conv_caches[0].cache, None)
-        k = self._norm(k.reshape(bs * hk, c), self.k_norm_weight)
-        v = short_conv(v.contiguous(), self.v_taps, layer.conv_caches[1].cache, None)
+        qkvr = linear(hidden_states, self.qkvr_weight)
+        k_history, v_history = layer.conv_caches[0].cache, layer.conv_caches[1].cache
+        if c % 8 == 0 and c <= 256 and (h * self.d_rel) % 8 == 0 and _aligned(qkvr, self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history):
+            q, k, v, r = attention_heads(qkvr.view(bs, -1), self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history, self.eps,
+                                         h, hk, c, self.d_rel)
+        else:   # heads of other widths, histories that start anywhere
+            q, k, v, r = qkvr.split(self.sizes, dim=-1)
+            q = self._norm(q.reshape(bs * h, c).contiguous(), self.q_norm_weight)
+            k = short_conv(k.contiguous(), self.k_taps, k_history, None)
+            k = self._norm(k.reshape(bs * hk, c), self.k_norm_weight)
+            v = short_conv(v.contiguous(), self.v_taps, v_history, None)
         out = decode_attention(q.view(bs, h, c), r.reshape(bs, h, self.d_rel), self.rel_proj, layer.k_cache, layer.v_cache,
                                cache.position, cache.pad_counts, window=self.window, log_scaling_n_floor=self.n_floor,
                                log_scaling_alpha=self.alpha, scale=1.0 / c, new_key=k.view(bs, hk, 1, c),
                                new_value=v.reshape(bs, hk, 1, c))
-        y = F.linear(out.reshape(bs, 1, h * c), self.o_weight)
+        y = linear(out.reshape(bs, 1, h * c), self.o_weight)
         if self.group is not None:
             y = all_reduce(y, self.group)   # (nothing to do with one rank)
         return y
 
 
-class DecodeLayer(_ZeroRows, nn.Module):
+class DecodeLayer(nn.Module):
     """One sparse decoder layer at decode, `MyInklingDecoderLayer.forward` (my_inkling/model.py:661-675):
     h' = attn_sconv(attention(input_norm(h)), residual=h);  out = mlp_sconv(moe(post_norm(h')), residual=h').
     `attention` is a DecodeAttention, `moe` a FusedMoE (a sparse layer) or a DenseMLP (a dense one); the two short
@@ -106,24 +99,25 @@ class DecodeLayer(_ZeroRows, nn.Module):
             self.register_buffer(name, t.contiguous())
 
     def _norm(self, x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-        rows = x.reshape(-1, x.shape[-1]).clone()          # (the norm kernel adds its FP32 input to the rows in place: zero here)
-        normed = torch.empty_like(rows)
-        add_rmsnorm(self._zero_rows(rows), rows, weight, self.eps, normed)
-        return normed.view(x.shape)
+        return _norm_rows(x.reshape(-1, x.shape[-1]), weight, self.eps).view(x.shape)
 
     def forward(self, hidden_states: torch.Tensor, cache) -> torch.Tensor:
         """hidden_states BF16 [bs, 1, d] -> BF16 [bs, 1, d]; the layer's caches are updated in place."""
         bs, _, d = hidden_states.shape
         layer = cache.layers[self.attention.layer_idx]
         attended = self.attention(self._norm(hidden_states, self.input_norm_weight), cache)
-        h = short_conv(attended.contiguous(), self.attn_taps, layer.conv_caches[2].cache, hidden_states.contiguous())
-        normed = self._norm(h, self.post_norm_weight).view(bs, d)
+        attended, history, residual = attended.contiguous(), layer.conv_caches[2].cache, hidden_states.contiguous()
+        if d % 8 == 0 and _aligned(self.attn_taps, history):
+            h, normed = short_conv_norm(attended, self.attn_taps, history, residual, self.post_norm_weight, self.eps)
+        else:
+            h = short_conv(attended, self.attn_taps, history, residual)
+            normed = self._norm(h, self.post_norm_weight).view(bs, d)
         block = self.moe.forward_partial(normed) if hasattr(self.moe, "forward_partial") else self.moe(normed)   # [bs, d], all-reduced
         return short_conv(block.view(bs, 1, d).contiguous(), self.mlp_taps, layer.conv_caches[3].cache, h)
 
 
 class DenseMLP(nn.Module):
-    """`MyInklingMLP` (my_inkling/model.py:153-171), the block of a dense layer: three library GEMVs,
+    """`MyInklingMLP` (my_inkling/model.py:153-171), the block of a dense layer: two launches of `ink_linear`,
     down(silu(gate(x)) * up(x)) * global_scale, BF16 like the reference's; all-reduced over `group` when the rows of
     gate/up and the columns of down are sliced."""
 
@@ -134,7 +128,7 @@ class DenseMLP(nn.Module):
         self.group = group
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        y = F.linear(F.silu(F.linear(x, self.gate_weight)) * F.linear(x, self.up_weight), self.down_weight) * self.global_scale
+        y = linear(gated(x, self.gate_weight, self.up_weight), self.down_weight, self.global_scale)
         return y if self.group is None else all_reduce(y, self.group)
 
 
@@ -159,6 +153,6 @@ class DecodeModel(nn.Module):
         for layer in self.layers:
             hidden = layer(hidden, cache)
         hidden = norm(hidden, self.final_norm_weight) / self.mup
-        logits = F.linear(hidden, self.lm_head_weight)
+        logits = linear(hidden, self.lm_head_weight)
         cache.position.add_(1)
         return logits if self.unpadded is None else logits[..., : self.unpadded]

@@ -2,6 +2,7 @@
 // layer's K/V cache (a ring of `window` slots in a sliding layer, `slots` positions in a full one).
 #include "../../include/inkling_b200.h"
 #include "common.cuh"
+#include "mma_bf16.cuh"
 #include "stream_math.cuh"
 
 namespace ink {
@@ -13,10 +14,11 @@ constexpr int kAttnUnit = 16;                               // cache slots per s
 constexpr int kAttnMinSlots = kAttnUnit * kAttnWarps;       // a block is not worth launching for fewer
 constexpr int kAttnCluster = 8;                             // parts that can meet in one thread-block cluster
 constexpr int kAttnMaxSplits = 64;
-// Blocks resident at once, up to 128 channels. (Of 256 channels it is two an SM. Dealing for two measured 160 us against 213 for
-// eight sequences of 64 heads on 8 at 8 000 slots, 64 against 84 for four of 32 on 8 at 6 000, but 86 against 67 for six of 64
-// on 8 at 2 900, whose parts then form clusters that do not fill the chip.)
-constexpr int kAttnWaveBlocks = 148 * 3;
+// Blocks of the large form that an SM holds, and clusters of n = 0, 1, .. 8 parts that are resident at once on 148 SMs
+// (cudaOccupancyMaxActiveClusters: a cluster lies in one GPC, so those of seven or eight parts leave a tenth of the SMs empty).
+constexpr int kAttnPerSm(int channels) { return channels > 128 ? 2 : 3; }
+constexpr int kAttnSms = 148;
+constexpr int kAttnClusters[2][kAttnCluster + 1] = {{0, 444, 222, 142, 104, 82, 71, 56, 48}, {0, 296, 148, 93, 71, 56, 45, 37, 33}};
 constexpr int kAttnPartial = 4;                             // floats in front of a partial result: running maximum, sum, padding
 
 struct AttnArgs {
@@ -38,14 +40,6 @@ struct AttnArgs {
   float alpha, scale;
 };
 
-// D[16x8] += A[16x16] . B[16x8], BF16 in, FP32 out. Lane (g = lane / 4, t = lane % 4) holds of A: a0 = row g,
-// columns 2t, 2t+1; a1 = row g + 8, the same columns; a2, a3 = columns 2t+8, 2t+9 of these rows; of B: b0 = rows
-// 2t, 2t+1, b1 = rows 2t+8, 2t+9 of column g; of D: d0, d1 = row g, columns 2t, 2t+1; d2, d3 = row g + 8.
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -54,19 +48,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 
 // the two floats cut off to BF16
 __device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
-
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// two floats at this block's address `p` in the shared memory of block `rank` of the cluster
-__device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
-  float2 v;
-  asm volatile("{\n .reg .u32 at;\n mapa.shared::cluster.u32 at, %2, %3;\n ld.shared::cluster.v2.f32 {%0, %1}, [at];\n}\n"
-               : "=f"(v.x), "=f"(v.y)
-               : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank)
-               : "memory");
-  return v;
-}
 
 // One block per (part of the cache, group of up to eight heads of one key/value head, sequence). Bound by reading
 // the cache once: 512 bytes a slot against 32 k FMAs for eight heads of 128 channels, which the CUDA cores cannot
@@ -90,7 +71,7 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 // and read one another's sums through distributed shared memory; more leave their sums in global memory and the block that
 // finishes last adds them up. The second way costs a fence, an atomic and two more round trips.
 template <int C, bool CLUSTER>
-__global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attention_kernel(AttnArgs a) {
+__global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_kernel(AttnArgs a) {
   constexpr int kPieces = C / 32;       // 16-byte pieces of a key row per lane
   constexpr int kHalves = C / 64;       // pieces of a value row per lane
   extern __shared__ __align__(16) unsigned char s_raw[];
@@ -98,6 +79,8 @@ __global__ void __launch_bounds__(kAttnThreads, C > 128 ? 2 : 3) decode_attentio
   uint16_t* s_r = reinterpret_cast<uint16_t*>(s_raw);                               // [heads][d_rel rounded up to 16]: before the sums
   __shared__ bool s_last;
   __shared__ __align__(16) float s_block[CLUSTER ? kAttnHeads * (C + 2) : 1];   // this block's sums, for its cluster
+  pdl_trigger();
+  pdl_wait();
   const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
@@ -449,6 +432,8 @@ __global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(A
   uint16_t* s_r = reinterpret_cast<uint16_t*>(s_block + kAttnHeads * (C + 2));      // [heads][d_rel]
   __shared__ float s_top[kAttnHeads];
   __shared__ bool s_last;
+  pdl_trigger();
+  pdl_wait();
   const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
   const int kv_head = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
@@ -763,6 +748,30 @@ static int attention_max_splits(int slots) {
   return whole < kAttnMaxSplits ? whole : kAttnMaxSplits;
 }
 
+// Where all 64-slot parts are resident at once the small form takes them. Else the number of parts that takes the fewest
+// rounds of (steps a warp makes + what a block costs beside, about four steps' time), a round being what is resident at once.
+static int attention_splits(int batch, int kv_heads, int chunks, int head_dim, int slots, bool* small) {
+  const int pairs = batch * kv_heads * chunks, whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
+  *small = whole <= kAttnMaxSplits && (long long)whole * pairs <= kSmallMostBlocks;
+  int splits = whole, best = 0x7fffffff;
+  for (int n = 1, most = attention_max_splits(slots); n <= most && !*small; ++n) {
+    const bool cluster = n > 1 && n <= kAttnCluster;
+    const long long resident = cluster ? kAttnClusters[head_dim > 128][n] : kAttnSms * kAttnPerSm(head_dim);
+    const long long wanted = cluster ? pairs : (long long)pairs * n, cost = (wanted + resident - 1) / resident * (4 + (whole + n - 1) / n);
+    if (cost <= best) {   // (of equals the finer: sequences may be shorter than the cache)
+      best = (int)cost;
+      splits = n;
+    }
+  }
+  return splits;
+}
+
+extern "C" int ink_decode_attention_joins(int batch, int heads, int kv_heads, int head_dim, int slots) {
+  if (batch <= 0 || kv_heads <= 0 || heads <= 0 || slots <= 0) return 0;
+  bool small;
+  return attention_splits(batch, kv_heads, (heads / kv_heads + kAttnHeads - 1) / kAttnHeads, head_dim, slots, &small) > kAttnCluster;
+}
+
 extern "C" size_t ink_decode_attention_workspace_bytes(int batch, int heads, int head_dim, int slots) {
   const size_t splits = (size_t)attention_max_splits(slots);
   return splits <= kAttnCluster ? 0 : attention_counter_bytes(batch, heads) + sizeof(float) * (size_t)batch * heads * splits * (kAttnPartial + head_dim);
@@ -781,13 +790,21 @@ static int launch_decode_attention(const AttnArgs& a, bool small, dim3 grid, cud
   config.blockDim = dim3(small ? kSmallThreads : kAttnThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute;
-  attribute.id = cudaLaunchAttributeClusterDimension;
-  attribute.val.clusterDim.x = grid.x;
-  attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-  config.attrs = &attribute;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = grid.x;
+  attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
   const bool cluster = a.splits > 1 && a.splits <= kAttnCluster;
-  config.numAttrs = cluster ? 1 : 0;
+  // Clusters may start while the kernel in front still runs, which saves a call 1 to 2 us, unless they hardly all fit: those that
+  // find an SM still taken would make a second round (seven sequences of 64 heads on 8 at 3 000 slots, 56 clusters of seven where 56
+  // fit: 45 us in a layer, 29 so). Nor do the other forms, whose grids fill the chip: their blocks would take
+  // the places unevenly (50.1 us for 46.7, seven sequences of 32 heads on 32, 256 channels, 512 slots).
+  const int fit = cluster ? kAttnClusters[C > 128][a.splits] : 0;
+  const bool early = cluster && (small || (long long)grid.y * grid.z <= fit - fit / 16);
+  config.attrs = early ? attributes : attributes + 1;
+  config.numAttrs = cluster ? (early ? 2 : 1) : 0;
   void (*kernel)(AttnArgs) = small ? (cluster ? decode_attention_small_kernel<C, true> : decode_attention_small_kernel<C, false>)
                                    : (cluster ? decode_attention_kernel<C, true> : decode_attention_kernel<C, false>);
   if (smem > 40 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -823,18 +840,8 @@ extern "C" int ink_decode_attention(const void* q, const void* r, const void* pr
     if (int rc = ink_update_kv(new_k, new_v, k_cache, v_cache, position, batch, kv_heads, head_dim, slots, window, stream)) return rc;
     new_k = new_v = nullptr;
   }
-  const int pairs = batch * kv_heads * chunks, whole = (slots + kAttnMinSlots - 1) / kAttnMinSlots;
-  // Where all 64-slot parts are resident at once the small form takes them. Else the number of parts that takes the fewest
-  // rounds of (steps a warp makes + what a block costs beside, about four steps' time), over the blocks resident at once.
-  const bool small = whole <= kAttnMaxSplits && (long long)whole * pairs <= kSmallMostBlocks;
-  int splits = whole, best = 0x7fffffff;
-  for (int n = 1, most = attention_max_splits(slots); n <= most && !small; ++n) {
-    const long long rounds = ((long long)pairs * n + kAttnWaveBlocks - 1) / kAttnWaveBlocks, cost = rounds * (4 + (whole + n - 1) / n);
-    if (cost <= best) {   // (of equals the finer: sequences may be shorter than the cache)
-      best = (int)cost;
-      splits = n;
-    }
-  }
+  bool small;
+  const int splits = attention_splits(batch, kv_heads, chunks, head_dim, slots, &small);
   AttnArgs a{(const uint16_t*)q, (const uint16_t*)r, (const uint16_t*)proj, (const uint16_t*)k_cache, (const uint16_t*)v_cache,
              position, pad_counts, (const uint16_t*)new_k, (const uint16_t*)new_v, (uint16_t*)k_cache, (uint16_t*)v_cache,
              (float*)((char*)workspace + attention_counter_bytes(batch, heads)), (unsigned*)workspace, (uint16_t*)out, heads, kv_heads,

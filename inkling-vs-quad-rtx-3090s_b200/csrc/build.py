@@ -17,7 +17,7 @@ CSRC = Path(__file__).resolve().parent
 PACKAGE = CSRC.parent
 LIBRARY = PACKAGE / "libinkling_b200.so"
 HOST_MODULE = PACKAGE / "inkling_b200_host.so"   # CPython extension: the eager calls' host side
-SOURCES = ("router_plan.cu", "routed_decode.cu", "stream_decode.cu", "moe_stack.cu", "grouped_experts.cu", "grouped_tc.cu", "glue.cu", "attention.cu")
+SOURCES = ("router_plan.cu", "routed_decode.cu", "stream_decode.cu", "moe_stack.cu", "grouped_experts.cu", "grouped_tc.cu", "glue.cu", "linear.cu", "attention.cu")
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xptxas=-v",

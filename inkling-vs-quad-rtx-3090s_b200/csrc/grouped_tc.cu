@@ -22,6 +22,7 @@
 #include "../../include/inkling_b200.h"
 #include "common.cuh"
 #include "decode_args.cuh"
+#include "mma_bf16.cuh"
 #include "pipe.cuh"
 #include "tc_path.cuh"
 #include "tensor_map.cuh"
@@ -104,8 +105,6 @@ __device__ __forceinline__ bool gg_wait(uint64_t* bar, uint32_t parity, GgShared
   }
   return true;
 }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // routes of a group that have something to do
 __device__ __forceinline__ int gg_count(const int32_t* counts, const int32_t* experts, const int64_t* pointers, int stride, int bank, int g) {

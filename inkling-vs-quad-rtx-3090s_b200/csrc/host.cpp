@@ -77,13 +77,14 @@ at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const at::Devi
 // The join's workspace starts with counters that are zero between launches. An eager call keeps one for its stream (made
 // again, zeroed, when the sizes change; at most kMostWorkspaces, then the pool starts anew -- the memory goes back to the
 // allocator, which hands it out on the same stream only). A call under capture gets its own from the graph's pool, its
-// counters cleared by the graph: graphs may be replayed in any order, on any stream.
-at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, size_t bytes, size_t counters) {
+// counters cleared by the graph: graphs may be replayed in any order, on any stream. (`joins`: the call counts at all. A
+// node that clears memory between two kernels costs 8 us.)
+at::Tensor attention_workspace(const at::Device& device, cudaStream_t stream, size_t bytes, size_t counters, bool joins) {
   const auto options = at::TensorOptions().dtype(at::kByte).device(device);
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
     const at::Tensor t = at::empty({(int64_t)bytes}, options);
-    if (cudaMemsetAsync(t.data_ptr(), 0, counters, stream) != cudaSuccess) fail("decode_attention: the workspace could not be cleared");
+    if (joins && cudaMemsetAsync(t.data_ptr(), 0, counters, stream) != cudaSuccess) fail("decode_attention: the workspace could not be cleared");
     return t;
   }
   struct Workspace {
@@ -150,7 +151,8 @@ PyObject* decode_attention(PyObject* const* args) {
     if (!out.defined()) out = new_tensor({bs, h, 1, c}, at::kBFloat16, q.device());
     const size_t need = ink_decode_attention_workspace_bytes((int)bs, (int)h, (int)c, (int)slots);
     at::Tensor workspace;
-    if (need) workspace = attention_workspace(q.device(), stream, need, ink_decode_attention_counter_bytes((int)bs, (int)h));
+    if (need) workspace = attention_workspace(q.device(), stream, need, ink_decode_attention_counter_bytes((int)bs, (int)h),
+                                              ink_decode_attention_joins((int)bs, (int)h, (int)hk, (int)c, (int)slots) != 0);
     check(ink_decode_attention(q.data_ptr(), r.data_ptr(), proj.data_ptr(), k.data_ptr(), v.data_ptr(), (const int64_t*)position.data_ptr(), (const int64_t*)pads,
                                out.data_ptr(), (int)bs, (int)h, (int)hk, (int)c, (int)d_rel, (int)proj.size(1), (int)slots, window, n_floor, alpha, scale, new_k.defined() ? new_k.data_ptr() : nullptr,
                                new_v.defined() ? new_v.data_ptr() : nullptr, need ? workspace.data_ptr() : nullptr, need, stream));

@@ -4,12 +4,14 @@ from .expert_planner import expert_copy, expert_plan
 from .grouped_experts import (block_scaled_supported, encode_bank_maps, encode_bf16_bank_maps, encode_shared_maps,
                               expert_bank_names, expert_gemm, expert_reduce, moe_grouped)
 from .attention import decode_attention, update_kv
-from .routed_decode import add_rmsnorm, moe_decode, routed_decode, short_conv
+from .linear import gated, linear
+from .routed_decode import add_rmsnorm, attention_heads, moe_decode, rmsnorm, routed_decode, short_conv, short_conv_norm
 from .stack import StackDescriptor, set_wait_limit, stack_supported
 from .router import router_forward, router_forward_static, router_plan_forward, router_workspace
 
 __all__ = [
     "add_rmsnorm",
+    "attention_heads",
     "block_scaled_supported",
     "encode_bank_maps",
     "encode_bf16_bank_maps",
@@ -25,6 +27,10 @@ __all__ = [
     "StackDescriptor",
     "set_wait_limit",
     "short_conv",
+    "short_conv_norm",
+    "rmsnorm",
+    "linear",
+    "gated",
     "decode_attention",
     "update_kv",
     "stack_supported",

@@ -31,6 +31,11 @@ _SIGNATURES = {
     "ink_moe_down": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P, P]),
     "ink_add_rmsnorm": (I, [P, P, P, F, P, I, I, P]),
     "ink_short_conv": (I, [P, I, P, P, P, P, I, I, I, P]),
+    "ink_rmsnorm": (I, [P, P, F, P, I, I, P]),
+    "ink_short_conv_norm": (I, [P, P, P, P, P, F, P, P, I, I, I, P]),
+    "ink_attention_heads": (I, [P, P, P, P, P, P, P, F, P, P, P, P, I, I, I, I, I, I, P]),
+    "ink_linear": (I, [P, P, P, P, P, I, I, I, P]),
+    "ink_decode_attention_joins": (I, [I, I, I, I, I]),
     "ink_decode_attention_workspace_bytes": (Z, [I, I, I, I]),
     "ink_decode_attention_counter_bytes": (Z, [I, I]),
     "ink_decode_attention": (I, [P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, F, P, P, P, Z, P]),

@@ -93,3 +93,47 @@ def short_conv(x, weight, history, residual=None):
                                          history.data_ptr(), _abi.ptr(residual), y.data_ptr(), bs, d, k,
                                          _abi.stream()))
     return y
+
+
+def rmsnorm(x, weight, eps: float):
+    """RMS norm over the last dimension of contiguous BF16 rows [n, c], with the rounding of `add_rmsnorm`; a new tensor."""
+    rows, hidden = x.shape
+    assert x.dtype == weight.dtype == torch.bfloat16 and weight.shape == (hidden,) and x.is_contiguous() and weight.is_contiguous()
+    _abi.require_cuda(x, weight)
+    normed = torch.empty_like(x)
+    _abi.check(_abi.lib().ink_rmsnorm(x.data_ptr(), weight.data_ptr(), float(eps), normed.data_ptr(), rows, hidden, _abi.stream()))
+    return normed
+
+
+def short_conv_norm(x, weight, history, residual, norm_weight, eps: float):
+    """`short_conv` with a residual and the norm of its result in one launch: x, residual BF16 [bs, 1, d] -> (y [bs, 1, d],
+    normed [bs, d])."""
+    bs, _, d = x.shape
+    k = weight.shape[-1]
+    assert x.dtype == residual.dtype == norm_weight.dtype == torch.bfloat16 and weight.dtype == history.dtype == torch.float32
+    assert all(t.is_contiguous() for t in (x, weight, history, residual, norm_weight))
+    assert history.shape == (bs, d, k) and weight.shape == (d, 1, k) and residual.shape == x.shape and norm_weight.shape == (d,)
+    _abi.require_cuda(x, weight, history, residual, norm_weight)
+    y, normed = torch.empty_like(x), torch.empty((bs, d), dtype=torch.bfloat16, device=x.device)
+    _abi.check(_abi.lib().ink_short_conv_norm(x.data_ptr(), weight.data_ptr(), history.data_ptr(), residual.data_ptr(), norm_weight.data_ptr(),
+                                              float(eps), y.data_ptr(), normed.data_ptr(), bs, d, k, _abi.stream()))
+    return y, normed
+
+
+def attention_heads(qkvr, q_weight, k_weight, k_taps, v_taps, k_history, v_history, eps: float, heads: int, kv_heads: int, head_dim: int, d_rel: int):
+    """What stands between the fused projection and the cache update: qkvr BF16 [bs, (h + 2 hk) c + h d_rel] -> normed queries
+    [bs, h, c], keys after convolution and norm and values after convolution [bs, hk, c], relative states [bs, h, d_rel]; the
+    histories FP32 [bs, hk c, K] move on by one."""
+    bs, taps = qkvr.shape[0], k_taps.shape[-1]
+    assert qkvr.dtype == q_weight.dtype == k_weight.dtype == torch.bfloat16
+    assert all(t.dtype == torch.float32 for t in (k_taps, v_taps, k_history, v_history))
+    tensors = (qkvr, q_weight, k_weight, k_taps, v_taps, k_history, v_history)
+    assert all(t.is_contiguous() for t in tensors) and qkvr.shape == (bs, (heads + 2 * kv_heads) * head_dim + heads * d_rel)
+    assert q_weight.shape == k_weight.shape == (head_dim,) and k_taps.shape == v_taps.shape == (kv_heads * head_dim, 1, taps)
+    assert k_history.shape == v_history.shape == (bs, kv_heads * head_dim, taps)
+    _abi.require_cuda(*tensors)
+    q, k, v, r = (qkvr.new_empty(bs, n, c) for n, c in ((heads, head_dim), (kv_heads, head_dim), (kv_heads, head_dim), (heads, d_rel)))
+    _abi.check(_abi.lib().ink_attention_heads(
+        qkvr.data_ptr(), q_weight.data_ptr(), k_weight.data_ptr(), k_taps.data_ptr(), v_taps.data_ptr(), k_history.data_ptr(), v_history.data_ptr(),
+        float(eps), q.data_ptr(), k.data_ptr(), v.data_ptr(), r.data_ptr(), bs, heads, kv_heads, head_dim, d_rel, taps, _abi.stream()))
+    return q, k, v, r

@@ -171,3 +171,109 @@ def test_resident_experts_over_bf16_banks(ib, device):
     experts.check_status()
     assert out.dtype == BF16
     assert max_rel(out.float(), oracle_moe.routed_experts_bf16_fp32(x, idx, w, bf)) <= TOL
+
+
+@pytest.mark.parametrize("hidden,rows", [(8, 3), (64, 5), (2048, 1), (2056, 2), (4096, 7), (16384, 2)])
+def test_the_norm_alone_is_the_norm_of_the_sum_with_zeros(ib, device, hidden, rows):
+    gen = torch.Generator().manual_seed(hidden)
+    x, w = torch.randn(rows, hidden, generator=gen).to(BF16).to(device), torch.randn(hidden, generator=gen).to(BF16).to(device)
+    x[0, :4] = 0
+    kept, want = x.clone(), torch.empty_like(x)
+    ib.kernels.add_rmsnorm(torch.zeros(rows, hidden, device=device), x.clone(), w, cases.EPS, want)
+    assert torch.equal(ib.kernels.rmsnorm(x, w, cases.EPS), want) and torch.equal(x, kept)
+
+
+def _conv(gen, device, batch, hidden, taps, at=0):
+    """Taps and history, the latter `at` floats into its buffer."""
+    buffer = torch.randn(batch * hidden * taps + at, generator=gen).to(device)
+    return torch.randn(hidden, 1, taps, generator=gen).to(device) * 0.3, buffer[at:].view(batch, hidden, taps)
+
+
+@pytest.mark.parametrize("batch,hidden,taps", [(1, 8, 4), (2, 256, 3), (3, 2040, 4), (1, 2056, 2), (7, 4096, 4), (2, 6152, 4), (1, 16384, 4)])
+def test_convolution_residual_and_norm_in_one_launch(ib, device, batch, hidden, taps):
+    """The same bits as short_conv and rmsnorm one after the other, twice (the history moves on)."""
+    gen = torch.Generator().manual_seed(hidden)
+    weight, history = _conv(gen, device, batch, hidden, taps)
+    norm, again = torch.randn(hidden, generator=gen).to(BF16).to(device), history.clone()
+    for _ in range(2):
+        x, residual = (torch.randn(batch, 1, hidden, generator=gen).to(BF16).to(device) for _ in range(2))
+        want = ib.kernels.short_conv(x, weight, again, residual)
+        y, normed = ib.kernels.short_conv_norm(x, weight, history, residual, norm, cases.EPS)
+        assert torch.equal(y, want) and torch.equal(history, again)
+        assert torch.equal(normed, ib.kernels.rmsnorm(want.view(batch, hidden), norm, cases.EPS))
+
+
+def test_a_convolution_history_may_start_anywhere(ib, device):
+    gen = torch.Generator().manual_seed(1)
+    weight, history = _conv(gen, device, 2, 300, 4, at=1)
+    x, again = torch.randn(2, 1, 300, generator=gen).to(BF16).to(device), history.clone()
+    assert torch.equal(ib.kernels.short_conv(x, weight, history), ib.kernels.short_conv(x, weight, again)) and torch.equal(history, again)
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,head_dim,d_rel,taps", [(1, 64, 16, 128, 16, 4), (7, 64, 8, 128, 16, 4), (2, 3, 3, 64, 8, 3), (3, 4, 1, 256, 6, 4),
+                                                                     (1, 2, 1, 8, 300, 2), (2, 1, 1, 40, 16, 4)])
+def test_heads_between_projection_and_attention(ib, device, batch, heads, kv_heads, head_dim, d_rel, taps):
+    """The same bits as the split, the norms, the convolutions and the copies one by one."""
+    gen = torch.Generator().manual_seed(head_dim + heads)
+    sizes = [heads * head_dim, kv_heads * head_dim, kv_heads * head_dim, heads * d_rel]
+    qkvr = torch.randn(batch, sum(sizes), generator=gen).to(BF16).to(device)
+    q_weight, k_weight = (torch.randn(head_dim, generator=gen).to(BF16).to(device) for _ in range(2))
+    (k_taps, k_history), (v_taps, v_history) = (_conv(gen, device, batch, kv_heads * head_dim, taps) for _ in range(2))
+    kh, vh = k_history.clone(), v_history.clone()
+    got = ib.kernels.attention_heads(qkvr, q_weight, k_weight, k_taps, v_taps, k_history, v_history, cases.EPS, heads, kv_heads, head_dim, d_rel)
+    q, k, v, r = qkvr.split(sizes, dim=-1)
+    q = ib.kernels.rmsnorm(q.reshape(-1, head_dim).contiguous(), q_weight, cases.EPS).view(batch, heads, head_dim)
+    k = ib.kernels.short_conv(k.unsqueeze(1).contiguous(), k_taps, kh)
+    k = ib.kernels.rmsnorm(k.view(-1, head_dim), k_weight, cases.EPS).view(batch, kv_heads, head_dim)
+    v = ib.kernels.short_conv(v.unsqueeze(1).contiguous(), v_taps, vh).view(batch, kv_heads, head_dim)
+    for a, b in zip(got, (q, k, v, r.reshape(batch, heads, d_rel))):
+        assert torch.equal(a, b)
+    assert torch.equal(k_history, kh) and torch.equal(v_history, vh)
+
+
+# rows fewer and more than blocks, at the edges of a consumer's sixteen, in one round and several; columns at the edges of a stage
+@pytest.mark.parametrize("n,k", [(1, 32), (8, 256), (149, 288), (2377, 64), (17, 4096), (100, 4128), (33, 8192), (11841, 1024), (24000, 96)])
+@pytest.mark.parametrize("tokens", [1, 2, 5, 8])
+def test_a_projection_against_64_bits(ib, device, n, k, tokens):
+    """Exact products; FP32 sums of k of them, each off by at most 2^-23 of the magnitudes so far, and one rounding to BF16 (two
+    with the factor, of which the second is of a value that the first may have moved)."""
+    gen = torch.Generator().manual_seed(n + k + tokens)
+    x, w = torch.randn(tokens, k, generator=gen).to(BF16).to(device), (torch.randn(n, k, generator=gen) * 0.05).to(BF16).to(device)
+    scale = torch.tensor([1.375]).to(BF16).to(device)
+    exact, magnitude = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    for factor, got in ((1.0, ib.kernels.linear(x, w)), (1.375, ib.kernels.linear(x, w, scale))):
+        bound = (1 if factor == 1.0 else 2.01) * 2.0 ** -8 * (exact * factor).abs() + factor * k * 2.0 ** -23 * magnitude
+        assert got.shape == (tokens, n) and bool(((got.double() - exact * factor).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n,k,tokens", [(4, 64, 1), (5, 512, 8), (1187, 96, 3), (6, 4128, 2), (3, 8192, 7), (5921, 288, 4), (13000, 32, 1)])
+def test_a_gated_projection_rounds_as_the_tensor_operations_do(ib, device, n, k, tokens):
+    """The two projections have the sums of `linear`, checked above; what follows has one outcome."""
+    gen = torch.Generator().manual_seed(n * k)
+    x = torch.randn(tokens, k, generator=gen).to(BF16).to(device)
+    gate, up = ((torch.randn(n, k, generator=gen) * 1.5 / k ** 0.5).to(BF16).to(device) for _ in range(2))
+    want = torch.nn.functional.silu(ib.kernels.linear(x, gate)) * ib.kernels.linear(x, up)
+    assert torch.equal(ib.kernels.gated(x, gate, up), want)
+
+
+def test_a_projection_in_a_chain_sees_what_the_kernel_in_front_wrote(ib, device):
+    """Weights are asked for before the kernel in front has finished, the activations not: twenty in a row against one by one."""
+    gen = torch.Generator().manual_seed(2)
+    ws = [(torch.randn(2048, 2048, generator=gen) * 0.03).to(BF16).to(device) for _ in range(20)]
+    x = torch.randn(3, 2048, generator=gen).to(BF16).to(device)
+    one_by_one = x
+    for w in ws:
+        one_by_one = ib.kernels.linear(one_by_one, w)
+        torch.cuda.synchronize()
+    for _ in range(3):
+        y = x
+        for w in ws:
+            y = ib.kernels.linear(y, w)
+        assert torch.equal(y, one_by_one)
+
+
+@pytest.mark.parametrize("n,k,tokens", [(11264, 4096, 1), (4096, 8192, 7), (8192, 4096, 3)])
+def test_a_layers_projections_are_the_bits_of_a_plain_gemm(ib, device, n, k, tokens):
+    gen = torch.Generator(device=device).manual_seed(n)
+    x, w = torch.randn(tokens, k, generator=gen, device=device).to(BF16), (torch.randn(n, k, generator=gen, device=device) * 0.02).to(BF16)
+    assert torch.equal(ib.kernels.linear(x, w), torch.nn.functional.linear(x, w))

@@ -1,0 +1,91 @@
+"""Which calls of the dense projections the kernel takes: those it cannot, and those where more than the values is asked for, stay
+tensor operations. No GPU: the launch is replaced."""
+import sys
+
+import pytest
+import torch
+import torch.nn.functional as F
+from torch.utils.flop_counter import FlopCounterMode
+
+from inkling_b200.kernels import gated, linear
+
+module = sys.modules[linear.__module__]
+BF16 = torch.bfloat16
+
+
+@pytest.fixture
+def launched(monkeypatch):
+    """The kernel's operands are on the GPU: here the check of the device is left out and the launch noted."""
+    calls = []
+
+    def launch(x, weight, up, scale):
+        calls.append((x, weight, up, scale))
+        y = F.linear(x, weight) if up is None else F.silu(F.linear(x, weight)) * F.linear(x, up)
+        return y if scale is None else y * scale
+
+    fits = module._fits
+
+    class OnGpu:
+        def __init__(self, t):
+            self.t = t
+
+        is_cuda = True
+
+        def __getattr__(self, name):
+            return getattr(self.t, name)
+
+    monkeypatch.setattr(module, "_fits", lambda *t: fits(*(OnGpu(v) for v in t)))
+    monkeypatch.setattr(module, "_launch", launch)
+    return calls
+
+
+def operands(tokens=3, n=24, k=64, dtype=BF16):
+    gen = torch.Generator().manual_seed(0)
+    return torch.randn(tokens, k, generator=gen).to(dtype), torch.randn(n, k, generator=gen).to(dtype)
+
+
+def test_what_the_kernel_takes(launched):
+    x, w = operands()
+    for shape in ((3, 64), (3, 1, 64), (1, 3, 64)):
+        assert linear(x.view(shape), w).shape == (*shape[:-1], 24)
+    assert linear(operands(8)[0], w, torch.ones(1, dtype=BF16)).shape == (8, 24)
+    gated(x, w, w)
+    assert len(launched) == 5
+
+
+@pytest.mark.parametrize("x,w,scale", [
+    (operands(9)[0], operands()[1], None),                                       # more tokens
+    (*operands(dtype=torch.float32), None), (*operands(k=48), None), (*operands(n=2, k=8224), None),
+    (operands()[0][:0], operands()[1], None), (operands()[0].t().contiguous().t(), operands()[1], None),
+    (operands()[0], operands()[1].t().contiguous().t(), None),
+    (torch.randn(3 * 64 + 1).to(BF16)[1:].view(3, 64), operands()[1], None),     # off the 16-byte boundary
+    (*operands(), torch.ones((), dtype=BF16)), (*operands(), torch.ones(1)), (*operands(), torch.ones(24, dtype=BF16)),
+])
+def test_what_it_does_not_take(launched, x, w, scale):
+    got = linear(x, w, scale)
+    want = F.linear(x, w) if scale is None else F.linear(x, w) * scale
+    assert not launched and torch.equal(got, want) and got.dtype == want.dtype
+
+
+def test_gradients_transforms_modes_and_subclasses_are_left_to_tensor_operations(launched):
+    x, w = operands()
+    grown = x.clone().requires_grad_()
+    linear(grown, w).sum().backward()
+    assert grown.grad is not None
+    gated(x, w.clone().requires_grad_(), w).sum().backward()
+    assert torch.equal(torch.vmap(linear, in_dims=(0, None))(x, w), F.linear(x, w))
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+        assert torch.autograd.forward_ad.unpack_dual(linear(dual, w)).tangent is not None
+    with FlopCounterMode(display=False) as flops:
+        linear(x, w)
+    assert flops.get_total_flops() == 2 * 3 * 24 * 64
+
+    class Seen(torch.Tensor):
+        pass
+
+    assert type(linear(x.as_subclass(Seen), w)) is Seen
+    assert not launched
+    with torch.no_grad():
+        linear(grown, w)   # no gradient is asked for
+    assert len(launched) == 1
