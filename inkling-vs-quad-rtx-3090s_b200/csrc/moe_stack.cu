@@ -1018,6 +1018,10 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         return true;
       };
       int layer = 0, t = lane;   // the tile to copy
+      while (plan.per_layer > 0 && t >= plan.per_layer) {   // (no shared experts: a layer may have fewer tiles than the ring slots)
+        t -= plan.per_layer;
+        ++layer;
+      }
       long long i = lane;        // its index in the block's whole sequence
       int asked = -1;            // (trace) the last layer whose routing this lane asked for
       long long stalled_since = clock64();

@@ -216,3 +216,19 @@ def test_wait_that_runs_out_is_reported_and_recovered(ib, device):
     torch.cuda.synchronize()
     desc.check_status()
     assert torch.equal(again, good)
+
+
+@pytest.mark.parametrize("d,f,experts,n_shared,top_k", [(2048, 256, 64, 0, 1), (1024, 512, 64, 0, 6), (2048, 256, 64, 1, 1), (4096, 256, 300, 0, 8)])
+def test_layers_of_fewer_tiles_than_ring_slots(ib, device, d, f, experts, n_shared, top_k):
+    """The stack's second and third block against the same blocks one by one: the sums that enter a block's norm, each step from
+    what the kernel itself was fed (a prefix of the stack)."""
+    x = torch.randn(1, d, generator=torch.Generator().manual_seed(d + f)).to(BF16).to(device)
+    normed = x
+    for n in (1, 2, 3):
+        stack = ib.MoEStack.synthetic(n, d, f, experts, n_shared, top_k, device, seed=3, bias_std=0.05)
+        out = stack(x).clone()
+        stack._fused.check_status()
+        got = stack.layers[-1].partial[:1].clone()
+        alone = stack.layers[-1](normed.unsqueeze(0)).view(1, d)      # the block by itself, on what the stack fed it
+        assert max_rel(got, alone.float()) <= 1.6e-2, n
+        normed = out
