@@ -40,12 +40,6 @@ struct AttnArgs {
   float alpha, scale;
 };
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
-}
-
 // the two floats cut off to BF16
 __device__ __forceinline__ uint32_t high_halves(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 

@@ -72,6 +72,23 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float v) {
 }
 __device__ __forceinline__ float round_bf16(float v) { return bf16_to_f32(f32_to_bf16_bits(v)); }
 
+// two floats to BF16, each rounded as above; sums and products of two BF16 pairs, each rounded once
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
 // ------------------------------------------------------------------ packed converts
 // four bytes of E2M1 codes (8 weights, low nibble first) -> four f16x2 registers
 __device__ __forceinline__ void e2m1x8_to_f16x2(uint32_t w, uint32_t (&h)[4]) {

@@ -14,8 +14,8 @@
 // (shared gate/up done, routed gate/up done); the weight stream itself never stops at them,
 // because weight addresses do not depend on activations. Counters only grow: every target is a
 // multiple of the number of launches so far, nothing is cleared, comparisons are modulo 2^32.
-// What one block hands to all others in small pieces -- router scores, output rows -- travels
-// as 8-byte words {FP32 value, tag of this launch and layer}: the reader polls the word it is
+// What one block hands to all others in small pieces -- router scores, output rows, narrow experts' activations -- travels
+// as 8-byte words {value or two BF16 values, tag of this launch and layer}: the reader polls the word it is
 // about to use, so there is no fence, no counter and no last-arrival serialisation on that
 // path, within a GPU and across GPUs alike (an aligned 8-byte store is one transaction).
 //
@@ -51,6 +51,13 @@ constexpr int kSMaxRows = 64;                          // output rows one block 
 constexpr int kSMaxExperts = 512;
 constexpr int kSyncWordsPerLayer = 8;                  // counters of one layer
 constexpr int kSMaxWorld = 8;                          // tensor-parallel ranks
+// Copies of every tagged word: a line that all blocks poll is served 148 times a round by one slice of the L2, and the stores to it
+// wait in that line; block b polls copy b % kCopies. (40 blocks of 4096 x 256: 815 us with one copy, 778 with eight.)
+constexpr int kCopies = 8;
+// A line that is polled before it is written makes the writing slower, so a poll is late rather than early, and seldom: the routing
+// warp looks for the scores of all blocks this long after its own block has published its own, and a poll that finds something missing pauses
+// (the same stack: no first wait 783 us, 250 ns 762, 500 ns 752, 900 ns 754; pauses of the routing warp of 100 ns instead of 500 with no first wait +40 us).
+constexpr unsigned kFirstLook = 600, kPollPause = 250;
 constexpr int kTileCountersPerLayer = kSMaxTopK * 32 + 32;   // routed gate/up tiles (at most 8 x 32), then down row tiles
 
 constexpr int kTraceBlocks = 256;
@@ -74,14 +81,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+// (a kernel of its own stamps: in the one that runs, the stamps were code that no cache close to the schedulers holds; eight blocks of
+// 4096 x 2048 385 us with them, switched off, 381 without; forty of 4096 x 256 752 and 740)
 #define INK_TRACE_VALUE(layer, slot, value)                                                             \
   do {                                                                                                  \
-    if (a.trace && blockIdx.x < kTraceBlocks)                                                           \
+    if (kTrace && a.trace && blockIdx.x < kTraceBlocks)                                                           \
       a.trace[((size_t)(layer) * kTraceBlocks + blockIdx.x) * kTraceSlots + (slot)] = (value);          \
   } while (0)
 #define INK_TRACE(layer, slot)                                                                          \
   do {                                                                                                  \
-    if (a.trace && blockIdx.x < kTraceBlocks)                                                           \
+    if (kTrace && a.trace && blockIdx.x < kTraceBlocks)                                                           \
       a.trace[((size_t)(layer) * kTraceBlocks + blockIdx.x) * kTraceSlots + (slot)] = global_ns();      \
   } while (0)
 
@@ -133,7 +142,7 @@ struct StackArgs {
   uint16_t* residual;              // [2][hidden] BF16: slot 0 holds the incoming residual stream (glue mode)
   uint16_t* normed_out;            // [hidden] BF16 output of the last norm (glue mode); else the block's output in BF16, or null
   float* partial;                  // [hidden] FP32 output of the (last) block
-  unsigned long long* scores;      // scratch [2][experts + n_shared] router words {selection score, BF16 logit, 16-bit tag}
+  unsigned long long* scores;      // scratch [2][kCopies][experts + n_shared] router words {selection score, BF16 logit, 16-bit tag}
   uint16_t* activated;             // scratch [2][top_k][f]
   uint16_t* shared_activated;      // scratch [2][n_shared][f]
   RouteTable* routes;              // scratch [n_layers]
@@ -197,7 +206,8 @@ struct StackShape {
   static constexpr int GU_CHUNKS = D / kTcChunkK;           // units per tile
   static constexpr int DN_TILES = D / kTcRows;              // 128-row tiles of the down projection per expert
   static constexpr int DN_CHUNKS = F / kTcChunkK;
-  static constexpr int STAGING_A = kSMaxTopK * F * 2 + kSMaxShared * F * 2;
+  // (narrow experts: behind x, so that a warp may stage activations while others are still at their gate/up tiles)
+  static constexpr int STAGING_A = (F <= 512 ? D * 4 : 0) + kSMaxTopK * F * 2 + kSMaxShared * F * 2;
   // tensor-core variant: the shared experts' activations are staged while the digit rows of x are still
   // being read, so they sit behind both digit-row areas
   static constexpr int TC_SACT = D * 6 > F * 16 ? D * 6 : F * 16;
@@ -294,12 +304,14 @@ struct StackShared {
   long long limit;                      // SM clocks a wait may take
   unsigned pause;                       // nanoseconds between two polls of a word that other blocks write
   volatile int rows_seen;               // layers whose summed output rows consumer warp 0 has seen arrive
-  volatile int routed_layers;           // layers whose routing table is in `routes` (set by the auxiliary warp)
+  volatile int routed_layers;           // layers whose choices (addresses, scale2) are in `routes` (set by the auxiliary warp)
+  volatile int weighted_layers;         // layers whose weights and gammas are there too
   volatile int seen[2];                 // layers whose grid-wide counters (shared gate/up, routed gate/up) the auxiliary
                                         // warp has seen complete: one poller per block instead of one per warp
   volatile int sact_flag[kSMaxShared];  // layers whose shared-expert activations are staged, per shared expert
   volatile int act_flag[kSMaxTopK];     // layers whose routed activations are staged, per route
   volatile int failed;
+  int own_rows;                         // router rows this block has published, in all layers
   volatile int consts_layers;           // layers whose routing constants have been loaded into `consts` (set by the auxiliary warp)
   RouteConsts consts;
   // tensor-core path
@@ -387,6 +399,12 @@ __device__ __forceinline__ unsigned long long ld_tagged_sys(const unsigned long 
 __device__ __forceinline__ void ld_tagged2(const unsigned long long* p, unsigned long long (&v)[2]) {   // 16-byte aligned pair
   asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "l"(p) : "memory");
 }
+__device__ __forceinline__ void ld_tagged2_sys(const unsigned long long* p, unsigned long long (&v)[2]) {   // the same, written by a peer
+  asm volatile("ld.relaxed.sys.global.v2.b64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_word(unsigned long long* p, uint32_t value, unsigned tag) {   // one or two BF16 values
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)value | ((unsigned long long)tag << 32)) : "memory");
+}
 __device__ __forceinline__ bool has_tag(unsigned long long word, unsigned tag) { return (unsigned)(word >> 32) == tag; }
 __device__ __forceinline__ float value_of(unsigned long long word) { return __uint_as_float((unsigned)word); }
 // The tag of a layer of a launch. Never zero before the epoch wraps, so a zero-filled buffer matches nothing.
@@ -415,15 +433,50 @@ __device__ __forceinline__ float wait_tagged(const unsigned long long* p, unsign
   return 0.f;
 }
 
-// Bounded wait until this block's auxiliary warp has resolved the routing of `layer`.
+// One warp: K activations that other blocks publish as words of PER (one or two) BF16 values; lane l gets the groups n * 32 + l of
+// eight. All words of a round are asked for at once. Zeros once the launch has failed.
+template <int K, int PER>
+__device__ __forceinline__ void warp_take_words(const unsigned long long* words, unsigned tag, uint4 (&v)[K / 256], StackShared* sh, int lane) {
+  constexpr int N = K / 256, W = 8 / PER;
+  unsigned long long w[N][W];
+  const long long t0 = clock64();
+  bool there;
+  for (;;) {
+    there = true;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+      for (int i = 0; i < W; i += 2) {
+        unsigned long long pair[2];
+        ld_tagged2(words + (size_t)(n * 32 + lane) * W + i, pair);
+        w[n][i] = pair[0];
+        w[n][i + 1] = pair[1];
+        there = there && has_tag(pair[0], tag) && has_tag(pair[1], tag);
+      }
+    there = __all_sync(0xffffffffu, there);
+    if (there || __any_sync(0xffffffffu, sh->failed != 0)) break;
+    if (clock64() - t0 > sh->limit) sh->failed = 1;
+    __nanosleep(sh->pause);
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    uint32_t p[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      p[i] = !there ? 0u : PER == 2 ? (uint32_t)w[n][i % W] : __byte_perm((uint32_t)w[n][(2 * i) % W], (uint32_t)w[n][(2 * i + 1) % W], 0x5410);
+    v[n] = make_uint4(p[0], p[1], p[2], p[3]);
+  }
+}
+
+// Bounded wait until this block's auxiliary warp has resolved the routing of `layer`, weights and all.
 __device__ __forceinline__ bool wait_routing(int layer, StackShared* sh) {
   if (sh->failed) return false;
-  if (sh->routed_layers > layer) {
+  if (sh->weighted_layers > layer) {
     __threadfence_block();
     return true;
   }
   const long long t0 = clock64();
-  while (sh->routed_layers <= layer) {
+  while (sh->weighted_layers <= layer) {
     if (sh->failed) return false;
     if (clock64() - t0 > sh->limit) {
       sh->failed = 1;
@@ -513,31 +566,27 @@ __device__ __forceinline__ bool poll_router_words(const StackArgs& a, const unsi
                                                   float (&sc)[K], StackShared* sh) {
   const int lane = threadIdx.x & 31;
   float* logit = sh->logit;
-  const unsigned long long found = (unsigned long long)tag16 << 48;   // stands for a row this lane does not have
-#pragma unroll
-  for (int i = 0; i < K; ++i) sc[i] = -INFINITY;
   unsigned long long w[K];
-  unsigned missing = 0;
 #pragma unroll
-  for (int i = 0; i < K; ++i)
-    if (i * 32 + lane < rows) missing |= 1u << i;
+  for (int i = 0; i < K; ++i) w[i] = i * 32 + lane < rows ? 0ull : (unsigned long long)tag16 << 48;   // (a row this lane does not have)
   const long long t0 = clock64();
-  for (;;) {
+  for (;;) {   // (as few instructions as can be: two consumer warps share the scheduler)
+    bool there = true;
 #pragma unroll
-    for (int i = 0; i < K; ++i) w[i] = (missing >> i) & 1u ? ld_tagged(words + i * 32 + lane) : found;
+    for (int i = 0; i < K; ++i)
+      if ((unsigned)(w[i] >> 48) != tag16) w[i] = ld_tagged(words + i * 32 + lane);
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const int e = i * 32 + lane;
-      if (((missing >> i) & 1u) && (unsigned)(w[i] >> 48) == tag16) {
-        if (e < a.experts) sc[i] = __uint_as_float((unsigned)w[i]);
-        logit[e] = __uint_as_float((unsigned)(w[i] >> 32) << 16);
-        missing &= ~(1u << i);
-      }
-    }
-    if (__all_sync(0xffffffffu, missing == 0)) break;
-    if (sh->failed) return false;
+    for (int i = 0; i < K; ++i) there = there && (unsigned)(w[i] >> 48) == tag16;
+    if (__all_sync(0xffffffffu, there)) break;
+    if (__any_sync(0xffffffffu, sh->failed != 0)) return false;
     if (clock64() - t0 > sh->limit) sh->failed = 1;
     __nanosleep(sh->pause);
+  }
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const int e = i * 32 + lane;
+    sc[i] = e < a.experts ? __uint_as_float((unsigned)w[i]) : -INFINITY;
+    if (e < rows) logit[e] = __uint_as_float((unsigned)(w[i] >> 32) << 16);
   }
   return !sh->failed;
 }
@@ -576,14 +625,24 @@ __device__ __forceinline__ int select_top_k(float (&sc)[K], int top_k) {
 
 // One warp. Waits for the layer's scores as the blocks publish them (router words), then
 // resolves the routing. Returns false if the launch failed while waiting.
-__device__ bool stack_router_tail(const StackArgs& a, const StackLayer& ly, int layer, StackShared* sh) {
+template <bool kTrace>
+__device__ bool stack_router_tail(const StackArgs& a, const StackLayer& ly, int layer, int own_rows, StackShared* sh) {
   const int lane = threadIdx.x & 31;
   const int par = layer & 1;
   const unsigned tag16 = router_tag(layer_tag(sh->epoch1, a.n_layers, layer));
   const int rows = a.experts + a.n_shared;
-  const unsigned long long* words = a.scores + (size_t)par * rows;
+  const unsigned long long* words = a.scores + ((size_t)par * kCopies + blockIdx.x % kCopies) * rows;
   const float* logit = sh->logit;
   int my_choice;
+  {   // this block's own rows first: the others' are not earlier (see kFirstLook)
+    const long long t0 = clock64();
+    while (*(volatile int*)&sh->own_rows < own_rows && !sh->failed) {
+      if (clock64() - t0 > sh->limit) sh->failed = 1;
+      __nanosleep(64);
+    }
+    __syncwarp();
+    __nanosleep(kFirstLook);
+  }
   constexpr int kFew = 9, kMany = (kSMaxExperts + kSMaxShared + 31) / 32;   // router rows per lane: up to 288, up to 514
   if (rows <= kFew * 32) {
     float sc[kFew];
@@ -597,6 +656,24 @@ __device__ bool stack_router_tail(const StackArgs& a, const StackLayer& ly, int 
     my_choice = select_top_k<kMany>(sc, a.top_k);
   }
   __syncwarp();
+  const RouteConsts& c = sh->consts;    // loaded for this layer before the scores could be complete (see the caller)
+  RouteTable* table = &sh->routes[layer & 1];
+  if (lane < a.top_k) {   // what the weight stream waits for first; the weights are needed by the down projection only
+    RouteEntry& r = table->route[lane];
+    r.gu_codes = c.bank[my_choice][0];
+    r.gu_scales = c.bank[my_choice][1];
+    r.gu_scale2 = c.gu_scale2[my_choice];
+    r.dn_codes = c.bank[my_choice][2];
+    r.dn_scales = c.bank[my_choice][3];
+    r.dn_scale2 = c.dn_scale2[my_choice];
+    r.expert = my_choice;
+  }
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence_block();
+    sh->routed_layers = layer + 1;   // the producer and the consumers of this block may read them
+    INK_TRACE(layer, kTrXVisible);   // (CUDA-core variant: the routing is resolved)
+  }
   const int n = a.top_k + a.n_shared;
   const bool live = lane < n;
   float l = 0.f;
@@ -613,29 +690,14 @@ __device__ bool stack_router_tail(const StackArgs& a, const StackLayer& ly, int 
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   const float lse = round_bf16(round_bf16(__logf(round_bf16(s))) + m);
   float w = round_bf16(__expf(round_bf16(lp - lse)));
-  const RouteConsts& c = sh->consts;    // loaded for this layer before the scores could be complete (see the caller)
   w = round_bf16(w * c.route_scale);
   w = round_bf16(w * c.global_scale);
-  RouteTable* table = &sh->routes[layer & 1];
-  if (lane < a.top_k) {
-    RouteEntry r;
-    r.gu_codes = c.bank[my_choice][0];
-    r.gu_scales = c.bank[my_choice][1];
-    r.gu_scale2 = c.gu_scale2[my_choice];
-    r.dn_codes = c.bank[my_choice][2];
-    r.dn_scales = c.bank[my_choice][3];
-    r.dn_scale2 = c.dn_scale2[my_choice];
-    r.weight = w;
-    r.expert = my_choice;
-    table->route[lane] = r;
-  } else if (live) {
-    table->gamma[lane - a.top_k] = w;
-  }
+  if (lane < a.top_k) table->route[lane].weight = w;
+  else if (live) table->gamma[lane - a.top_k] = w;
   __syncwarp();
   if (lane == 0) {
     __threadfence_block();
-    sh->routed_layers = layer + 1;   // the producer and the consumers of this block may read the table
-    INK_TRACE(layer, kTrXVisible);   // (CUDA-core variant: the routing is resolved)
+    sh->weighted_layers = layer + 1;
   }
   if (blockIdx.x == 0) {   // one block also writes the optional router outputs (off the critical path)
     if (lane < a.top_k) {
@@ -795,6 +857,39 @@ __device__ __forceinline__ void gather_row(const StackArgs& a, StackShared* sh, 
   if (!sh->failed) st_tagged(a.summed + (size_t)xpar * D + row, sum, tag);
 }
 
+// The same for two neighbouring rows on the CUDA cores: the sums, or zeros once the launch has failed.
+template <int D>
+__device__ __forceinline__ float2 gather_pair(const StackArgs& a, StackShared* sh, int xpar, unsigned tag, int row) {
+  const unsigned long long* from = a.inbox + (size_t)xpar * a.world * D + row;
+  unsigned long long w[kSMaxWorld][2];
+  bool all = true;
+  auto ask = [&](int r) {
+    ld_tagged2_sys(from + (size_t)r * D, w[r]);
+    all = all && has_tag(w[r][0], tag) && has_tag(w[r][1], tag);
+  };
+#pragma unroll
+  for (int r = 0; r < kSMaxWorld; ++r)
+    if (r < a.world) ask(r);
+  const long long t0 = clock64();
+  while (!all && !sh->failed) {
+    __nanosleep(64);
+    all = true;
+#pragma unroll
+    for (int r = 0; r < kSMaxWorld; ++r)
+      if (r < a.world && !(has_tag(w[r][0], tag) && has_tag(w[r][1], tag))) ask(r);
+    if (clock64() - t0 > sh->limit) sh->failed = 1;
+  }
+  float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < kSMaxWorld; ++r) {
+    if (r < a.world) {
+      sum.x += value_of(w[r][0]);
+      sum.y += value_of(w[r][1]);
+    }
+  }
+  return all ? sum : make_float2(0.f, 0.f);
+}
+
 // Tensor-core variant: every part of row tile `tile` (the routed projections' parts and the shared
 // experts' rows) is in global memory. Sums them in a fixed order -- the parts of a route in block
 // order, the routes in choice order, then the shared experts -- and stores the rows into every
@@ -846,7 +941,7 @@ __device__ __forceinline__ void finish_row_tile(const StackArgs& a, StackShared*
   if (a.world > 1)
     for (int row = first; row < kTcRows; row += stride) gather_row<D>(a, sh, xpar, tag, tile * kTcRows + row);
 }
-template <int D, int F, bool TC>
+template <int D, int F, bool TC, bool kTrace>
 __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_kernel(StackArgs a) {
   using S = StackShape<D, F>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -854,17 +949,24 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // TC: the layers carry TMA descriptors and the routed experts run on the tensor cores
   constexpr bool tc = TC;
+  // The activations of narrow experts travel as tagged words, like the scores and the output rows: the warp that stages an expert
+  // polls the words themselves. With a counter there are a fence, the counter's own round trip, a flag and the loads in a chain
+  // (a block of 4096 x 256: 5.9 us from a block's last gate/up tile to its staged activations, 2.3 so). Wide experts' 16 384 values are too many
+  // for every block to poll.
+  constexpr bool kWordActs = !TC && F <= 512;
   unsigned char* slots = smem + ((1024u - (smem_u32(smem) & 1023u)) & 1023u);   // swizzled tiles need 1024-byte alignment
   unsigned char* staging = slots + kSStages * kSSlot;
   uint16_t* s_x16 = reinterpret_cast<uint16_t*>(staging);            // [D] FP16 normalised (gate/up phases, CUDA-core path)
   unsigned char* s_xdig = staging;                                    // [D/256][8 rows][128 B] digit rows of x (tensor-core path)
   uint16_t* s_xbf = reinterpret_cast<uint16_t*>(staging + (tc ? D * 4 : D * 2));   // [D] BF16
-  uint16_t* s_act = reinterpret_cast<uint16_t*>(staging);            // [top_k][F] FP16 normalised (down phases)
+  uint16_t* s_act = reinterpret_cast<uint16_t*>(staging + (kWordActs ? D * 4 : 0));   // [top_k][F] FP16 normalised (down phases)
   unsigned char* s_adig = staging;                                    // [F/256][32 rows][128 B] digit rows of the routed activations
   uint16_t* s_sact = tc ? reinterpret_cast<uint16_t*>(staging + S::TC_SACT)
                         : s_act + (size_t)kSMaxTopK * F;              // [n_shared][F] BF16 (act * gamma)
   const TilePlan plan = make_plan<D, F>(a, tc);
-  const int total_rows = a.experts + a.n_shared;
+  const int total_rows = a.experts + a.n_shared, my_copy = blockIdx.x % kCopies;
+  // the output rows' words: FP32 each on the tensor cores; two BF16 values each, in copies, on the CUDA cores
+  constexpr size_t kRowWords = TC ? D : (size_t)kCopies * (D / 2);
   const int n_jobs = a.top_k + a.n_shared;
 
   if (threadIdx.x == 0) {
@@ -884,7 +986,8 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
     sh.act_ready = 0;
     sh.sg_done = 0;
     sh.issued = 0;
-    sh.routed_layers = 0;
+    sh.routed_layers = sh.weighted_layers = 0;
+    sh.own_rows = 0;
     sh.consts_layers = 0;
     for (int i = 0; i < 2; ++i) sh.seen[i] = 0;
     for (int i = 0; i < kSMaxShared; ++i) sh.sact_flag[i] = 0;
@@ -1062,7 +1165,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         } else if (more && clock64() - stalled_since > sh.limit) {
           sh.failed = 1;   // nothing for this lane within the limit: every wait of the launch gives up
         }
-        if (a.trace && lane == 0 && more) {   // cycles with a tile to issue, its routing known, but the slot still in use
+        if (kTrace && lane == 0 && more) {   // cycles with a tile to issue, its routing known, but the slot still in use
           const long long now = clock64();
           const bool routing_known = !((t >= plan.s_qg && t < plan.s_sd) || (t >= plan.s_qd && t < plan.s_pad)) || sh.routed_layers > layer;
           if (!ready && routing_known) slot_wait += now - looked_at;
@@ -1256,13 +1359,20 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       const unsigned* sync = a.sync + (size_t)layer * kSyncWordsPerLayer;
       // every block resolves the routing for itself (same inputs, same arithmetic, same result): the
       // code stays warm in this SM's instruction cache and nothing has to be published between blocks
-      if (!stack_router_tail(a, a.layers[layer], layer, &sh)) break;
+      if (!stack_router_tail<kTrace>(a, a.layers[layer], layer, (layer + 1) * plan.n_r, &sh)) break;
       // The constants of this layer are in the route table now; the next layer's are fetched while this one streams: on
       // the CUDA-core path after the counters below, which blocks are waiting for (40 layers of 2048 x 256: 837.8 us with the
       // loads in front of them, 827.9 so; of 4096 x 256: 959.6, 958.2); nobody needs the constants before the next layer starts.
       // (The consumers read this layer's biases only before they publish its scores, i.e. before this point.)
       if (tc && layer + 1 < a.n_layers) load_route_consts(a, layer + 1, &sh);
-      if (!tc && lane == 0) {
+      if (kWordActs) {
+        wait_flag(&sh.act_flag[a.top_k - 1], layer, &sh, lane);   // nobody waits for memory now
+        // Without shared experts a block may have nothing to add to a layer: nobody may be two layers ahead of it, since it reads words that
+        // the next layer but one overwrites. (The next layer's scores wait for the constants below.) And the last block to know the launch's
+        // number must have started before block 0 counts it up.
+        if (lane == 0 && (a.n_shared == 0 || (layer == 0 && blockIdx.x == 0))) wait_global(sync + kShGuDone, sh.epoch1 * gridDim.x, &sh);
+        __syncwarp();
+      } else if (!tc && lane == 0) {
         // One lane polls the layer's grid-wide counters for the whole block and raises a flag in shared memory
         // for each: eight polling warps per block crowd the counter's L2 line and hold up its increments.
         const unsigned epoch1 = sh.epoch1;
@@ -1326,7 +1436,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
     }
   } else if (warp <= kSC) {
     // =========================================================== consumers
-    const int cw = warp - 1, ct = threadIdx.x - 32;
+    const int cw = (warp + kSC - 2) % kSC, ct = threadIdx.x - 32;   // (a layer's first tiles, the router's rows, go to warps 2 and 3: the auxiliary warp is on warp 1's scheduler)
     constexpr int VG = VecShape<D>::VG, VT = VecShape<D>::VT;   // groups of eight elements per thread, threads that hold some
     const bool holder = ct < VT;
 
@@ -1344,9 +1454,9 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         if (ok && lane == 0) ok = tc_wait_issued(i, &sh);
         ok = __all_sync(0xffffffffu, ok);
       }
-      const long long wait_from = a.trace ? clock64() : 0;
+      const long long wait_from = kTrace ? clock64() : 0;
       if (ok) ok = mbar_wait(&sh.full[slot], (uint32_t)(i / kSStages) & 1, sh.limit);
-      if (a.trace) {
+      if (kTrace) {
         tile_from = clock64();
         waited += tile_from - wait_from;
       }
@@ -1361,7 +1471,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
     auto release = [&](int slot) {
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh.empty[slot]);
-      if (a.trace) busy += clock64() - tile_from;
+      if (kTrace) busy += clock64() - tile_from;
     };
     // one more tile of `section` (0 shared g/u, 1 routed g/u, 2 down) of this block is done;
     // returns true in the warp that finished the section's last tile
@@ -1428,7 +1538,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       float amax = bf16_to_f32(amax_bits);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      if (lane == 0) sh.red[cw][0] = amax;
+      if (lane == 0) sh.red[warp - 1][0] = amax;
       consumer_sync();
       amax = 0.f;
       for (int w = 0; w < kSC; ++w) amax = fmaxf(amax, sh.red[w][0]);
@@ -1436,6 +1546,10 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       consumer_sync();
     }
 
+    // the residual stream, in the layout of the vector above: every block keeps it
+    uint4 res[VG];
+#pragma unroll
+    for (int g = 0; g < VG; ++g) res[g] = a.glue && holder ? reinterpret_cast<const uint4*>(a.residual)[g * VT + ct] : make_uint4(0, 0, 0, 0);
     for (int layer = 0; layer < a.n_layers; ++layer, base += plan.per_layer) {
       const uint16_t* norm_weight = a.layers[layer].norm_weight;
       unsigned* sync = a.sync + (size_t)layer * kSyncWordsPerLayer;
@@ -1445,12 +1559,12 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       const int xpar = (int)(((epoch1 - 1u) * (unsigned)a.n_layers + (unsigned)layer) & 1u);
       const unsigned tag = layer_tag(epoch1, a.n_layers, layer);
       const float x_inverse = sh.x_inverse;
-      const bool tracer = (ct == 0);
+      const bool tracer = kTrace && ct == 0;
       if (tracer) INK_TRACE(layer, kTrLayerStart);
       // blocks that own no tile of a section still have to be counted
       if (ct == 0) {
-        if (plan.n_sg == 0) red_release_add(sync + kShGuDone, 1u);
-        if (plan.n_q == 0 && !tc) red_release_add(sync + kRtGuDone, 1u);   // (the tensor-core path counts tiles)
+        if (kWordActs ? layer == 0 || a.n_shared == 0 : plan.n_sg == 0) red_release_add(sync + kShGuDone, 1u);
+        if (plan.n_q == 0 && !tc && !kWordActs) red_release_add(sync + kRtGuDone, 1u);   // (the tensor-core path counts tiles)
       }
       // ------------------------------------------------ router rows
       if (plan.n_r > 0) wait_flag(&sh.consts_layers, layer, &sh, lane);   // the layer's biases (loaded a layer ahead)
@@ -1468,12 +1582,13 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
           acc = warp_sum(acc);
           release(slot);
           const int row = plan.r0 + t;
-          if (lane == 0) {   // one word per row: the routing warps of all blocks poll for them
+          if (lane < kCopies) {   // one word per row: the routing warps of all blocks poll for them
             const float l = round_bf16(acc);
             const float score = row < a.experts ? round_bf16(1.f / (1.f + __expf(-l))) + sh.consts.bias[row] : 0.f;
-            unsigned long long* at = a.scores + (size_t)par * total_rows + row;
+            unsigned long long* at = a.scores + ((size_t)par * kCopies + lane) * total_rows + row;
             asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(at), "l"(router_word(score, l, router_tag(tag))) : "memory");
           }
+          if (lane == 0) atomicAdd(&sh.own_rows, 1);
         } else {
           release(slot);
         }
@@ -1513,18 +1628,21 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
             if (h == S::SG_SPLIT - 1) {
               float gate = multi_reduce<S::SG_PAIRS>(g, lane);
               float up = multi_reduce<S::SG_PAIRS>(u, lane);
-              if (reduced_owner<S::SG_PAIRS>(lane)) {
+              constexpr int kGroup = 32 / S::SG_PAIRS;   // lanes that hold a pair's sums
+              static_assert(kGroup >= kCopies, "a lane per copy");
+              if (kWordActs ? lane % kGroup < kCopies : reduced_owner<S::SG_PAIRS>(lane)) {
                 gate = round_bf16(gate);
                 up = round_bf16(up);
                 const float act = round_bf16(gate / (1.f + expf(-gate)));
                 const int pair = (plan.u0 + unit) * S::SG_PAIRS + reduced_row<S::SG_PAIRS>(lane);  // over [n_shared * F]
-                a.shared_activated[(size_t)par * a.n_shared * F + pair] = (uint16_t)f32_to_bf16_bits(act * up);
+                if (kWordActs) st_word(reinterpret_cast<unsigned long long*>(a.shared_activated) + ((size_t)par * kCopies + lane % kGroup) * a.n_shared * F + pair, f32_to_bf16_bits(act * up), tag);
+                else a.shared_activated[(size_t)par * a.n_shared * F + pair] = (uint16_t)f32_to_bf16_bits(act * up);
               }
             }
           } else {
             release(slot);
           }
-          if (t + kSC >= plan.s_qg && warp_done(layer, 0, min(kSC, plan.n_sg), true) && lane == 0) red_release_add(sync + kShGuDone, 1u);
+          if (!kWordActs && t + kSC >= plan.s_qg && warp_done(layer, 0, min(kSC, plan.n_sg), true) && lane == 0) red_release_add(sync + kShGuDone, 1u);
         }
       }
       if (tracer) INK_TRACE(layer, kTrShGuDone);
@@ -1581,11 +1699,20 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
             constexpr int kOwnerStride = 32 / S::QG_ROWS;
             const float up = __shfl_down_sync(0xffffffffu, mine, kOwnerStride);
             const int row = reduced_row<S::QG_ROWS>(lane);
-            if (reduced_owner<S::QG_ROWS>(lane) && (row & 1) == 0) y[row >> 1] = (uint16_t)f32_to_bf16_bits(silu_mul(mine, up));
+            if constexpr (kWordActs) {   // two activations a word
+              const uint32_t act = f32_to_bf16_bits(silu_mul(mine, up)), next = __shfl_down_sync(0xffffffffu, act, 2 * kOwnerStride);
+              if ((row & 3) == 0) {
+#pragma unroll
+                for (int copy = lane % kOwnerStride; copy < kCopies; copy += kOwnerStride)
+                  st_word(reinterpret_cast<unsigned long long*>(a.activated) + (((size_t)par * kCopies + copy) * a.top_k + choice) * (F / 2) + (row0 + row) / 4, act | (next << 16), tag);
+              }
+            } else {
+              if (reduced_owner<S::QG_ROWS>(lane) && (row & 1) == 0) y[row >> 1] = (uint16_t)f32_to_bf16_bits(silu_mul(mine, up));
+            }
           } else {
             release(slot);
           }
-          if (t + kSC >= plan.s_sd && warp_done(layer, 1, min(kSC, plan.n_q), true) && lane == 0) red_release_add(sync + kRtGuDone, 1u);
+          if (!kWordActs && t + kSC >= plan.s_sd && warp_done(layer, 1, min(kSC, plan.n_q), true) && lane == 0) red_release_add(sync + kRtGuDone, 1u);
         }
       }
       if (tracer) INK_TRACE(layer, kTrRtGuDone);
@@ -1596,25 +1723,26 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       // tiles goes on with its down tiles, and waits only for the staging flag of the vector it needs. Only
       // where the shared experts' staging area overlaps the x staging (narrow experts) must every warp be
       // past its gate/up tiles first.
-      if (!tc && kSMaxTopK * F * 2 < D * 4) consumer_sync();
+      if (!tc && !kWordActs && kSMaxTopK * F * 2 < D * 4) consumer_sync();
       // ------------------------------------------------ shared down
       if (tc) {
         if (lane == 0) wait_global(sync + kShGuDone, epoch1 * gridDim.x, &sh);
-      } else {
+      } else if (!kWordActs) {
         wait_flag(&sh.seen[0], layer, &sh, lane);
       }
       if (lane == 0) wait_routing(layer, &sh);
       __syncwarp();
       if (tracer) INK_TRACE(layer, kTrShGuAll);
       for (int e = cw; e < a.n_shared; e += kSC) {   // warp e stages shared expert e: act * gamma, BF16
-        if (!sh.failed) {
+        if (!__any_sync(0xffffffffu, sh.failed != 0)) {
           const uint4* src = reinterpret_cast<const uint4*>(a.shared_activated + ((size_t)par * a.n_shared + e) * F);
           const float gamma = sh.routes[par].gamma[e];
           uint4* dst = reinterpret_cast<uint4*>(s_sact + (size_t)e * F);
           constexpr int N = F / 256;
           uint4 v[N];
 #pragma unroll
-          for (int n = 0; n < N; ++n) v[n] = __ldcg(src + n * 32 + lane);
+          for (int n = 0; n < N; ++n) v[n] = kWordActs ? make_uint4(0, 0, 0, 0) : __ldcg(src + n * 32 + lane);
+          if constexpr (kWordActs) warp_take_words<F, 1>(reinterpret_cast<const unsigned long long*>(a.shared_activated) + (((size_t)par * kCopies + my_copy) * a.n_shared + e) * F, tag, v, &sh, lane);
 #pragma unroll
           for (int n = 0; n < N; ++n) {
             uint4 o;
@@ -1650,21 +1778,23 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
           sact_seen |= 1u << e;
         }
         const uint4* xs = reinterpret_cast<const uint4*>(s_sact + (size_t)e * F);
-        float acc[S::SD_ROWS];
+        constexpr int kAtOnce = S::SD_ROWS < 4 ? S::SD_ROWS : 4;   // rows of a pass: a short body, whatever the width
+#pragma unroll 1
+        for (int first = 0; first < S::SD_ROWS; first += kAtOnce) {
+          float acc[kAtOnce];
 #pragma unroll
-        for (int row = 0; row < S::SD_ROWS; ++row) {
-          float sum = 0.f;
+          for (int row = 0; row < kAtOnce; ++row) {
+            float sum = 0.f;
 #pragma unroll 2
-          for (int c = 0; c < S::SD_CPL; ++c) {
-            const int chunk = c * 32 + lane;
-            sum = dot8(*reinterpret_cast<const uint4*>(src + (size_t)row * F * 2 + chunk * 16), xs[chunk], sum);
+            for (int c = 0; c < S::SD_CPL; ++c) {
+              const int chunk = c * 32 + lane;
+              sum = dot8(*reinterpret_cast<const uint4*>(src + (size_t)(first + row) * F * 2 + chunk * 16), xs[chunk], sum);
+            }
+            acc[row] = sum;
           }
-          acc[row] = sum;
-        }
-        {
-          const float total = multi_reduce<S::SD_ROWS>(acc, lane);   // one reduction for all rows of the tile
-          if (reduced_owner<S::SD_ROWS>(lane)) {
-            const int row = reduced_row<S::SD_ROWS>(lane);
+          const float total = multi_reduce<kAtOnce>(acc, lane);   // one reduction for all rows of the pass
+          if (reduced_owner<kAtOnce>(lane)) {
+            const int row = first + reduced_row<kAtOnce>(lane);
             if (tc) a.sd_out[((size_t)par * a.n_shared + e) * D + (size_t)plan.g0 * S::RT + local0 + row] = round_bf16(total);
             else sh.contrib[a.top_k + e][local0 + row] = round_bf16(total);
           }
@@ -1695,12 +1825,21 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       waited = 0;
       if constexpr (!tc) {
       // ------------------------------------------------ routed down
-      wait_flag(&sh.seen[1], layer, &sh, lane);
+      if (!kWordActs) wait_flag(&sh.seen[1], layer, &sh, lane);
       if (tracer) INK_TRACE(layer, kTrRtGuAll);
       for (int job = cw; job < a.top_k; job += kSC) {   // warp j stages route j
-        if (!sh.failed) {
-          const float inverse = warp_stage_f16<F>(a.activated + ((size_t)par * a.top_k + job) * F, s_act + (size_t)job * F, lane);
-          if (lane == 0) sh.inverse[job] = inverse;
+        if (!__any_sync(0xffffffffu, sh.failed != 0)) {
+          if constexpr (kWordActs) {
+            if (sh.routes[par].route[job].gu_codes) {   // (nobody publishes an inactive route's)
+              uint4 v[F / 256];
+              warp_take_words<F, 2>(reinterpret_cast<const unsigned long long*>(a.activated) + (((size_t)par * kCopies + my_copy) * a.top_k + job) * (F / 2), tag, v, &sh, lane);
+              const float inverse = warp_stage_f16<F>(v, s_act + (size_t)job * F, lane);
+              if (lane == 0) sh.inverse[job] = inverse;
+            }
+          } else {
+            const float inverse = warp_stage_f16<F>(a.activated + ((size_t)par * a.top_k + job) * F, s_act + (size_t)job * F, lane);
+            if (lane == 0) sh.inverse[job] = inverse;
+          }
         }
         __syncwarp();
         if (lane == 0) {
@@ -1762,7 +1901,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
                 sh.contrib[choice][local0 + reduced_row<S::RT>(lane)] = round_bf16(down * r.weight);
               }
             } else {
-#pragma unroll 1
+#pragma unroll 4
               for (int p = 0; p < S::PASSES; ++p) {
                 const int row = p * S::RPP + rp;
                 float acc = 0.f;
@@ -1793,29 +1932,40 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         // the last tile is always a routed one.)
         if (last_of_block && !sh.failed) {
           __syncwarp();
-          // hand this block's rows over (to every rank, itself included), then sum what the ranks sent for them
-          if (a.world == 1) {
-            for (int row = lane; row < plan.n_g * S::RT; row += 32) {
-              float total = 0.f;
-              for (int j = 0; j < n_jobs; ++j) total += sh.contrib[j][row];
-              send_row<D>(a, xpar, tag, plan.g0 * S::RT + row, total);
+          // Hand this block's rows over, two at a time (they start at a multiple of RT, RT is even): one rank publishes
+          // them straight away; several store them into every rank's inbox, itself included, and sum what the ranks sent.
+          unsigned long long* summed_words = a.summed + (size_t)xpar * kRowWords + plan.g0 * S::RT / 2;
+          const bool last = layer + 1 == a.n_layers;
+          auto publish = [&](int pair, float v0, float v1) {
+            const uint32_t packed = f32_to_bf16_bits(v0) | (f32_to_bf16_bits(v1) << 16);   // (the residual add takes the BF16 value)
+            const size_t i = (size_t)plan.g0 * S::RT + 2 * pair;
+            if (a.glue) {
+#pragma unroll
+              for (int copy = 0; copy < kCopies; ++copy) st_word(summed_words + (size_t)copy * (D / 2) + pair, packed, tag);
             }
-          } else {
-            // to the peers two rows at a time (the block's rows start at a multiple of RT, RT is even): half as
-            // many packets on the links
-            for (int pair = lane; pair < plan.n_g * S::RT / 2; pair += 32) {
-              float t0 = 0.f, t1 = 0.f;
-              for (int j = 0; j < n_jobs; ++j) {
-                t0 += sh.contrib[j][2 * pair];
-                t1 += sh.contrib[j][2 * pair + 1];
-              }
+            if (last) *reinterpret_cast<float2*>(a.partial + i) = make_float2(v0, v1);
+            if (!a.glue && a.normed_out) *reinterpret_cast<uint32_t*>(a.normed_out + i) = packed;
+          };
+          for (int pair = lane; pair < plan.n_g * S::RT / 2; pair += 32) {
+            float t0 = 0.f, t1 = 0.f;
+            for (int j = 0; j < n_jobs; ++j) {
+              t0 += sh.contrib[j][2 * pair];
+              t1 += sh.contrib[j][2 * pair + 1];
+            }
+            if (a.world == 1) {
+              publish(pair, t0, t1);
+            } else {
               const size_t at = ((size_t)xpar * a.world + a.rank) * D + (size_t)plan.g0 * S::RT + 2 * pair;
               for (int r = 0; r < a.world; ++r) st_tagged2_sys(a.peer_inbox[r] + at, t0, t1, tag);
             }
           }
           if (lane == 0) INK_TRACE(layer, kTrRowsSent);
-          if (a.world > 1)
-            for (int row = lane; row < plan.n_g * S::RT; row += 32) gather_row<D>(a, &sh, xpar, tag, plan.g0 * S::RT + row);
+          if (a.world > 1) {
+            for (int pair = lane; pair < plan.n_g * S::RT / 2; pair += 32) {
+              const float2 sum = gather_pair<D>(a, &sh, xpar, tag, plan.g0 * S::RT + 2 * pair);
+              if (!sh.failed) publish(pair, sum.x, sum.y);
+            }
+          }
           __syncwarp();   // the lanes waited for different rows: together again before anything warp-wide
         }
       }
@@ -1830,10 +1980,11 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       if (tracer) INK_TRACE(layer, kTrRtDownDone);
       if (tracer) INK_TRACE_VALUE(layer, kTrWaitRtDown, (unsigned long long)waited);
       waited = 0;
-      const unsigned long long* summed = a.summed + (size_t)xpar * D;
+      const unsigned long long* summed = a.summed + (size_t)xpar * kRowWords + (TC ? 0 : my_copy * (D / 2));
       if (!a.glue) {
-        // one block only: each block writes its own rows, summed over the ranks, as they arrive
-        for (int row = ct; row < plan.n_g * S::RT; row += kSC * 32) {
+        // one block only: its rows have been written by the warp that summed them (tensor-core variant: each block writes
+        // its own rows as they arrive)
+        for (int row = ct; tc && row < plan.n_g * S::RT; row += kSC * 32) {
           const size_t i = (size_t)plan.g0 * S::RT + row;
           const float v = wait_tagged(summed + i, tag, &sh);
           a.partial[i] = v;
@@ -1846,62 +1997,56 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       if (tc && blockIdx.x == 0 && ct < kSMaxTopK) a.act_amax[((layer + 1) & 1) * kSMaxTopK + ct] = 0u;
       // ------------------------------------------------ residual add + RMS norm (every block, redundantly)
       {
-        const uint16_t* res_in = a.residual + (size_t)par * D;
-        uint16_t* res_out = a.residual + (size_t)(par ^ 1) * D;
-        float sumsq = 0.f, amax_h = 0.f, amax_w = 0.f;
-        // all loads first (they are independent), arithmetic after: one L2 round trip; 16-byte loads of eight
-        // consecutive elements keep both the loads and the code that follows short
         // (one answer per warp: what follows synchronises the warp, so its lanes must not disagree about a
         // failure that another warp reports while they read the flag)
         __syncwarp();
         const bool live = !__any_sync(0xffffffffu, sh.failed != 0) && holder;
-        uint4 res[VG], nw[VG];
-        float part[VG][8];
+        uint4 nw[VG];
+        uint32_t part[VG][4];   // the rows as BF16 pairs
 #pragma unroll
         for (int g = 0; g < VG; ++g) {
-          const int group = g * VT + ct;
-          res[g] = live ? __ldcg(reinterpret_cast<const uint4*>(res_in) + group) : make_uint4(0, 0, 0, 0);
-          nw[g] = live ? reinterpret_cast<const uint4*>(norm_weight)[group] : make_uint4(0, 0, 0, 0);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) part[g][k] = 0.f;
+          nw[g] = live ? reinterpret_cast<const uint4*>(norm_weight)[g * VT + ct] : make_uint4(0, 0, 0, 0);
+          part[g][0] = part[g][1] = part[g][2] = part[g][3] = 0u;
         }
         // The layer's output rows, summed over the ranks, as their owners publish them: every thread polls the
         // tagged words of its own elements (all of a round in flight together), so a block goes on as soon as
         // the last row it needs is there -- no counter, no fence.
         if (live) {
-          unsigned long long w[VG][8];
-          // Polling has to be gentle: every block polls the same 32 KB, and on B200 the polls delay the very stores
-          // they wait for (a round of everything from every thread costs the L2 more than the rows take to arrive).
-          // So ONE warp of the block watches one word per sending block -- the last row of its slice -- with a pause
-          // between rounds, and raises a flag for the other warps ...
-          if (cw == 0) {
-            const int groups = D / S::RT;
-            const long long t0 = clock64();
-            for (;;) {
-              bool there = true;
-              for (int b = lane; b < (int)gridDim.x; b += 32) {
-                const int first = (int)((long long)b * groups / gridDim.x), end = (int)((long long)(b + 1) * groups / gridDim.x);
-                if (end > first) there = there && has_tag(ld_tagged(summed + (size_t)end * S::RT - 1), tag);
+          constexpr int kWords = TC ? 8 : 4;   // of eight rows: FP32 each, or two BF16 values
+          unsigned long long w[VG][kWords];
+          // Tensor-core variant, whose words have no copies: ONE warp of the block watches one word per sending block -- the last
+          // row of its slice -- and raises a flag for the other warps. (Every thread polling all of its words delayed the very stores it waited for.)
+          if constexpr (TC) {
+            if (cw == 0) {
+              const int groups = D / S::RT;
+              const long long t0 = clock64();
+              for (;;) {
+                bool there = true;
+                for (int b = lane; b < (int)gridDim.x; b += 32) {
+                  const int first = (int)((long long)b * groups / gridDim.x), end = (int)((long long)(b + 1) * groups / gridDim.x);
+                  if (end > first) there = there && has_tag(ld_tagged(summed + (size_t)end * S::RT - 1), tag);
+                }
+                if (__all_sync(0xffffffffu, there) || sh.failed) break;
+                if (clock64() - t0 > sh.limit) sh.failed = 1;
+                __nanosleep(sh.pause);
               }
-              if (__all_sync(0xffffffffu, there) || sh.failed) break;
-              if (clock64() - t0 > sh.limit) sh.failed = 1;
-              __nanosleep(sh.pause);
+              __syncwarp();
+              if (lane == 0) {
+                __threadfence_block();
+                sh.rows_seen = layer + 1;
+              }
+            } else {
+              wait_flag(&sh.rows_seen, layer, &sh, lane);
             }
-            __syncwarp();
-            if (lane == 0) {
-              __threadfence_block();
-              sh.rows_seen = layer + 1;
-            }
-          } else {
-            wait_flag(&sh.rows_seen, layer, &sh, lane);
           }
-          // ... then every thread loads its own elements; a sender's other rows may be a moment behind its last one
+          // Every thread polls its own elements. (With copies this is faster than a look at the senders' last rows, a flag and the loads in a
+          // chain: a block of 4096 x 2048 46.5 us, now 44.8; of 4096 x 256 19.8, now 16.6.)
           bool all = true;
 #pragma unroll
           for (int g = 0; g < VG; ++g) {
-            const unsigned long long* src = summed + (size_t)(g * VT + ct) * 8;
+            const unsigned long long* src = summed + (size_t)(g * VT + ct) * kWords;
 #pragma unroll
-            for (int k = 0; k < 8; k += 2) {
+            for (int k = 0; k < kWords; k += 2) {
               unsigned long long pair[2];
               ld_tagged2(src + k, pair);
               w[g][k] = pair[0];
@@ -1915,9 +2060,9 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
             all = true;
 #pragma unroll
             for (int g = 0; g < VG; ++g) {
-              const unsigned long long* src = summed + (size_t)(g * VT + ct) * 8;
+              const unsigned long long* src = summed + (size_t)(g * VT + ct) * kWords;
 #pragma unroll
-              for (int k = 0; k < 8; k += 2) {
+              for (int k = 0; k < kWords; k += 2) {
                 if (!has_tag(w[g][k], tag) || !has_tag(w[g][k + 1], tag)) {
                   unsigned long long pair[2];
                   ld_tagged2(src + k, pair);
@@ -1930,53 +2075,48 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
             if (clock64() - t0 > sh.limit) sh.failed = 1;
           }
 #pragma unroll
-          for (int g = 0; g < VG; ++g)
+          for (int g = 0; g < VG; ++g) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) part[g][k] = sh.failed ? 0.f : value_of(w[g][k]);
-        }
-        if (tracer) INK_TRACE(layer, kTrDownAll);
-        float h[VG][8];
-#pragma unroll
-        for (int g = 0; g < VG; ++g) {
-          const uint32_t r4[4] = {res[g].x, res[g].y, res[g].z, res[g].w}, w4[4] = {nw[g].x, nw[g].y, nw[g].z, nw[g].w};
-          uint32_t packed[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float lo = round_bf16(bf16lo(r4[k]) + round_bf16(part[g][2 * k]));
-            const float hi = round_bf16(bf16hi(r4[k]) + round_bf16(part[g][2 * k + 1]));
-            h[g][2 * k] = lo;
-            h[g][2 * k + 1] = hi;
-            sumsq = fmaf(lo, lo, fmaf(hi, hi, sumsq));
-            amax_h = fmaxf(amax_h, fmaxf(fabsf(lo), fabsf(hi)));
-            amax_w = fmaxf(amax_w, fmaxf(fabsf(bf16lo(w4[k])), fabsf(bf16hi(w4[k]))));
-            packed[k] = f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
-          }
-          if (blockIdx.x == 0 && live) {
-            const int group = g * VT + ct;
-            reinterpret_cast<uint4*>(res_out)[group] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-            if (layer + 1 == a.n_layers) {
-              float4* out = reinterpret_cast<float4*>(a.partial) + (size_t)group * 2;
-              out[0] = make_float4(part[g][0], part[g][1], part[g][2], part[g][3]);
-              out[1] = make_float4(part[g][4], part[g][5], part[g][6], part[g][7]);
+            for (int k = 0; k < 4; ++k) part[g][k] = sh.failed ? 0u : TC ? pack_bf16(value_of(w[g][2 * k % kWords]), value_of(w[g][(2 * k + 1) % kWords])) : (uint32_t)w[g][k];
+            if (tc && layer + 1 == a.n_layers && blockIdx.x == 0) {   // (CUDA-core variant: written by the blocks that own the rows)
+              float4* out = reinterpret_cast<float4*>(a.partial) + (size_t)(g * VT + ct) * 2;
+              out[0] = make_float4(value_of(w[g][0]), value_of(w[g][1]), value_of(w[g][2]), value_of(w[g][3]));
+              out[1] = make_float4(value_of(w[g][4 % kWords]), value_of(w[g][5 % kWords]), value_of(w[g][6 % kWords]), value_of(w[g][7 % kWords]));
             }
           }
         }
+        if (tracer) INK_TRACE(layer, kTrDownAll);
+        // Packed BF16 arithmetic where one rounding is what the reference has: the code of a phase is straight, run once a layer, and
+        // fetching it takes longer than executing it (in single precision this phase took 2.3 us a layer up to the barrier, 1.3 so).
+        float sumsq = 0.f;
+        uint32_t top_h = 0u, top_w = 0u;   // largest magnitudes, as BF16 pairs
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          sumsq += __shfl_xor_sync(0xffffffffu, sumsq, o);
-          amax_h = fmaxf(amax_h, __shfl_xor_sync(0xffffffffu, amax_h, o));
-          amax_w = fmaxf(amax_w, __shfl_xor_sync(0xffffffffu, amax_w, o));
+        for (int g = 0; g < VG; ++g) {
+          uint32_t r4[4] = {res[g].x, res[g].y, res[g].z, res[g].w};
+          const uint32_t w4[4] = {nw[g].x, nw[g].y, nw[g].z, nw[g].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            r4[k] = add_bf16x2(r4[k], part[g][k]);
+            const float lo = bf16lo(r4[k]), hi = bf16hi(r4[k]);
+            sumsq = fmaf(lo, lo, fmaf(hi, hi, sumsq));
+            top_h = __vmaxu2(top_h, r4[k] & 0x7fff7fffu);
+            top_w = __vmaxu2(top_w, w4[k] & 0x7fff7fffu);
+          }
+          res[g] = make_uint4(r4[0], r4[1], r4[2], r4[3]);
+          if (blockIdx.x == 0 && live && layer + 1 == a.n_layers) reinterpret_cast<uint4*>(a.residual + (size_t)(par ^ 1) * D)[g * VT + ct] = res[g];
         }
+        sumsq = warp_sum(sumsq);
+        const uint32_t most_h = __reduce_max_sync(0xffffffffu, max(top_h & 0xffffu, top_h >> 16)), most_w = __reduce_max_sync(0xffffffffu, max(top_w & 0xffffu, top_w >> 16));
         if (lane == 0) {
-          sh.red[cw][0] = sumsq;
-          sh.red[cw][1] = amax_h;
-          sh.red[cw][2] = amax_w;
+          sh.red[warp - 1][0] = sumsq;
+          sh.red[warp - 1][1] = bf16_to_f32(most_h);
+          sh.red[warp - 1][2] = bf16_to_f32(most_w);
         }
         consumer_sync();   // also: every consumer is past its down tiles, staging may be overwritten
         if (tracer) INK_TRACE(layer, kTrNormReduced);
         sumsq = 0.f;
-        amax_h = 0.f;
-        amax_w = 0.f;
+        float amax_h = 0.f, amax_w = 0.f;
+#pragma unroll
         for (int w = 0; w < kSC; ++w) {
           sumsq += sh.red[w][0];
           amax_h = fmaxf(amax_h, sh.red[w][1]);
@@ -1986,14 +2126,10 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
         uint4 xb[VG];
 #pragma unroll
         for (int g = 0; g < VG; ++g) {
-          const uint32_t w4[4] = {nw[g].x, nw[g].y, nw[g].z, nw[g].w};
+          const uint32_t r4[4] = {res[g].x, res[g].y, res[g].z, res[g].w}, w4[4] = {nw[g].x, nw[g].y, nw[g].z, nw[g].w};
           uint32_t packed[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float lo = round_bf16(h[g][2 * k] * scale) * bf16lo(w4[k]);
-            const float hi = round_bf16(h[g][2 * k + 1] * scale) * bf16hi(w4[k]);
-            packed[k] = f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
-          }
+          for (int k = 0; k < 4; ++k) packed[k] = mul_bf16x2(pack_bf16(bf16lo(r4[k]) * scale, bf16hi(r4[k]) * scale), w4[k]);
           xb[g] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
         if (layer + 1 == a.n_layers) {
@@ -2098,7 +2234,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
       const int par = layer & 1;
       const unsigned epoch1 = sh.epoch1;
       const int xpar = (int)(((epoch1 - 1u) * (unsigned)a.n_layers + (unsigned)layer) & 1u);
-      const bool tracer = (et == 0);
+      const bool tracer = kTrace && et == 0;
       // ------------------------------------------------ routed gate/up
       if (tw < 4) {
         scales_loop(plan.s_qg, plan.n_qu);
@@ -2235,7 +2371,7 @@ __global__ void __launch_bounds__(TC ? kSThreadsTc : kSThreads, 1) moe_stack_ker
 }
 
 // ------------------------------------------------------------------- host side
-template <int D, int F, bool TC>
+template <int D, int F, bool TC, bool kTrace>
 static int launch_stack(const StackArgs& a, cudaStream_t stream) {
   using S = StackShape<D, F>;
   constexpr int threads = TC ? kSThreadsTc : kSThreads;
@@ -2247,16 +2383,16 @@ static int launch_stack(const StackArgs& a, cudaStream_t stream) {
   cudaGetDevice(&device);
   INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "moe_stack: device ordinal %d", device);
   if (sms_of[device] == 0) {
-    cudaError_t e = cudaFuncSetAttribute(moe_stack_kernel<D, F, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(moe_stack_kernel<D, F, TC, kTrace>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "moe_stack: %d bytes of shared memory refused: %s", S::SMEM,
                 cudaGetErrorString(e));
-    cudaFuncSetAttribute(moe_stack_kernel<D, F, TC>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(moe_stack_kernel<D, F, TC, kTrace>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);
     int coop = 0, per_sm = 0, count = 0;
     cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     INK_REQUIRE(coop, kLaunchFailed, "moe_stack: the device cannot launch cooperative kernels");
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_stack_kernel<D, F, TC>, threads, S::SMEM);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_stack_kernel<D, F, TC, kTrace>, threads, S::SMEM);
     INK_REQUIRE(e == cudaSuccess && per_sm >= 1 && count >= 1, kLaunchFailed, "moe_stack: the kernel does not fit on an SM");
     sms_of[device] = count;
   }
@@ -2266,7 +2402,7 @@ static int launch_stack(const StackArgs& a, cudaStream_t stream) {
   INK_REQUIRE(rows_per_block <= kSMaxRows, kUnsupportedShape, "moe_stack: %d output rows per block", rows_per_block);
   StackArgs args = a;
   void* params[] = {&args};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)moe_stack_kernel<D, F, TC>, dim3(sms), dim3(threads), params,
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)moe_stack_kernel<D, F, TC, kTrace>, dim3(sms), dim3(threads), params,
                                               (size_t)S::SMEM, stream);
   INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "moe_stack: launch failed: %s", cudaGetErrorString(e));
   return kOk;
@@ -2309,6 +2445,14 @@ static size_t gu_part_bytes(int hidden, int intermediate, int top_k) {
          (size_t)((hidden + kTcChunkK - 1) / kTcChunkK);
 }
 
+// two sets of the experts' activations: BF16, or, of narrow experts, copies of 8-byte words of one or two
+static size_t activated_bytes(int experts, int intermediate, int per_word) {
+  const size_t values = 2 * (size_t)experts * intermediate;
+  return intermediate <= 512 ? values / per_word * 8 * kCopies : values * 2;
+}
+// two sets of the output rows' words (the tensor-core variant has one copy of a word a row)
+static size_t row_word_bytes(int hidden) { return sizeof(unsigned long long) * 2 * kCopies * (size_t)(hidden / 2); }
+
 // The region other ranks write into: two sets (alternating from layer to layer) of one slot of
 // `hidden` tagged 8-byte words per rank.
 extern "C" size_t ink_moe_stack_symmetric_bytes(int n_layers, int hidden, int world) {
@@ -2336,11 +2480,11 @@ extern "C" size_t ink_moe_stack_scratch_bytes(int n_layers, int hidden, int inte
   bytes += pad256(sizeof(float) * 2 * (size_t)n_shared * hidden);               // shared experts' down rows
   bytes += pad256(sizeof(unsigned) * 2 * kSMaxTopK);                            // activation maxima
   bytes += pad256(sizeof(unsigned) * kTileCounters * (size_t)n_layers);         // tile counters
-  bytes += pad256(sizeof(unsigned long long) * 2 * (size_t)(experts + n_shared));   // router words
-  bytes += pad256(2 * 2 * (size_t)top_k * intermediate);                        // activated
-  bytes += pad256(2 * 2 * (size_t)n_shared * intermediate);                     // shared activated
+  bytes += pad256(sizeof(unsigned long long) * 2 * kCopies * (size_t)(experts + n_shared));   // router words
+  bytes += pad256(activated_bytes(top_k, intermediate, 2));                     // activated
+  bytes += pad256(activated_bytes(n_shared, intermediate, 1));                  // shared activated
   bytes += pad256(2 * 2 * (size_t)hidden);                                      // residual double buffer
-  bytes += pad256(sizeof(unsigned long long) * 2 * (size_t)hidden);             // rows summed over the ranks (tagged)
+  bytes += pad256(row_word_bytes(hidden));                                      // rows summed over the ranks (tagged)
   bytes += pad256(sizeof(unsigned long long) * (size_t)n_layers * kTraceBlocks * kTraceSlots);   // phase stamps (tracing)
   return bytes;
 }
@@ -2395,16 +2539,16 @@ static int stack_decode(const void* layers, int n_layers, const void* x, void* r
   a.sd_out = (float*)take(sizeof(float) * 2 * (size_t)n_shared * hidden);
   a.act_amax = (unsigned*)take(sizeof(unsigned) * 2 * kSMaxTopK);
   a.tilesync = (unsigned*)take(sizeof(unsigned) * kTileCounters * (size_t)n_layers);
-  a.scores = (unsigned long long*)take(sizeof(unsigned long long) * 2 * (size_t)(experts + n_shared));
-  a.activated = (uint16_t*)take(2 * 2 * (size_t)top_k * intermediate);
-  a.shared_activated = (uint16_t*)take(2 * 2 * (size_t)n_shared * intermediate);
+  a.scores = (unsigned long long*)take(sizeof(unsigned long long) * 2 * kCopies * (size_t)(experts + n_shared));
+  a.activated = (uint16_t*)take(activated_bytes(top_k, intermediate, 2));
+  a.shared_activated = (uint16_t*)take(activated_bytes(n_shared, intermediate, 1));
   a.residual = (uint16_t*)take(2 * 2 * (size_t)hidden);
-  a.summed = (unsigned long long*)take(sizeof(unsigned long long) * 2 * (size_t)hidden);
+  a.summed = (unsigned long long*)take(row_word_bytes(hidden));
   a.wait_limit = g_stack_wait_limit;
   {
     const char* pause = getenv("INKLING_STACK_POLL_PAUSE_NS");
-    a.poll_pause_ns = pause ? (unsigned)atoi(pause) : 500u;   // measured on B200: 250..2000 ns are equally good, 64 ns costs 4 us per block
-    if (a.poll_pause_ns > 100000u) a.poll_pause_ns = 500u;
+    a.poll_pause_ns = pause ? (unsigned)atoi(pause) : kPollPause;
+    if (a.poll_pause_ns > 100000u) a.poll_pause_ns = kPollPause;
   }
   for (int r = 0; r < kSMaxWorld; ++r) a.peer_inbox[r] = nullptr;
   for (int r = 0; r < world && world > 1; ++r) {
@@ -2428,7 +2572,7 @@ static int stack_decode(const void* layers, int n_layers, const void* x, void* r
 #define INK_STACK_CASE(DD, FF)                   \
   if (hidden == DD && intermediate == FF) {      \
     built = true;                                \
-    rc = banks_mapped ? launch_stack<DD, FF, true>(a, s) : launch_stack<DD, FF, false>(a, s); \
+    rc = banks_mapped ? launch_stack<DD, FF, true, true>(a, s) : a.trace ? launch_stack<DD, FF, false, true>(a, s) : launch_stack<DD, FF, false, false>(a, s); \
   }
   INK_STACK_CASE(4096, 2048)
   INK_STACK_CASE(4096, 1024)

@@ -126,24 +126,20 @@ __device__ __forceinline__ bool reduced_owner(int lane) {  // one lane per row
   return (lane & ((32 / R) - 1)) == 0;
 }
 
-// One warp: K BF16 values written by other blocks (read through L2, never from a stale L1 line)
-// -> FP16 scaled by a power of two into [1, 2); returns the inverse. One round trip: every lane
-// loads its K / 256 groups of eight values at once and keeps them for the second pass.
+// One warp: K BF16 values, lane l with the groups n * 32 + l of eight -> FP16 scaled by a power of two into [1, 2), to shared
+// memory; returns the inverse.
 template <int K>
-__device__ __forceinline__ float warp_stage_f16(const uint16_t* src, uint16_t* dst, int lane) {
+__device__ __forceinline__ float warp_stage_f16(const uint4 (&v)[K / 256], uint16_t* dst, int lane) {
   constexpr int N = K / 256;
   static_assert(K % 256 == 0, "a warp stages whole rounds of 32 x 8 values");
-  uint4 v[N];
   uint32_t amax = 0;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    v[n] = __ldcg(reinterpret_cast<const uint4*>(src) + n * 32 + lane);
     const uint32_t w4[4] = {v[n].x, v[n].y, v[n].z, v[n].w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) amax = max(amax, max(w4[k] & 0x7fffu, (w4[k] >> 16) & 0x7fffu));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  amax = __reduce_max_sync(0xffffffffu, amax);
   float inverse;
   const float scale = pow2_normaliser(amax, &inverse);
 #pragma unroll
@@ -152,6 +148,14 @@ __device__ __forceinline__ float warp_stage_f16(const uint16_t* src, uint16_t* d
     reinterpret_cast<uint4*>(dst)[n * 32 + lane] = h;
   }
   return inverse;
+}
+// The same for values that other blocks have written (read through L2, never from a stale L1 line): one round trip.
+template <int K>
+__device__ __forceinline__ float warp_stage_f16(const uint16_t* src, uint16_t* dst, int lane) {
+  uint4 v[K / 256];
+#pragma unroll
+  for (int n = 0; n < K / 256; ++n) v[n] = __ldcg(reinterpret_cast<const uint4*>(src) + n * 32 + lane);
+  return warp_stage_f16<K>(v, dst, lane);
 }
 
 }  // namespace ink

@@ -232,3 +232,39 @@ def test_layers_of_fewer_tiles_than_ring_slots(ib, device, d, f, experts, n_shar
         alone = stack.layers[-1](normed.unsqueeze(0)).view(1, d)      # the block by itself, on what the stack fed it
         assert max_rel(got, alone.float()) <= 1.6e-2, n
         normed = out
+
+
+# narrow experts hand their activations over as words: one and two words a shared unit, four, eight and sixteen rows a routed tile; fewer
+# router rows, routed tiles or row groups than blocks; no shared experts, one choice, all choices; more router rows than 288
+@pytest.mark.parametrize("d,f,experts,n_shared,top_k", [(4096, 256, 8, 2, 6), (4096, 512, 16, 1, 1), (2048, 256, 300, 0, 8), (2048, 256, 4, 0, 1),
+                                                        (1024, 512, 4, 2, 4), (4096, 1024, 8, 1, 2)])
+def test_hand_overs_at_every_width(ib, device, d, f, experts, n_shared, top_k):
+    gen = torch.Generator().manual_seed(d + f)
+    x = torch.randn(1, d, generator=gen).to(BF16).to(device)
+    one = ib.MoEStack.synthetic(1, d, f, experts, n_shared, top_k, device, seed=2, bias_std=0.05)
+    assert one.one_launch
+    fused, partial = one(x).clone(), one.layers[0].partial[:1].clone()
+    one._fused.check_status()
+    one.one_launch = False
+    assert max_rel(fused.float(), one(x).float()) <= 1.6e-2          # as for the stacks above
+    block = one.layers[0](x.unsqueeze(0)).view(1, d)                   # the block alone, its rows written as BF16 and FP32
+    assert torch.equal(block, one.layers[0].partial[:1].to(BF16)) and max_rel(partial, one.layers[0].partial[:1]) <= 1.6e-2
+    five = ib.MoEStack.synthetic(5, d, f, experts, n_shared, top_k, device, seed=3, bias_std=0.05)
+    first = five(x).clone()
+    for _ in range(40):                                                  # every launch hands over in the same buffers
+        assert torch.equal(five(x), first)
+    five._fused.check_status()
+
+
+def test_routes_to_experts_that_are_not_there_hand_nothing_over(ib, device):
+    d, f = 1024, 512
+    p, banks, x = cases.make_layer(d, f, 8, 2, 3, 1, seed=4, bias="randn")
+    layer = build_layer(ib, device, p, banks)
+    layer(x.to(device).unsqueeze(0))
+    gone = int(layer.topk_indices[0, 1])
+    layer.experts.sources.view(-1, 6)[gone] = 0
+    out = layer(x.to(device).unsqueeze(0))[0].float()
+    layer._fused.check_status()
+    idx, w, gam = layer.topk_indices[:1].cpu(), layer.topk_weights[:1].cpu(), layer.gammas[:1].cpu()
+    w = torch.where(idx == gone, torch.zeros_like(w), w)
+    assert max_rel(out, oracle_moe.moe_layer_fp32(x, p, banks, idx, w, gam)) <= TOL
