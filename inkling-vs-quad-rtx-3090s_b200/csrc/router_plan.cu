@@ -306,12 +306,21 @@ __global__ void __launch_bounds__(1024) plan_kernel(PlanArgs p, int runs) {
 }
 
 // ------------------------------------------------------------- router, many tokens
-// The logits of more than a handful of tokens: a block takes eight router rows and sixteen tokens, every thread the
-// partial sums of all 128 pairs over its columns. A thread's columns, the order of its sums and the order in which the
+// The logits of more than a handful of tokens: a block takes tiles of sixteen router rows and sixteen tokens, a thread the partial
+// sums of sixteen tokens and half of the rows over its columns. A thread's columns, the order of its sums and the order in which the
 // threads' sums are added are those of router_kernel, so a token's logits do not depend on how many others there are (the
-// selection compares BF16 values: a last-bit difference picks another expert). Bound by the FMA pipes (2.1 G FMAs for
-// 1 999 tokens: 58 us); router_kernel, two rows a block and its tail on one block, took 3 270 us for them.
-constexpr int kManyRows = 8, kManyTokens = 16, kManyThreads = 128;
+// selection compares BF16 values: a last-bit difference picks another expert): products on the CUDA cores, two rows' FMAs an instruction.
+// Persistent blocks, one an SM: the next chunks of columns, of this tile or the next, are copied to shared memory while one is computed on.
+// 1 999 tokens, 258 rows of 4 096 columns (2.1 G FMAs, 58 us at the FMA pipes' rate): 160 us, 52 % of the issue slots, 2.6 instructions
+// for each that multiplies (tokens spread to pairs, the sums over the threads); loads straight to registers, eight warps an SM to hide them, 193; router_kernel,
+// two rows a block and its tail on one block, 3 270.
+constexpr int kManyRows = 8, kManyTokens = 16, kManyGroups = 2;            // rows of a thread, tokens, threads' shares of a tile's rows
+constexpr int kManyColumns = 128;                                           // threads along the columns, eight of them each
+constexpr int kManyThreads = kManyGroups * kManyColumns;
+constexpr int kManyTileRows = kManyGroups * kManyRows;
+constexpr int kManyStages = 3;
+constexpr int kManyStageBytes = (kManyTileRows + kManyTokens) * kManyColumns * 16;
+constexpr int kManySmem = kManyStages * kManyStageBytes;
 
 // Sums N per-lane values over the warp in the order of warp_sum; lane l keeps the values first, first + 1, ... (N / 32).
 template <int N>
@@ -331,58 +340,114 @@ __device__ __forceinline__ int wide_reduce(float (&v)[N], int lane) {
   return first;
 }
 
-__global__ void __launch_bounds__(kManyThreads, 2) router_logits_kernel(RouterArgs a) {
-  constexpr int kPairs = kManyRows * kManyTokens, kParts = kManyThreads / 32;
-  __shared__ float s_part[kParts][kPairs];
-  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
-  const int total = a.n_routed + a.n_shared, chunks = a.hidden / 8;
-  const int row0 = blockIdx.x * kManyRows, token0 = blockIdx.y * kManyTokens;
-  float acc[kPairs];   // [token][row]
-#pragma unroll
-  for (int i = 0; i < kPairs; ++i) acc[i] = 0.f;
-#pragma unroll 1
-  for (int c = tid; c < chunks; c += kManyThreads) {
-    float w[kManyRows][8];
-#pragma unroll
-    for (int r = 0; r < kManyRows; ++r) {
-      const int row = min(row0 + r, total - 1);
-      const uint4 q = __ldg(reinterpret_cast<const uint4*>(a.weight + (size_t)row * a.hidden) + c);
-      w[r][0] = bf16lo(q.x); w[r][1] = bf16hi(q.x); w[r][2] = bf16lo(q.y); w[r][3] = bf16hi(q.y);
-      w[r][4] = bf16lo(q.z); w[r][5] = bf16hi(q.z); w[r][6] = bf16lo(q.w); w[r][7] = bf16hi(q.w);
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__global__ void __launch_bounds__(kManyThreads, 1) router_logits_kernel(RouterArgs a) {
+  constexpr int kPairs = kManyRows * kManyTokens, kParts = kManyColumns / 32, kRowPairs = kManyRows / 2;
+  extern __shared__ __align__(16) unsigned char s_many[];   // [stages][sixteen rows, sixteen tokens][columns][16 B]
+  __shared__ float s_part[kManyGroups][kParts][kPairs];
+  const int tid = threadIdx.x, lane = tid & 31, group = tid / kManyColumns, column = tid % kManyColumns, part = column >> 5;
+  const int total = a.n_routed + a.n_shared, pieces = a.hidden / 8, chunks = (pieces + kManyColumns - 1) / kManyColumns;
+  const int row_tiles = (total + kManyTileRows - 1) / kManyTileRows;
+  const long long tiles = (long long)row_tiles * (a.tokens / kManyTokens + (a.tokens % kManyTokens != 0));
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_many);
+  // the copies of one chunk of a tile, half of its rows each: a group of copies (maybe an empty one)
+  long long copy_tile = blockIdx.x;
+  int copy_chunk = 0, copy_stage = 0;
+  auto copy_next = [&]() {
+    if (copy_tile < tiles) {
+      const int row0 = (int)(copy_tile % row_tiles) * kManyTileRows, token0 = (int)(copy_tile / row_tiles) * kManyTokens;
+      const int piece = copy_chunk * kManyColumns + column;
+      const uint32_t to = ring + (uint32_t)(copy_stage * kManyStageBytes + column * 16);
+#pragma unroll 4
+      for (int r = group; r < kManyTileRows + kManyTokens; r += kManyGroups) {
+        const uint16_t* from = r < kManyTileRows ? a.weight + (size_t)min(row0 + r, total - 1) * a.hidden
+                                                 : a.x + (size_t)min(token0 + r - kManyTileRows, a.tokens - 1) * a.hidden;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + (uint32_t)(r * kManyColumns * 16)),
+                     "l"(from + (piece < pieces ? piece * 8 : 0)), "r"(piece < pieces ? 16 : 0)   // (0: zeros, which add nothing)
+                     : "memory");
+      }
+      copy_stage = (copy_stage + 1) % kManyStages;
+      if (++copy_chunk == chunks) {
+        copy_chunk = 0;
+        copy_tile += gridDim.x;
+      }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i + 1 < kManyStages; ++i) copy_next();
+  int stage = 0;
+  for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int row0 = (int)(tile % row_tiles) * kManyTileRows + group * kManyRows, token0 = (int)(tile / row_tiles) * kManyTokens;
+    uint64_t acc2[kManyTokens][kRowPairs];   // sums of two rows
 #pragma unroll
-    for (int t0 = 0; t0 < kManyTokens; t0 += 4) {
-      uint4 x4[4];
+    for (int t = 0; t < kManyTokens; ++t)
 #pragma unroll
-      for (int t = 0; t < 4; ++t) x4[t] = __ldg(reinterpret_cast<const uint4*>(a.x + (size_t)min(token0 + t0 + t, a.tokens - 1) * a.hidden) + c);
+      for (int r = 0; r < kRowPairs; ++r) acc2[t][r] = 0ull;
+#pragma unroll 1
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kManyStages - 2) : "memory");
+      __syncthreads();   // everybody's copies of this chunk are there, everybody is done with the one before
+      copy_next();
+      const unsigned char* at = s_many + stage * kManyStageBytes + column * 16;
+      stage = (stage + 1) % kManyStages;
+      uint64_t w[kRowPairs][8];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float x[8] = {bf16lo(x4[t].x), bf16hi(x4[t].x), bf16lo(x4[t].y), bf16hi(x4[t].y),
-                            bf16lo(x4[t].z), bf16hi(x4[t].z), bf16lo(x4[t].w), bf16hi(x4[t].w)};
+      for (int r = 0; r < kRowPairs; ++r) {
+        const uint4 q0 = *reinterpret_cast<const uint4*>(at + (group * kManyRows + 2 * r) * kManyColumns * 16);
+        const uint4 q1 = *reinterpret_cast<const uint4*>(at + (group * kManyRows + 2 * r + 1) * kManyColumns * 16);
+        const uint32_t v0[4] = {q0.x, q0.y, q0.z, q0.w}, v1[4] = {q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
-        for (int r = 0; r < kManyRows; ++r) {
-          float s = acc[(t0 + t) * kManyRows + r];
+        for (int k = 0; k < 4; ++k) {
+          w[r][2 * k] = pair_of(bf16lo(v0[k]), bf16lo(v1[k]));
+          w[r][2 * k + 1] = pair_of(bf16hi(v0[k]), bf16hi(v1[k]));
+        }
+      }
+      constexpr int kAtOnce = 4;   // tokens: sixteen sums that do not wait for one another
 #pragma unroll
-          for (int k = 0; k < 8; ++k) s = fmaf(w[r][k], x[k], s);
-          acc[(t0 + t) * kManyRows + r] = s;
+      for (int t0 = 0; t0 < kManyTokens; t0 += kAtOnce) {
+        uint32_t v[kAtOnce][4];
+#pragma unroll
+        for (int t = 0; t < kAtOnce; ++t) {
+          const uint4 q = *reinterpret_cast<const uint4*>(at + (kManyTileRows + t0 + t) * kManyColumns * 16);
+          v[t][0] = q.x; v[t][1] = q.y; v[t][2] = q.z; v[t][3] = q.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+#pragma unroll
+          for (int t = 0; t < kAtOnce; ++t) {
+            const float x = (k & 1) ? bf16hi(v[t][k / 2]) : bf16lo(v[t][k / 2]);
+            const uint64_t xx = pair_of(x, x);
+#pragma unroll
+            for (int r = 0; r < kRowPairs; ++r) asm volatile("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc2[t0 + t][r]) : "l"(w[r][k]), "l"(xx));
+          }
         }
       }
     }
-  }
-  const int first = wide_reduce<kPairs>(acc, lane);
+    float acc[kPairs];   // [token][row]
 #pragma unroll
-  for (int i = 0; i < kPairs / 32; ++i) s_part[part][first + i] = acc[i];
-  __syncthreads();
-  for (int i = tid; i < kPairs; i += kManyThreads) {
-    const int row = row0 + i % kManyRows, token = token0 + i / kManyRows;
-    if (row >= total || token >= a.tokens) continue;
-    float s = 0.f;
+    for (int t = 0; t < kManyTokens; ++t)
 #pragma unroll
-    for (int w = 0; w < kParts; ++w) s += s_part[w][i];
-    const float l = round_bf16(s);
-    a.logits[(size_t)token * total + row] = l;
-    if (row < a.n_routed) a.scores[(size_t)token * a.n_routed + row] = round_bf16(1.f / (1.f + __expf(-l))) + a.bias[row];
+      for (int r = 0; r < kRowPairs; ++r) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[t * kManyRows + 2 * r]), "=f"(acc[t * kManyRows + 2 * r + 1]) : "l"(acc2[t][r]));
+    const int first = wide_reduce<kPairs>(acc, lane);
+#pragma unroll
+    for (int i = 0; i < kPairs / 32; ++i) s_part[group][part][first + i] = acc[i];
+    __syncthreads();   // (the next tile's first barrier keeps these sums until they have been read)
+    const int row = row0 + column % kManyRows, token = token0 + column / kManyRows;   // a pair a thread
+    static_assert(kPairs == kManyColumns, "a thread writes one logit");
+    if (row < total && token < a.tokens) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < kParts; ++w) s += s_part[group][w][column];
+      const float l = round_bf16(s);
+      a.logits[(size_t)token * total + row] = l;
+      if (row < a.n_routed) a.scores[(size_t)token * a.n_routed + row] = round_bf16(1.f / (1.f + __expf(-l))) + a.bias[row];
+    }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // One warp per token; the block that is done last makes the plan, if one is asked for.
@@ -466,18 +531,21 @@ static int launch_router(const RouterArgs& a, const PlanArgs* p, cudaStream_t st
     INK_CHECK_LAUNCH("ink_router_forward");
     return kOk;
   }
-  constexpr int kMost = 65535 * kManyTokens;   // (what a grid's second dimension holds)
-  for (int t0 = 0; t0 < a.tokens; t0 += kMost) {
-    RouterArgs part = a;
-    part.tokens = a.tokens - t0 < kMost ? a.tokens - t0 : kMost;
-    part.x += (size_t)t0 * a.hidden;
-    part.logits += (size_t)t0 * rows;
-    part.scores += (size_t)t0 * a.n_routed;
-    const dim3 grid((unsigned)((rows + kManyRows - 1) / kManyRows), (unsigned)((part.tokens + kManyTokens - 1) / kManyTokens));
-    router_logits_kernel<<<grid, kManyThreads, 0, stream>>>(part);
-    INK_CHECK_LAUNCH("ink_router_forward (logits)");
-    if (a.tokens - t0 <= kMost) break;   // (t0 stays inside an int)
+  constexpr int kMaxDevices = 64;
+  static int sms_of[kMaxDevices] = {};   // 0: this device is not configured yet
+  int device = 0;
+  cudaGetDevice(&device);
+  INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "router: device ordinal %d", device);
+  if (sms_of[device] == 0) {
+    const cudaError_t e = cudaFuncSetAttribute(router_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kManySmem);
+    INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "router: %d bytes of shared memory refused: %s", kManySmem, cudaGetErrorString(e));
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    sms_of[device] = sms > 0 ? sms : 148;
   }
+  const long long tiles = (long long)((rows + kManyTileRows - 1) / kManyTileRows) * ((a.tokens + (long long)kManyTokens - 1) / kManyTokens);
+  router_logits_kernel<<<(unsigned)(tiles < sms_of[device] ? tiles : sms_of[device]), kManyThreads, kManySmem, stream>>>(a);
+  INK_CHECK_LAUNCH("ink_router_forward (logits)");
   const unsigned selects = (unsigned)((a.tokens + 31) / 32);
   if (!p) {
     router_select_kernel<false><<<selects, 1024, 0, stream>>>(a, PlanArgs{}, 0);
