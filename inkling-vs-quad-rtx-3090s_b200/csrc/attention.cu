@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
   const uint16_t* fresh_v = a.new_k ? a.new_v + ((size_t)b * a.kv_heads + kv_head) * C : nullptr;
   if (a.new_k && chunk == 0 && split == 0 && fresh_slot < a.slots) {
     for (int i = tid; i < C / 2; i += kAttnThreads) {
-      reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[i] = __ldg(reinterpret_cast<const uint32_t*>(fresh_k) + i);
-      reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[i] = __ldg(reinterpret_cast<const uint32_t*>(fresh_v) + i);
+      reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[i] = __ldcg(reinterpret_cast<const uint32_t*>(fresh_k) + i);
+      reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[i] = __ldcg(reinterpret_cast<const uint32_t*>(fresh_v) + i);
     }
   }
   // The slots that can count at all (a full layer: from the end of the padding to the position; a ring: all that have
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
       const bool ok = unit < unit1 && allowed_at(slot);
       const uint4* row = reinterpret_cast<const uint4*>(slot == fresh_slot ? fresh_k : keys + (size_t)slot * C);
 #pragma unroll
-      for (int i = 0; i < kPieces; ++i) kq[n][i] = ok ? ldg_stream_16(row + t + 4 * i) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < kPieces; ++i) kq[n][i] = ok ? ld_stream_16(row + t + 4 * i) : make_uint4(0, 0, 0, 0);
     }
   };
   int unit = unit0 + warp;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
   uint4 qf[kPieces];
 #pragma unroll
   for (int i = 0; i < kPieces; ++i) {
-    qf[i] = g < n_heads ? __ldg(reinterpret_cast<const uint4*>(a.q + ((size_t)b * a.heads + head0 + g) * C) + t + 4 * i) : make_uint4(0, 0, 0, 0);
+    qf[i] = g < n_heads ? __ldcg(reinterpret_cast<const uint4*>(a.q + ((size_t)b * a.heads + head0 + g) * C) + t + 4 * i) : make_uint4(0, 0, 0, 0);
     if (scaled) {
       qf[i].x = pack_bf16(bf16lo(qf[i].x) * tau, bf16hi(qf[i].x) * tau);
       qf[i].y = pack_bf16(bf16lo(qf[i].y) * tau, bf16hi(qf[i].y) * tau);
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
     uint4 vv[kAhead][4];
     auto load_values = [&](int h, uint4 (&to)[4]) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) to[i] = vok[i] ? ldg_stream_16(vrow[i] + g + 8 * h) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < 4; ++i) to[i] = vok[i] ? ld_stream_16(vrow[i] + g + 8 * h) : make_uint4(0, 0, 0, 0);
     };
 #pragma unroll
     for (int h = 0; h < kAhead; ++h) load_values(h, vv[h]);
@@ -494,8 +494,8 @@ __global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(A
     else if (!ok) vw[n] = 0u;
   }
   if (a.new_k && chunk == 0 && fresh_here && tid < kWords) {
-    reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_k) + tid);
-    reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[tid] = __ldg(reinterpret_cast<const uint32_t*>(fresh_v) + tid);
+    reinterpret_cast<uint32_t*>(a.k_store + (row0 + fresh_slot) * C)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(fresh_k) + tid);
+    reinterpret_cast<uint32_t*>(a.v_store + (row0 + fresh_slot) * C)[tid] = __ldcg(reinterpret_cast<const uint32_t*>(fresh_v) + tid);
   }
   const bool scaled = a.window == 0 && a.n_floor > 0;
   float tau = 1.f;

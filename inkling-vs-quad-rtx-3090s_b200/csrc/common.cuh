@@ -144,6 +144,14 @@ __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
                : "l"(p));
   return v;
 }
+// the same for memory that the kernel in front may have written
+__device__ __forceinline__ uint4 ld_stream_16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
 __device__ __forceinline__ uint32_t ldg_stream_u16(const void* p) {
   uint16_t v;
   asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));

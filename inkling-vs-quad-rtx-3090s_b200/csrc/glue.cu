@@ -30,9 +30,9 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(const float* 
   for (int i = 0; i < kNormMaxPerThread; ++i) {
     const int gidx = i * kNormThreads + tid;
     if (gidx < groups) {
-      const float4 a = ADD ? *reinterpret_cast<const float4*>(p + gidx * 8) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 b = ADD ? *reinterpret_cast<const float4*>(p + gidx * 8 + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const uint4 q = *reinterpret_cast<const uint4*>(r + gidx * 8);
+      const float4 a = ADD ? __ldcg(reinterpret_cast<const float4*>(p + gidx * 8)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 b = ADD ? __ldcg(reinterpret_cast<const float4*>(p + gidx * 8 + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint4 q = __ldcg(reinterpret_cast<const uint4*>(r + gidx * 8));
       const float add[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
       const uint32_t res[4] = {q.x, q.y, q.z, q.w};
       uint32_t packed[4];
@@ -123,12 +123,12 @@ __global__ void __launch_bounds__(256) short_conv_kernel(const void* __restrict_
   if (d >= hidden) return;
   const size_t at = (size_t)blockIdx.y * hidden + d;
   float current;
-  if (XF32) current = round_bf16(reinterpret_cast<const float*>(x_raw)[at]);
-  else current = bf16_to_f32(reinterpret_cast<const uint16_t*>(x_raw)[at]);
+  if (XF32) current = round_bf16(__ldcg(reinterpret_cast<const float*>(x_raw) + at));
+  else current = bf16_to_f32(__ldcg(reinterpret_cast<const uint16_t*>(x_raw) + at));
   ConvChannel<TAPS, WIDE> conv;
   conv.fetch(taps + (size_t)d * TAPS, history + at * TAPS);
   float out = conv.step(current, history + at * TAPS);
-  if (residual) out = round_bf16(__fadd_rn(out, bf16_to_f32(residual[at])));
+  if (residual) out = round_bf16(__fadd_rn(out, bf16_to_f32(__ldcg(residual + at))));
   y[at] = (uint16_t)f32_to_bf16_bits(out);
 }
 
@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(kConvNormThreads) conv_norm_kernel(const uint1
       const int d = channel_of(i0 + n * kConvNormThreads);
       if (d >= hidden) continue;
       conv[n].fetch(taps + (size_t)d * TAPS, history + (row + d) * TAPS);
-      in[n] = bf16_to_f32(x[row + d]);
-      skip[n] = bf16_to_f32(residual[row + d]);
+      in[n] = bf16_to_f32(__ldcg(x + row + d));
+      skip[n] = bf16_to_f32(__ldcg(residual + row + d));
     }
 #pragma unroll
     for (int n = 0; n < kAhead; ++n) {
@@ -283,7 +283,8 @@ __global__ void __launch_bounds__(128) heads_kernel(const HeadsArgs a) {
   }
 }
 
-// A launch that may start while the kernel in front runs (see pdl_wait).
+// A launch that may start while the kernel in front runs (see pdl_wait). What that one writes is read through L2, never by loads
+// that are meant for memory nobody writes while a kernel is there.
 template <typename... Params, typename... Args>
 static cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, int threads, int cluster, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t config = {};
