@@ -206,8 +206,13 @@ int ink_attention_heads(const void* qkvr, const void* q_weight, const void* k_we
  * y = bf16(x . weight^T), x BF16 [tokens, k], weight BF16 [n, k], y BF16 [tokens, n], sums in FP32 over
  * the columns in order, sixteen at a time. With `up` BF16 [n, k]:
  * y = bf16(bf16(silu(bf16(x . weight^T))) * bf16(x . up^T)). With `scale` BF16 [1]: y is multiplied by it and rounded once more.
- * k a multiple of 32 up to 8192; x, weight and up 16-byte aligned. */
+ * k a multiple of 32 up to 8192; x, weight and up 16-byte aligned. All operands are read in stream order. */
 int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k, ink_stream_t stream);
+/* The same. `settled` not 0: the caller vouches that the launch in front on the stream does not write weight or up; they may be
+ * read while it runs. (What the launches before that one wrote is there, if the one in front is any kernel of this library but the
+ * grouped projections, or one launched without the programmatic stream serialization attribute.) */
+int ink_linear_settled(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k, int settled,
+                       ink_stream_t stream);
 
 /* Decode attention with the learned relative-position bias, one query token per sequence: the static_decode
  * branch of MyInklingAttention.forward (my_inkling/model.py:533-612) from the normed query to the output of

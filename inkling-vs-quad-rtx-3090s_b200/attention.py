@@ -26,6 +26,12 @@ def _aligned(*tensors: torch.Tensor) -> bool:
     return all(t.data_ptr() % 16 == 0 for t in tensors)
 
 
+def _runs_alone(module, kind) -> bool:
+    """A call of `module` launches `kind`'s kernels and nothing before them: no hook, no other forward."""
+    return (type(module) is kind and "forward" not in vars(module) and not module._forward_pre_hooks
+            and not nn.modules.module._global_forward_pre_hooks)
+
+
 class DecodeAttention(nn.Module):
     def __init__(self, qkvr_weight, o_weight, q_norm_weight, k_norm_weight, k_taps, v_taps, rel_proj, *, layer_idx: int,
                  heads: int, kv_heads: int, head_dim: int, d_rel: int, window: int = 0, log_scaling_n_floor=None,
@@ -57,14 +63,15 @@ class DecodeAttention(nn.Module):
     def _norm(self, rows: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         return _norm_rows(rows, weight, self.eps)
 
-    def forward(self, hidden_states: torch.Tensor, cache) -> torch.Tensor:
+    def forward(self, hidden_states: torch.Tensor, cache, *, settled: bool = False) -> torch.Tensor:
         """hidden_states BF16 [bs, 1, d], cache in decode mode -> BF16 [bs, 1, d]; the caches and the convolution
-        histories of this layer are updated in place, `cache.position` is left to the caller (`cache.advance`)."""
+        histories of this layer are updated in place, `cache.position` is left to the caller (`cache.advance`).
+        `settled`: the launch in front is a kernel that does not write this module's weights (see `linear`)."""
         bs, s, _ = hidden_states.shape
         assert s == 1, "one token per sequence"
         layer = cache.layers[self.layer_idx]
         h, hk, c = self.heads, self.kv_heads, self.head_dim
-        qkvr = linear(hidden_states, self.qkvr_weight)
+        qkvr = linear(hidden_states, self.qkvr_weight, settled=settled)
         k_history, v_history = layer.conv_caches[0].cache, layer.conv_caches[1].cache
         if c % 8 == 0 and c <= 256 and (h * self.d_rel) % 8 == 0 and _aligned(qkvr, self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history):
             q, k, v, r = attention_heads(qkvr.view(bs, -1), self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history, self.eps,
@@ -79,7 +86,7 @@ class DecodeAttention(nn.Module):
                                cache.position, cache.pad_counts, window=self.window, log_scaling_n_floor=self.n_floor,
                                log_scaling_alpha=self.alpha, scale=1.0 / c, new_key=k.view(bs, hk, 1, c),
                                new_value=v.reshape(bs, hk, 1, c))
-        y = linear(out.reshape(bs, 1, h * c), self.o_weight)
+        y = linear(out.reshape(bs, 1, h * c), self.o_weight, settled=True)   # (the attention is in front)
         if self.group is not None:
             y = all_reduce(y, self.group)   # (nothing to do with one rank)
         return y
@@ -105,14 +112,18 @@ class DecodeLayer(nn.Module):
         """hidden_states BF16 [bs, 1, d] -> BF16 [bs, 1, d]; the layer's caches are updated in place."""
         bs, _, d = hidden_states.shape
         layer = cache.layers[self.attention.layer_idx]
-        attended = self.attention(self._norm(hidden_states, self.input_norm_weight), cache)
+        normed = self._norm(hidden_states, self.input_norm_weight)
+        attended = self.attention(normed, cache, settled=True) if _runs_alone(self.attention, DecodeAttention) else self.attention(normed, cache)
         attended, history, residual = attended.contiguous(), layer.conv_caches[2].cache, hidden_states.contiguous()
         if d % 8 == 0 and _aligned(self.attn_taps, history):
             h, normed = short_conv_norm(attended, self.attn_taps, history, residual, self.post_norm_weight, self.eps)
         else:
             h = short_conv(attended, self.attn_taps, history, residual)
             normed = self._norm(h, self.post_norm_weight).view(bs, d)
-        block = self.moe.forward_partial(normed) if hasattr(self.moe, "forward_partial") else self.moe(normed)   # [bs, d], all-reduced
+        if _runs_alone(self.moe, DenseMLP):
+            block = self.moe(normed, settled=True)
+        else:
+            block = self.moe.forward_partial(normed) if hasattr(self.moe, "forward_partial") else self.moe(normed)   # [bs, d], all-reduced
         return short_conv(block.view(bs, 1, d).contiguous(), self.mlp_taps, layer.conv_caches[3].cache, h)
 
 
@@ -127,8 +138,9 @@ class DenseMLP(nn.Module):
             self.register_buffer(name, t.contiguous())
         self.group = group
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        y = linear(gated(x, self.gate_weight, self.up_weight), self.down_weight, self.global_scale)
+    def forward(self, x: torch.Tensor, *, settled: bool = False) -> torch.Tensor:
+        """`settled`: as of DecodeAttention."""
+        y = linear(gated(x, self.gate_weight, self.up_weight, settled=settled), self.down_weight, self.global_scale, settled=True)
         return y if self.group is None else all_reduce(y, self.group)
 
 
@@ -153,6 +165,6 @@ class DecodeModel(nn.Module):
         for layer in self.layers:
             hidden = layer(hidden, cache)
         hidden = norm(hidden, self.final_norm_weight) / self.mup
-        logits = linear(hidden, self.lm_head_weight)
+        logits = linear(hidden, self.lm_head_weight, settled=True)   # (the division is in front)
         cache.position.add_(1)
         return logits if self.unpadded is None else logits[..., : self.unpadded]

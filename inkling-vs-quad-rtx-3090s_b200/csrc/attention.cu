@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
   uint16_t* s_r = reinterpret_cast<uint16_t*>(s_raw);                               // [heads][d_rel rounded up to 16]: before the sums
   __shared__ bool s_last;
   __shared__ __align__(16) float s_block[CLUSTER ? kAttnHeads * (C + 2) : 1];   // this block's sums, for its cluster
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(A
   uint16_t* s_r = reinterpret_cast<uint16_t*>(s_block + kAttnHeads * (C + 2));      // [heads][d_rel]
   __shared__ float s_top[kAttnHeads];
   __shared__ bool s_last;
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int split = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int group = a.heads / a.kv_heads, chunks = (group + kAttnHeads - 1) / kAttnHeads;
   const int kv_head = blockIdx.y / chunks, chunk = blockIdx.y % chunks;

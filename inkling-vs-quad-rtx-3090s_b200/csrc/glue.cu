@@ -17,8 +17,8 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(const float* 
                                                                     const uint16_t* __restrict__ weight, float eps,
                                                                     uint16_t* __restrict__ normed, int hidden) {
   __shared__ float s_red[kNormThreads / 32];
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int token = blockIdx.x, tid = threadIdx.x;
   const float* p = ADD ? partial + (size_t)token * hidden : nullptr;
   uint16_t* r = residual + (size_t)token * hidden;
@@ -117,8 +117,8 @@ template <int TAPS, bool XF32, bool WIDE>
 __global__ void __launch_bounds__(256) short_conv_kernel(const void* __restrict__ x_raw, const float* __restrict__ taps,
                                                           float* __restrict__ history, const uint16_t* __restrict__ residual,
                                                           uint16_t* __restrict__ y, int hidden) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int d = blockIdx.x * blockDim.x + threadIdx.x;
   if (d >= hidden) return;
   const size_t at = (size_t)blockIdx.y * hidden + d;
@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(kConvNormThreads) conv_norm_kernel(const uint1
                                                                       uint16_t* __restrict__ normed, int hidden) {
   __shared__ float s_h[kNormMaxPerThread * 256];   // this block's sums: 256 channels of every 2 048
   __shared__ float s_sum;
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   const size_t row = (size_t)blockIdx.y * hidden;
   auto channel_of = [&](int i) -> int { return i / 256 * (kNormThreads * 8) + rank * 256 + i % 256; };
@@ -209,8 +209,8 @@ struct HeadsArgs {
 };
 template <int TAPS>
 __global__ void __launch_bounds__(128) heads_kernel(const HeadsArgs a) {
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31, c = a.head_dim, width = (a.heads + 2 * a.kv_heads) * c + a.heads * a.d_rel;
   const int vectors = a.heads + 2 * a.kv_heads + 1;   // of a token; the last is its relative states
   const int at = blockIdx.x * 4 + (threadIdx.x >> 5);

@@ -4,7 +4,8 @@
 // Bound by reading the weights once. One block per SM takes an equal share of the rows, up to eighty at a time. Four warps copy
 // them into a ring of stages (256 columns of all rows; cp.async, so that rows lie on a pitch without bank conflicts), a fifth the
 // tokens' columns; a consumer warp takes sixteen rows and makes m16n8k16 products (M = weight rows, N = tokens: eight tokens are
-// far too few for the tcgen05 tiles). The weights depend on nothing: the ring fills before the kernel in front has finished.
+// far too few for the tcgen05 tiles). Where the caller vouches for the weights (`settled`: the launch in front does not write them) the ring
+// fills before the kernel in front has finished; else the weights, like the tokens, are asked for when it has.
 //
 // The sum over columns runs from the first to the last, sixteen at a time into one FP32 accumulator. That is the order of a
 // plain tensor-core GEMM, so the results are the bits of the library GEMV that these calls were (up to 8192 columns; above, the
@@ -42,6 +43,7 @@ struct LinearArgs {
   uint16_t* y;            // [tokens, n]
   int tokens, n, k;
   int groups, stages;     // consumers that have rows; stages of the ring
+  int settled;            // the kernel in front does not write the weights
 };
 
 struct LinearShared {
@@ -74,7 +76,6 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_kernel(const LinearArgs
   constexpr int kOut = GATED ? kLinRows / 2 : kLinRows;   // outputs of a consumer
   extern __shared__ __align__(128) unsigned char s_ring[];   // [stages][groups * 16 + 8 rows][kLinPitch]: weights, then tokens
   __shared__ LinearShared sh;
-  pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int stage_rows = a.groups * kLinRows, stage_bytes = (stage_rows + kLinTokens) * kLinPitch;
   const int first = (int)((long long)a.n * blockIdx.x / gridDim.x), end = (int)((long long)a.n * (blockIdx.x + 1) / gridDim.x);
@@ -93,7 +94,8 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_kernel(const LinearArgs
     // =========================================================== copies
     const int producer = warp - kLinConsumers;
     const bool weights = producer < kLinWeightWarps;
-    if (!weights) pdl_wait();   // x is there now
+    if (!weights || !a.settled) pdl_wait();   // x is there now, and any weights
+    if (!weights) pdl_trigger();
     const uint32_t ring = smem_u32(s_ring);
     int stage = 0;
     uint32_t lap = 0;
@@ -224,13 +226,18 @@ static int launch_linear(LinearArgs a, cudaStream_t stream) {
 
 using namespace ink;
 
-extern "C" int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k,
-                          ink_stream_t stream) {
+extern "C" int ink_linear_settled(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k,
+                                  int settled, ink_stream_t stream) {
   INK_REQUIRE(x && weight && y, kBadArgument, "linear: null pointer argument");
   INK_REQUIRE(tokens >= 0 && tokens <= kLinTokens && n > 0 && n <= (1 << 24) && k > 0 && k % 32 == 0 && k <= kLinMostK, kUnsupportedShape,
               "linear: tokens=%d n=%d k=%d unsupported (up to %d tokens, k a multiple of 32 up to %d)", tokens, n, k, kLinTokens, kLinMostK);
   INK_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(up), kMisaligned, "linear: x and weights must be 16-byte aligned");
   if (tokens == 0) return kOk;
-  const LinearArgs a{(const uint16_t*)x, (const uint16_t*)weight, (const uint16_t*)up, (const uint16_t*)scale, (uint16_t*)y, tokens, n, k, 0, 0};
+  const LinearArgs a{(const uint16_t*)x, (const uint16_t*)weight, (const uint16_t*)up, (const uint16_t*)scale, (uint16_t*)y, tokens, n, k, 0, 0, settled};
   return up ? launch_linear<true>(a, (cudaStream_t)stream) : launch_linear<false>(a, (cudaStream_t)stream);
+}
+
+extern "C" int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k,
+                          ink_stream_t stream) {
+  return ink_linear_settled(x, weight, up, scale, y, tokens, n, k, 0, stream);
 }

@@ -37,7 +37,9 @@ __device__ __forceinline__ float2 ld_cluster_float2(const float* p, int rank) {
 
 // Programmatic dependent launch. A kernel launched as a dependent starts when the one in front has let it (every block has
 // triggered or ended); what that one wrote is there after pdl_wait, which also means that it has ended. Every block waits
-// before it ends, so whoever waits for a kernel may rely on all the kernels before it too.
+// before it ends, so whoever waits for a kernel may rely on all the kernels before it too. Kernels trigger after their own wait (the
+// grouped projections before it: nothing but their own staging and sums follows them): a kernel that has started may rely, without
+// waiting, on all that was written before the kernel in front of it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -1,6 +1,8 @@
 """Dense BF16 projections of a decode step (ink_linear)."""
 from __future__ import annotations
 
+from functools import partial
+
 import torch
 import torch.nn.functional as F
 
@@ -28,26 +30,31 @@ def _fits(x, *weights) -> bool:
                     and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in weights))
 
 
-def _launch(x, weight, up, scale):
+def _launch(x, weight, up, scale, settled=False):
     n, k = weight.shape
     y = x.new_empty(*x.shape[:-1], n)
     with torch.cuda.device(x.device):
-        _abi.check(_abi.lib().ink_linear(x.data_ptr(), weight.data_ptr(), _abi.ptr(up), _abi.ptr(scale), y.data_ptr(), x.numel() // k, n, k, _abi.stream()))
+        _abi.check(_abi.lib().ink_linear_settled(x.data_ptr(), weight.data_ptr(), _abi.ptr(up), _abi.ptr(scale), y.data_ptr(), x.numel() // k, n, k, int(settled),
+                                                 _abi.stream()))
     return y
 
 
-def linear(x, weight, scale=None):
+_launch_settled = partial(_launch, settled=True)
+
+
+def linear(x, weight, scale=None, *, settled: bool = False):
     """x . weight^T, times `scale` (one BF16 value) if there is one: F.linear and a multiplication, as one kernel where it takes
-    the operands and as these operations where it does not."""
+    the operands and as these operations where it does not. `settled`: the caller vouches that the launch in front on this
+    stream does not write the weights, which may then be read before it has ended."""
     if _plain(x, weight, *(() if scale is None else (scale,))) and _fits(x, weight):
         if scale is None or (scale.dtype == torch.bfloat16 and scale.shape == (1,) and scale.device == x.device):
-            return _launch(x, weight, None, scale)
+            return (_launch_settled if settled else _launch)(x, weight, None, scale)
     y = F.linear(x, weight)
     return y if scale is None else y * scale
 
 
-def gated(x, gate, up):
-    """silu(x . gate^T) * (x . up^T)."""
+def gated(x, gate, up, *, settled: bool = False):
+    """silu(x . gate^T) * (x . up^T); `settled` as above."""
     if _plain(x, gate, up) and _fits(x, gate, up) and gate.shape == up.shape:
-        return _launch(x, gate, up, None)
+        return (_launch_settled if settled else _launch)(x, gate, up, None)
     return F.silu(F.linear(x, gate)) * F.linear(x, up)

@@ -272,6 +272,64 @@ def test_a_projection_in_a_chain_sees_what_the_kernel_in_front_wrote(ib, device)
         assert torch.equal(y, one_by_one)
 
 
+def _weights_normed(k, x, w0, norm):
+    return k.linear(x, k.rmsnorm(w0, norm, cases.EPS))
+
+
+def _weights_normed_one_further(k, x, w0, norm):
+    w = k.rmsnorm(w0, norm, cases.EPS)
+    return k.linear(k.rmsnorm(x, norm, cases.EPS), w)
+
+
+def _weights_projected(k, x, w0, norm):
+    return k.linear(x, k.linear(w0[:8], w0))
+
+
+def _pair_projected(k, x, w0, norm):
+    return k.gated(x, k.linear(w0[:8], w0), k.linear(w0[8:16], w0))
+
+
+@pytest.mark.parametrize("rows,width,chain", [(16, 4096, _weights_normed), (16, 4096, _weights_normed_one_further), (32, 32, _weights_projected), (32, 32, _pair_projected)])
+def test_a_projections_weights_may_be_what_the_kernels_in_front_wrote(ib, device, rows, width, chain):
+    """A captured chain whose weights are other values at every replay, behind a kernel that takes long on a third of the SMs and lets
+    the chain start beside it: what the weights' memory held before must not be read."""
+    gen = torch.Generator(device=device).manual_seed(3)
+
+    def values(*shape):
+        return torch.randn(*shape, generator=gen, device=device).to(BF16)
+
+    x, w0, norm = values(5, width), values(rows, 4096), torch.ones(4096, dtype=BF16, device=device)
+    long_x, long_w = values(8, 8192), values(48, 8192)
+
+    def step():
+        ib.kernels.linear(long_x, long_w)
+        return chain(ib.kernels, x, w0, norm)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = step()
+
+    class OneByOne:
+        def __getattr__(self, name):
+            def call(*args):
+                y = getattr(ib.kernels, name)(*args)
+                torch.cuda.synchronize()
+                return y
+            return call
+
+    for _ in range(4):
+        x.copy_(values(5, width))
+        w0.copy_(values(rows, 4096))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, chain(OneByOne(), x, w0, norm))
+
+
 @pytest.mark.parametrize("n,k,tokens", [(11264, 4096, 1), (4096, 8192, 7), (8192, 4096, 3)])
 def test_a_layers_projections_are_the_bits_of_a_plain_gemm(ib, device, n, k, tokens):
     gen = torch.Generator(device=device).manual_seed(n)

@@ -89,3 +89,28 @@ def test_gradients_transforms_modes_and_subclasses_are_left_to_tensor_operations
     with torch.no_grad():
         linear(grown, w)   # no gradient is asked for
     assert len(launched) == 1
+
+
+def test_who_vouches_for_the_weights(monkeypatch):
+    """Only a layer, whose own norm stands in front of a module that launches nothing else first, and a module for its later projections."""
+    from inkling_b200 import attention
+
+    seen = []
+    monkeypatch.setattr(attention, "linear", lambda x, w, scale=None, settled=False: seen.append(settled) or F.linear(x, w))
+    monkeypatch.setattr(attention, "gated", lambda x, g, u, settled=False: seen.append(settled) or F.linear(x, g))
+    w = torch.zeros(8, 8)
+
+    def mlp(kind=attention.DenseMLP):
+        return kind(w, w, w, torch.ones(1))
+
+    mlp()(w)
+    assert seen == [False, True]
+
+    class Other(attention.DenseMLP):
+        pass
+
+    hooked, replaced = mlp(), mlp()
+    hooked.register_forward_pre_hook(lambda *_: None)
+    replaced.forward = replaced.forward
+    assert attention._runs_alone(mlp(), attention.DenseMLP)
+    assert not any(attention._runs_alone(m, attention.DenseMLP) for m in (mlp(Other), hooked, replaced))
