@@ -18,7 +18,8 @@ from .kernels.paired_all_reduce import all_reduce
 
 
 def _norm_rows(rows: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
-    """RMS norm over the last dimension of BF16 [n, c] with the reference's rounding (kernels/decode.py:36-43)."""
+    """RMS norm over the last dimension of BF16 [n, c], of any strides, with the reference's rounding (kernels/decode.py:36-43)."""
+    rows = rows.contiguous()
     return rmsnorm(rows if rows.data_ptr() % 16 == 0 else rows.clone(), weight, eps)
 
 

@@ -357,6 +357,41 @@ def test_a_decode_step_of_the_whole_model(ib, step):
     assert torch.equal(got.argmax(-1), want.argmax(-1))          # the same next token
 
 
+def _small_layer(ib, device, bs, seed=0, k_taps=4, v_taps=4):
+    """A dense decoder layer of 256 columns, four heads of 64 on two, and a cache in mid-sequence."""
+    from types import SimpleNamespace
+
+    gen = torch.Generator().manual_seed(seed)
+    draw = lambda *shape, std=1.0: (torch.randn(*shape, generator=gen) * std).to(device)  # noqa: E731
+    bf = lambda *shape, std=1.0: draw(*shape, std=std).bfloat16()  # noqa: E731
+    d, h, hk, c, slots = 256, 4, 2, 64, 64
+    attn = ib.DecodeAttention(bf((h + 2 * hk) * c + h * 16, d, std=0.06), bf(d, h * c, std=0.06), bf(c), bf(c), draw(hk * c, 1, k_taps, std=0.3),
+                              draw(hk * c, 1, v_taps, std=0.3), bf(16, slots, std=0.3), layer_idx=0, heads=h, kv_heads=hk, head_dim=c, d_rel=16)
+    mlp = ib.DenseMLP(bf(512, d, std=0.06), bf(512, d, std=0.06), bf(d, 512, std=0.06), torch.ones(1, dtype=torch.bfloat16, device=device))
+    layer = ib.DecodeLayer(attn, mlp, bf(d), bf(d), draw(d, 1, 4, std=0.3), draw(d, 1, 4, std=0.3))
+    tensors = [bf(bs, hk, slots, c), bf(bs, hk, slots, c), draw(bs, hk * c, k_taps), draw(bs, hk * c, v_taps), draw(bs, d, 4), draw(bs, d, 4)]
+
+    def cache():
+        k, v, *histories = (t.clone() for t in tensors)
+        state = SimpleNamespace(k_cache=k, v_cache=v, conv_caches=[SimpleNamespace(cache=t) for t in histories])
+        return SimpleNamespace(layers=[state], position=torch.tensor(45, device=device), pad_counts=torch.zeros(bs, dtype=torch.int64, device=device))
+
+    return layer, cache, bf
+
+
+@pytest.mark.parametrize("view", [lambda t: t[:, -1:, :256], lambda t: t[:, :1, 256:], lambda t: t[:, :1, 1:257], lambda t: t[:, 1:2, ::2],
+                                  lambda t: t[:1, :1, :256].expand(3, 1, 256)])
+def test_a_layers_hidden_states_may_have_any_strides(ib, view):
+    device = torch.device("cuda", 0)
+    layer, cache, bf = _small_layer(ib, device, 3)
+    x = view(bf(3, 5, 512))
+    a, b = cache(), cache()
+    assert torch.equal(layer(x, a), layer(x.contiguous(), b))
+    for s, t in zip(a.layers[0].conv_caches, b.layers[0].conv_caches):
+        assert torch.equal(s.cache, t.cache)
+    assert torch.equal(a.layers[0].k_cache, b.layers[0].k_cache) and torch.equal(a.layers[0].v_cache, b.layers[0].v_cache)
+
+
 @pytest.mark.parametrize("c,h,hk,slots,window,position,d_rel", [
     (128, 8, 8, 64, 0, 0, 16),            # one slot in use, one head per key/value head
     (128, 9, 1, 65, 0, 64, 16),           # nine heads on one key/value head (a second, nearly empty group), one slot past a part
