@@ -74,10 +74,10 @@ class DecodeAttention(nn.Module):
         h, hk, c = self.heads, self.kv_heads, self.head_dim
         qkvr = linear(hidden_states, self.qkvr_weight, settled=settled)
         k_history, v_history = layer.conv_caches[0].cache, layer.conv_caches[1].cache
-        if c % 8 == 0 and c <= 256 and (h * self.d_rel) % 8 == 0 and _aligned(qkvr, self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history):
+        if c % 8 == 0 and c <= 256 and (h * self.d_rel) % 8 == 0 and self.k_taps.shape == self.v_taps.shape and _aligned(qkvr, self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history):
             q, k, v, r = attention_heads(qkvr.view(bs, -1), self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history, self.eps,
                                          h, hk, c, self.d_rel)
-        else:   # heads of other widths, histories that start anywhere
+        else:   # heads of other widths, convolutions of two lengths, histories that start anywhere
             q, k, v, r = qkvr.split(self.sizes, dim=-1)
             q = self._norm(q.reshape(bs * h, c).contiguous(), self.q_norm_weight)
             k = short_conv(k.contiguous(), self.k_taps, k_history, None)
@@ -116,7 +116,7 @@ class DecodeLayer(nn.Module):
         normed = self._norm(hidden_states, self.input_norm_weight)
         attended = self.attention(normed, cache, settled=True) if _runs_alone(self.attention, DecodeAttention) else self.attention(normed, cache)
         attended, history, residual = attended.contiguous(), layer.conv_caches[2].cache, hidden_states.contiguous()
-        if d % 8 == 0 and _aligned(self.attn_taps, history):
+        if d % 8 == 0 and attended.dtype == torch.bfloat16 and _aligned(self.attn_taps, history):
             h, normed = short_conv_norm(attended, self.attn_taps, history, residual, self.post_norm_weight, self.eps)
         else:
             h = short_conv(attended, self.attn_taps, history, residual)

@@ -392,6 +392,30 @@ def test_a_layers_hidden_states_may_have_any_strides(ib, view):
     assert torch.equal(a.layers[0].k_cache, b.layers[0].k_cache) and torch.equal(a.layers[0].v_cache, b.layers[0].v_cache)
 
 
+def test_convolutions_of_two_lengths_and_an_attention_in_single_precision(ib):
+    """Three taps are four of which the first is zero; what an attention of another make returns in FP32 is rounded to BF16."""
+    device = torch.device("cuda", 0)
+    layer, cache, bf = _small_layer(ib, device, 3, v_taps=3)
+    x, a, b = bf(3, 1, 256), cache(), cache()
+    same, _, _ = _small_layer(ib, device, 3, v_taps=3)
+    same.attention.v_taps = torch.nn.functional.pad(layer.attention.v_taps, (1, 0))
+    history = b.layers[0].conv_caches[1]
+    history.cache = torch.nn.functional.pad(history.cache, (1, 0))
+    y = layer(x, a)
+    assert torch.equal(y, same(x, b)) and torch.equal(a.layers[0].conv_caches[1].cache, history.cache[..., 1:])
+
+    class Single(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner, self.layer_idx = inner, inner.layer_idx
+
+        def forward(self, hidden, cache):
+            return self.inner(hidden, cache).float()
+
+    layer.attention = Single(layer.attention)
+    assert torch.equal(layer(x, cache()), y)
+
+
 @pytest.mark.parametrize("c,h,hk,slots,window,position,d_rel", [
     (128, 8, 8, 64, 0, 0, 16),            # one slot in use, one head per key/value head
     (128, 9, 1, 65, 0, 64, 16),           # nine heads on one key/value head (a second, nearly empty group), one slot past a part
