@@ -210,9 +210,10 @@ int ink_attention_heads(const void* qkvr, const void* q_weight, const void* k_we
 int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k, ink_stream_t stream);
 /* The same. `settled` not 0: the caller vouches that the launch in front on the stream does not write weight or up; they may be
  * read while it runs. (What the launches before that one wrote is there, if the one in front is any kernel of this library but the
- * grouped projections, or one launched without the programmatic stream serialization attribute.) */
+ * grouped projections, or one launched without the programmatic stream serialization attribute.)
+ * `status`: null, or a device word that gets bit 1 set if a bounded wait gave up (y then holds NaN). */
 int ink_linear_settled(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k, int settled,
-                       ink_stream_t stream);
+                       int32_t* status, ink_stream_t stream);
 
 /* Decode attention with the learned relative-position bias, one query token per sequence: the static_decode
  * branch of MyInklingAttention.forward (my_inkling/model.py:533-612) from the normed query to the output of

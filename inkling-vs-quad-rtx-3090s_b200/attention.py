@@ -33,7 +33,24 @@ def _runs_alone(module, kind) -> bool:
             and not nn.modules.module._global_forward_pre_hooks)
 
 
-class DecodeAttention(nn.Module):
+class _Projections(nn.Module):
+    """Modules whose projections report a bounded wait that gave up in one status word."""
+
+    def _make_status(self, weight: torch.Tensor) -> None:
+        self.register_buffer("status", torch.zeros(1, dtype=torch.int32, device=weight.device), persistent=False)
+
+    def check_status(self) -> None:
+        """Host read (synchronises): raises if a wait inside a projection of this module, or of those it holds, gave up
+        since the last check; the outputs of that call are invalid. Call outside graph capture."""
+        words = [m.status for m in self.modules() if isinstance(m, _Projections)]
+        flags = [int(w.item()) for w in words]
+        for w in words:
+            w.zero_()
+        if any(flags):
+            raise RuntimeError(f"{type(self).__name__}: a bounded wait inside a projection timed out; the output of that call is invalid")
+
+
+class DecodeAttention(_Projections):
     def __init__(self, qkvr_weight, o_weight, q_norm_weight, k_norm_weight, k_taps, v_taps, rel_proj, *, layer_idx: int,
                  heads: int, kv_heads: int, head_dim: int, d_rel: int, window: int = 0, log_scaling_n_floor=None,
                  log_scaling_alpha: float = 0.1, eps: float = 1e-6, group=None):
@@ -49,6 +66,7 @@ class DecodeAttention(nn.Module):
         for name, t in (("qkvr_weight", qkvr_weight), ("o_weight", o_weight), ("q_norm_weight", q_norm_weight),
                         ("k_norm_weight", k_norm_weight), ("k_taps", k_taps), ("v_taps", v_taps), ("rel_proj", rel_proj)):
             self.register_buffer(name, t.contiguous())
+        self._make_status(self.qkvr_weight)
 
     @classmethod
     def from_reference(cls, attention, group=None) -> "DecodeAttention":
@@ -72,7 +90,7 @@ class DecodeAttention(nn.Module):
         assert s == 1, "one token per sequence"
         layer = cache.layers[self.layer_idx]
         h, hk, c = self.heads, self.kv_heads, self.head_dim
-        qkvr = linear(hidden_states, self.qkvr_weight, settled=settled)
+        qkvr = linear(hidden_states, self.qkvr_weight, settled=settled, status=self.status)
         k_history, v_history = layer.conv_caches[0].cache, layer.conv_caches[1].cache
         if c % 8 == 0 and c <= 256 and (h * self.d_rel) % 8 == 0 and self.k_taps.shape == self.v_taps.shape and _aligned(qkvr, self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history):
             q, k, v, r = attention_heads(qkvr.view(bs, -1), self.q_norm_weight, self.k_norm_weight, self.k_taps, self.v_taps, k_history, v_history, self.eps,
@@ -87,7 +105,7 @@ class DecodeAttention(nn.Module):
                                cache.position, cache.pad_counts, window=self.window, log_scaling_n_floor=self.n_floor,
                                log_scaling_alpha=self.alpha, scale=1.0 / c, new_key=k.view(bs, hk, 1, c),
                                new_value=v.reshape(bs, hk, 1, c))
-        y = linear(out.reshape(bs, 1, h * c), self.o_weight, settled=True)   # (the attention is in front)
+        y = linear(out.reshape(bs, 1, h * c), self.o_weight, settled=True, status=self.status)   # (the attention is in front)
         if self.group is not None:
             y = all_reduce(y, self.group)   # (nothing to do with one rank)
         return y
@@ -128,7 +146,7 @@ class DecodeLayer(nn.Module):
         return short_conv(block.view(bs, 1, d).contiguous(), self.mlp_taps, layer.conv_caches[3].cache, h)
 
 
-class DenseMLP(nn.Module):
+class DenseMLP(_Projections):
     """`MyInklingMLP` (my_inkling/model.py:153-171), the block of a dense layer: two launches of `ink_linear`,
     down(silu(gate(x)) * up(x)) * global_scale, BF16 like the reference's; all-reduced over `group` when the rows of
     gate/up and the columns of down are sliced."""
@@ -137,15 +155,17 @@ class DenseMLP(nn.Module):
         super().__init__()
         for name, t in (("gate_weight", gate_weight), ("up_weight", up_weight), ("down_weight", down_weight), ("global_scale", global_scale)):
             self.register_buffer(name, t.contiguous())
+        self._make_status(self.gate_weight)
         self.group = group
 
     def forward(self, x: torch.Tensor, *, settled: bool = False) -> torch.Tensor:
         """`settled`: as of DecodeAttention."""
-        y = linear(gated(x, self.gate_weight, self.up_weight, settled=settled), self.down_weight, self.global_scale, settled=True)
+        y = linear(gated(x, self.gate_weight, self.up_weight, settled=settled, status=self.status), self.down_weight, self.global_scale, settled=True,
+                   status=self.status)
         return y if self.group is None else all_reduce(y, self.group)
 
 
-class DecodeModel(nn.Module):
+class DecodeModel(_Projections):
     """One decode step of the reference's model, `MyInkling.forward` with a decoding cache (my_inkling/model.py:679-800):
     normed embedding, the decoder layers, the final norm, the logits (hidden / mup multiplier through the LM head), and
     the cache's position counter moved on by one token."""
@@ -156,6 +176,7 @@ class DecodeModel(nn.Module):
         for name, t in (("embedding", embedding), ("embed_norm_weight", embed_norm_weight), ("final_norm_weight", final_norm_weight),
                         ("lm_head_weight", lm_head_weight)):
             self.register_buffer(name, t.contiguous())
+        self._make_status(self.lm_head_weight)
         self.layers = nn.ModuleList(layers)
         self.mup, self.eps, self.unpadded = float(mup_multiplier), eps, unpadded_vocab_size
 
@@ -166,6 +187,6 @@ class DecodeModel(nn.Module):
         for layer in self.layers:
             hidden = layer(hidden, cache)
         hidden = norm(hidden, self.final_norm_weight) / self.mup
-        logits = linear(hidden, self.lm_head_weight, settled=True)   # (the division is in front)
+        logits = linear(hidden, self.lm_head_weight, settled=True, status=self.status)   # (the division is in front)
         cache.position.add_(1)
         return logits if self.unpadded is None else logits[..., : self.unpadded]

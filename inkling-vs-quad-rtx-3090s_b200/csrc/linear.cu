@@ -44,19 +44,22 @@ struct LinearArgs {
   int tokens, n, k;
   int groups, stages;     // consumers that have rows; stages of the ring
   int settled;            // the kernel in front does not write the weights
+  int32_t* status;        // or null: kFlagWaitTimedOut when a wait gave up
 };
 
 struct LinearShared {
   uint64_t full[kLinMostStages], empty[kLinMostStages];
   volatile int failed;
 };
-__device__ __forceinline__ bool lin_wait(uint64_t* bar, uint32_t parity, LinearShared* sh) {
+// (called when the kernel in front has ended: the limit is for this kernel's own copies and products)
+__device__ __forceinline__ bool lin_wait(uint64_t* bar, uint32_t parity, LinearShared* sh, int32_t* status) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!mbar_try_wait(bar, parity)) {
     if (sh->failed) return false;
     if (clock64() - t0 > kWaitLimitCycles) {
       sh->failed = 1;
+      if (status) atomicOr(status, kFlagWaitTimedOut);
       return false;
     }
   }
@@ -103,7 +106,10 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_kernel(const LinearArgs
     for (int round = 0; ok && round < rounds; ++round) {
       const int row0 = first + round * per_round, outputs = min(per_round, end - row0);
       for (int c = 0; c < chunks; ++c) {
-        if (lap > 0) ok = __all_sync(0xffffffffu, lin_wait(&sh.empty[stage], (lap - 1) & 1u, &sh));
+        if (lap > 0) {
+          if (lap == 1 && stage == 0) pdl_wait();   // (the products start when the kernel in front has ended)
+          ok = __all_sync(0xffffffffu, lin_wait(&sh.empty[stage], (lap - 1) & 1u, &sh, a.status));
+        }
         if (!ok) break;
         const int k0 = c * kLinChunk + lane * 8;
         const uint32_t to = ring + (uint32_t)(stage * stage_bytes) + (uint32_t)lane * 16;
@@ -131,13 +137,14 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_kernel(const LinearArgs
     const int g = lane >> 2, t = lane & 3;
     const unsigned char* rows = s_ring + (warp * kLinRows + g) * kLinPitch + t * 8;        // (rows beyond the share hold anything: they
     const unsigned char* tokens = s_ring + (stage_rows + g) * kLinPitch + t * 8;           //  and tokens beyond the last are not written)
+    pdl_wait();   // (the tokens; and y may still be read by the kernels in front)
     int stage = 0;
     uint32_t lap = 0;
     bool ok = true;
     for (int round = 0; round < rounds; ++round) {
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       for (int c = 0; ok && c < chunks; ++c) {
-        ok = __all_sync(0xffffffffu, lin_wait(&sh.full[stage], lap & 1u, &sh));
+        ok = __all_sync(0xffffffffu, lin_wait(&sh.full[stage], lap & 1u, &sh, a.status));
         if (!ok) break;
         const unsigned char *w = rows + stage * stage_bytes, *x = tokens + stage * stage_bytes;
         // (a lane's four columns of a step are neighbours, on both sides: the sum over sixteen does not depend on who holds which)
@@ -169,7 +176,6 @@ __global__ void __launch_bounds__(kLinThreads, 1) linear_kernel(const LinearArgs
       }
       if (!ok) d[0] = d[1] = d[2] = d[3] = __int_as_float(0x7fffffff);   // (a wait that gave up shows in the results)
       const int row0 = first + round * per_round, outputs = min(per_round, end - row0);
-      if (round == 0) pdl_wait();   // (y may still be read by the kernels in front)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int out = warp * kOut + g + (GATED ? 0 : j >> 1) * 8, token = 2 * t + (j & 1);
@@ -227,17 +233,17 @@ static int launch_linear(LinearArgs a, cudaStream_t stream) {
 using namespace ink;
 
 extern "C" int ink_linear_settled(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k,
-                                  int settled, ink_stream_t stream) {
+                                  int settled, int32_t* status, ink_stream_t stream) {
   INK_REQUIRE(x && weight && y, kBadArgument, "linear: null pointer argument");
   INK_REQUIRE(tokens >= 0 && tokens <= kLinTokens && n > 0 && n <= (1 << 24) && k > 0 && k % 32 == 0 && k <= kLinMostK, kUnsupportedShape,
               "linear: tokens=%d n=%d k=%d unsupported (up to %d tokens, k a multiple of 32 up to %d)", tokens, n, k, kLinTokens, kLinMostK);
   INK_REQUIRE(aligned16(x) && aligned16(weight) && aligned16(up), kMisaligned, "linear: x and weights must be 16-byte aligned");
   if (tokens == 0) return kOk;
-  const LinearArgs a{(const uint16_t*)x, (const uint16_t*)weight, (const uint16_t*)up, (const uint16_t*)scale, (uint16_t*)y, tokens, n, k, 0, 0, settled};
+  const LinearArgs a{(const uint16_t*)x, (const uint16_t*)weight, (const uint16_t*)up, (const uint16_t*)scale, (uint16_t*)y, tokens, n, k, 0, 0, settled, status};
   return up ? launch_linear<true>(a, (cudaStream_t)stream) : launch_linear<false>(a, (cudaStream_t)stream);
 }
 
 extern "C" int ink_linear(const void* x, const void* weight, const void* up, const void* scale, void* y, int tokens, int n, int k,
                           ink_stream_t stream) {
-  return ink_linear_settled(x, weight, up, scale, y, tokens, n, k, 0, stream);
+  return ink_linear_settled(x, weight, up, scale, y, tokens, n, k, 0, nullptr, stream);
 }

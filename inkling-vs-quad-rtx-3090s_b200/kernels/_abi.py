@@ -35,7 +35,7 @@ _SIGNATURES = {
     "ink_short_conv_norm": (I, [P, P, P, P, P, F, P, P, I, I, I, P]),
     "ink_attention_heads": (I, [P, P, P, P, P, P, P, F, P, P, P, P, I, I, I, I, I, I, P]),
     "ink_linear": (I, [P, P, P, P, P, I, I, I, P]),
-    "ink_linear_settled": (I, [P, P, P, P, P, I, I, I, I, P]),
+    "ink_linear_settled": (I, [P, P, P, P, P, I, I, I, I, P, P]),
     "ink_decode_attention_joins": (I, [I, I, I, I, I]),
     "ink_decode_attention_workspace_bytes": (Z, [I, I, I, I]),
     "ink_decode_attention_counter_bytes": (Z, [I, I]),

@@ -30,31 +30,33 @@ def _fits(x, *weights) -> bool:
                     and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in weights))
 
 
-def _launch(x, weight, up, scale, settled=False):
+def _launch(x, weight, up, scale, settled=False, status=None):
     n, k = weight.shape
     y = x.new_empty(*x.shape[:-1], n)
     with torch.cuda.device(x.device):
         _abi.check(_abi.lib().ink_linear_settled(x.data_ptr(), weight.data_ptr(), _abi.ptr(up), _abi.ptr(scale), y.data_ptr(), x.numel() // k, n, k, int(settled),
-                                                 _abi.stream()))
+                                                 _abi.ptr(status), _abi.stream()))
     return y
 
 
-_launch_settled = partial(_launch, settled=True)
+def _launcher(settled, status):
+    return partial(_launch, settled=settled, status=status) if settled or status is not None else _launch
 
 
-def linear(x, weight, scale=None, *, settled: bool = False):
+def linear(x, weight, scale=None, *, settled: bool = False, status=None):
     """x . weight^T, times `scale` (one BF16 value) if there is one: F.linear and a multiplication, as one kernel where it takes
     the operands and as these operations where it does not. `settled`: the caller vouches that the launch in front on this
-    stream does not write the weights, which may then be read before it has ended."""
+    stream does not write the weights, which may then be read before it has ended. `status` (optional int32[1]) gets bit 1 set if
+    a bounded wait inside the kernel gave up (the result is NaN then)."""
     if _plain(x, weight, *(() if scale is None else (scale,))) and _fits(x, weight):
         if scale is None or (scale.dtype == torch.bfloat16 and scale.shape == (1,) and scale.device == x.device):
-            return (_launch_settled if settled else _launch)(x, weight, None, scale)
+            return _launcher(settled, status)(x, weight, None, scale)
     y = F.linear(x, weight)
     return y if scale is None else y * scale
 
 
-def gated(x, gate, up, *, settled: bool = False):
-    """silu(x . gate^T) * (x . up^T); `settled` as above."""
+def gated(x, gate, up, *, settled: bool = False, status=None):
+    """silu(x . gate^T) * (x . up^T); `settled` and `status` as above."""
     if _plain(x, gate, up) and _fits(x, gate, up) and gate.shape == up.shape:
-        return (_launch_settled if settled else _launch)(x, gate, up, None)
+        return _launcher(settled, status)(x, gate, up, None)
     return F.silu(F.linear(x, gate)) * F.linear(x, up)

@@ -96,8 +96,8 @@ def test_who_vouches_for_the_weights(monkeypatch):
     from inkling_b200 import attention
 
     seen = []
-    monkeypatch.setattr(attention, "linear", lambda x, w, scale=None, settled=False: seen.append(settled) or F.linear(x, w))
-    monkeypatch.setattr(attention, "gated", lambda x, g, u, settled=False: seen.append(settled) or F.linear(x, g))
+    monkeypatch.setattr(attention, "linear", lambda x, w, scale=None, settled=False, status=None: seen.append(settled) or F.linear(x, w))
+    monkeypatch.setattr(attention, "gated", lambda x, g, u, settled=False, status=None: seen.append(settled) or F.linear(x, g))
     w = torch.zeros(8, 8)
 
     def mlp(kind=attention.DenseMLP):
@@ -114,3 +114,23 @@ def test_who_vouches_for_the_weights(monkeypatch):
     replaced.forward = replaced.forward
     assert attention._runs_alone(mlp(), attention.DenseMLP)
     assert not any(attention._runs_alone(m, attention.DenseMLP) for m in (mlp(Other), hooked, replaced))
+
+
+def test_a_wait_that_gave_up_is_reported_once(launched, monkeypatch):
+    """The modules hand their status word to every projection; a model checks those of its layers too."""
+    from inkling_b200 import attention
+
+    words = []
+    monkeypatch.setattr(module, "_launch", lambda x, weight, up, scale, settled=False, status=None: words.append(status) or F.linear(x, weight))
+    w = torch.zeros(64, 64, dtype=BF16)
+    mlp = attention.DenseMLP(w, w, w, torch.ones(1, dtype=BF16))
+    mlp(w[:1])
+    assert len(words) == 2 and all(s is mlp.status for s in words) and "status" not in mlp.state_dict()
+    attn = attention.DecodeAttention(torch.zeros(64 + 2 * 32 + 2 * 16, 64), w, w[0], w[0], w, w, w, layer_idx=0, heads=2, kv_heads=1, head_dim=32, d_rel=16)
+    model = attention.DecodeModel(w, w[0], [attention.DecodeLayer(attn, mlp, w[0], w[0], w, w)], w[0], w, 1.0)
+    model.check_status()
+    for holder in (mlp, attn, model):
+        holder.status.fill_(2)
+        with pytest.raises(RuntimeError, match="timed out"):
+            model.check_status()
+        model.check_status()
