@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kAttnThreads, kAttnPerSm(C)) decode_attention_
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int j = step * 16 + 2 * t + (i & 1) + (i >> 1) * 8;
-            w[i] = (rel && j < a.d_rel) ? (uint32_t)__ldg(a.proj + (size_t)j * a.extent + d_mine) : 0u;
+            w[i] = (rel && j < a.d_rel) ? (uint32_t)a.proj[(size_t)j * a.extent + d_mine] : 0u;
           }
           const uint32_t* r2 = reinterpret_cast<const uint32_t*>(s_r + g * rel_pitch + step * 16) + t;
           mma_bf16(bias, r2[0], 0u, r2[4], 0u, w[0] | (w[1] << 16), w[2] | (w[3] << 16));
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(A
     if (rel) {
 #pragma unroll 8
       for (int j = 0; j < a.d_rel; ++j) {
-        const float p = bf16_to_f32(__ldg(a.proj + (size_t)j * a.extent + d));
+        const float p = bf16_to_f32(a.proj[(size_t)j * a.extent + d]);
 #pragma unroll
         for (int n = 0; n < kMine; ++n)
           if (h0 + n * kStep < n_heads) sum[n] = fmaf(bf16_to_f32(s_r[(h0 + n * kStep) * a.d_rel + j]), p, sum[n]);

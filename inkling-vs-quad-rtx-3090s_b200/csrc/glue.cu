@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(const float* 
   for (int i = 0; i < kNormMaxPerThread; ++i) {
     const int gidx = i * kNormThreads + tid;
     if (gidx < groups) {
-      const uint4 wq = *reinterpret_cast<const uint4*>(weight + gidx * 8);
+      const uint4 wq = __ldcg(reinterpret_cast<const uint4*>(weight + gidx * 8));
       const uint32_t wv[4] = {wq.x, wq.y, wq.z, wq.w};
       uint32_t packed[4];
 #pragma unroll
@@ -81,14 +81,14 @@ struct ConvChannel {
   float past[TAPS], tap[TAPS];
   __device__ __forceinline__ void fetch(const float* taps, const float* history) {
     if constexpr (WIDE) {
-      const float4 h = *reinterpret_cast<const float4*>(history), w = *reinterpret_cast<const float4*>(taps);
+      const float4 h = __ldcg(reinterpret_cast<const float4*>(history)), w = __ldcg(reinterpret_cast<const float4*>(taps));
       past[0] = h.x; past[1] = h.y; past[2] = h.z; past[3] = h.w;
       tap[0] = w.x; tap[1] = w.y; tap[2] = w.z; tap[3] = w.w;
     } else {
 #pragma unroll
       for (int j = 0; j < TAPS; ++j) {
-        past[j] = history[j];
-        tap[j] = taps[j];
+        past[j] = __ldcg(history + j);
+        tap[j] = __ldcg(taps + j);
       }
     }
   }
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kConvNormThreads) conv_norm_kernel(const uint1
   const float scale = rsqrtf(total / (float)hidden + eps);
   for (int i = tid; channel_of(i) < hidden; i += kConvNormThreads) {
     const int d = channel_of(i);
-    normed[row + d] = (uint16_t)f32_to_bf16_bits(round_bf16(s_h[i] * scale) * bf16_to_f32(weight[d]));
+    normed[row + d] = (uint16_t)f32_to_bf16_bits(round_bf16(s_h[i] * scale) * bf16_to_f32(__ldcg(weight + d)));
   }
   cluster_sync();   // (a block's sum stays until all have read it)
 }
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(128) heads_kernel(const HeadsArgs a) {
     }
     sum = warp_sum(sum);
     const float scale = rsqrtf(sum / (float)c + a.eps);
-    const uint4 raw = live ? *(reinterpret_cast<const uint4*>(weight) + lane) : make_uint4(0, 0, 0, 0);
+    const uint4 raw = live ? __ldcg(reinterpret_cast<const uint4*>(weight) + lane) : make_uint4(0, 0, 0, 0);
     const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {

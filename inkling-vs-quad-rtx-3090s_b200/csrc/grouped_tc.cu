@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const uint16_t* __restrict
     }
     if (pointers[expert * stride] == 0) continue;
     const float w = bf16_to_f32(weights[route]);
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(y + route * width) + piece);
+    const uint4 q = __ldcg(reinterpret_cast<const uint4*>(y + route * width) + piece);   // (y is written while this kernel is on the chip)
     const uint32_t q4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const uint16_t* __restrict
     }
   }
   for (int e = 0; e < n_shared; ++e) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(shared_y + ((size_t)token * n_shared + e) * width) + piece);
+    const uint4 q = __ldcg(reinterpret_cast<const uint4*>(shared_y + ((size_t)token * n_shared + e) * width) + piece);
     const uint32_t q4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
