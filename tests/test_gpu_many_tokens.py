@@ -111,7 +111,8 @@ def test_experts_that_are_not_there_are_skipped_and_reported(ib, device):
         module.check_status()
 
 
-@pytest.mark.parametrize("hidden,routed,shared,top_k,tokens", [(4096, 256, 2, 6, 17), (1024, 61, 1, 4, 33), (264, 300, 0, 8, 9), (8, 8, 2, 8, 100)])
+@pytest.mark.parametrize("hidden,routed,shared,top_k,tokens", [(4096, 256, 2, 6, 17), (1024, 61, 1, 4, 33), (264, 300, 0, 8, 9), (8, 8, 2, 8, 100),
+                                                               (2056, 256, 2, 6, 333), (4096, 256, 2, 6, 1999), (520, 40, 1, 4, 5000)])   # several tiles a block
 def test_a_token_is_routed_the_same_in_any_company(ib, device, hidden, routed, shared, top_k, tokens):
     """Bit-exact: the many-token router against the one-launch router on the same tokens in groups of at most eight."""
     gen = torch.Generator().manual_seed(hidden)
