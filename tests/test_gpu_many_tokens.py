@@ -71,6 +71,7 @@ def test_unquantised_banks_of_several_tokens(ib, device, d, f, experts, tokens):
     (256, 2048, 100, 100), (256, 2048, 100, 500),   # one ring stage an item, more deals than blocks, more items a deal than the queue holds
     (512, 1024, 60, 290),                            # deals that end inside an expert; gate/up and down of different lengths
     (4096, 128, 3, 5), (256, 256, 1, 2),             # one item a deal; fewer items than blocks
+    (1024, 512, 40, 13), (1024, 512, 40, 60), (512, 512, 64, 700),   # first deals of one, of some and of most items; later ones of one and of several
 ])
 def test_every_item_is_dealt_whatever_their_number(ib, device, d, f, experts, tokens):
     if f % 256:   # (packed banks need a multiple of 256 columns: BF16 ones)
