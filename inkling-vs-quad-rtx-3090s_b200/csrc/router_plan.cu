@@ -312,8 +312,10 @@ __global__ void __launch_bounds__(1024) plan_kernel(PlanArgs p, int runs) {
 // selection compares BF16 values: a last-bit difference picks another expert): products on the CUDA cores, two rows' FMAs an instruction.
 // Persistent blocks, one an SM: the next chunks of columns, of this tile or the next, are copied to shared memory while one is computed on.
 // 1 999 tokens, 258 rows of 4 096 columns (2.1 G FMAs, 58 us at the FMA pipes' rate): 160 us, 52 % of the issue slots, 2.6 instructions
-// for each that multiplies (tokens spread to pairs, the sums over the threads); loads straight to registers, eight warps an SM to hide them, 193; router_kernel,
-// two rows a block and its tail on one block, 3 270.
+// for each that multiplies (tokens spread to pairs, the sums over the threads); router_kernel, two rows a block and its tail on one block, 3 270.
+// Loads straight to registers (router_logits_tile_kernel, which was here for all tiles) depend on where the operands are. In DRAM, as a block's
+// experts leave them: a block of 4096 x 512 with 256 experts 707 us at 1 999 tokens and 426 at 926, 672 and 406 so. The tokens in L2, written just
+// before: 659 and 403, 680 and 409 so. Tokens and weights in L2, the router alone called again and again: 135 at 1 999 tokens, 166 so.
 constexpr int kManyRows = 8, kManyTokens = 16, kManyGroups = 2;            // rows of a thread, tokens, threads' shares of a tile's rows
 constexpr int kManyColumns = 128;                                           // threads along the columns, eight of them each
 constexpr int kManyThreads = kManyGroups * kManyColumns;
@@ -338,6 +340,67 @@ __device__ __forceinline__ int wide_reduce(float (&v)[N], int lane) {
     first += upper ? n / 2 : 0;
   }
   return first;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// The logit of pair `i` of a tile, of this row and token, from the warps' sums of it.
+template <int PARTS>
+__device__ __forceinline__ void write_logit(const RouterArgs& a, const float (&part)[PARTS][kManyRows * kManyTokens], int i, int row, int token) {
+  static_assert(kManyRows * kManyTokens == kManyColumns, "a thread writes one logit");
+  if (row >= a.n_routed + a.n_shared || token >= a.tokens) return;
+  float s = 0.f;
+#pragma unroll
+  for (int w = 0; w < PARTS; ++w) s += part[w][i];
+  const float l = round_bf16(s);
+  a.logits[(size_t)token * (a.n_routed + a.n_shared) + row] = l;
+  if (row < a.n_routed) a.scores[(size_t)token * a.n_routed + row] = round_bf16(1.f / (1.f + __expf(-l))) + a.bias[row];
+}
+
+// One tile of tokens (nine to sixteen): no next tile to copy ahead, and half as many rows a block put twice as many SMs to work. Loads go
+// straight to registers; rows and tokens are asked for into L2 all at once, where the router's weights rarely are.
+__global__ void __launch_bounds__(kManyColumns, 2) router_logits_tile_kernel(RouterArgs a) {
+  constexpr int kPairs = kManyRows * kManyTokens, kParts = kManyColumns / 32;
+  __shared__ float s_part[kParts][kPairs];
+  const int tid = threadIdx.x, lane = tid & 31, part = tid >> 5;
+  const int total = a.n_routed + a.n_shared, chunks = a.hidden / 8, row0 = blockIdx.x * kManyRows;
+  const size_t row_bytes = (size_t)a.hidden * 2, w_bytes = min(kManyRows, total - row0) * row_bytes, x_bytes = a.tokens * row_bytes;
+  const char *w_from = reinterpret_cast<const char*>(a.weight) + row0 * row_bytes, *x_from = reinterpret_cast<const char*>(a.x);
+  for (size_t i = (size_t)tid * 128; i < w_bytes; i += kManyColumns * 128) prefetch_l2(w_from + i);
+  for (size_t i = ((size_t)blockIdx.x * kManyColumns + tid) * 128; i < x_bytes; i += (size_t)gridDim.x * kManyColumns * 128) prefetch_l2(x_from + i);
+  float acc[kPairs];   // [token][row]
+#pragma unroll
+  for (int i = 0; i < kPairs; ++i) acc[i] = 0.f;
+#pragma unroll 1
+  for (int c = tid; c < chunks; c += kManyColumns) {
+    float w[kManyRows][8];
+#pragma unroll
+    for (int r = 0; r < kManyRows; ++r) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(a.weight + (size_t)min(row0 + r, total - 1) * a.hidden) + c);
+      w[r][0] = bf16lo(q.x); w[r][1] = bf16hi(q.x); w[r][2] = bf16lo(q.y); w[r][3] = bf16hi(q.y);
+      w[r][4] = bf16lo(q.z); w[r][5] = bf16hi(q.z); w[r][6] = bf16lo(q.w); w[r][7] = bf16hi(q.w);
+    }
+#pragma unroll
+    for (int t0 = 0; t0 < kManyTokens; t0 += 4) {
+      uint4 x4[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) x4[t] = __ldg(reinterpret_cast<const uint4*>(a.x + (size_t)min(t0 + t, a.tokens - 1) * a.hidden) + c);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float x[8] = {bf16lo(x4[t].x), bf16hi(x4[t].x), bf16lo(x4[t].y), bf16hi(x4[t].y),
+                            bf16lo(x4[t].z), bf16hi(x4[t].z), bf16lo(x4[t].w), bf16hi(x4[t].w)};
+#pragma unroll
+        for (int r = 0; r < kManyRows; ++r)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc[(t0 + t) * kManyRows + r] = fmaf(w[r][k], x[k], acc[(t0 + t) * kManyRows + r]);
+      }
+    }
+  }
+  const int first = wide_reduce<kPairs>(acc, lane);
+#pragma unroll
+  for (int i = 0; i < kPairs / 32; ++i) s_part[part][first + i] = acc[i];
+  __syncthreads();
+  write_logit<kParts>(a, s_part, tid, row0 + tid % kManyRows, tid / kManyRows);
 }
 
 __device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
@@ -436,16 +499,7 @@ __global__ void __launch_bounds__(kManyThreads, 1) router_logits_kernel(RouterAr
 #pragma unroll
     for (int i = 0; i < kPairs / 32; ++i) s_part[group][part][first + i] = acc[i];
     __syncthreads();   // (the next tile's first barrier keeps these sums until they have been read)
-    const int row = row0 + column % kManyRows, token = token0 + column / kManyRows;   // a pair a thread
-    static_assert(kPairs == kManyColumns, "a thread writes one logit");
-    if (row < total && token < a.tokens) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < kParts; ++w) s += s_part[group][w][column];
-      const float l = round_bf16(s);
-      a.logits[(size_t)token * total + row] = l;
-      if (row < a.n_routed) a.scores[(size_t)token * a.n_routed + row] = round_bf16(1.f / (1.f + __expf(-l))) + a.bias[row];
-    }
+    write_logit<kParts>(a, s_part[group], column, row0 + column % kManyRows, token0 + column / kManyRows);   // a pair a thread
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -536,15 +590,21 @@ static int launch_router(const RouterArgs& a, const PlanArgs* p, cudaStream_t st
   int device = 0;
   cudaGetDevice(&device);
   INK_REQUIRE(device >= 0 && device < kMaxDevices, kLaunchFailed, "router: device ordinal %d", device);
-  if (sms_of[device] == 0) {
+  if (a.tokens > kManyTokens && sms_of[device] == 0) {
     const cudaError_t e = cudaFuncSetAttribute(router_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kManySmem);
     INK_REQUIRE(e == cudaSuccess, kLaunchFailed, "router: %d bytes of shared memory refused: %s", kManySmem, cudaGetErrorString(e));
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     sms_of[device] = sms > 0 ? sms : 148;
   }
-  const long long tiles = (long long)((rows + kManyTileRows - 1) / kManyTileRows) * ((a.tokens + (long long)kManyTokens - 1) / kManyTokens);
-  router_logits_kernel<<<(unsigned)(tiles < sms_of[device] ? tiles : sms_of[device]), kManyThreads, kManySmem, stream>>>(a);
+  // us, register loads / persistent: alone, all in L2, 9 tokens 10.3 / 14.6 and 16 tokens 11.3 / 14.9 (so with the prefetch 11.0 and 11.5); a block
+  // of 4096 x 512, 256 experts, tokens in DRAM: 9 tokens 74.5 / 75.3, 16 tokens 83.8 / 84.2, 30 tokens 103.5 / 102.4, 63 tokens 135.7 / 134.4.
+  if (a.tokens <= kManyTokens) {
+    router_logits_tile_kernel<<<(rows + kManyRows - 1) / kManyRows, kManyColumns, 0, stream>>>(a);
+  } else {
+    const long long tiles = (long long)((rows + kManyTileRows - 1) / kManyTileRows) * ((a.tokens + (long long)kManyTokens - 1) / kManyTokens);
+    router_logits_kernel<<<(unsigned)(tiles < sms_of[device] ? tiles : sms_of[device]), kManyThreads, kManySmem, stream>>>(a);
+  }
   INK_CHECK_LAUNCH("ink_router_forward (logits)");
   const unsigned selects = (unsigned)((a.tokens + 31) / 32);
   if (!p) {
