@@ -936,11 +936,12 @@ static int launch_stage(bool fp4, const StageArgs& a, size_t most_rows, cudaStre
 }
 
 // Tokens T of a tile, from the mean number of routes per expert. T = 16, 32, 64, us a call, experts chosen evenly / as rank^-0.6:
-//   256 of 4096 x 2048   mean 8: 600 621 713 / 629 633 716;  16:  825 690 784 /  874  742  812;  32: 1283  981  971 / 1347  969 1059;  46: 1713 1308 1201 / 1895 1246 1252
-//   256 of 4096 x 512         8: 227 229 239 / 239 253 283;  16:  308 293 303 /  313  306  327;  32:  514  451  440 /  518  454  481;  46:  717  616  590 /  721  606  602
-//   128 of 2048 x 1024        8: 120 117 123 / 117 120 134;  16:  144 140 142 /  144  145  164;  32:  232  205  198 /  232  199  215;  48:  311  275  271 /  313  268  279
-//    64 of 1024 x 512         8:  51  54  53 /  52  60  75;  16:   62  64  63 /   63   67   94;  32:   87   88   98 /   87   89  104;  48:  105   99  114 /  101  100  125
-// T = 16 and 32 meet between means of 10 (615 629 / 661 647 for the largest layers) and 12 (646 650 / 699 676).
+//   256 of 4096 x 2048   mean 8: 580 597 652 / 603 604 652;  16:  713 646 707 /  748  678  725;  32: 1181  873  849 / 1225  920  890;  48: 1608 1232 1006 / 1594 1121 1061
+//   256 of 4096 x 512         8: 222 225 237 / 224 228 257;  16:  292 280 289 /  295  293  312;  32:  486  418  417 /  489  423  441;  48:  694  583  553 /  701  581  576
+//   128 of 2048 x 1024        8: 111 109 116 / 114 117 128;  16:  137 128 132 /  141  138  155;  32:  220  195  184 /  221  188  194;  48:  302  258  247 /  294  254  261
+//    64 of 1024 x 512         8:  42  42  41 /  44  48  47;  16:   51  50  50 /   51   54   70;  32:   71   70   71 /   73   71   85;  48:   94   91   92 /   94   93  100
+// T = 16 and 32 meet between means of 10 (595 609 / 639 622 for the largest layers) and 12 (618 622 / 676 640). The lines are those of long items: where
+// items are short and the choice uneven a smaller tile would do better, by up to 12 % (the last row, means of 12, 16, 40 and 48).
 static int gg_tokens(long long routes, int experts) { return routes > 32LL * experts ? 64 : routes > 10LL * experts ? 32 : 16; }
 
 }  // namespace ink

@@ -7,16 +7,17 @@
 // far too few for the tcgen05 tiles). Where the caller vouches for the weights (`settled`: the launch in front does not write them) the ring
 // fills before the kernel in front has finished; else the weights, like the tokens, are asked for when it has.
 //
-// The sum over columns runs from the first to the last, sixteen at a time into one FP32 accumulator. That is the order of a
-// plain tensor-core GEMM, so the results are the bits of the library GEMV that these calls were (up to 8192 columns; above, the
-// library cuts the sum in parts): a decode step of several layers turns any last-bit difference
+// The sum over columns runs from the first to the last, sixteen at a time into one FP32 accumulator: a row and a token have the same bits in any
+// company. That is also the order of a plain tensor-core GEMM; on the shapes compared (the tests', torch 2.11) the results were the bits of
+// the library calls that stood here, and that matters: a decode step of several layers turns any last-bit difference
 // into another rounding of a router logit, hence another routing weight. It costs a chain of K / 16 dependent instructions
 // a round (55 clocks each), which the loads hide but for few rows of many columns. (Tiles of eight rows with sums cut between eight
 // warps, and between two blocks above 4096 columns: 13.9 us for the 17.3 of 4096 x 8192, 15.9 for 16.3 of 11264 x 4096; but the logits of a six-layer
 // step then differ by 2.8 % of their norm.)
 //
-// us a call, calls on different weights one after the other in a graph, one token / seven; the library GEMV that stood here; the weights at the
-// copy rate:  11264 x 4096 16.3 / 16.8, 17.1 / 17.5, 14.1;  4096 x 8192 17.3 / 18.2, 21.5 / 21.7, 10.2;  32768 x 4096 41.0 / 42.6, 45.4 / 45.8, 41.0;
+// us a call, calls on different weights one after the other in a graph, settled weights, one token / seven; the library GEMV that stood here; the
+// weights at the copy rate (weights that wait for the kernel in front: 11264 x 4096 17.2 / 17.4, 32768 x 4096 44.5 / 44.8 for 43.0 / 43.7, the others
+// within 0.1):  11264 x 4096 16.3 / 16.8, 17.1 / 17.5, 14.1;  4096 x 8192 17.3 / 18.2, 21.5 / 21.7, 10.2;  32768 x 4096 41.0 / 42.6, 45.4 / 45.8, 41.0;
 // gated 2 x 8192 x 4096 22.0 / 22.8, 31.5 / 30.2 in four launches, 20.5.
 #include "../../include/inkling_b200.h"
 #include "common.cuh"

@@ -57,6 +57,8 @@ constexpr int kCopies = 8;
 // A line that is polled before it is written makes the writing slower, so a poll is late rather than early, and seldom: the routing
 // warp looks for the scores of all blocks this long after its own block has published its own, and a poll that finds something missing pauses
 // (the same stack: no first wait 783 us, 250 ns 762, 500 ns 752, 900 ns 754; pauses of the routing warp of 100 ns instead of 500 with no first wait +40 us).
+// The same at every width and depth, us with no first wait / 250 ns / 600 ns: one block of 4096 x 2048 48.9 / 48.8 / 48.7, of 4096 x 1024 32.9 / 32.8 /
+// 32.8, of 4096 x 256 20.0 / 19.8 / 19.6, of 1024 x 512 15.8 / 15.6 / 15.4; sixteen of 4096 x 1024 443 / 440 / 438, eight of 4096 x 2048 364 / 363 / 363.
 constexpr unsigned kFirstLook = 600, kPollPause = 250;
 constexpr int kTileCountersPerLayer = kSMaxTopK * 32 + 32;   // routed gate/up tiles (at most 8 x 32), then down row tiles
 
@@ -143,8 +145,8 @@ struct StackArgs {
   uint16_t* normed_out;            // [hidden] BF16 output of the last norm (glue mode); else the block's output in BF16, or null
   float* partial;                  // [hidden] FP32 output of the (last) block
   unsigned long long* scores;      // scratch [2][kCopies][experts + n_shared] router words {selection score, BF16 logit, 16-bit tag}
-  uint16_t* activated;             // scratch [2][top_k][f]
-  uint16_t* shared_activated;      // scratch [2][n_shared][f]
+  uint16_t* activated;             // scratch [2][top_k][f] BF16; of experts up to 512 wide [2][kCopies][top_k][f / 2] words of two
+  uint16_t* shared_activated;      // scratch [2][n_shared][f] BF16; of experts up to 512 wide [2][kCopies][n_shared][f] words of one
   RouteTable* routes;              // scratch [n_layers]
   float* gu_part;                  // scratch [top_k * 2f/128 tiles][hidden/256][128]: partial gate/up rows of a tile split between blocks
   float* dn_part;                  // scratch [top_k * hidden/128 tiles][f/256][128]: the same for the down projection
@@ -157,10 +159,10 @@ struct StackArgs {
   int rank, world;
   unsigned long long* inbox;       // this rank's [2][world][hidden] tagged words: partial output rows as the ranks deliver them
   unsigned long long* peer_inbox[kSMaxWorld];   // the same region of every rank, as mapped into this process
-  unsigned long long* summed;      // scratch [2][hidden] tagged words: the rows summed over the ranks, for every block of this rank
+  unsigned long long* summed;      // scratch: the rows summed over the ranks, for every block of this rank: tagged words [2][kCopies][hidden / 2]
+                                   // of two BF16 rows (tensor-core variant: [2][hidden] of one FP32 row)
   long long wait_limit;            // SM clocks a wait may take before the launch gives up
   unsigned poll_pause_ns;          // pause between two polls of a hand-over word
-                                   // when a lane issues its last tile of a layer: they arrive while the blocks hand their rows over
   int32_t* status;
   unsigned long long* trace;       // optional [n_layers][kTraceBlocks][kTraceSlots] nanosecond stamps
 };
