@@ -516,7 +516,9 @@ __global__ void __launch_bounds__(kSmallThreads) decode_attention_small_kernel(A
     for (int n = 0; n < kMine; ++n) sum[n] = 0.f;
     const bool rel = slot < a.slots && d >= 0 && d < a.extent;
     if (rel) {
-#pragma unroll 8
+      // (sixteen patterns in one round trip; eight at a time the calls of one round took up to 4 % more: seven sequences of 64 heads on 8, 256
+      // channels, 128 slots 14.2 us, 13.8 so; one of 16 on 16, 128 channels, 512 slots 8.4 / 8.2)
+#pragma unroll 16
       for (int j = 0; j < a.d_rel; ++j) {
         const float p = bf16_to_f32(a.proj[(size_t)j * a.extent + d]);
 #pragma unroll
